@@ -97,96 +97,75 @@ __device__ __forceinline__ int cell_aliases(int i, int n, int per, int out[3])
     return m;
 }
 
-// candidate c (0..3) of the padded positions aliasing unique node i, or kNoAlias
-constexpr int kNoAlias = -1000;
-__device__ __forceinline__ int node_alias_cand(int i, int n, int per, int c)
+// distance from unique node i to its padded alias along one direction, 0 when it has none (per, n >= 3: nodes 0
+// and 1 alias to n and n + 1, node n - 1 to -1)
+__device__ __forceinline__ int node_alias_step(int i, int n, int per)
 {
-    if (c == 0) return i;
-    if (!per) return kNoAlias;
-    if (c == 1) return i == 0 ? n : kNoAlias;
-    if (c == 2) return i == 1 ? n + 1 : kNoAlias;
-    return i == n - 1 ? -1 : kNoAlias;
+    return !per ? 0 : (i <= 1 ? n : (i == n - 1 ? -n : 0));
 }
 
+// Store at unique node (i, j, k) and at every padded alias. With n >= 3 a node has at most one alias per
+// direction, so the aliases are the corners of one box of steps: at most 8 predicated stores, no loop. (Loops
+// over candidate lists cost more than the stencil on the small levels, where most nodes lie on a seam: with
+// rolled loops the prolongation alone took 14.4 us of a 16^3 V-cycle's launches.)
 template <typename T>
 __device__ __forceinline__ void store_node(T* a, const NodalGeom& g, int i, int j, int k, T v)
 {
-    // nodes away from a periodic seam (all but a few planes) have no alias: one store
-    const bool ax = g.per[0] && (i <= 1 || i >= g.n[0] - 1);
-    const bool ay = g.per[1] && (j <= 1 || j >= g.n[1] - 1);
-    const bool az = g.per[2] && (k <= 1 || k >= g.n[2] - 1);
-    if (!(ax || ay || az)) {
-        a[pidx(g.sy, g.sz, i, j, k)] = v;
-        return;
+    const long long p = pidx(g.sy, g.sz, i, j, k);
+    a[p] = v;
+    const int ex = node_alias_step(i, g.n[0], g.per[0]);
+    const long long ey = node_alias_step(j, g.n[1], g.per[1]) * g.sy;
+    const long long ez = node_alias_step(k, g.n[2], g.per[2]) * g.sz;
+    if (ex) a[p + ex] = v;
+    if (ey) a[p + ey] = v;
+    if (ex && ey) a[p + ex + ey] = v;
+    if (ez) {
+        a[p + ez] = v;
+        if (ex) a[p + ex + ez] = v;
+        if (ey) a[p + ey + ez] = v;
+        if (ex && ey) a[p + ex + ey + ez] = v;
     }
-    // a node on a periodic seam: every combination of its per-direction aliases (kept as rolled
-    // loops: this path is rare, and inlining it unrolled bloats every kernel that stores nodes)
+    // a periodic direction of 2 cells: node 1 is also node -1
+    const int zx = g.per[0] && g.n[0] == 2 && i == 1, zy = g.per[1] && g.n[1] == 2 && j == 1,
+              zz = g.per[2] && g.n[2] == 2 && k == 1;
+    if (zx | zy | zz) {
+        int xs[3], ys[3], zs[3];
+        const int nx = node_aliases(i, g.n[0], g.per[0], xs);
+        const int ny = node_aliases(j, g.n[1], g.per[1], ys);
+        const int nz = node_aliases(k, g.n[2], g.per[2], zs);
 #pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
-        const int kk = node_alias_cand(k, g.n[2], g.per[2], c);
-        if (kk == kNoAlias) continue;
-#pragma unroll 1
-        for (int b = 0; b < 4; ++b) {
-            const int jj = node_alias_cand(j, g.n[1], g.per[1], b);
-            if (jj == kNoAlias) continue;
-#pragma unroll 1
-            for (int q = 0; q < 4; ++q) {
-                const int ii = node_alias_cand(i, g.n[0], g.per[0], q);
-                if (ii == kNoAlias) continue;
-                a[pidx(g.sy, g.sz, ii, jj, kk)] = v;
-            }
-        }
-    }
-}
-
-// store_node with the alias lists unrolled (at most 3 positions per direction, on levels of 2 cells): for kernels
-// where most nodes lie on a periodic seam (the smallest levels), the rolled candidate loops cost more
-// than the stencil
-template <typename T>
-__device__ __forceinline__ void store_node_unrolled(T* a, const NodalGeom& g, int i, int j, int k, T v)
-{
-    int xs[3], ys[3], zs[3];
-    const int nx = node_aliases(i, g.n[0], g.per[0], xs);
-    const int ny = node_aliases(j, g.n[1], g.per[1], ys);
-    const int nz = node_aliases(k, g.n[2], g.per[2], zs);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        if (c >= nz) break;
-#pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            if (b >= ny) break;
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                if (q >= nx) break;
-                a[pidx(g.sy, g.sz, xs[q], ys[b], zs[c])] = v;
-            }
-        }
+        for (int c = 0; c < nz * ny * nx; ++c) a[pidx(g.sy, g.sz, xs[c % nx], ys[(c / nx) % ny], zs[c / (nx * ny)])] = v;
     }
 }
 
-template <typename T>
-__device__ __forceinline__ void store_cell(T* a, const CellGeom& g, int i, int j, int k, T v)
+// distance from cell i to its padded alias along one direction, 0 when it has none (cells 0 and n - 1 alias to n
+// and -1; n >= 2)
+__device__ __forceinline__ int cell_alias_step(int i, int n, int per) { return !per ? 0 : (i == 0 ? n : (i == n - 1 ? -n : 0)); }
+
+template <typename T, typename G>
+__device__ __forceinline__ void store_cell(T* a, const G& g, int i, int j, int k, T v)
 {
-    int xs[2], ys[2], zs[2];
-    int nx = cell_aliases(i, g.n[0], g.per[0], xs);
-    int ny = cell_aliases(j, g.n[1], g.per[1], ys);
-    int nz = cell_aliases(k, g.n[2], g.per[2], zs);
-    for (int c = 0; c < nz; ++c)
-        for (int b = 0; b < ny; ++b)
-            for (int q = 0; q < nx; ++q) a[pidx(g.sy, g.sz, xs[q], ys[b], zs[c])] = v;
+    const long long p = pidx(g.sy, g.sz, i, j, k);
+    a[p] = v;
+    const int ex = cell_alias_step(i, g.n[0], g.per[0]);
+    const long long ey = cell_alias_step(j, g.n[1], g.per[1]) * g.sy;
+    const long long ez = cell_alias_step(k, g.n[2], g.per[2]) * g.sz;
+    if (ex) a[p + ex] = v;
+    if (ey) a[p + ey] = v;
+    if (ex && ey) a[p + ex + ey] = v;
+    if (ez) {
+        a[p + ez] = v;
+        if (ex) a[p + ex + ez] = v;
+        if (ey) a[p + ey + ez] = v;
+        if (ex && ey) a[p + ex + ey + ez] = v;
+    }
 }
 
 // Sigma of the 8 cells around a node, used with periodic aliases of cells.
 template <typename T>
 __device__ __forceinline__ void store_sigma_cell(T* a, const NodalGeom& g, int i, int j, int k, T v)
 {
-    int xs[2], ys[2], zs[2];
-    int nx = cell_aliases(i, g.n[0], g.per[0], xs);
-    int ny = cell_aliases(j, g.n[1], g.per[1], ys);
-    int nz = cell_aliases(k, g.n[2], g.per[2], zs);
-    for (int c = 0; c < nz; ++c)
-        for (int b = 0; b < ny; ++b)
-            for (int q = 0; q < nx; ++q) a[pidx(g.sy, g.sz, xs[q], ys[b], zs[c])] = v;
+    store_cell(a, g, i, j, k, v);
 }
 
 __device__ __forceinline__ bool node_is_dirichlet(const NodalGeom& g, int i, int j, int k)

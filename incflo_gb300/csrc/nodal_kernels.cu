@@ -612,7 +612,7 @@ __device__ __forceinline__ void cc_jacobi(const NodalGeom& g, const T* s, const 
                 v = __ldcg(xin + c) + omega * (__ldcg(b + c) - ax) * approx_recip(diag);
             }
         }
-        store_node_unrolled(xout, g, i, j, k, v);
+        store_node(xout, g, i, j, k, v);
     }
 }
 
@@ -632,7 +632,7 @@ __device__ __forceinline__ void cc_resid(const NodalGeom& g, const T* s, const T
                                : NodalOp<T>::template apply<false, LdCg>(x, s, c, g.sy, g.sz, g, diag);
             v = __ldcg(b + c) - ax;
         }
-        store_node_unrolled(r, g, i, j, k, v);
+        store_node(r, g, i, j, k, v);
     }
 }
 
@@ -662,7 +662,7 @@ __device__ __forceinline__ void cc_restrict(const NodalGeom& gf, const NodalGeom
             }
             v = acc;
         }
-        store_node_unrolled(bc, gc, I, J, K, v);
+        store_node(bc, gc, I, J, K, v);
     }
 }
 
@@ -695,7 +695,7 @@ __device__ __forceinline__ void cc_prolong(const NodalGeom& gf, const NodalGeom&
         const int sh = oi + oj + ok;
         const T w = sh == 0 ? T(1) : (sh == 1 ? T(0.5) : (sh == 2 ? T(0.25) : T(0.125)));
         const long long p = pidx(gf.sy, gf.sz, i, j, k);
-        store_node_unrolled(xf, gf, i, j, k, __ldcg(xf + p) + w * acc);
+        store_node(xf, gf, i, j, k, __ldcg(xf + p) + w * acc);
     }
 }
 
@@ -737,7 +737,7 @@ __device__ __forceinline__ void cc_bottom(const NodalGeom& g, const double* M, c
         if (v < N) a0 = fma(M[(size_t)v * N + t], bb[v], a0);
         int i, j, k;
         decode_node(g, t, i, j, k);
-        store_node_unrolled(xout, g, i, j, k, (T)(a0 + a1));
+        store_node(xout, g, i, j, k, (T)(a0 + a1));
     }
 }
 

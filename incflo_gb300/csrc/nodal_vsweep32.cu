@@ -172,27 +172,25 @@ __device__ __forceinline__ void store4(float* out, const NodalGeom& g, int i0, i
         *reinterpret_cast<float4*>(out + pidx(g.sy, g.sz, i0, j, k)) = make_float4(v[0], v[1], v[2], v[3]);
         return;
     }
-#pragma unroll 1
+    // the row and its images across the y and z seams (at most one per direction, node_alias_step)
+    float* row = out + pidx(g.sy, g.sz, 0, j, k);
+    const long long ey = node_alias_step(j, g.n[1], g.per[1]) * g.sy;
+    const long long ez = node_alias_step(k, g.n[2], g.per[2]) * g.sz;
+#pragma unroll
     for (int c = 0; c < 4; ++c) {
-        const int kk = node_alias_cand(k, g.n[2], g.per[2], c);
-        if (kk == kNoAlias) continue;
-#pragma unroll 1
-        for (int b = 0; b < 4; ++b) {
-            const int jj = node_alias_cand(j, g.n[1], g.per[1], b);
-            if (jj == kNoAlias) continue;
-            float* row = out + pidx(g.sy, g.sz, 0, jj, kk);
-            if (nact == 4) {
-                *reinterpret_cast<float4*>(row + i0) = make_float4(v[0], v[1], v[2], v[3]);
-            } else {
-                for (int q = 0; q < nact; ++q) row[i0 + q] = v[q];
+        if (((c & 1) && !ey) || ((c & 2) && !ez)) continue;
+        float* r = row + ((c & 1) ? ey : 0) + ((c & 2) ? ez : 0);
+        if (nact == 4) {
+            *reinterpret_cast<float4*>(r + i0) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+            for (int q = 0; q < nact; ++q) r[i0 + q] = v[q];
+        }
+        if (g.per[0]) {
+            if (i0 == 0) {
+                r[g.n[0]] = v[0];
+                r[g.n[0] + 1] = v[1];
             }
-            if (g.per[0]) {
-                if (i0 == 0) {
-                    row[g.n[0]] = v[0];
-                    row[g.n[0] + 1] = v[1];
-                }
-                if (i0 + 3 == g.n[0] - 1) row[-1] = v[3];
-            }
+            if (i0 + 3 == g.n[0] - 1) r[-1] = v[3];
         }
     }
 }
