@@ -871,11 +871,10 @@ int CompositeNodal::init(const gbp_geometry& coarse, const int bc_lo[3], const i
     add(3 * ncf, 8);                               // velo_f
     add(ncf, 8);                                   // sig_f
     add(nnf, 8);                                   // p_fb
-    // the shared-sum FP64 residual on both levels (isotropic cells): four edge-weight arrays each
+    // the shared-sum FP64 residual on both levels (isotropic cells)
     qsw = qsweep_supported(gf_nomask) && qsweep_supported(gc);
     if (qsw) {
-        for (int q = 0; q < 4; ++q) add(gf.count, 8);
-        for (int q = 0; q < 4; ++q) add(gc.count, 8);
+        for (int q = 0; q < 5; ++q) add(gc.count, 8);
     }
     nparts = std::max(nodal_partials_needed(gc), 1184);
     add(nparts + 64, 8);
@@ -890,10 +889,7 @@ int CompositeNodal::init(const gbp_geometry& coarse, const int bc_lo[3], const i
     ccls = pool.take<unsigned char>(gc.count);
     fcls = pool.take<unsigned char>(gf.count);
     if (qsw) {
-        double** wf[4] = {&qwf.wsum, &qwf.wx, &qwf.wy, &qwf.wz};
-        double** wc[4] = {&qwc.wsum, &qwc.wx, &qwc.wy, &qwc.wz};
-        for (int q = 0; q < 4; ++q) *wf[q] = pool.take<double>(gf.count);
-        for (int q = 0; q < 4; ++q) *wc[q] = pool.take<double>(gc.count);
+        for (double** w : {&qwc.w5, &qwc.rd, &qwc.wx, &qwc.wy, &qwc.wz}) *w = pool.take<double>(gc.count);
     }
     sc_m = pool.take<double>(gc.count);
     sc_t = pool.take<double>(gc.count);
@@ -1021,7 +1017,7 @@ int CompositeNodal::check_fields(const AmrFields& f)
 void CompositeNodal::resid_f(const double* x, const double* b, double* r)
 {
     if (qsw)
-        nodal_qsweep64(gf_nomask, 1, fin.sigma64(), qwf, x, b, r, 1.0, nullptr, st);
+        nodal_qsweep64(gf_nomask, 1, fin.sigma64(), fin.qweights0(), x, b, r, 1.0, nullptr, st);
     else
         nodal_resid<double>(gf_nomask, fin.sigma64(), x, b, r, nullptr, st);
 }
@@ -1273,7 +1269,7 @@ int CompositeNodal::project(const AmrFields& f, gbp_stats* stats)
     rc = fin.set_sigma(&sa, 0.0);
     if (rc) return rc;
     if (qsw) {
-        nodal_qweights64(gf_nomask, fin.sigma64(), qwf, st);
+        fin.qweights0();  // the fine part shares its solver's weights (a mask does not enter them)
         nodal_qweights64(gc, sc_m, qwc, st);
     }
     // right-hand sides: leaf cells of each level, then the fine interface into the coarse interface

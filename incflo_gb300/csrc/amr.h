@@ -87,7 +87,7 @@ private:
     unsigned long long *dnorm = nullptr, *hnorm = nullptr;
     bool qsw = false;      // shared-sum FP64 residuals (isotropic cells)
     bool have_last = false;  // phi_c / phi_f hold the last converged solution (initial_guess = previous)
-    QWeights qwf{}, qwc{};  // their edge weights, fine and coarse
+    QWeights qwc{};         // the coarse level's weights (the fine level's are its solver's)
     void* dboxes = nullptr;  // device table for the batched box kernels
     size_t dboxes_bytes = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;

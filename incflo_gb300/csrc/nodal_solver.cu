@@ -272,9 +272,9 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
     }
     const NodalGeom& G0 = L[0].g;
     for (int q = 0; q < 3; ++q) add(G0.count, 8);
-    use_qsweep = qsweep_supported(G0);
-    if (use_qsweep)
-        for (int q = 0; q < 4; ++q) add(G0.count, 8);
+    for (auto& lv : L)
+        if (qsweep_supported(lv.g))
+            for (int q = 0; q < 5; ++q) add(lv.g.count, 8);
     add(nodal_partials_needed(G0) + 64, 8);
     add(5 * B.g.count, 8);
     add(16, 4);
@@ -304,12 +304,9 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
     phi = pool.take<double>(G0.count);
     rhs0 = pool.take<double>(G0.count);
     res = pool.take<double>(G0.count);
-    if (use_qsweep) {
-        qw.wsum = pool.take<double>(G0.count);
-        qw.wx = pool.take<double>(G0.count);
-        qw.wy = pool.take<double>(G0.count);
-        qw.wz = pool.take<double>(G0.count);
-    }
+    for (auto& lv : L)
+        if (qsweep_supported(lv.g))
+            for (double** w : {&lv.qw.w5, &lv.qw.rd, &lv.qw.wx, &lv.qw.wy, &lv.qw.wz}) *w = pool.take<double>(lv.g.count);
     partials = pool.take<double>(nodal_partials_needed(G0) + 64);
     bscr = pool.take<double>(5 * B.g.count);
     dinfo = pool.take<int>(16);
@@ -356,7 +353,32 @@ int NodalSolver::finish_sigma()
     nk += (long long)L.size();
     GBP_CUDA(cudaGetLastError());
     sigma_ready = true;
+    for (auto& lv : L) lv.qw_ready = false;
     return build_bottom();
+}
+
+void NodalSolver::ensure_qweights()
+{
+    const size_t most = opt.precision == GBP_PREC_MIXED ? 1 : L.size();
+    for (size_t l = 0; l < most; ++l)
+        if (L[l].qw.w5 && !L[l].qw_ready) {
+            nodal_qweights64(L[l].g, L[l].s64, L[l].qw, st);
+            L[l].qw_ready = true;
+            ++nk;
+        }
+}
+
+const QWeights& NodalSolver::qweights0()
+{
+    ensure_qweights();
+    return L[0].qw;
+}
+
+int NodalSolver::level_of(const NodalGeom& g) const
+{
+    for (size_t l = 0; l < L.size(); ++l)
+        if (&g == &L[l].g) return (int)l;
+    return -1;
 }
 
 // Dense inverse of the coarsest operator, assembled on the host from the coarsest sigma: the
@@ -364,7 +386,6 @@ int NodalSolver::finish_sigma()
 // face) use (A + c 1 1^T)^-1, which solves A x = b exactly for consistent b (sum b = 0).
 int NodalSolver::build_bottom()
 {
-    if (use_qsweep) nodal_qweights64(L[0].g, L[0].s64, qw, st);
     if (!dense_bottom) return GBP_OK;
     const NodalLevel& B = L.back();
     const NodalGeom& g = B.g;
@@ -519,8 +540,9 @@ struct LevelBufs<float> {
 template <typename T>
 void NodalSolver::jacobi(const NodalGeom& g, const T* s, const T* x, const T* b, T* out, double w, cudaStream_t s_)
 {
-    if (sizeof(T) == 8 && use_qsweep && &g == &L[0].g) {
-        nodal_qsweep64(g, 0, reinterpret_cast<const double*>(s), qw, reinterpret_cast<const double*>(x),
+    const int l = sizeof(T) == 8 ? level_of(g) : -1;
+    if (l >= 0 && L[l].qw_ready) {
+        nodal_qsweep64(g, 0, reinterpret_cast<const double*>(s), L[l].qw, reinterpret_cast<const double*>(x),
                        reinterpret_cast<const double*>(b), reinterpret_cast<double*>(out), w, nullptr, s_);
     } else if (sizeof(T) == 4 && use_tma && vsweep32_supported(g)) {
         int rc = vsweep32(g, 0, reinterpret_cast<const float*>(s), reinterpret_cast<const float*>(x),
@@ -538,8 +560,9 @@ template <typename T>
 void NodalSolver::resid(const NodalGeom& g, const T* s, const T* x, const T* b, T* r, unsigned long long* norm,
                         cudaStream_t s_)
 {
-    if (sizeof(T) == 8 && use_qsweep && &g == &L[0].g) {
-        nodal_qsweep64(g, 1, reinterpret_cast<const double*>(s), qw, reinterpret_cast<const double*>(x),
+    const int l = sizeof(T) == 8 ? level_of(g) : -1;
+    if (l >= 0 && L[l].qw_ready) {
+        nodal_qsweep64(g, 1, reinterpret_cast<const double*>(s), L[l].qw, reinterpret_cast<const double*>(x),
                        reinterpret_cast<const double*>(b), reinterpret_cast<double*>(r), omega_eff, norm, s_);
     } else if (sizeof(T) == 4 && !norm && use_tma && vsweep32_supported(g)) {
         int rc = vsweep32(g, 1, reinterpret_cast<const float*>(s), reinterpret_cast<const float*>(x),
@@ -615,7 +638,10 @@ void NodalSolver::vcycle(int l, const T* b, bool zero)
     int q0 = 0;  // pre-smoothing sweeps done
     if (zero) {
         if (pre > 0) {
-            nodal_jacobi<T>(lv.g, B::s(lv), nullptr, b, x, wpre[0], true, s);
+            if (sizeof(T) == 8 && lv.qw_ready)
+                nodal_qzero64(lv.g, lv.qw, reinterpret_cast<const double*>(b), reinterpret_cast<double*>(x), wpre[0], s);
+            else
+                nodal_jacobi<T>(lv.g, B::s(lv), nullptr, b, x, wpre[0], true, s);
             if (cut) eb_nodes<T>(lv.g, eb.e, 0, nullptr, b, x, wpre[0], s);
             ++nk;
             q0 = 1;
@@ -720,6 +746,7 @@ void NodalSolver::apply_vcycles(const double* r, double* x, int m, double scale,
 {
     const NodalLevel& l0 = L[0];
     cap_or_st = s;
+    if (opt.precision != GBP_PREC_MIXED) ensure_qweights();
     if (opt.precision == GBP_PREC_MIXED) {
         nodal_to_f32(l0.g, r, l0.b32, scale, s);
         vcycle<float>(0, l0.b32, true);
@@ -826,6 +853,7 @@ int NodalSolver::solve(bool have_guess, gbp_stats* stats, bool from_prev)
     const NodalLevel& l0 = L[0];
     cap_or_st = st;
     GBP_CUDA(cudaEventRecord(ev1, st));
+    ensure_qweights();
     if (!have_guess) GBP_CUDA(cudaMemsetAsync(phi, 0, sizeof(double) * l0.g.count, st));
     // dnorm[0] holds |b| (written by project); dnorm[1] receives the initial residual norm
     GBP_CUDA(cudaMemsetAsync(dnorm + 1, 0, 3 * sizeof(unsigned long long), st));
@@ -1306,6 +1334,7 @@ double* NodalSolver::residual_of(const double* x)
 {
     cap_or_st = st;
     launch_rc = 0;
+    ensure_qweights();
     resid0(x, rhs0, L[0].r64, nullptr, st);
     return L[0].r64;
 }
@@ -1637,6 +1666,7 @@ int NodalSolver::time_kernel(int which, int reps, double* ms, double* bytes)
     if (which == 8) *bytes = 4.0 * (2.0 * nn + nc + nn / 8.0);
     if (which == 9) *bytes = 4.0 * (3.0 * nn + nc + nn / 8.0);
     if (f32) nodal_to_f32(g, res, l0.b32, scale32, st);
+    ensure_qweights();
     GBP_CUDA(cudaEventRecord(ev0, st));
     for (int r = 0; r < reps; ++r) {
         switch (which) {

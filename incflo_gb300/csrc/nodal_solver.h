@@ -70,6 +70,8 @@ struct NodalLevel {
     double *s64 = nullptr, *x64 = nullptr, *t64 = nullptr, *b64 = nullptr, *r64 = nullptr;
     float *s32 = nullptr, *x32 = nullptr, *t32 = nullptr, *b32 = nullptr, *r32 = nullptr;
     unsigned char* mask8 = nullptr;  // overset mask storage (active when g.mask is set)
+    QWeights qw{};                   // sigma sums of the shared-sum FP64 sweep (levels it supports)
+    bool qw_ready = false;           // ... of the present sigma
 };
 
 class NodalSolver {
@@ -130,6 +132,8 @@ public:
     // cleared; synchronises s).
     int take_sweep_status(cudaStream_t s);
     float* sigma32() const { return L[0].s32; }
+    // level-0 weights of the shared-sum FP64 sweep for the present sigma (w5 == nullptr: not a level it supports)
+    const QWeights& qweights0();
 
     void reset_count() { nk = 0; }
     long long kernel_count() const { return nk; }
@@ -215,6 +219,9 @@ private:
     bool singular_faces = false;  // singular from the boundary types alone (no overset mask)
     int rebuild_masks();
     int finish_sigma();
+    // the shared-sum FP64 sweep's weights of the levels it runs on: level 0, and with FP64 V-cycles the others
+    void ensure_qweights();
+    int level_of(const NodalGeom& g) const;
     void resid0(const double* x, const double* b, double* r, unsigned long long* norm, cudaStream_t s);
     unsigned user_zeros = 0;
     unsigned char* umask8 = nullptr;  // the user's overset mask, level 0 (null: none)
@@ -254,8 +261,6 @@ private:
     size_t net_x0_bytes = 0;
     double* net_scr = nullptr;   // 8 device doubles: input statistics, Galerkin dot products
     cudaEvent_t evw = nullptr;
-    QWeights qw{};               // level-0 sigma sums of the shared-sum FP64 sweep (isotropic levels)
-    bool use_qsweep = false;
     int warm_streak = 0;         // consecutive bypassed warm starts
     // cost model of a warm start, from the last solve: the per-V-cycle residual contraction and the device
     // time of one V-cycle (a candidate is taken only when the V-cycles its smaller residual saves cost more
