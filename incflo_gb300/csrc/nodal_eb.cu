@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(128) k_eb_node(NodalGeom g, EbNodal e, const T
         if (MODE == 0)
             v = diag > T(0) ? xc + omega * (b[p] - ax) / diag : xc;
         else
-            v = b[p] - ax;
+            v = (b ? b[p] : T(0)) - ax;
     }
     store_node(out, g, nd.i, nd.j, nd.k, v);
 }

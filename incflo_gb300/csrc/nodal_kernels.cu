@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(256) k_jacobi(NodalGeom g, const T* __restrict
 
 // r = b - A x, with the strong-form max norm accumulated into *norm when norm != nullptr.
 // NodalOp::apply() evaluates sum_c sigma_c sum_{b != i} K(i,b) (x_b - x_i), which equals
-// (A x)_i because every element row of K sums to zero.
+// (A x)_i because every element row of K sums to zero. b == nullptr: r = -A x.
 template <typename T, bool ISO>
 __global__ void __launch_bounds__(256) k_resid(NodalGeom g, const T* __restrict__ s, const T* __restrict__ x,
                                                const T* __restrict__ b, T* __restrict__ r,
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(256) k_resid(NodalGeom g, const T* __restrict_
             const long long c = pidx(g.sy, g.sz, i, j, k);
             T diag;
             T ax = NodalOp<T>::template apply<ISO>(x, s, c, g.sy, g.sz, g, diag);
-            v = b[c] - ax;
+            v = (b ? b[c] : T(0)) - ax;
             if (norm) nv = fabs((double)v) * node_inv_volume(g, i, j, k);
         }
         store_node(r, g, i, j, k, v);

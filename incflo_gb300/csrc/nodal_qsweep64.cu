@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(QTX* QTY) k_qweights64(NodalGeom g, const doub
 }
 
 // MODE 0: Jacobi sweep out = x + omega (b - A x) / diag; 1: residual out = b - A x (with the max norm);
-// 2: out = A x
+// 2: out = -A x
 template <int MODE>
 __global__ void __launch_bounds__(kQThreads) k_qsweep64(NodalGeom g, const double* __restrict__ x,
                                                         const double* __restrict__ b, const double* __restrict__ s,
@@ -165,9 +165,7 @@ __global__ void __launch_bounds__(kQThreads) k_qsweep64(NodalGeom g, const doubl
                     v = fma(mkc, u_lo + u, e);  // b - A x (MODE 2: -A x)
                     if (MODE == 0) {
                         v = fma(omega * v, w.rd[pc], xc);
-                    } else if (MODE == 2) {
-                        v = -v;
-                    } else if (norm) {
+                    } else if (MODE == 1 && norm) {
                         // |v| / V_node as an integer key (boundary nodes: V / 2^e, exact scaling)
                         const int f = (!g.per[0] && (i == 0 || i == g.n[0])) + (!g.per[1] && (j == 0 || j == g.n[1])) +
                                       (!g.per[2] && (k == 0 || k == g.n[2]));

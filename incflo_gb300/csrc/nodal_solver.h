@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "gbp_internal.cuh"
+#include "krylov.h"
 #include "nodal_kernels.h"
 #include "nodal_eb.h"
 #include "nodal_sweep.h"
@@ -173,6 +174,12 @@ private:
     template <typename T>
     void resid(const NodalGeom& g, const T* s, const T* x, const T* b, T* r, unsigned long long* norm,
                cudaStream_t s_);
+    // m iterations of the accelerated V-cycle (krylov.h) for A x = r: x and r in place
+    template <typename T>
+    void krylov_steps(int m, T* x, T* r, cudaStream_t s);
+    template <typename T>
+    void apply_neg(const T* p, T* q, cudaStream_t s);  // q = -A p on level 0
+    bool accelerated() const;
     void record_iteration(int m);
     int warm_start(double bnorm, double* rn, gbp_stats* stats, bool from_prev);
     void drop_graphs();
@@ -194,6 +201,11 @@ private:
     size_t net_prev_count = 0;
     double* rhs0 = nullptr;      // level-0 right-hand side (FP64, weak form)
     double* res = nullptr;       // level-0 outer residual (FP64)
+    // conjugate-gradient vectors: two FP64 arrays of level 0, or in the mixed form p, the inner solution, q and zeros
+    double *kp = nullptr, *kq = nullptr;
+    double* kpart = nullptr;     // partial sums of its dot products
+    KrylovState* kstate = nullptr;
+    KrylovBox kbox{};
     double* partials = nullptr;  // reduction scratch
     double* bscr = nullptr;      // bottom CG scratch
     int* dinfo = nullptr;        // bottom iteration count

@@ -23,7 +23,7 @@ struct QWeights {
 };
 bool qsweep_supported(const NodalGeom& g);
 void nodal_qweights64(const NodalGeom& g, const double* s64, const QWeights& w, cudaStream_t st);
-// mode 0: Jacobi sweep, 1: residual (+ strong-form max norm into *norm when norm != nullptr), 2: out = A x (b unused)
+// mode 0: Jacobi sweep, 1: residual (+ strong-form max norm into *norm when norm != nullptr), 2: out = -A x (b unused)
 void nodal_qsweep64(const NodalGeom& g, int mode, const double* s64, const QWeights& w, const double* x,
                     const double* b, double* out, double omega, unsigned long long* norm, cudaStream_t st);
 // Jacobi sweep from zero: out = omega b / diag

@@ -41,3 +41,17 @@ def test_fp64_sweep_tiles(gpu_lib, n, lo, hi):
 ], ids=["4", "12x6x10", "8x12x4"])
 def test_periodic_seams_of_small_levels(gpu_lib, n, lo, hi, precision):
     _nodal(n, lo, hi, precision)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,ext,lo,hi", [
+    ((34, 24, 40), (1.0, 24 * 0.8 / 34, 40 * 1.25 / 34), (P, P, N), (P, P, N)),  # rows end inside a 16-byte vector
+    ((32, 32, 24), (1.0, 0.8, 0.9375), (D, N, P), (N, I, P)),
+], ids=["34x24x40", "32x32x24"])
+def test_accelerated_vcycles_on_stretched_cells(gpu_lib, n, ext, lo, hi, precision):
+    """Cells of aspect 1 : 0.8 : 1.25: stationary V(2,2) cycles need 38 for 1e-11, accelerated ones 16."""
+    _nodal(n, lo, hi, precision, ext=ext)
+    proj = NodalProjector(*(cuda(a) for a in nodal_case(n, ext, lo, hi, seed=1)[:0:-1]), Geometry(n, (0, 0, 0), ext),
+                          options=make_options(0, precision=precision))
+    proj.setDomainBC(lo, hi)
+    assert proj.project(rtol=1e-11, atol=0.0)["vcycles"] <= 24
