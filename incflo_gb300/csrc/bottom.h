@@ -1,0 +1,51 @@
+// The coarsest level of a multigrid hierarchy (nodal or cell-centred): its operator as rows of a fixed number of
+// entries, rebuilt on the device whenever the coefficients change, and the two solvers on it:
+//   - up to kDenseBottom unknowns: the dense FP64 inverse (Gauss-Jordan in one CTA), applied as one product;
+//   - above: Jacobi-preconditioned conjugate gradients in FP64 by one thread-block cluster (bottom_cg).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "gbp_internal.cuh"
+
+namespace gbp {
+
+// 64 unknowns: the inverse costs 64 x 64 x 64 FP64 multiply-adds on one SM (2 per clock: about 75 us) per coefficient
+// set, and a product 1 us per V-cycle, where the cluster's conjugate gradients take 25 to 60 us per V-cycle. (The
+// inverse of up to 216 unknowns by the host took 0.3 to 10 ms per coefficient set.)
+constexpr int kDenseBottom = 64;
+// most unknowns of the cluster solver: the search direction is replicated in every CTA's shared memory
+constexpr int kClusterBottom = 16384;
+constexpr int kBottomThreads = 1024;
+
+struct BottomRows {
+    int n = 0, w = 0;          // unknowns, entries per row (27 nodal, 7 cell-centred)
+    double* coef = nullptr;    // [w][n]
+    int* idx = nullptr;        // [w][n] unknown of each entry
+    double* diag = nullptr;    // [n], 0: no equation (held at 0)
+    double* weight = nullptr;  // [n] null-space weight of each unknown (node volume / 1), 0 where held
+    size_t bytes() const { return (size_t)n * w * 12 + (size_t)n * 16 + 1024; }
+    void carve(char* base);    // sets the arrays inside `bytes()` bytes at base (256-byte aligned)
+};
+
+void bottom_rows_nodal(const NodalGeom& g, const double* s64, const BottomRows& r, cudaStream_t st);
+void bottom_rows_mac(const CellGeom& g, const double* bx, const double* by, const double* bz, const BottomRows& r,
+                     cudaStream_t st);
+// M (n x n) = inverse of the rows' matrix (singular: of A + c 1 1^T over the unknowns that carry an equation), rows and
+// columns of held unknowns 0; act (may be null): 1 where an unknown carries an equation. *bad = 1 when a pivot is not
+// positive.
+void bottom_inverse(const BottomRows& r, int singular, double* M, unsigned char* act, unsigned* bad, cudaStream_t st);
+
+struct BottomCG {
+    BottomRows r;
+    int singular, maxiter;
+    double rtol, atol;
+    int* info;  // most iterations so far (nullptr: not kept)
+};
+// x = A^-1 b on the coarsest level by one cluster
+template <typename T>
+int bottom_cg_nodal(const NodalGeom& g, const BottomCG& c, const T* b, T* x, cudaStream_t st);
+template <typename T>
+int bottom_cg_mac(const CellGeom& g, const BottomCG& c, const T* b, T* x, cudaStream_t st);
+
+}  // namespace gbp

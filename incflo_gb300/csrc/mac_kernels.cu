@@ -10,6 +10,7 @@
 // The right-hand side is g = -V div(umac), the correction umac -= beta_eff grad phi.
 #include <cuda_runtime.h>
 
+#include "bottom.h"
 #include "gbp_internal.cuh"
 #include "mac_kernels.h"
 
@@ -629,15 +630,15 @@ void mac_bottom(const CellGeom& g, const double* bx, const double* by, const dou
 GBP_MAC_INST(double)
 GBP_MAC_INST(float)
 
-// Dense bottom solve: x = M b with M the FP64 inverse of the coarsest operator, precomputed on the host
+// Dense bottom solve: x = M b with M the FP64 inverse of the coarsest operator, computed by bottom_inverse
 // whenever the face coefficients change (singular systems: the inverse of A + c 1 1^T over the cells
-// that carry an equation, exact for a right-hand side of zero mean over them). One CTA; N <= 128.
+// that carry an equation, exact for a right-hand side of zero mean over them). One CTA; N <= kDenseBottom.
 template <typename T>
 __global__ void __launch_bounds__(128) k_mac_bottom_dense(CellGeom g, const double* __restrict__ M,
                                                           const unsigned char* __restrict__ act,
                                                           const T* __restrict__ bin, T* __restrict__ xout, int singular)
 {
-    __shared__ double bb[128];
+    __shared__ double bb[kDenseBottom];
     __shared__ double red[32];
     const int N = g.n[0] * g.n[1] * g.n[2];
     double s = 0.0, na = 0.0;
@@ -802,7 +803,7 @@ int mac_coarse_cluster_size()
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(16);
         cfg.blockDim = dim3(kMacCoarseThreads);
-        cfg.dynamicSmemBytes = kMacDenseBottomMax * sizeof(double);
+        cfg.dynamicSmemBytes = kDenseBottom * sizeof(double);
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = 16;
@@ -827,7 +828,7 @@ int mac_coarse_vcycle(const MacCoarseCycle<T>& c, int cluster, cudaStream_t st)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cluster);
     cfg.blockDim = dim3(kMacCoarseThreads);
-    cfg.dynamicSmemBytes = kMacDenseBottomMax * sizeof(double);
+    cfg.dynamicSmemBytes = kDenseBottom * sizeof(double);
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;

@@ -20,7 +20,6 @@ template <typename T>
 void mac_bottom(const CellGeom& g, const double* bx, const double* by, const double* bz, const T* b, T* x,
                 double* scratch, int maxiter, double rtol, double atol, int singular, cudaStream_t st);
 // x = M b on the coarsest level (M: the precomputed dense inverse, act: cells with an equation)
-constexpr int kMacDenseBottomMax = 128;
 template <typename T>
 void mac_bottom_dense(const CellGeom& g, const double* M, const unsigned char* act, const T* b, T* x, int singular,
                       cudaStream_t st);

@@ -7,6 +7,7 @@
 
 #include <vector>
 
+#include "bottom.h"
 #include "gbp_internal.cuh"
 #include "mac_kernels.h"
 #include "nodal_solver.h"
@@ -76,7 +77,7 @@ private:
     // r = b - A x on the finest level in FP64 (with the cut-face terms), norm = max |r| / (kap V)
     void resid64(const double* x, const double* b, double* r, unsigned long long* norm, cudaStream_t s);
     void eb_refresh_beta();
-    int build_dense_bottom();
+    int build_bottom();
     void record_iteration(int m);  // m V-cycles per refinement step
     int run_iteration(int m);
     int solve(bool have_guess, gbp_stats* stats);
@@ -101,9 +102,9 @@ private:
     bool robin_ready = false;
     unsigned* dflags = nullptr;
     DevicePool apool;  // alpha a V per level (ABecLaplacian)
-    // dense inverse of the coarsest operator (at most kMacDenseBottomMax cells), rebuilt with the face
-    // coefficients; the single-CTA CG otherwise
-    DevicePool dpool;
+    // the coarsest operator's rows and, for a small one, its dense inverse (bottom.h), rebuilt with the face
+    // coefficients; the single-CTA CG beyond the cluster solver's size
+    BottomRows brows;
     double* dmat = nullptr;
     unsigned char* dact = nullptr;
     bool dense_bottom = false;

@@ -15,6 +15,7 @@
 
 #include <algorithm>
 
+#include "bottom.h"
 #include "gbp_internal.cuh"
 #include "nodal_kernels.h"
 #include "nodal_sweep.h"
@@ -808,7 +809,7 @@ int nodal_coarse_cluster_size()
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(16);
         cfg.blockDim = dim3(kCoarseThreads);
-        cfg.dynamicSmemBytes = 216 * sizeof(double);
+        cfg.dynamicSmemBytes = kDenseBottom * sizeof(double);
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = 16;

@@ -278,12 +278,19 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
         if (qsweep_supported(lv.g))
             for (int q = 0; q < 5; ++q) add(lv.g.count, 8);
     add(nodal_partials_needed(G0) + 64, 8);
-    add(5 * B.g.count, 8);
+    nbottom = B.g.nu[0] * B.g.nu[1] * B.g.nu[2];
+    dense_bottom = nbottom <= kDenseBottom;
+    brows = BottomRows{};
+    if (nbottom <= kClusterBottom) {
+        brows.n = nbottom;
+        brows.w = 27;
+        add(brows.bytes() + 512, 1);
+    } else {
+        add(5 * B.g.count, 8);
+    }
     add(16, 4);
     add(8, 8);
     add(8, 8);
-    nbottom = B.g.nu[0] * B.g.nu[1] * B.g.nu[2];
-    dense_bottom = nbottom <= kDenseBottomMax;
     if (dense_bottom) add((size_t)nbottom * nbottom, 8);
     need += 4096;
     rc = pool.reserve(need);
@@ -315,7 +322,11 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
         if (qsweep_supported(lv.g))
             for (double** w : {&lv.qw.w5, &lv.qw.rd, &lv.qw.wx, &lv.qw.wy, &lv.qw.wz}) *w = pool.take<double>(lv.g.count);
     partials = pool.take<double>(nodal_partials_needed(G0) + 64);
-    bscr = pool.take<double>(5 * B.g.count);
+    bscr = nullptr;
+    if (brows.n)
+        brows.carve(pool.take<char>(brows.bytes()));
+    else
+        bscr = pool.take<double>(5 * B.g.count);
     dinfo = pool.take<int>(16);
     derr = reinterpret_cast<unsigned*>(dinfo + 8);
     dnorm = pool.take<unsigned long long>(8);
@@ -388,140 +399,39 @@ int NodalSolver::level_of(const NodalGeom& g) const
     return -1;
 }
 
-// Dense inverse of the coarsest operator, assembled on the host from the coarsest sigma: the
-// bottom solve becomes one FP64 matrix-vector product in one CTA. Singular systems (no Dirichlet
-// face) use (A + c 1 1^T)^-1, which solves A x = b exactly for consistent b (sum b = 0).
+// The coarsest operator's rows from the present sigma, and for a small one its dense inverse (bottom.h).
 int NodalSolver::build_bottom()
 {
+    if (!brows.n) return GBP_OK;
+    bottom_rows_nodal(L.back().g, L.back().s64, brows, st);
     if (!dense_bottom) return GBP_OK;
-    const NodalLevel& B = L.back();
-    const NodalGeom& g = B.g;
-    std::vector<double> sg((size_t)g.count);
-    GBP_CUDA(cudaMemcpyAsync(sg.data(), B.s64, sizeof(double) * g.count, cudaMemcpyDeviceToHost, st));
+    unsigned* bad = reinterpret_cast<unsigned*>(dinfo + 12);
+    GBP_CUDA(cudaMemsetAsync(bad, 0, sizeof(unsigned), st));
+    bottom_inverse(brows, bsing ? 1 : 0, dmat, nullptr, bad, st);
+    unsigned h = 0;
+    GBP_CUDA(cudaMemcpyAsync(&h, bad, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     GBP_CUDA(cudaStreamSynchronize(st));
-    const int N = nbottom;
-    std::vector<double> A((size_t)N * N, 0.0);
-    auto wrapn = [&](int i, int d) { return g.per[d] ? ((i % g.n[d]) + g.n[d]) % g.n[d] : i; };
-    std::vector<unsigned char> hm;
-    if (g.mask) {
-        hm.resize((size_t)g.count);
-        GBP_CUDA(cudaMemcpyAsync(hm.data(), g.mask, g.count, cudaMemcpyDeviceToHost, st));
-        GBP_CUDA(cudaStreamSynchronize(st));
+    if (h) {
+        set_error("nodal plan: the coarsest operator is singular beyond its constant null space");
+        return GBP_BAD_ARG;
     }
-    auto dir = [&](int i, int j, int k) {
-        return (g.dlo[0] && i == 0) || (g.dhi[0] && i == g.n[0]) || (g.dlo[1] && j == 0) || (g.dhi[1] && j == g.n[1]) ||
-               (g.dlo[2] && k == 0) || (g.dhi[2] && k == g.n[2]) ||
-               (g.mask && !hm[(size_t)pidx(g.sy, g.sz, i, j, k)]);
-    };
-    for (int k = 0; k < g.nu[2]; ++k)
-        for (int j = 0; j < g.nu[1]; ++j)
-            for (int i = 0; i < g.nu[0]; ++i) {
-                const int u = i + g.nu[0] * (j + g.nu[1] * k);
-                if (dir(i, j, k)) {
-                    A[(size_t)u * N + u] = 1.0;
-                    continue;
-                }
-                for (int c = 0; c < 2; ++c)
-                    for (int b = 0; b < 2; ++b)
-                        for (int a = 0; a < 2; ++a) {
-                            int cell[3] = {i - 1 + a, j - 1 + b, k - 1 + c};
-                            bool inside = true;
-                            for (int d = 0; d < 3; ++d) {
-                                if (g.per[d])
-                                    cell[d] = wrapn(cell[d], d);
-                                else if (cell[d] < 0 || cell[d] >= g.n[d])
-                                    inside = false;
-                            }
-                            if (!inside) continue;
-                            const double s = sg[(size_t)pidx(g.sy, g.sz, cell[0], cell[1], cell[2])];
-                            for (int r = 0; r < 2; ++r)
-                                for (int q = 0; q < 2; ++q)
-                                    for (int pp = 0; pp < 2; ++pp) {
-                                        int nd[3] = {cell[0] + pp, cell[1] + q, cell[2] + r};
-                                        for (int d = 0; d < 3; ++d)
-                                            if (g.per[d]) nd[d] = wrapn(nd[d], d);
-                                        if (dir(nd[0], nd[1], nd[2])) continue;
-                                        const int mask = (pp != 1 - a) | ((q != 1 - b) << 1) | ((r != 1 - c) << 2);
-                                        const int v = nd[0] + g.nu[0] * (nd[1] + g.nu[1] * nd[2]);
-                                        A[(size_t)u * N + v] += s * g.K[mask];
-                                    }
-                        }
-            }
-    if (bsing) {
-        double tr = 0.0;
-        for (int u = 0; u < N; ++u) tr += A[(size_t)u * N + u];
-        const double c = tr / ((double)N * N);
-        for (auto& v : A) v += c;
-    }
-    // Gauss-Jordan inverse with partial pivoting
-    std::vector<double> M((size_t)N * N, 0.0);
-    for (int u = 0; u < N; ++u) M[(size_t)u * N + u] = 1.0;
-    for (int col = 0; col < N; ++col) {
-        int piv = col;
-        for (int r = col + 1; r < N; ++r)
-            if (fabs(A[(size_t)r * N + col]) > fabs(A[(size_t)piv * N + col])) piv = r;
-        if (A[(size_t)piv * N + col] == 0.0) {
-            set_error("nodal plan: the coarsest operator is singular beyond its constant null space");
-            return GBP_BAD_ARG;
-        }
-        if (piv != col)
-            for (int q = 0; q < N; ++q) {
-                std::swap(A[(size_t)piv * N + q], A[(size_t)col * N + q]);
-                std::swap(M[(size_t)piv * N + q], M[(size_t)col * N + q]);
-            }
-        const double inv = 1.0 / A[(size_t)col * N + col];
-        for (int q = 0; q < N; ++q) {
-            A[(size_t)col * N + q] *= inv;
-            M[(size_t)col * N + q] *= inv;
-        }
-        for (int r = 0; r < N; ++r) {
-            if (r == col) continue;
-            const double f = A[(size_t)r * N + col];
-            if (f == 0.0) continue;
-            for (int q = 0; q < N; ++q) {
-                A[(size_t)r * N + q] -= f * A[(size_t)col * N + q];
-                M[(size_t)r * N + q] -= f * M[(size_t)col * N + q];
-            }
-        }
-    }
-    // Dirichlet nodes stay 0: zero their rows and columns
-    for (int k = 0; k < g.nu[2]; ++k)
-        for (int j = 0; j < g.nu[1]; ++j)
-            for (int i = 0; i < g.nu[0]; ++i)
-                if (dir(i, j, k)) {
-                    const int u = i + g.nu[0] * (j + g.nu[1] * k);
-                    for (int q = 0; q < N; ++q) M[(size_t)u * N + q] = M[(size_t)q * N + u] = 0.0;
-                }
-    // stored transposed: step v of the product reads M[v][*] across the threads
-    std::vector<double> Mt((size_t)N * N);
-    for (int u = 0; u < N; ++u)
-        for (int v = 0; v < N; ++v) Mt[(size_t)v * N + u] = M[(size_t)u * N + v];
-    GBP_CUDA(cudaMemcpyAsync(dmat, Mt.data(), sizeof(double) * Mt.size(), cudaMemcpyHostToDevice, st));
-    GBP_CUDA(cudaStreamSynchronize(st));
     return GBP_OK;
 }
 
-template <>
-void NodalSolver::bottom<double>(int l, const double* b, double* x)
+template <typename T>
+void NodalSolver::bottom(int l, const T* b, T* x)
 {
     const NodalLevel& lv = L[l];
-    if (dense_bottom)
-        nodal_bottom_dense<double>(lv.g, dmat, b, x, bsing ? 1 : 0, cap_or_st);
-    else
-        nodal_bottom<double>(lv.g, lv.s64, b, x, bscr, opt.bottom_maxiter, opt.bottom_rtol, opt.bottom_atol, dinfo,
-                             bsing ? 1 : 0, cap_or_st);
-    xres[l] = x;
-}
-
-template <>
-void NodalSolver::bottom<float>(int l, const float* b, float* x)
-{
-    const NodalLevel& lv = L[l];
-    if (dense_bottom)
-        nodal_bottom_dense<float>(lv.g, dmat, b, x, bsing ? 1 : 0, cap_or_st);
-    else
-        nodal_bottom<float>(lv.g, lv.s64, b, x, bscr, opt.bottom_maxiter, opt.bottom_rtol, opt.bottom_atol, dinfo,
-                            bsing ? 1 : 0, cap_or_st);
+    if (dense_bottom) {
+        nodal_bottom_dense<T>(lv.g, dmat, b, x, bsing ? 1 : 0, cap_or_st);
+    } else if (brows.n) {
+        const BottomCG c{brows, bsing ? 1 : 0, opt.bottom_maxiter, opt.bottom_rtol, opt.bottom_atol, dinfo};
+        const int rc = bottom_cg_nodal<T>(lv.g, c, b, x, cap_or_st);
+        if (rc && !launch_rc) launch_rc = rc;
+    } else {
+        nodal_bottom<T>(lv.g, lv.s64, b, x, bscr, opt.bottom_maxiter, opt.bottom_rtol, opt.bottom_atol, dinfo,
+                        bsing ? 1 : 0, cap_or_st);
+    }
     xres[l] = x;
 }
 

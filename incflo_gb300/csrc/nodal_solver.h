@@ -7,6 +7,7 @@
 
 #include <vector>
 
+#include "bottom.h"
 #include "gbp_internal.cuh"
 #include "krylov.h"
 #include "nodal_kernels.h"
@@ -207,7 +208,8 @@ private:
     KrylovState* kstate = nullptr;
     KrylovBox kbox{};
     double* partials = nullptr;  // reduction scratch
-    double* bscr = nullptr;      // bottom CG scratch
+    double* bscr = nullptr;      // scratch of the single-CTA bottom CG (coarsest levels beyond the cluster's)
+    BottomRows brows;            // the coarsest operator's rows
     int* dinfo = nullptr;        // bottom iteration count
     unsigned long long* dnorm = nullptr;  // [0] rhs norm, [1] residual norm
     unsigned long long* hnorm = nullptr;  // pinned mirror
@@ -256,7 +258,6 @@ private:
     int gexec_prec = -1;
     double gexec_scale = 0.0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
-    static constexpr int kDenseBottomMax = 216;
     int nbottom = 0;
     bool dense_bottom = false;
     double* dmat = nullptr;      // dense inverse of the coarsest operator (transposed)

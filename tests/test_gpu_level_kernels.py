@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import oracle as O
-from incflo_gb300 import Geometry, NodalProjector, make_options
+from incflo_gb300 import Geometry, MacProjector, NodalProjector, make_options
 from tests.helpers import D, I, N, P, cuda, nodal_case, rel_l2, unique_nodes
 
 pytestmark = pytest.mark.gpu
@@ -55,3 +55,48 @@ def test_accelerated_vcycles_on_stretched_cells(gpu_lib, n, ext, lo, hi, precisi
                           options=make_options(0, precision=precision))
     proj.setDomainBC(lo, hi)
     assert proj.project(rtol=1e-11, atol=0.0)["vcycles"] <= 24
+
+
+# coarsest levels of 65 to several thousand unknowns (cell counts with odd factors): the cluster's conjugate
+# gradients, with rows that leave lanes, warps and whole CTAs idle, and with coefficients kept in shared memory or not
+BOTTOMS = [
+    ((24, 20, 36), (P, N, P), (P, N, P)),     # singular
+    ((40, 56, 24), (N, D, P), (I, N, P)),
+    ((26, 22, 34), (P, P, D), (P, P, N)),     # 13 x 11 x 17 cells
+    ((42, 38, 50), (N, N, N), (N, N, N)),     # 21 x 19 x 25 cells: coefficients from L2
+]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,lo,hi", BOTTOMS, ids=["x".join(map(str, c[0])) for c in BOTTOMS])
+def test_cluster_bottom_solve_nodal(gpu_lib, n, lo, hi, precision):
+    _nodal(n, lo, hi, precision)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,lo,hi", BOTTOMS, ids=["x".join(map(str, c[0])) for c in BOTTOMS])
+def test_cluster_bottom_solve_mac(gpu_lib, n, lo, hi, precision):
+    lo, hi = ([N if b == I else b for b in s] for s in (lo, hi))
+    g = O.Grid(n, hi=tuple(v / n[0] for v in n), bclo=lo, bchi=hi)
+    rng = np.random.default_rng(3)
+    beta = [rng.uniform(0.3, 1.0, g.face_shape(d)) for d in range(3)]
+    u = [rng.standard_normal(g.face_shape(d)) for d in range(3)]
+    for d in range(3):  # one value per periodic face, none through walls
+        ax = 2 - d
+        first, last = [slice(None)] * 3, [slice(None)] * 3
+        first[ax], last[ax] = 0, -1
+        for f in (beta[d], u[d]):
+            if lo[d] == P:
+                f[tuple(last)] = f[tuple(first)]
+        if lo[d] == N:
+            u[d][tuple(first)] = 0.0
+        if hi[d] == N:
+            u[d][tuple(last)] = 0.0
+    un, phi_or, st_or = O.mac_project(g, beta, u, rtol=1e-13)
+    mp = MacProjector(Geometry(n, (0, 0, 0), tuple(v / n[0] for v in n)), options=make_options(1, precision=precision))
+    mp.initProjector(beta=[cuda(b) for b in beta])
+    mp.setDomainBC(lo, hi)
+    ut, phi = [cuda(x) for x in u], cuda(np.zeros(g.cell_shape))
+    mp.setUMAC(ut)
+    st = mp.project(rtol=1e-12, atol=0.0, phi=phi, phi_guess=False)
+    assert st["status"] == 0 and rel_l2(phi.cpu().numpy(), phi_or) <= 1e-9
