@@ -101,9 +101,19 @@ __device__ __forceinline__ T mac_Ax(const CellGeom& g, const T* __restrict__ x, 
     return ax;
 }
 
-template <typename T>
+// Red-black half sweep: x = (b + sum w beta x_nb) / diag on the cells of one colour. FROM 1: the first half sweep from
+// x = 0, b / diag (nothing of x is read, and the other colour need not hold 0: its own half sweep follows and reads only
+// this one). FROM 2: x_nb + the coarse correction of the neighbour's parent, the piecewise-constant prolongation applied
+// on the way: neither colour's corrected value is ever stored, because the first half sweep replaces this colour from
+// the corrected other one, and the second replaces the other.
+// FP32: HBM bound on large levels. FP64: the pipe (2 lanes per clock and SM) bounds it, so 1 / diag comes from an array
+// (id) and each direction's weight multiplies once: 10 instructions per cell against about 36 with the division and six
+// weighted coefficients.
+template <typename T, int FROM>
 __global__ void __launch_bounds__(256) k_mac_rbgs(CellGeom g, const T* __restrict__ bx, const T* __restrict__ by,
-                                                  const T* __restrict__ bz, const T* __restrict__ b, T* x, int color)
+                                                  const T* __restrict__ bz, const T* __restrict__ b,
+                                                  const T* __restrict__ id, T* x, int color, CellGeom gc,
+                                                  const T* __restrict__ xc)
 {
     // thread t handles the t-th cell of this colour along x
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -125,10 +135,81 @@ __global__ void __launch_bounds__(256) k_mac_rbgs(CellGeom g, const T* __restric
     }
     if (i >= g.n[0]) return;
     const long long p = pidx(g.sy, g.sz, i, j, k);
-    T diag, off;
-    (void)mac_Ax<T>(g, x, bx, by, bz, p, diag, off);
-    const T v = diag != T(0) ? (b[p] + off) / diag : T(0);
+    T v;
+    if (sizeof(T) == 8 && FROM == 1) {
+        v = b[p] * id[p];
+    } else {
+        const T wx = (T)g.w[0], wy = (T)g.w[1], wz = (T)g.w[2];
+        const T b0 = bx[p], b1 = bx[p + 1], b2 = by[p], b3 = by[p + g.sy], b4 = bz[p], b5 = bz[p + g.sz];
+        T acc = b[p];
+        if (FROM != 1) {
+            T xw = x[p - 1], xe = x[p + 1], xs = x[p - g.sy], xn = x[p + g.sy], xb = x[p - g.sz], xt = x[p + g.sz];
+            if (FROM == 2) {
+                const int I = i >> 1, J = j >> 1, K = k >> 1;
+                const long long q = pidx(gc.sy, gc.sz, I, J, K);
+                const T e = xc[q];  // the parent of this cell and of its neighbour on one side in each direction
+                xw += (i & 1) ? e : xc[q - 1];
+                xe += (i & 1) ? xc[q + 1] : e;
+                xs += (j & 1) ? e : xc[q - gc.sy];
+                xn += (j & 1) ? xc[q + gc.sy] : e;
+                xb += (k & 1) ? e : xc[q - gc.sz];
+                xt += (k & 1) ? xc[q + gc.sz] : e;
+            }
+            acc += wx * (b0 * xw + b1 * xe);
+            acc += wy * (b2 * xs + b3 * xn);
+            acc += wz * (b4 * xb + b5 * xt);
+        }
+        if (sizeof(T) == 8) {
+            v = acc * id[p];
+        } else {
+            T diag = wx * (b0 + b1) + wy * (b2 + b3) + wz * (b4 + b5);
+            const T* ac = mac_acoef<T>(g);
+            if (ac) diag += ac[p];
+            v = diag != T(0) ? acc / diag : T(0);
+        }
+    }
     store_cell(x, g, i, j, k, v);
+}
+
+// 1 / diag of every cell (0 where the cell carries no equation)
+__global__ void __launch_bounds__(256) k_mac_idiag(CellGeom g, const double* __restrict__ bx, const double* __restrict__ by,
+                                                   const double* __restrict__ bz, double* __restrict__ id)
+{
+    int i, j, k;
+    if (!decode_cell(g, blockIdx.x * (long long)blockDim.x + threadIdx.x, i, j, k)) return;
+    const long long p = pidx(g.sy, g.sz, i, j, k);
+    double diag = fma(g.w[0], bx[p] + bx[p + 1], fma(g.w[1], by[p] + by[p + g.sy], g.w[2] * (bz[p] + bz[p + g.sz])));
+    if (g.a64) diag += g.a64[p];
+    id[p] = diag != 0.0 ? 1.0 / diag : 0.0;
+}
+
+// Coarse right-hand side after a pre-smoothing that ended on the black cells: their residual is rounding, so the sum
+// of the 8 fine residuals is that of the 4 red ones. One thread per coarse cell; neither the residual nor a second pass
+// over it touches memory (the two kernels moved 6 + 1 vectors of the fine level, this one reads 5).
+template <typename T>
+__global__ void __launch_bounds__(256) k_mac_resid_restrict(CellGeom g, CellGeom gc, const T* __restrict__ bx,
+                                                            const T* __restrict__ by, const T* __restrict__ bz,
+                                                            const T* __restrict__ x, const T* __restrict__ b,
+                                                            T* __restrict__ bc)
+{
+    int I, J, K;
+    if (!decode_cell(gc, blockIdx.x * (long long)blockDim.x + threadIdx.x, I, J, K)) return;
+    const long long f = pidx(g.sy, g.sz, 2 * I, 2 * J, 2 * K);
+    const T wx = (T)g.w[0], wy = (T)g.w[1], wz = (T)g.w[2];
+    const T* ac = mac_acoef<T>(g);
+    T sum = T(0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int a = q == 1 || q == 2, bb = q == 1 || q == 3, c = q >= 2;  // (0,0,0), (1,1,0), (1,0,1), (0,1,1)
+        const long long p = f + a + (bb ? g.sy : 0) + (c ? g.sz : 0);
+        const T xc = x[p];
+        T ax = wx * (bx[p] * (xc - x[p - 1]) + bx[p + 1] * (xc - x[p + 1]));
+        ax += wy * (by[p] * (xc - x[p - g.sy]) + by[p + g.sy] * (xc - x[p + g.sy]));
+        ax += wz * (bz[p] * (xc - x[p - g.sz]) + bz[p + g.sz] * (xc - x[p + g.sz]));
+        if (ac) ax += ac[p] * xc;
+        sum += b[p] - ax;
+    }
+    bc[pidx(gc.sy, gc.sz, I, J, K)] = sum;
 }
 
 template <typename T>
@@ -142,7 +223,7 @@ __global__ void __launch_bounds__(256) k_mac_resid(CellGeom g, const T* __restri
     if (decode_cell(g, blockIdx.x * (long long)blockDim.x + threadIdx.x, i, j, k)) {
         const long long p = pidx(g.sy, g.sz, i, j, k);
         T diag, off;
-        const T v = b[p] - mac_Ax<T>(g, x, bx, by, bz, p, diag, off);
+        const T v = (b ? b[p] : T(0)) - mac_Ax<T>(g, x, bx, by, bz, p, diag, off);
         r[p] = v;
         if (norm) nv = fabs((double)v) / g.vol;
     }
@@ -171,7 +252,7 @@ __global__ void __launch_bounds__(256) k_mac_resid<double>(CellGeom g, const dou
         const double dz = fma(bz[p], xc - x[p - g.sz], bz[p + g.sz] * (xc - x[p + g.sz]));
         double ax = fma(g.w[0], dx, fma(g.w[1], dy, g.w[2] * dz));
         if (g.a64) ax = fma(g.a64[p], xc, ax);
-        const double v = b[p] - ax;
+        const double v = (b ? b[p] : 0.0) - ax;
         r[p] = v;
         key = abs_key(v);
     }
@@ -591,10 +672,35 @@ static inline long long nface(const CellGeom& g, int d)
 }
 
 template <typename T>
-void mac_rbgs(const CellGeom& g, const T* bx, const T* by, const T* bz, const T* b, T* x, int color, cudaStream_t st)
+void mac_rbgs(const CellGeom& g, const T* bx, const T* by, const T* bz, const T* b, const T* id, T* x, int color,
+              cudaStream_t st)
 {
     const long long n = (long long)g.n[1] * g.n[2] * ((g.n[0] + 1) / 2);
-    k_mac_rbgs<T><<<nblk(n, 256), 256, 0, st>>>(g, bx, by, bz, b, x, color);
+    k_mac_rbgs<T, 0><<<nblk(n, 256), 256, 0, st>>>(g, bx, by, bz, b, id, x, color, g, nullptr);
+}
+template <typename T>
+void mac_rbgs_zero(const CellGeom& g, const T* bx, const T* by, const T* bz, const T* b, const T* id, T* x, int color,
+                   cudaStream_t st)
+{
+    const long long n = (long long)g.n[1] * g.n[2] * ((g.n[0] + 1) / 2);
+    k_mac_rbgs<T, 1><<<nblk(n, 256), 256, 0, st>>>(g, bx, by, bz, b, id, x, color, g, nullptr);
+}
+template <typename T>
+void mac_rbgs_prolong(const CellGeom& g, const CellGeom& gc, const T* bx, const T* by, const T* bz, const T* b,
+                      const T* id, const T* xc, T* x, int color, cudaStream_t st)
+{
+    const long long n = (long long)g.n[1] * g.n[2] * ((g.n[0] + 1) / 2);
+    k_mac_rbgs<T, 2><<<nblk(n, 256), 256, 0, st>>>(g, bx, by, bz, b, id, x, color, gc, xc);
+}
+void mac_idiag(const CellGeom& g, const double* bx, const double* by, const double* bz, double* id, cudaStream_t st)
+{
+    k_mac_idiag<<<nblk(ncell(g), 256), 256, 0, st>>>(g, bx, by, bz, id);
+}
+template <typename T>
+void mac_resid_restrict(const CellGeom& g, const CellGeom& gc, const T* bx, const T* by, const T* bz, const T* x,
+                        const T* b, T* bc, cudaStream_t st)
+{
+    k_mac_resid_restrict<T><<<nblk(ncell(gc), 256), 256, 0, st>>>(g, gc, bx, by, bz, x, b, bc);
 }
 template <typename T>
 void mac_resid(const CellGeom& g, const T* bx, const T* by, const T* bz, const T* x, const T* b, T* r,
@@ -620,7 +726,14 @@ void mac_bottom(const CellGeom& g, const double* bx, const double* by, const dou
 }
 
 #define GBP_MAC_INST(T)                                                                                        \
-    template void mac_rbgs<T>(const CellGeom&, const T*, const T*, const T*, const T*, T*, int, cudaStream_t); \
+    template void mac_rbgs<T>(const CellGeom&, const T*, const T*, const T*, const T*, const T*, T*, int,      \
+                              cudaStream_t);                                                                   \
+    template void mac_rbgs_zero<T>(const CellGeom&, const T*, const T*, const T*, const T*, const T*, T*, int, \
+                                   cudaStream_t);                                                              \
+    template void mac_rbgs_prolong<T>(const CellGeom&, const CellGeom&, const T*, const T*, const T*, const T*, \
+                                      const T*, const T*, T*, int, cudaStream_t);                              \
+    template void mac_resid_restrict<T>(const CellGeom&, const CellGeom&, const T*, const T*, const T*,        \
+                                        const T*, const T*, T*, cudaStream_t);                                 \
     template void mac_resid<T>(const CellGeom&, const T*, const T*, const T*, const T*, const T*, T*,          \
                                unsigned long long*, cudaStream_t);                                            \
     template void mac_restrict<T>(const CellGeom&, const CellGeom&, const T*, T*, cudaStream_t);              \

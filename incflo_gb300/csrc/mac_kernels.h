@@ -7,8 +7,22 @@
 
 namespace gbp {
 
+// one red-black half sweep (colour 0 red, 1 black); id: 1 / diag (FP64 only); mac_rbgs_zero: from x = 0;
+// mac_rbgs_prolong: from x + the prolonged coarse correction xc on the other colour
 template <typename T>
-void mac_rbgs(const CellGeom& g, const T* bx, const T* by, const T* bz, const T* b, T* x, int color, cudaStream_t st);
+void mac_rbgs(const CellGeom& g, const T* bx, const T* by, const T* bz, const T* b, const T* id, T* x, int color,
+              cudaStream_t st);
+template <typename T>
+void mac_rbgs_zero(const CellGeom& g, const T* bx, const T* by, const T* bz, const T* b, const T* id, T* x, int color,
+                   cudaStream_t st);
+template <typename T>
+void mac_rbgs_prolong(const CellGeom& g, const CellGeom& gc, const T* bx, const T* by, const T* bz, const T* b,
+                      const T* id, const T* xc, T* x, int color, cudaStream_t st);
+void mac_idiag(const CellGeom& g, const double* bx, const double* by, const double* bz, double* id, cudaStream_t st);
+// coarse right-hand side bc = restriction of b - A x after a pre-smoothing that ended on the black cells
+template <typename T>
+void mac_resid_restrict(const CellGeom& g, const CellGeom& gc, const T* bx, const T* by, const T* bz, const T* x,
+                        const T* b, T* bc, cudaStream_t st);
 template <typename T>
 void mac_resid(const CellGeom& g, const T* bx, const T* by, const T* bz, const T* x, const T* b, T* r,
                unsigned long long* norm, cudaStream_t st);

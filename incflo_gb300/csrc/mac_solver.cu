@@ -145,7 +145,7 @@ int MacSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc_h
     size_t need = 0;
     auto add = [&](size_t cnt, size_t sz) { need = ((need + 255) & ~size_t(255)) + cnt * sz; };
     for (auto& lv : L) {
-        for (int q = 0; q < 6; ++q) add(lv.g.count, 8);
+        for (int q = 0; q < 7; ++q) add(lv.g.count, 8);
         for (int q = 0; q < 6; ++q) add(lv.g.count, 4);
     }
     const CellGeom& G0 = L[0].g;
@@ -179,6 +179,7 @@ int MacSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc_h
         lv.x64 = pool.take<double>(lv.g.count);
         lv.rhs64 = pool.take<double>(lv.g.count);
         lv.r64 = pool.take<double>(lv.g.count);
+        lv.id64 = pool.take<double>(lv.g.count);
         for (int d = 0; d < 3; ++d) lv.b32[d] = pool.take<float>(lv.g.count);
         lv.x32 = pool.take<float>(lv.g.count);
         lv.rhs32 = pool.take<float>(lv.g.count);
@@ -329,6 +330,7 @@ int MacSolver::abec_solve(const gbp_array4* rhs, gbp_array4* phi_io, gbp_stats* 
 // Cells whose row is empty (covered by an embedded boundary) carry no equation and stay 0.
 int MacSolver::build_bottom()
 {
+    idiag_ready = false;  // the coefficients changed
     if (!brows.n) return GBP_OK;
     const MacLevel& B = L.back();
     const bool was = dense_bottom;
@@ -354,6 +356,7 @@ void MacSolver::add_vcycle_correction(const double* r, double* e, double sc)
 {
     const MacLevel& l0 = L[0];
     cap_or_st = st;
+    ensure_idiag();
     if (opt.precision == GBP_PREC_MIXED) {
         mac_to_f32(l0.g, r, l0.rhs32, sc, st);
         vcycle<float>(0, l0.rhs32, true);
@@ -670,6 +673,7 @@ struct MacBufs<double> {
     template <typename E>
     static const double* cb(const E& e) { return e.cb64; }
     static double* const* b(const MacLevel& l) { return l.b64; }
+    static const double* id(const MacLevel& l) { return l.id64; }
     static double* x(const MacLevel& l) { return l.x64; }
     static double* rhs(const MacLevel& l) { return l.rhs64; }
     static double* r(const MacLevel& l) { return l.r64; }
@@ -681,6 +685,7 @@ struct MacBufs<float> {
     template <typename E>
     static const float* cb(const E& e) { return e.cb32; }
     static float* const* b(const MacLevel& l) { return l.b32; }
+    static const float* id(const MacLevel&) { return nullptr; }
     static float* x(const MacLevel& l) { return l.x32; }
     static float* rhs(const MacLevel& l) { return l.rhs32; }
     static float* r(const MacLevel& l) { return l.r32; }
@@ -743,6 +748,27 @@ void MacSolver::vcycle(int l, const T* b, bool zero)
         return;
     }
     T* const* be = B::b(lv);
+    const T* id = B::id(lv);
+    const MacLevel& cv = L[l + 1];
+    if (!(l == 0 && eb.on) && opt.nu1 >= 1 && opt.nu2 >= 1) {
+        for (int q = 0; q < opt.nu1; ++q) {
+            if (zero && q == 0)
+                mac_rbgs_zero<T>(lv.g, be[0], be[1], be[2], b, id, x, 0, s);
+            else
+                mac_rbgs<T>(lv.g, be[0], be[1], be[2], b, id, x, 0, s);
+            mac_rbgs<T>(lv.g, be[0], be[1], be[2], b, id, x, 1, s);
+        }
+        mac_resid_restrict<T>(lv.g, cv.g, be[0], be[1], be[2], x, b, B::rhs(cv), s);
+        vcycle<T>(l + 1, B::rhs(cv), true);
+        for (int q = 0; q < opt.nu2; ++q) {
+            if (q == 0)
+                mac_rbgs_prolong<T>(lv.g, cv.g, be[0], be[1], be[2], b, id, B::x(cv), x, 1, s);
+            else
+                mac_rbgs<T>(lv.g, be[0], be[1], be[2], b, id, x, 1, s);
+            mac_rbgs<T>(lv.g, be[0], be[1], be[2], b, id, x, 0, s);
+        }
+        return;
+    }
     if (zero) cudaMemsetAsync(x, 0, sizeof(T) * lv.g.count, s);
     // cut cells on the finest level: the smoother sees b minus the cut-face terms of the current x
     // (lagged by one red-black pair), the residual carries them exactly
@@ -757,21 +783,27 @@ void MacSolver::vcycle(int l, const T* b, bool zero)
         if (cut) eb_cells<T>(lv.g, eb.cells, eb.ncells, eb.faces, B::cb(eb), x, b, B::beff(eb), s);
     };
     for (int q = 0; q < opt.nu1; ++q) {
-        lag();
-        mac_rbgs<T>(lv.g, be[0], be[1], be[2], bs, x, 0, s);
-        mac_rbgs<T>(lv.g, be[0], be[1], be[2], bs, x, 1, s);
+        if (!(zero && q == 0)) lag();  // (x = 0: nothing to lag)
+        mac_rbgs<T>(lv.g, be[0], be[1], be[2], bs, id, x, 0, s);
+        mac_rbgs<T>(lv.g, be[0], be[1], be[2], bs, id, x, 1, s);
     }
     mac_resid<T>(lv.g, be[0], be[1], be[2], x, b, B::r(lv), nullptr, s);
     if (cut) eb_cells<T>(lv.g, eb.cells, eb.ncells, eb.faces, B::cb(eb), x, B::r(lv), B::r(lv), s);
-    const MacLevel& cv = L[l + 1];
     mac_restrict<T>(lv.g, cv.g, B::r(lv), B::rhs(cv), s);
     vcycle<T>(l + 1, B::rhs(cv), true);
     mac_prolong_add<T>(lv.g, cv.g, B::x(cv), x, s);
     for (int q = 0; q < opt.nu2; ++q) {
         lag();
-        mac_rbgs<T>(lv.g, be[0], be[1], be[2], bs, x, 1, s);
-        mac_rbgs<T>(lv.g, be[0], be[1], be[2], bs, x, 0, s);
+        mac_rbgs<T>(lv.g, be[0], be[1], be[2], bs, id, x, 1, s);
+        mac_rbgs<T>(lv.g, be[0], be[1], be[2], bs, id, x, 0, s);
     }
+}
+
+void MacSolver::ensure_idiag()
+{
+    if (idiag_ready || opt.precision == GBP_PREC_MIXED) return;
+    for (auto& lv : L) mac_idiag(lv.g, lv.b64[0], lv.b64[1], lv.b64[2], lv.id64, st);
+    idiag_ready = true;
 }
 
 void MacSolver::resid64(const double* x, const double* b, double* r, unsigned long long* norm, cudaStream_t s)
@@ -854,6 +886,7 @@ int MacSolver::solve(bool have_guess, gbp_stats* stats)
     const MacLevel& l0 = L[0];
     cap_or_st = st;
     GBP_CUDA(cudaEventRecord(ev1, st));
+    ensure_idiag();
     if (!have_guess) GBP_CUDA(cudaMemsetAsync(phi, 0, sizeof(double) * l0.g.count, st));
     GBP_CUDA(cudaMemsetAsync(dnorm, 0, 4 * sizeof(unsigned long long), st));
     mac_norm(l0.g, rhs0, dnorm, st, eb.on ? eb.m.kap : nullptr);

@@ -16,7 +16,7 @@ namespace gbp {
 
 struct MacLevel {
     CellGeom g;
-    double *b64[3] = {}, *x64 = nullptr, *rhs64 = nullptr, *r64 = nullptr;
+    double *b64[3] = {}, *x64 = nullptr, *rhs64 = nullptr, *r64 = nullptr, *id64 = nullptr;  // id64: 1 / diag
     float *b32[3] = {}, *x32 = nullptr, *rhs32 = nullptr, *r32 = nullptr;
 };
 
@@ -78,6 +78,9 @@ private:
     void resid64(const double* x, const double* b, double* r, unsigned long long* norm, cudaStream_t s);
     void eb_refresh_beta();
     int build_bottom();
+    // 1 / diag of every level for the FP64 half sweeps
+    void ensure_idiag();
+    bool idiag_ready = false;
     void record_iteration(int m);  // m V-cycles per refinement step
     int run_iteration(int m);
     int solve(bool have_guess, gbp_stats* stats);
