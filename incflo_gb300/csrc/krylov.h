@@ -26,6 +26,9 @@ struct KrylovState {
     double rz, rz_old, qz, pq, alpha, beta;
     int it, restart;
     unsigned done[2];  // blocks that finished a dot product (reset by the last one)
+    // power-of-two scale of an FP32 right-hand side, and its inverse: read on the device, so that a captured step
+    // serves every right-hand side
+    double scale, inv_scale;
 };
 
 // most blocks of a dot product (2 partial sums each in the scratch)

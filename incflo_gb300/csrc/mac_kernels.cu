@@ -12,6 +12,7 @@
 
 #include "bottom.h"
 #include "gbp_internal.cuh"
+#include "krylov.h"
 #include "mac_kernels.h"
 
 namespace gbp {
@@ -645,16 +646,20 @@ __global__ void k_mac_remove_mean(CellGeom g, double* __restrict__ v, const doub
 }
 
 template <typename TE>
-__global__ void k_mac_add_correction(CellGeom g, double* __restrict__ x, const TE* __restrict__ e, double inv_scale)
+__global__ void k_mac_add_correction(CellGeom g, double* __restrict__ x, const TE* __restrict__ e, double inv_scale,
+                                     const KrylovState* __restrict__ ks)
 {
+    if (ks) inv_scale = ks->inv_scale;
     int i, j, k;
     if (!decode_cell(g, blockIdx.x * (long long)blockDim.x + threadIdx.x, i, j, k)) return;
     const long long p = pidx(g.sy, g.sz, i, j, k);
     store_cell(x, g, i, j, k, x[p] + (double)e[p] * inv_scale);
 }
 
-__global__ void k_mac_to_f32(CellGeom g, const double* __restrict__ r, float* __restrict__ r32, double scale)
+__global__ void k_mac_to_f32(CellGeom g, const double* __restrict__ r, float* __restrict__ r32, double scale,
+                             const KrylovState* __restrict__ ks)
 {
+    if (ks) scale = ks->scale;
     int i, j, k;
     if (!decode_cell(g, blockIdx.x * (long long)blockDim.x + threadIdx.x, i, j, k)) return;
     const long long p = pidx(g.sy, g.sz, i, j, k);
@@ -1327,15 +1332,18 @@ void eb_zero_covered(const CellGeom& g, const double* kap, double* phi, cudaStre
     k_eb_zero_covered<<<nblk(ncell(g), 256), 256, 0, st>>>(g, kap, phi);
 }
 template <typename TE>
-void mac_add_correction(const CellGeom& g, double* x, const TE* e, double inv_scale, cudaStream_t st)
+void mac_add_correction(const CellGeom& g, double* x, const TE* e, double inv_scale, cudaStream_t st,
+                        const KrylovState* ks)
 {
-    k_mac_add_correction<TE><<<nblk(ncell(g), 256), 256, 0, st>>>(g, x, e, inv_scale);
+    k_mac_add_correction<TE><<<nblk(ncell(g), 256), 256, 0, st>>>(g, x, e, inv_scale, ks);
 }
-template void mac_add_correction<double>(const CellGeom&, double*, const double*, double, cudaStream_t);
-template void mac_add_correction<float>(const CellGeom&, double*, const float*, double, cudaStream_t);
-void mac_to_f32(const CellGeom& g, const double* r, float* r32, double scale, cudaStream_t st)
+template void mac_add_correction<double>(const CellGeom&, double*, const double*, double, cudaStream_t,
+                                         const KrylovState*);
+template void mac_add_correction<float>(const CellGeom&, double*, const float*, double, cudaStream_t,
+                                        const KrylovState*);
+void mac_to_f32(const CellGeom& g, const double* r, float* r32, double scale, cudaStream_t st, const KrylovState* ks)
 {
-    k_mac_to_f32<<<nblk(ncell(g), 256), 256, 0, st>>>(g, r, r32, scale);
+    k_mac_to_f32<<<nblk(ncell(g), 256), 256, 0, st>>>(g, r, r32, scale, ks);
 }
 
 }  // namespace gbp

@@ -7,6 +7,8 @@
 
 namespace gbp {
 
+struct KrylovState;
+
 // one red-black half sweep (colour 0 red, 1 black); id: 1 / diag (FP64 only); mac_rbgs_zero: from x = 0;
 // mac_rbgs_prolong: from x + the prolonged coarse correction xc on the other colour
 template <typename T>
@@ -162,7 +164,10 @@ int mac_partials_needed(const CellGeom& g);
 void mac_remove_mean(const CellGeom& g, double* v, double* partials, int mode, cudaStream_t st,
                      const double* kap = nullptr, double nfluid = 0.0);
 template <typename TE>
-void mac_add_correction(const CellGeom& g, double* x, const TE* e, double inv_scale, cudaStream_t st);
-void mac_to_f32(const CellGeom& g, const double* r, float* r32, double scale, cudaStream_t st);
+void mac_add_correction(const CellGeom& g, double* x, const TE* e, double inv_scale, cudaStream_t st,
+                        const KrylovState* ks = nullptr);
+// (ks: the scale is read from the device instead)
+void mac_to_f32(const CellGeom& g, const double* r, float* r32, double scale, cudaStream_t st,
+                const KrylovState* ks = nullptr);
 
 }  // namespace gbp

@@ -9,6 +9,7 @@
 
 #include "bottom.h"
 #include "gbp_internal.cuh"
+#include "krylov.h"
 #include "mac_kernels.h"
 #include "nodal_solver.h"
 
@@ -96,9 +97,16 @@ private:
     bool singular = false;
     bool beta_ready = false;
     double scale32 = 1.0;
-    cudaGraphExec_t gexec = nullptr;
+    static constexpr int kMaxGraphs = 8;  // captured steps of 1 to 8 inner V-cycles (more are launched directly)
+    cudaGraphExec_t gexec[kMaxGraphs + 1] = {};
     int gexec_prec = -1;
-    double gexec_scale = 0.0;
+    void drop_graphs();
+    // conjugate-gradient vectors (as NodalSolver's)
+    double *kp = nullptr, *kq = nullptr, *kpart = nullptr;
+    KrylovState *kstate = nullptr, *hstate = nullptr;
+    KrylovBox kbox{};
+    template <typename T>
+    void krylov_steps(int m, T* x, T* r, cudaStream_t s);
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     RobinFaces rb{};             // finest-level Robin faces (sides with GBP_BC_ROBIN)
     bool any_dirichlet = false;  // a Dirichlet side exists (the system is nonsingular)

@@ -17,6 +17,7 @@
 
 #include "bottom.h"
 #include "gbp_internal.cuh"
+#include "krylov.h"
 #include "nodal_kernels.h"
 #include "nodal_sweep.h"
 
@@ -1130,8 +1131,9 @@ __global__ void __launch_bounds__(256) k_remove_mean(NodalGeom g, double* __rest
 
 template <typename TE>
 __global__ void __launch_bounds__(256) k_add_correction(NodalGeom g, double* __restrict__ x, const TE* __restrict__ e,
-                                                        double inv_scale)
+                                                        double inv_scale, const KrylovState* __restrict__ ks)
 {
+    if (ks) inv_scale = ks->inv_scale;
     int i, j, k;
     if (!grid3_node(g, i, j, k)) return;
     const long long p = pidx(g.sy, g.sz, i, j, k);
@@ -1139,8 +1141,9 @@ __global__ void __launch_bounds__(256) k_add_correction(NodalGeom g, double* __r
 }
 
 __global__ void __launch_bounds__(256) k_to_f32(NodalGeom g, const double* __restrict__ r, float* __restrict__ r32,
-                                                double scale)
+                                                double scale, const KrylovState* __restrict__ ks)
 {
+    if (ks) scale = ks->scale;
     int i, j, k;
     if (!grid3_node(g, i, j, k)) return;
     const long long p = pidx(g.sy, g.sz, i, j, k);
@@ -1455,16 +1458,19 @@ void nodal_norm(const NodalGeom& g, const double* v, unsigned long long* norm, c
 int nodal_partials_needed(const NodalGeom& g) { return std::max(nodal_rhs_partials(g), 1184); }
 
 template <typename TE>
-void nodal_add_correction(const NodalGeom& g, double* x, const TE* e, double inv_scale, cudaStream_t st)
+void nodal_add_correction(const NodalGeom& g, double* x, const TE* e, double inv_scale, cudaStream_t st,
+                          const KrylovState* ks)
 {
-    k_add_correction<TE><<<grid3(g), kBlock3, 0, st>>>(g, x, e, inv_scale);
+    k_add_correction<TE><<<grid3(g), kBlock3, 0, st>>>(g, x, e, inv_scale, ks);
 }
-template void nodal_add_correction<double>(const NodalGeom&, double*, const double*, double, cudaStream_t);
-template void nodal_add_correction<float>(const NodalGeom&, double*, const float*, double, cudaStream_t);
+template void nodal_add_correction<double>(const NodalGeom&, double*, const double*, double, cudaStream_t,
+                                           const KrylovState*);
+template void nodal_add_correction<float>(const NodalGeom&, double*, const float*, double, cudaStream_t,
+                                          const KrylovState*);
 
-void nodal_to_f32(const NodalGeom& g, const double* r, float* r32, double scale, cudaStream_t st)
+void nodal_to_f32(const NodalGeom& g, const double* r, float* r32, double scale, cudaStream_t st, const KrylovState* ks)
 {
-    k_to_f32<<<grid3(g), kBlock3, 0, st>>>(g, r, r32, scale);
+    k_to_f32<<<grid3(g), kBlock3, 0, st>>>(g, r, r32, scale, ks);
 }
 
 void nodal_correct(const NodalGeom& g, const CorrArgs& a, const double* s64, const double* phi, cudaStream_t st,

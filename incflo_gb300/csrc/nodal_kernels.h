@@ -7,6 +7,8 @@
 
 namespace gbp {
 
+struct KrylovState;
+
 // Inputs of the fused right-hand-side kernel: u' = u + (add_gp ? sigma*gp : 0) - (sub_old ? u_old : 0)
 struct RhsArgs {
     gbp_array4 vel;
@@ -107,8 +109,11 @@ void nodal_fold(const NodalGeom& g, const double* part, int nparts, double* scal
 int nodal_partials_needed(const NodalGeom& g);
 void nodal_norm(const NodalGeom& g, const double* v, unsigned long long* norm, cudaStream_t st);
 template <typename TE>
-void nodal_add_correction(const NodalGeom& g, double* x, const TE* e, double inv_scale, cudaStream_t st);
-void nodal_to_f32(const NodalGeom& g, const double* r, float* r32, double scale, cudaStream_t st);
+void nodal_add_correction(const NodalGeom& g, double* x, const TE* e, double inv_scale, cudaStream_t st,
+                          const KrylovState* ks = nullptr);
+// (ks: the scale is read from the device instead)
+void nodal_to_f32(const NodalGeom& g, const double* r, float* r32, double scale, cudaStream_t st,
+                  const KrylovState* ks = nullptr);
 // cell planes k0 .. k1-1 (k1 < 0: to the last plane)
 void nodal_correct(const NodalGeom& g, const CorrArgs& a, const double* s64, const double* phi, cudaStream_t st,
                    int k0 = 0, int k1 = -1);

@@ -98,6 +98,7 @@ void NodalSolver::destroy()
     drop_graphs();
     if (hnorm) cudaFreeHost(hnorm);
     hnorm = nullptr;
+    hstate = nullptr;
     if (cap) cudaStreamDestroy(cap);
     cap = nullptr;
     if (ev0) cudaEventDestroy(ev0);
@@ -332,8 +333,9 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
     dnorm = pool.take<unsigned long long>(8);
     dscal = pool.take<double>(8);
     if (dense_bottom) dmat = pool.take<double>((size_t)nbottom * nbottom);
-    GBP_CUDA(cudaMallocHost(&hnorm, 8 * sizeof(unsigned long long)));
-    memset(hnorm, 0, 8 * sizeof(unsigned long long));
+    GBP_CUDA(cudaMallocHost(&hnorm, 8 * sizeof(unsigned long long) + sizeof(KrylovState)));
+    memset(hnorm, 0, 8 * sizeof(unsigned long long) + sizeof(KrylovState));
+    hstate = reinterpret_cast<KrylovState*>(hnorm + 8);
     GBP_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
     GBP_CUDA(cudaEventCreate(&ev0));
     GBP_CUDA(cudaEventCreate(&ev1));
@@ -696,7 +698,7 @@ void NodalSolver::record_iteration(int m)
     cudaMemsetAsync(dnorm + 1, 0, sizeof(unsigned long long), s);
     if (opt.precision == GBP_PREC_MIXED) {
         const float* e = nullptr;
-        nodal_to_f32(l0.g, res, l0.b32, scale32, s);
+        nodal_to_f32(l0.g, res, l0.b32, 1.0, s, kstate);
         if (accelerated()) {
             float* x = reinterpret_cast<float*>(kp) + l0.g.count;
             cudaMemsetAsync(x, 0, sizeof(float) * l0.g.count, s);
@@ -707,7 +709,7 @@ void NodalSolver::record_iteration(int m)
             for (int c = 1; c < m; ++c) vcycle<float>(0, l0.b32, false);
             e = (const float*)xres[0];
         }
-        nodal_add_correction<float>(l0.g, phi, e, 1.0 / scale32, s);
+        nodal_add_correction<float>(l0.g, phi, e, 1.0, s, kstate);
         resid0(phi, rhs0, res, dnorm + 1, s);
         nk += 3;
     } else {
@@ -789,10 +791,9 @@ int NodalSolver::run_iteration(int m)
         GBP_CUDA(cudaGetLastError());
         return GBP_OK;
     }
-    if (gexec_prec != opt.precision || gexec_scale != scale32) {
+    if (gexec_prec != opt.precision) {
         drop_graphs();
         gexec_prec = opt.precision;
-        gexec_scale = scale32;
     }
     cudaGraphExec_t& ge = gexec[m];
     if (!ge) {
@@ -891,7 +892,10 @@ int NodalSolver::solve(bool have_guess, gbp_stats* stats, bool from_prev)
     // V-cycles of the first inner solve: accelerated, about what FP32 delivers (1e-6) at the contraction of a smooth
     // problem (0.03 to 0.04 per V-cycle)
     int m = mixed ? (accelerated() ? std::min(mmax, 4) : mmax) : 1;
-    GBP_CUDA(cudaMemsetAsync(kstate, 0, sizeof(KrylovState), st));
+    memset(hstate, 0, sizeof(KrylovState));
+    hstate->scale = scale32;
+    hstate->inv_scale = 1.0 / scale32;
+    GBP_CUDA(cudaMemcpyAsync(kstate, hstate, sizeof(KrylovState), cudaMemcpyHostToDevice, st));
     if (mixed && accelerated())
         GBP_CUDA(cudaMemsetAsync(reinterpret_cast<float*>(kq) + l0.g.count, 0, sizeof(float) * l0.g.count, st));
     if (!evi0) {

@@ -206,6 +206,7 @@ private:
     double *kp = nullptr, *kq = nullptr;
     double* kpart = nullptr;     // partial sums of its dot products
     KrylovState* kstate = nullptr;
+    KrylovState* hstate = nullptr;  // pinned: the state a solve starts from
     KrylovBox kbox{};
     double* partials = nullptr;  // reduction scratch
     double* bscr = nullptr;      // scratch of the single-CTA bottom CG (coarsest levels beyond the cluster's)
@@ -256,7 +257,6 @@ private:
     void* xres[kMaxLevels] = {};
     cudaGraphExec_t gexec[kMaxInner + 1] = {};  // one refinement-step graph per inner-cycle count
     int gexec_prec = -1;
-    double gexec_scale = 0.0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     int nbottom = 0;
     bool dense_bottom = false;
