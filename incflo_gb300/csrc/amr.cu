@@ -874,7 +874,7 @@ int CompositeNodal::init(const gbp_geometry& coarse, const int bc_lo[3], const i
     // the shared-sum FP64 residual on both levels (isotropic cells)
     qsw = qsweep_supported(gf_nomask) && qsweep_supported(gc);
     if (qsw) {
-        for (int q = 0; q < 5; ++q) add(gc.count, 8);
+        for (int q = 0; q < 4; ++q) add(gc.count, 8);
     }
     nparts = std::max(nodal_partials_needed(gc), 1184);
     add(nparts + 64, 8);
@@ -889,7 +889,7 @@ int CompositeNodal::init(const gbp_geometry& coarse, const int bc_lo[3], const i
     ccls = pool.take<unsigned char>(gc.count);
     fcls = pool.take<unsigned char>(gf.count);
     if (qsw) {
-        for (double** w : {&qwc.w5, &qwc.rd, &qwc.wx, &qwc.wy, &qwc.wz}) *w = pool.take<double>(gc.count);
+        for (double** w : {&qwc.w5, &qwc.wx, &qwc.wy, &qwc.wz}) *w = pool.take<double>(gc.count);
     }
     sc_m = pool.take<double>(gc.count);
     sc_t = pool.take<double>(gc.count);
@@ -1195,8 +1195,8 @@ void CompositeNodal::issue_outer32(double scale32)
             }
         }
     }
-    nodal_add_correction<float>(gc, phi_c, ec32, 1.0 / scale32, st);
-    nodal_add_correction<float>(gf_nomask, phi_f, ef32, 1.0 / scale32, st);
+    nodal_add_unique(gc, phi_c, ec32, 1.0 / scale32, st);
+    nodal_add_unique(gf_nomask, phi_f, ef32, 1.0 / scale32, st);
     cudaMemsetAsync(dnorm + 1, 0, sizeof(unsigned long long), st);
     composite_residual(b_c, b_f, dnorm + 1);
     cudaMemcpyAsync(hnorm + 1, dnorm + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);

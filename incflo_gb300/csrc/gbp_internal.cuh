@@ -116,6 +116,7 @@ __device__ __forceinline__ void store_node(T* a, const NodalGeom& g, int i, int 
     const int ex = node_alias_step(i, g.n[0], g.per[0]);
     const long long ey = node_alias_step(j, g.n[1], g.per[1]) * g.sy;
     const long long ez = node_alias_step(k, g.n[2], g.per[2]) * g.sz;
+    if (!(ex | ey | ez)) return;
     if (ex) a[p + ex] = v;
     if (ey) a[p + ey] = v;
     if (ex && ey) a[p + ex + ey] = v;
@@ -150,6 +151,7 @@ __device__ __forceinline__ void store_cell(T* a, const G& g, int i, int j, int k
     const int ex = cell_alias_step(i, g.n[0], g.per[0]);
     const long long ey = cell_alias_step(j, g.n[1], g.per[1]) * g.sy;
     const long long ez = cell_alias_step(k, g.n[2], g.per[2]) * g.sz;
+    if (!(ex | ey | ez)) return;
     if (ex) a[p + ex] = v;
     if (ey) a[p + ey] = v;
     if (ex && ey) a[p + ex + ey] = v;

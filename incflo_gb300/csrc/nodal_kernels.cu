@@ -923,37 +923,54 @@ __global__ void k_sigma_coarsen(NodalGeom gf, NodalGeom gc, const double* __rest
     if (sc32) store_sigma_cell(sc32, gc, i, j, k, (float)v);
 }
 
-// Tiles of the z-marching FP64 kernels: a CTA of 33 x 9 threads covers 32 x 8 node columns; thread
-// (tx, ty) owns cell column and node column (x0 - 1 + tx, y0 - 1 + ty) (a cell is named by its low
-// node), the threads with tx, ty >= 1 own nodes, and the CTA walks a z range one layer at a time.
-constexpr int ZX = 32, ZY = 8, ZTX = ZX + 1, ZTY = ZY + 1;
+// Tiles of the z-marching FP64 kernels: a CTA of 10 warps covers 32 x 8 nodes (cells); warps 0-8 hold the 9 rows of
+// cells (nodes) they read, warp 9 the 9 entries of the column beside the tile. An FP64 instruction takes its pipe for
+// a whole warp whatever its active lanes, so the sums run on 8 full warps (a 33 x 9 thread tile spread them over 10).
+constexpr int ZX = 32, ZY = 8, kZThreads = 32 * (ZY + 2);
 
-// z chunk length for a bx x by tile grid over nz planes: about 4 waves of CTAs
+// z chunk length of a bx x by tile grid over nz planes: the planes and the extra layer of all CTAs of one SM pass its
+// FP64 pipe, one CTA alone also waits for its own loads
 static int zchunk(int bx, int by, int nz)
 {
-    const int want = std::max(1, 4 * sm_count_cached() * 6 / std::max(1, bx * by));
-    return std::max(4, (nz + want - 1) / want);
+    const int sms = sm_count_cached();
+    int best = nz;
+    double cost = 1e300;
+    for (int c = 1; c <= nz; ++c) {
+        const int per = (bx * by * ((nz + c - 1) / c) + sms - 1) / sms;
+        const double t = per * (c + 1.0) * (1.0 + 0.35 / per);
+        if (t < cost * (1.0 - 1e-9)) {
+            cost = t;
+            best = c;
+        }
+    }
+    return best;
 }
 
 // g = -(weak divergence) of u' = u + (add_gp ? sigma*gp : 0) - (sub_old ? u_old : 0), for the nodes.
-// Each cell of a layer computes its weak fluxes F_d = (h_e h_f / 4) u'_d once (ghost cells carry F
-// only across an inflow face, and only the normal component; other ghosts carry 0); a node sums +-F
-// over its 8 cells in separable form: per layer the x difference of y-pair sums of F_x, the y
-// difference of x-pair sums of F_y and the 4-cell sum of F_z, then layers k-1 and k.
+// Each cell of a layer forms u' once (ghost cells carry a value only across an inflow face, and only the normal
+// component; other ghosts carry 0); a node sums +-u'_d h_e h_f / 4 over its 8 cells in separable form: per layer the x
+// difference of y-pair sums of u'_x, the y difference of x-pair sums of u'_y and the 4-cell sum of u'_z, then layers k-1
+// and k and the three factors. A node's y-pair sums serve its +x neighbour too (a shuffle; the column beside the tile
+// is paired by its own warp): 17 FP64 instructions per node, which bound this kernel (26 with the factors per cell, no
+// shared pair sums and the node work on 10 warps: 870 us at 256^3).
 // part: per-CTA sums of g (consistency correction of singular systems).
-__global__ void __launch_bounds__(ZTX* ZTY) k_nodal_rhs(NodalGeom g, RhsArgs a, const double* __restrict__ s64,
+__global__ void __launch_bounds__(kZThreads, 3) k_nodal_rhs(NodalGeom g, RhsArgs a, const double* __restrict__ s64,
                                                         double* __restrict__ b, double* __restrict__ part, int kchunk,
                                                         int zb0, int nzb)
 {
-    __shared__ double F[2][3][ZTY][ZTX];
-    const int tx = threadIdx.x % ZTX, ty = threadIdx.x / ZTX;
+    __shared__ double F[2][3][ZY + 1][ZX + 1];
+    __shared__ double H[2][2][ZY + 1];  // y-pair sums of u'_x and u'_z in the column beside the tile
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool halo = warp == ZY + 1;
+    const int tx = halo ? 0 : lane + 1, ty = halo ? lane : warp;  // cell of the tile: column x0-1+tx, row y0-1+ty
     const int ci = blockIdx.x * ZX - 1 + tx, cj = blockIdx.y * ZY - 1 + ty;
     const int zb = zb0 + blockIdx.z;  // z chunk (a launch may cover a subset of them)
     const int kbeg = zb * kchunk;
     const int kend = min(kbeg + kchunk, g.nu[2]);
-    const bool owner = tx >= 1 && ty >= 1 && ci < g.nu[0] && cj < g.nu[1];
+    const bool owner = !halo && ty >= 1 && ci < g.nu[0] && cj < g.nu[1];
     // cells beyond the last node column are never read by an owner
-    const bool used = ci < g.nu[0] && cj < g.nu[1];
+    const bool used = ty <= ZY && ci < g.nu[0] && cj < g.nu[1];
+    const double c0f = -a.cf[0], c1f = -a.cf[1], c2f = -a.cf[2];
     // x / y part of this cell column: periodic wrap, or out of the domain (ghost)
     int c0 = ci, c1 = cj, nout_xy = 0, dout_xy = -1;
     if (g.per[0]) {
@@ -1006,39 +1023,53 @@ __global__ void __launch_bounds__(ZTX* ZTY) k_nodal_rhs(NodalGeom g, RhsArgs a, 
                     u1 -= a.vel_old.data[oo + a.vel_old.nstride];
                     u2 -= a.vel_old.data[oo + 2 * a.vel_old.nstride];
                 }
-                f0 = a.cf[0] * u0;
-                f1 = a.cf[1] * u1;
-                f2 = a.cf[2] * u2;
+                f0 = u0;
+                f1 = u1;
+                f2 = u2;
             } else if (nout == 1) {
                 // the ghost cell across one face: its raw (unwrapped) index in that direction
                 int q[3] = {c0, c1, c2};
                 q[dout] = dout == 0 ? ci : (dout == 1 ? cj : L);
                 const int inflow = q[dout] < 0 ? a.inflow_lo[dout] : a.inflow_hi[dout];
                 if (inflow) {
-                    const double fv = a.cf[dout] * a4(a.vel, q[0], q[1], q[2], dout);
+                    const double fv = a4(a.vel, q[0], q[1], q[2], dout);
                     if (dout == 0) f0 = fv;
                     else if (dout == 1) f1 = fv;
                     else f2 = fv;
                 }
             }
         }
-        F[buf][0][ty][tx] = f0;
-        F[buf][1][ty][tx] = f1;
-        F[buf][2][ty][tx] = f2;
+        if (ty <= ZY) {
+            F[buf][0][ty][tx] = f0;
+            F[buf][1][ty][tx] = f1;
+            F[buf][2][ty][tx] = f2;
+        }
+        if (halo) {
+            const double p0 = f0 + __shfl_up_sync(0xffffffffu, f0, 1), p2 = f2 + __shfl_up_sync(0xffffffffu, f2, 1);
+            if (lane <= ZY) {
+                H[buf][0][lane] = p0;
+                H[buf][1][lane] = p2;
+            }
+        }
         __syncthreads();
-        if (owner) {
-            const double(*F0)[ZTX] = F[buf][0];
-            const double(*F1)[ZTX] = F[buf][1];
-            const double(*F2)[ZTX] = F[buf][2];
-            const double A0 = (F0[ty - 1][tx] + F0[ty][tx]) - (F0[ty - 1][tx - 1] + F0[ty][tx - 1]);
-            const double A1 = (F1[ty][tx - 1] + F1[ty][tx]) - (F1[ty - 1][tx - 1] + F1[ty - 1][tx]);
-            const double Q2 = (F2[ty - 1][tx - 1] + F2[ty - 1][tx]) + (F2[ty][tx - 1] + F2[ty][tx]);
-            if (L >= kbeg) {
+        if (!halo && ty >= 1) {
+            const double(*F1)[ZX + 1] = F[buf][1];
+            const double P0 = F[buf][0][ty - 1][tx] + f0, P2 = F[buf][2][ty - 1][tx] + f2;
+            double P0l = __shfl_up_sync(0xffffffffu, P0, 1), P2l = __shfl_up_sync(0xffffffffu, P2, 1);
+            if (lane == 0) {
+                P0l = H[buf][0][ty];
+                P2l = H[buf][1][ty];
+            }
+            const double A0 = P0 - P0l;
+            const double A1 = (F1[ty][tx - 1] + f1) - (F1[ty - 1][tx - 1] + F1[ty - 1][tx]);
+            const double Q2 = P2 + P2l;
+            if (owner && L >= kbeg) {
                 // node (ci, cj, L): layers L-1 and L
                 double gv = 0.0;
-                if (!node_is_dirichlet(g, ci, cj, L)) gv = -(((A0p + A0) + (A1p + A1)) + (Q2 - Q2p));
+                if (!node_is_dirichlet(g, ci, cj, L))
+                    gv = fma(c0f, A0p + A0, fma(c1f, A1p + A1, c2f * (Q2 - Q2p)));
                 b[pidx(g.sy, g.sz, ci, cj, L)] = gv;
-                acc += gv;
+                if (part) acc += gv;
             }
             A0p = A0;
             A1p = A1;
@@ -1110,17 +1141,25 @@ __global__ void __launch_bounds__(256) k_remove_mean(NodalGeom g, double* __rest
     const double cv = c * (exy == 0 ? g.vol : (exy == 1 ? 0.5 * g.vol : 0.25 * g.vol));
     const double cvz = 0.5 * cv;  // on a z boundary plane
     unsigned long long key = 0;
+    // 4 planes at a time: their loads in flight together (the stores to the same array keep the compiler from it)
     if (i < g.nu[0] && j < g.nu[1])
-        for (int k = kbeg; k < kend; ++k) {
-            const long long p = pidx(g.sy, g.sz, i, j, k);
-            if (mode == 0) {
-                const int e = exy + (!g.per[2] && (k == 0 || k == g.n[2]));
-                const double bv = v[p] - (e == exy ? cv : cvz);
-                v[p] = bv;
-                const unsigned long long kb = e == 0 ? abs_key(bv) : abs_key(bv * (double)(1 << e));
-                key = kb > key ? kb : key;
-            } else {
-                store_node(v, g, i, j, k, v[p] - c);
+        for (int k0 = kbeg; k0 < kend; k0 += 4) {
+            double x[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) x[q] = k0 + q < kend ? v[pidx(g.sy, g.sz, i, j, k0 + q)] : 0.0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int k = k0 + q;
+                if (k >= kend) break;
+                if (mode == 0) {
+                    const int e = exy + (!g.per[2] && (k == 0 || k == g.n[2]));
+                    const double bv = x[q] - (e == exy ? cv : cvz);
+                    v[pidx(g.sy, g.sz, i, j, k)] = bv;
+                    const unsigned long long kb = e == 0 ? abs_key(bv) : abs_key(bv * (double)(1 << e));
+                    key = kb > key ? kb : key;
+                } else {
+                    store_node(v, g, i, j, k, x[q] - c);
+                }
             }
         }
     if (mode == 0 && norm) {
@@ -1129,62 +1168,108 @@ __global__ void __launch_bounds__(256) k_remove_mean(NodalGeom g, double* __rest
     }
 }
 
+// x += e over the whole padded array, 4 positions per thread (both carry their periodic aliases; a Dirichlet node's e
+// is 0)
 template <typename TE>
-__global__ void __launch_bounds__(256) k_add_correction(NodalGeom g, double* __restrict__ x, const TE* __restrict__ e,
+__global__ void __launch_bounds__(256) k_add_correction(long long n4, double* __restrict__ x, const TE* __restrict__ e,
                                                         double inv_scale, const KrylovState* __restrict__ ks)
 {
+    const long long t = blockIdx.x * 256ll + threadIdx.x;
+    if (t >= n4) return;
     if (ks) inv_scale = ks->inv_scale;
+    double2* xp = reinterpret_cast<double2*>(x) + 2 * t;
+    double2 a = xp[0], b = xp[1];
+    if constexpr (sizeof(TE) == 4) {
+        const float4 f = reinterpret_cast<const float4*>(e)[t];
+        a.x = fma((double)f.x, inv_scale, a.x);
+        a.y = fma((double)f.y, inv_scale, a.y);
+        b.x = fma((double)f.z, inv_scale, b.x);
+        b.y = fma((double)f.w, inv_scale, b.y);
+    } else {
+        const double2 f = reinterpret_cast<const double2*>(e)[2 * t], h = reinterpret_cast<const double2*>(e)[2 * t + 1];
+        a.x = fma(f.x, inv_scale, a.x);
+        a.y = fma(f.y, inv_scale, a.y);
+        b.x = fma(h.x, inv_scale, b.x);
+        b.y = fma(h.y, inv_scale, b.y);
+    }
+    xp[0] = a;
+    xp[1] = b;
+}
+
+__global__ void __launch_bounds__(256) k_add_unique(NodalGeom g, double* __restrict__ x, const float* __restrict__ e,
+                                                    double inv_scale)
+{
     int i, j, k;
     if (!grid3_node(g, i, j, k)) return;
     const long long p = pidx(g.sy, g.sz, i, j, k);
     store_node(x, g, i, j, k, x[p] + (double)e[p] * inv_scale);
 }
 
-__global__ void __launch_bounds__(256) k_to_f32(NodalGeom g, const double* __restrict__ r, float* __restrict__ r32,
+// r32 = scale r over the whole padded array
+__global__ void __launch_bounds__(256) k_to_f32(long long n4, const double* __restrict__ r, float* __restrict__ r32,
                                                 double scale, const KrylovState* __restrict__ ks)
 {
+    const long long t = blockIdx.x * 256ll + threadIdx.x;
+    if (t >= n4) return;
     if (ks) scale = ks->scale;
-    int i, j, k;
-    if (!grid3_node(g, i, j, k)) return;
-    const long long p = pidx(g.sy, g.sz, i, j, k);
-    r32[p] = (float)(r[p] * scale);
+    const double2 a = reinterpret_cast<const double2*>(r)[2 * t], b = reinterpret_cast<const double2*>(r)[2 * t + 1];
+    reinterpret_cast<float4*>(r32)[t] =
+        make_float4((float)(a.x * scale), (float)(a.y * scale), (float)(b.x * scale), (float)(b.y * scale));
 }
 
 // u <- u + (add_gp ? sigma*gp : 0) - sigma*G phi; gradphi <- G phi; gp <- G phi (+= if incremental).
-// z-marching tile (33 x 9 node columns for 32 x 8 cell columns): each node column forms the z-pair sum
+// z-marching tile (32 x 8 cell columns, 33 x 9 node columns): each node column forms the z-pair sum
 // S and difference D of its two planes once; a cell's gradient is then
 //   4h G_x = (S10 + S11) - (S00 + S01), 4h G_y = (S01 + S11) - (S00 + S10), 4h G_z = (D00 + D10) + (D01 + D11)
-// (Sab = node column (i+a, j+b)), 9 additions instead of 21.
-__global__ void __launch_bounds__(ZTX* ZTY) k_nodal_correct(NodalGeom g, CorrArgs a, const double* __restrict__ s64,
+// (Sab = node column (i+a, j+b)), the y-pair sums shared with the -x neighbour by a shuffle: 18 FP64 instructions per
+// cell, which bound this kernel (25 without the shared sums and with the cell work on 10 warps: 845 us at 256^3).
+__global__ void __launch_bounds__(kZThreads, 3) k_nodal_correct(NodalGeom g, CorrArgs a, const double* __restrict__ s64,
                                                             const double* __restrict__ phi, int kchunk, int k0, int k1)
 {
-    __shared__ double S[2][ZTY][ZTX], D[2][ZTY][ZTX];
-    const int tx = threadIdx.x % ZTX, ty = threadIdx.x / ZTX;
+    __shared__ double S[2][ZY + 1][ZX + 1], D[2][ZY + 1][ZX + 1];
+    __shared__ double H[2][2][ZY + 1];  // y-pair sums of S and D in the column beside the tile
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool halo = warp == ZY + 1;
+    const int tx = halo ? ZX : lane, ty = halo ? lane : warp;
     const int ni = blockIdx.x * ZX + tx, nj = blockIdx.y * ZY + ty;  // node column; cell column = same
     const int kbeg = k0 + blockIdx.z * kchunk;
     const int kend = min(kbeg + kchunk, k1);
     // node columns 0..n (index n: the periodic alias or the high boundary node)
-    const bool has_node = ni <= g.n[0] && nj <= g.n[1];
-    const bool cell = tx < ZX && ty < ZY && ni < g.n[0] && nj < g.n[1];
+    const bool has_node = ty <= ZY && ni <= g.n[0] && nj <= g.n[1];
+    const bool cell = !halo && ty < ZY && ni < g.n[0] && nj < g.n[1];
     const long long pc = pidx(g.sy, g.sz, ni, nj, kbeg);
     double plo = has_node ? phi[pc] : 0.0;
     for (int k = kbeg; k < kend; ++k) {
         const int buf = (k - kbeg) & 1;
         const long long pk = pc + (long long)(k - kbeg) * g.sz;
         const double phi_hi = has_node ? phi[pk + g.sz] : 0.0;
-        S[buf][ty][tx] = plo + phi_hi;
-        D[buf][ty][tx] = phi_hi - plo;
+        const double s = plo + phi_hi, d = phi_hi - plo;
         plo = phi_hi;
+        if (ty <= ZY) {
+            S[buf][ty][tx] = s;
+            D[buf][ty][tx] = d;
+        }
+        if (halo) {
+            const double ps = s + __shfl_down_sync(0xffffffffu, s, 1), pd = d + __shfl_down_sync(0xffffffffu, d, 1);
+            if (lane < ZY) {
+                H[buf][0][lane] = ps;
+                H[buf][1][lane] = pd;
+            }
+        }
         __syncthreads();
+        if (halo || ty >= ZY) continue;  // whole warps; their next barrier is the next layer's
+        const double S01 = S[buf][ty + 1][tx];
+        const double Ys = s + S01, Yd = d + D[buf][ty + 1][tx];
+        double Ysr = __shfl_down_sync(0xffffffffu, Ys, 1), Ydr = __shfl_down_sync(0xffffffffu, Yd, 1);
+        if (lane == 31) {
+            Ysr = H[buf][0][ty];
+            Ydr = H[buf][1][ty];
+        }
         if (cell && (!a.cmask || a.cmask[pk])) {
-            const double S00 = S[buf][ty][tx], S10 = S[buf][ty][tx + 1], S01 = S[buf][ty + 1][tx],
-                         S11 = S[buf][ty + 1][tx + 1];
-            const double D00 = D[buf][ty][tx], D10 = D[buf][ty][tx + 1], D01 = D[buf][ty + 1][tx],
-                         D11 = D[buf][ty + 1][tx + 1];
             double G[3];
-            G[0] = ((S10 + S11) - (S00 + S01)) * a.inv4h[0];
-            G[1] = ((S01 + S11) - (S00 + S10)) * a.inv4h[1];
-            G[2] = ((D00 + D10) + (D01 + D11)) * a.inv4h[2];
+            G[0] = (Ysr - Ys) * a.inv4h[0];
+            G[1] = ((S01 + S[buf][ty + 1][tx + 1]) - (s + S[buf][ty][tx + 1])) * a.inv4h[1];
+            G[2] = (Yd + Ydr) * a.inv4h[2];
             const double sg = s64[pk];
             const long long ov = (long long)(ni - a.vel.lo[0]) + (long long)(nj - a.vel.lo[1]) * a.vel.jstride +
                                  (long long)(k - a.vel.lo[2]) * a.vel.kstride;
@@ -1395,7 +1480,7 @@ void nodal_rhs(const NodalGeom& g, const RhsArgs& a, const double* s64, double* 
     const dim3 grid = rhs_grid(g, kchunk);
     if (zb1 < 0) zb1 = (int)grid.z;
     if (zb1 <= zb0) return;
-    k_nodal_rhs<<<dim3(grid.x, grid.y, zb1 - zb0), ZTX * ZTY, 0, st>>>(g, a, s64, b, part, kchunk, zb0, (int)grid.z);
+    k_nodal_rhs<<<dim3(grid.x, grid.y, zb1 - zb0), kZThreads, 0, st>>>(g, a, s64, b, part, kchunk, zb0, (int)grid.z);
 }
 
 int nodal_rhs_zchunks(const NodalGeom& g, int* kchunk)
@@ -1461,16 +1546,23 @@ template <typename TE>
 void nodal_add_correction(const NodalGeom& g, double* x, const TE* e, double inv_scale, cudaStream_t st,
                           const KrylovState* ks)
 {
-    k_add_correction<TE><<<grid3(g), kBlock3, 0, st>>>(g, x, e, inv_scale, ks);
+    const long long n4 = g.count / 4;  // rows are multiples of 8 elements
+    k_add_correction<TE><<<nblocks(n4, 256), 256, 0, st>>>(n4, x, e, inv_scale, ks);
 }
 template void nodal_add_correction<double>(const NodalGeom&, double*, const double*, double, cudaStream_t,
                                            const KrylovState*);
 template void nodal_add_correction<float>(const NodalGeom&, double*, const float*, double, cudaStream_t,
                                           const KrylovState*);
 
+void nodal_add_unique(const NodalGeom& g, double* x, const float* e, double inv_scale, cudaStream_t st)
+{
+    k_add_unique<<<grid3(g), kBlock3, 0, st>>>(g, x, e, inv_scale);
+}
+
 void nodal_to_f32(const NodalGeom& g, const double* r, float* r32, double scale, cudaStream_t st, const KrylovState* ks)
 {
-    k_to_f32<<<grid3(g), kBlock3, 0, st>>>(g, r, r32, scale, ks);
+    const long long n4 = g.count / 4;
+    k_to_f32<<<nblocks(n4, 256), 256, 0, st>>>(n4, r, r32, scale, ks);
 }
 
 void nodal_correct(const NodalGeom& g, const CorrArgs& a, const double* s64, const double* phi, cudaStream_t st,
@@ -1480,7 +1572,7 @@ void nodal_correct(const NodalGeom& g, const CorrArgs& a, const double* s64, con
     if (k1 <= k0) return;
     const int bx = (g.n[0] + ZX - 1) / ZX, by = (g.n[1] + ZY - 1) / ZY;
     const int kchunk = zchunk(bx, by, k1 - k0);
-    k_nodal_correct<<<dim3(bx, by, (k1 - k0 + kchunk - 1) / kchunk), ZTX * ZTY, 0, st>>>(g, a, s64, phi, kchunk, k0,
+    k_nodal_correct<<<dim3(bx, by, (k1 - k0 + kchunk - 1) / kchunk), kZThreads, 0, st>>>(g, a, s64, phi, kchunk, k0,
                                                                                          k1);
 }
 

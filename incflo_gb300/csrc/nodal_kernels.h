@@ -111,6 +111,8 @@ void nodal_norm(const NodalGeom& g, const double* v, unsigned long long* norm, c
 template <typename TE>
 void nodal_add_correction(const NodalGeom& g, double* x, const TE* e, double inv_scale, cudaStream_t st,
                           const KrylovState* ks = nullptr);
+// the same from the unique nodes of e alone (its periodic aliases need not hold their values)
+void nodal_add_unique(const NodalGeom& g, double* x, const float* e, double inv_scale, cudaStream_t st);
 // (ks: the scale is read from the device instead)
 void nodal_to_f32(const NodalGeom& g, const double* r, float* r32, double scale, cudaStream_t st,
                   const KrylovState* ks = nullptr);

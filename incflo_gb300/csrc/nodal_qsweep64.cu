@@ -22,6 +22,7 @@
 #include <algorithm>
 
 #include "gbp_internal.cuh"
+#include "krylov.h"
 #include "nodal_sweep.h"
 
 namespace gbp {
@@ -29,7 +30,6 @@ namespace gbp {
 namespace {
 
 constexpr int QX = 32, QY = 8;
-constexpr int QTX = QX + 1, QTY = QY + 1;   // k_qweights64's thread tile
 constexpr int kQThreads = 32 * (QY + 2);    // k_qsweep64: QY + 1 cell rows and the halo column
 
 __device__ __forceinline__ bool q_alias(const NodalGeom& g, int i, int j, int k)
@@ -39,58 +39,52 @@ __device__ __forceinline__ bool q_alias(const NodalGeom& g, int i, int j, int k)
 }
 
 // w5 = 5 kc (sum of the 8 cells around each node), rd = 1 / diagonal (single precision, where the diagonal is in
-// its range: a smoother needs no more); wx / wy / wz = kc (sigma sum of the 4 cells around the edge
-// from node (i,j,k) to (i+1,j,k) / (i,j+1,k) / (i,j,k+1)). Written over index ranges -1..nu so that the
-// sweep can read the edge to a node's low neighbour; padding cells are 0, periodic ones aliased.
-// z-marching tile (33 x 9 threads: node columns x0-1 .. x0+31, y0-1 .. y0+7 and the cell columns one
-// lower), separable sums per cell layer: Px = x pair, Q = Px + Px(j-1) (4 cells around a z edge),
-// Y = y pair; then the 8 cells = Q(k-1) + Q(k), wz = Q(k), wx = Y(k-1) + Y(k), wy = Px(k-1) + Px(k).
-__global__ void __launch_bounds__(QTX* QTY) k_qweights64(NodalGeom g, const double* __restrict__ s,
-                                                         double* __restrict__ w5, double* __restrict__ rd,
-                                                         double* __restrict__ wx, double* __restrict__ wy,
-                                                         double* __restrict__ wz, int kchunk)
+// its range: a smoother needs no more; nullptr: not wanted); wx / wy / wz = kc (sigma sum of the 4 cells around the edge
+// from node (i,j,k) to (i+1,j,k) / (i,j+1,k) / (i,j,k+1)). The sweep also reads the edge to a node's low neighbour:
+// across a periodic seam the last node's edge is stored at index -1 too, elsewhere index -1 keeps its 0.
+// A CTA marches a z range over 32 x 8 node columns; separable sums of kc sigma per cell layer: Px = x pair, Q = Px +
+// Px(j-1) (4 cells around a z edge), Y = y pair; then the 8 cells = Q(k-1) + Q(k), wz = Q(k), wx = Y(k-1) + Y(k), wy =
+// Px(k-1) + Px(k): 9 FP64 instructions per node.
+__global__ void __launch_bounds__(32 * QY) k_qweights64(NodalGeom g, const double* __restrict__ s, QWeights w,
+                                                        int kchunk)
 {
-    __shared__ double T[2][QTY + 1][QTX + 1];
-    const int tx = threadIdx.x % QTX, ty = threadIdx.x / QTX;
-    // node column of this thread: (i, j) = (x0 - 1 + tx, y0 - 1 + ty); its cells are i-1..i, j-1..j
-    const int i = blockIdx.x * QX - 1 + tx, j = blockIdx.y * QY - 1 + ty;
-    const int kbeg = blockIdx.z * kchunk - 1;  // node planes -1 .. nu-1
-    const int kend = min(kbeg + kchunk, g.nu[2]);
-    // neighbouring tiles share their edge column / row: the lower tile writes it
-    const bool node = (tx >= 1 || blockIdx.x == 0) && (ty >= 1 || blockIdx.y == 0) && i < g.nu[0] && j < g.nu[1];
+    __shared__ double T[2][QY + 1][QX + 1];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int i = blockIdx.x * QX + tx, j = blockIdx.y * QY + ty;
+    const int kbeg = blockIdx.z * kchunk, kend = min(kbeg + kchunk, g.nu[2]);
+    const bool node = i < g.nu[0] && j < g.nu[1];
     const double kc = g.K[3];
+    const long long sx = g.per[0] && i == g.n[0] - 1 ? -g.n[0] : 0, sy = g.per[1] && j == g.n[1] - 1 ? -g.n[1] * g.sy : 0;
     double Qp = 0.0, Yp = 0.0, Pp = 0.0;
     for (int L = kbeg - 1; L < kend; ++L) {
         const int buf = (L - kbeg + 1) & 1;
-        // stage cells (x0-2 .. x0+31, y0-2 .. y0+7) of layer L: tile (tx, ty) = cell (i - 1, j - 1),
-        // plus the extra high column / row; cells below -1 are never read (zero)
-        for (int q = threadIdx.x; q < (QTX + 1) * (QTY + 1); q += QTX * QTY) {
-            const int cx = q % (QTX + 1), cy = q / (QTX + 1);
-            const int a = blockIdx.x * QX - 2 + cx, b = blockIdx.y * QY - 2 + cy;
-            double v = 0.0;
-            if (L >= -1 && a >= -1 && b >= -1 && a <= g.nu[0] - 1 && b <= g.nu[1] - 1) v = s[pidx(g.sy, g.sz, a, b, L)];
-            T[buf][cy][cx] = v;
+        // cells (x0-1 .. x0+31, y0-1 .. y0+7) of layer L
+        for (int q = threadIdx.x; q < (QX + 1) * (QY + 1); q += 32 * QY) {
+            const int cx = q % (QX + 1), cy = q / (QX + 1);
+            const int a = blockIdx.x * QX - 1 + cx, b = blockIdx.y * QY - 1 + cy;
+            T[buf][cy][cx] = a < g.nu[0] && b < g.nu[1] ? kc * s[pidx(g.sy, g.sz, a, b, L)] : 0.0;
         }
         __syncthreads();
-        // this node's cells in the tile: (i-1, j-1) = (tx, ty), (i, j-1) = (tx+1, ty), (i-1, j) = (tx, ty+1), (i, j) = (tx+1, ty+1)
-        const double Px = T[buf][ty + 1][tx] + T[buf][ty + 1][tx + 1];   // cells (i-1..i, j)
-        const double Pxm = T[buf][ty][tx] + T[buf][ty][tx + 1];          // cells (i-1..i, j-1)
-        const double Q = Px + Pxm;
-        const double Y = T[buf][ty][tx + 1] + T[buf][ty + 1][tx + 1];    // cells (i, j-1..j)
+        // this node's cells: (i-1, j-1) = (tx, ty) ... (i, j) = (tx+1, ty+1)
+        const double Px = T[buf][ty + 1][tx] + T[buf][ty + 1][tx + 1];
+        const double Q = Px + (T[buf][ty][tx] + T[buf][ty][tx + 1]);
+        const double Y = T[buf][ty][tx + 1] + T[buf][ty + 1][tx + 1];
         if (node && L >= kbeg) {
-            // node (i, j, L): layers L-1 (previous) and L
-            const int k = L;
-            const long long p = pidx(g.sy, g.sz, i, j, k);
-            if (i >= 0 && j >= 0 && k >= 0) {
-                const double ssum = Qp + Q;
-                w5[p] = 5.0 * kc * ssum;
-                const double diag = g.K[0] * ssum;
+            const long long p = pidx(g.sy, g.sz, i, j, L);
+            const double w5 = 5.0 * (Qp + Q), wx = Yp + Y, wy = Pp + Px;
+            w.w5[p] = w5;
+            w.wx[p] = wx;
+            w.wy[p] = wy;
+            w.wz[p] = Q;
+            if (sx) w.wx[p + sx] = wx;
+            if (sy) w.wy[p + sy] = wy;
+            if (g.per[2] && L == g.n[2] - 1) w.wz[p - g.n[2] * g.sz] = Q;
+            if (w.rd) {
+                // the diagonal is K0 = -4 kc times the 8 cells
+                const double diag = -0.8 * w5;
                 const float fd = (float)diag;
-                rd[p] = (fd > 1e-30f && fd < 1e30f) ? (double)__frcp_rn(fd) : 1.0 / diag;
+                w.rd[p] = (fd > 1e-30f && fd < 1e30f) ? (double)__frcp_rn(fd) : 1.0 / diag;
             }
-            if (j >= 0 && k >= 0) wx[p] = kc * (Yp + Y);
-            if (i >= 0 && k >= 0) wy[p] = kc * (Pp + Px);
-            if (i >= 0 && j >= 0) wz[p] = kc * Q;
         }
         Qp = Q;
         Yp = Y;
@@ -99,14 +93,16 @@ __global__ void __launch_bounds__(QTX* QTY) k_qweights64(NodalGeom g, const doub
 }
 
 // MODE 0: Jacobi sweep out = x + omega (b - A x) / diag; 1: residual out = b - A x (with the max norm);
-// 2: out = -A x
+// 2: out = -A x; 3: the residual of mode 1 as the next FP32 right-hand side, out32 = scale (b - A x)
 template <int MODE>
-__global__ void __launch_bounds__(kQThreads) k_qsweep64(NodalGeom g, const double* __restrict__ x,
+__global__ void __launch_bounds__(kQThreads, 3) k_qsweep64(NodalGeom g, const double* __restrict__ x,
                                                         const double* __restrict__ b, const double* __restrict__ s,
                                                         QWeights w, double* __restrict__ out, double omega,
-                                                        int kchunk, unsigned long long* norm)
+                                                        int kchunk, unsigned long long* norm,
+                                                        float* __restrict__ out32, const KrylovState* __restrict__ ks)
 {
     __shared__ double T[2][QY + 1][QX + 1];
+    const double scale = MODE == 3 ? ks->scale : 0.0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // the cell of this thread: tile column cx (0 = the halo column x0-1), tile row cy (0 = the halo row y0-1)
     const bool halo = warp == QY + 1;
@@ -165,7 +161,7 @@ __global__ void __launch_bounds__(kQThreads) k_qsweep64(NodalGeom g, const doubl
                     v = fma(mkc, u_lo + u, e);  // b - A x (MODE 2: -A x)
                     if (MODE == 0) {
                         v = fma(omega * v, w.rd[pc], xc);
-                    } else if (MODE == 1 && norm) {
+                    } else if ((MODE == 1 || MODE == 3) && norm) {
                         // |v| / V_node as an integer key (boundary nodes: V / 2^e, exact scaling)
                         const int f = (!g.per[0] && (i == 0 || i == g.n[0])) + (!g.per[1] && (j == 0 || j == g.n[1])) +
                                       (!g.per[2] && (k == 0 || k == g.n[2]));
@@ -173,7 +169,9 @@ __global__ void __launch_bounds__(kQThreads) k_qsweep64(NodalGeom g, const doubl
                         nkey = kb > nkey ? kb : nkey;
                     }
                 }
-                if (q_alias(g, i, j, k))
+                if (MODE == 3)
+                    out32[pc] = (float)(scale * v);
+                else if (q_alias(g, i, j, k))
                     store_node(out, g, i, j, k, v);
                 else
                     out[pc] = v;
@@ -184,7 +182,7 @@ __global__ void __launch_bounds__(kQThreads) k_qsweep64(NodalGeom g, const doubl
             u_lo = u;
         }
     }
-    if (MODE == 1 && norm) {
+    if ((MODE == 1 || MODE == 3) && norm) {
         nkey = block_max_key(nkey);
         if (threadIdx.x == 0) atomic_max_nonneg(norm, key_value(nkey) * g.ivol);
     }
@@ -215,17 +213,6 @@ bool qsweep_supported(const NodalGeom& g)
     return g.iso != 0 && (long long)g.nu[0] * g.nu[1] * g.nu[2] >= kQMinNodes;
 }
 
-void nodal_qweights64(const NodalGeom& g, const double* s64, const QWeights& w, cudaStream_t st)
-{
-    // node columns -1 .. nu-1 in tiles of 32 x 8 (tile origin x0 - 1), node planes -1 .. nu-1
-    const int bx = (g.nu[0] + QX - 1) / QX, by = (g.nu[1] + QY - 1) / QY;
-    const int nz = g.nu[2] + 1;
-    const int want = std::max(1, 4 * sm_count_cached() * 6 / std::max(1, bx * by));
-    const int kchunk = std::max(4, (nz + want - 1) / want);
-    k_qweights64<<<dim3(bx, by, (nz + kchunk - 1) / kchunk), QTX * QTY, 0, st>>>(g, s64, w.w5, w.rd, w.wx, w.wy, w.wz,
-                                                                                kchunk);
-}
-
 // z chunk of a CTA: its planes and the extra cell layer below them all pass the SM's FP64 pipe, so the time is the
 // largest number of CTAs on one SM times (chunk + 1); one CTA alone on an SM also waits for its own loads.
 static int q_chunk(int tiles, int nz)
@@ -244,18 +231,28 @@ static int q_chunk(int tiles, int nz)
     return best;
 }
 
+void nodal_qweights64(const NodalGeom& g, const double* s64, const QWeights& w, cudaStream_t st)
+{
+    const int bx = (g.nu[0] + QX - 1) / QX, by = (g.nu[1] + QY - 1) / QY;
+    const int kchunk = q_chunk(bx * by, g.nu[2]);
+    k_qweights64<<<dim3(bx, by, (g.nu[2] + kchunk - 1) / kchunk), 32 * QY, 0, st>>>(g, s64, w, kchunk);
+}
+
 void nodal_qsweep64(const NodalGeom& g, int mode, const double* s64, const QWeights& w, const double* x,
-                    const double* b, double* out, double omega, unsigned long long* norm, cudaStream_t st)
+                    const double* b, double* out, double omega, unsigned long long* norm, cudaStream_t st,
+                    float* out32, const KrylovState* ks)
 {
     const int bx = (g.nu[0] + QX - 1) / QX, by = (g.nu[1] + QY - 1) / QY;
     const int kchunk = q_chunk(bx * by, g.nu[2]);
     const dim3 grid(bx, by, (g.nu[2] + kchunk - 1) / kchunk);
     if (mode == 0)
-        k_qsweep64<0><<<grid, kQThreads, 0, st>>>(g, x, b, s64, w, out, omega, kchunk, norm);
+        k_qsweep64<0><<<grid, kQThreads, 0, st>>>(g, x, b, s64, w, out, omega, kchunk, norm, nullptr, nullptr);
     else if (mode == 1)
-        k_qsweep64<1><<<grid, kQThreads, 0, st>>>(g, x, b, s64, w, out, omega, kchunk, norm);
+        k_qsweep64<1><<<grid, kQThreads, 0, st>>>(g, x, b, s64, w, out, omega, kchunk, norm, nullptr, nullptr);
+    else if (mode == 2)
+        k_qsweep64<2><<<grid, kQThreads, 0, st>>>(g, x, b, s64, w, out, omega, kchunk, norm, nullptr, nullptr);
     else
-        k_qsweep64<2><<<grid, kQThreads, 0, st>>>(g, x, b, s64, w, out, omega, kchunk, norm);
+        k_qsweep64<3><<<grid, kQThreads, 0, st>>>(g, x, b, s64, w, nullptr, omega, kchunk, norm, out32, ks);
 }
 
 void nodal_qzero64(const NodalGeom& g, const QWeights& w, const double* b, double* out, double omega, cudaStream_t st)

@@ -73,7 +73,7 @@ struct NodalLevel {
     float *s32 = nullptr, *x32 = nullptr, *t32 = nullptr, *b32 = nullptr, *r32 = nullptr;
     unsigned char* mask8 = nullptr;  // overset mask storage (active when g.mask is set)
     QWeights qw{};                   // sigma sums of the shared-sum FP64 sweep (levels it supports)
-    bool qw_ready = false;           // ... of the present sigma
+    int qw_ready = 0;                // ... of the present sigma: 1 for residuals, 2 with the reciprocal diagonal
 };
 
 class NodalSolver {

@@ -17,15 +17,18 @@ int nodal_sweep(const NodalGeom& g, int mode, const T* s, const T* x, const T* b
                 unsigned* err, unsigned long long* norm, cudaStream_t st);
 // Precomputed per padded node for the shared-sum FP64 sweep (nodal_qsweep64.cu), kc the far-corner coupling of the
 // element: w5 = 5 kc (the 8 cells around the node), rd = 1 / the operator's diagonal; wx / wy / wz = kc (the 4 cells
-// around the edge to the +x / +y / +z neighbour).
+// around the edge to the +x / +y / +z neighbour). rd may be null where only residuals are wanted.
+struct KrylovState;
 struct QWeights {
     double *w5, *rd, *wx, *wy, *wz;
 };
 bool qsweep_supported(const NodalGeom& g);
 void nodal_qweights64(const NodalGeom& g, const double* s64, const QWeights& w, cudaStream_t st);
-// mode 0: Jacobi sweep, 1: residual (+ strong-form max norm into *norm when norm != nullptr), 2: out = -A x (b unused)
+// mode 0: Jacobi sweep, 1: residual (+ strong-form max norm into *norm when norm != nullptr), 2: out = -A x (b unused),
+// 3: mode 1 with the residual written as out32 = ks->scale (b - A x) instead
 void nodal_qsweep64(const NodalGeom& g, int mode, const double* s64, const QWeights& w, const double* x,
-                    const double* b, double* out, double omega, unsigned long long* norm, cudaStream_t st);
+                    const double* b, double* out, double omega, unsigned long long* norm, cudaStream_t st,
+                    float* out32 = nullptr, const KrylovState* ks = nullptr);
 // Jacobi sweep from zero: out = omega b / diag
 void nodal_qzero64(const NodalGeom& g, const QWeights& w, const double* b, double* out, double omega, cudaStream_t st);
 
