@@ -173,6 +173,8 @@ int MacSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc_h
     } else {
         add(5 * B.g.count, 8);
     }
+    plan_tail();
+    add(tail.t.table.size() + 1, 4);
     add(8, 8);
     add(8, 4);
     for (int q = 0; q < 6; ++q) {
@@ -213,6 +215,9 @@ int MacSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc_h
     } else {
         bscr = pool.take<double>(5 * B.g.count);
     }
+    tail.table = pool.take<int>(tail.t.table.size() + 1);
+    if (!tail.t.table.empty())
+        GBP_CUDA(cudaMemcpyAsync(tail.table, tail.t.table.data(), sizeof(int) * tail.t.table.size(), cudaMemcpyHostToDevice, st));
     dnorm = pool.take<unsigned long long>(8);
     dflags = pool.take<unsigned>(8);
     rb = RobinFaces{};
@@ -705,17 +710,27 @@ struct MacBufs<float> {
     static float* r(const MacLevel& l) { return l.r32; }
 };
 
-// First level cycled by the cluster kernel: the first level below the finest with at most kCoarseCells
-// cells, when the bottom is the dense inverse and the tail fits the kernel's table; -1 otherwise.
-int MacSolver::coarse_first() const
+void MacSolver::plan_tail()
 {
-    if (!dense_bottom || !use_coarse) return -1;
-    for (int l = 1; l + 1 < (int)L.size(); ++l) {
+    tail = Tail{};
+    const int ctas = brows.n && brows.n <= kDenseBottom ? tail_cluster_size() : 0;
+    if (!ctas) return;
+    for (int l = 0; l + 1 < (int)L.size(); ++l) {
         const CellGeom& g = L[l].g;
-        if ((long long)g.n[0] * g.n[1] * g.n[2] <= kCoarseCells)
-            return ((int)L.size() - l <= kMacCoarseMaxLevels) ? l : -1;
+        if ((long long)g.n[0] * g.n[1] * g.n[2] > kTailCells) continue;
+        std::vector<int> planes, elems;
+        std::vector<long long> cells;
+        for (size_t q = l; q < L.size(); ++q) {
+            planes.push_back(L[q].g.n[2]);
+            elems.push_back((int)L[q].g.sz);
+            cells.push_back((long long)L[q].g.n[0] * L[q].g.n[1] * L[q].g.n[2]);
+        }
+        if (tail_layout((int)planes.size(), planes.data(), g.per[2], elems.data(), cells.data(), 7, sizeof(float),
+                        brows.n, kSoloCells, ctas, &tail.t)) {
+            tail.first = l;
+            return;
+        }
     }
-    return -1;
 }
 
 template <typename T>
@@ -726,28 +741,38 @@ void MacSolver::vcycle(int l, const T* b, bool zero)
     const cudaStream_t s = cap_or_st;
     T* x = B::x(lv);
     // the small levels (this one down to the bottom) in one cluster-resident launch
-    if (sizeof(T) == 4 && zero && l >= 1 && l == coarse_first()) {
-        MacCoarseCycle<T> c{};
-        c.nl = (int)L.size() - l;
-        for (int q = 0; q < c.nl; ++q) {
-            const MacLevel& v = L[l + q];
-            c.g[q] = v.g;
-            c.bx[q] = B::b(v)[0];
-            c.by[q] = B::b(v)[1];
-            c.bz[q] = B::b(v)[2];
-            c.x[q] = B::x(v);
-            c.b[q] = B::rhs(v);
-            c.r[q] = B::r(v);
+    if constexpr (sizeof(T) == 4) {
+        if (zero && l == tail.first && use_coarse && dense_bottom && opt.nu1 >= 1 && opt.nu2 >= 1 && !(l == 0 && eb.on)) {
+            MacTail<T> c{};
+            c.nl = tail.t.nl;
+            c.ctas = tail.t.ctas;
+            c.solo = tail.t.solo;
+            c.tab_ints = tail.t.tab_ints;
+            for (int q = 0; q < c.nl; ++q) {
+                const MacLevel& v = L[l + q];
+                c.g[q] = v.g;
+                c.bx[q] = B::b(v)[0];
+                c.by[q] = B::b(v)[1];
+                c.bz[q] = B::b(v)[2];
+                c.np[q] = tail.t.np[q];
+                c.off[q] = tail.t.off[q];
+                c.own[q] = tail.t.own[q];
+                c.copies[q] = tail.t.copies[q];
+            }
+            c.b0 = b;
+            c.xout = x;
+            c.M = dmat;
+            c.act = dact;
+            c.singular = singular ? 1 : 0;
+            c.nu1 = opt.nu1;
+            c.nu2 = opt.nu2;
+            c.table = tail.table;
+            c.tab_off = tail.t.tab_off;
+            c.dense_off = tail.t.dense_off;
+            int rc = mac_tail<T>(c, tail.t.bytes, s);
+            if (rc && !launch_rc) launch_rc = rc;
+            return;
         }
-        c.b[0] = const_cast<T*>(b);
-        c.M = dmat;
-        c.act = dact;
-        c.singular = singular ? 1 : 0;
-        c.nu1 = opt.nu1;
-        c.nu2 = opt.nu2;
-        int rc = mac_coarse_vcycle<T>(c, mac_coarse_cluster_size(), s);
-        if (rc && !launch_rc) launch_rc = rc;
-        return;
     }
     if (l == (int)L.size() - 1) {
         if (dense_bottom) {
@@ -1112,7 +1137,7 @@ __global__ void k_mac_maxdiff(const float* __restrict__ a, const float* __restri
 int MacSolver::check_coarse_cycle(double* diff)
 {
     const int lc = coarse_first();
-    if (lc < 1 || !beta_ready) {
+    if (lc < 0 || !beta_ready) {
         set_error("check_coarse_cycle: the MAC plan has no cluster-cycled levels (levels " + std::to_string(L.size()) +
                   ", dense bottom " + std::to_string((int)dense_bottom) + ") or no beta");
         return GBP_BAD_ARG;

@@ -12,6 +12,7 @@
 #include "krylov.h"
 #include "mac_kernels.h"
 #include "nodal_solver.h"
+#include "tail.h"
 
 namespace gbp {
 
@@ -119,11 +120,16 @@ private:
     double* dmat = nullptr;
     unsigned char* dact = nullptr;
     bool dense_bottom = false;
-    // the FP32 levels with at most this many cells (below the finest) run as one cluster launch per V-cycle
-    // (measured on the 256^3 MAC projection: 24.55 ms against 24.95 with per-level launches)
-    static constexpr long long kCoarseCells = 40000;
+    // as NodalSolver's, FP32 only (tail.cu)
+    static constexpr long long kTailCells = 5000, kSoloCells = 1100;
     bool use_coarse = true;
-    int coarse_first() const;
+    struct Tail {
+        int first = -1;
+        TailLayout t;
+        int* table = nullptr;
+    } tail;
+    void plan_tail();
+    int coarse_first() const { return use_coarse && dense_bottom && opt.nu1 >= 1 && opt.nu2 >= 1 ? tail.first : -1; }
     int launch_rc = 0;  // first failure while issuing a launch (recorded during capture)
     bool abec = false;
     struct EbState {

@@ -289,6 +289,9 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
     } else {
         add(5 * B.g.count, 8);
     }
+    plan_tail(tail32, kTailNodes32, 4);
+    plan_tail(tail64, kTailNodes64, 8);
+    for (Tail* t : {&tail32, &tail64}) add(t->t.table.size() + 1, 4);
     add(16, 4);
     add(8, 8);
     add(8, 8);
@@ -328,6 +331,11 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
         brows.carve(pool.take<char>(brows.bytes()));
     else
         bscr = pool.take<double>(5 * B.g.count);
+    for (Tail* t : {&tail32, &tail64}) {
+        t->table = pool.take<int>(t->t.table.size() + 1);
+        if (!t->t.table.empty())
+            GBP_CUDA(cudaMemcpyAsync(t->table, t->t.table.data(), sizeof(int) * t->t.table.size(), cudaMemcpyHostToDevice, st));
+    }
     dinfo = pool.take<int>(16);
     derr = reinterpret_cast<unsigned*>(dinfo + 8);
     dnorm = pool.take<unsigned long long>(8);
@@ -499,19 +507,35 @@ void NodalSolver::resid(const NodalGeom& g, const T* s, const T* x, const T* b, 
     }
 }
 
-// First level of the hierarchy cycled by the cluster kernel (k_coarse_vcycle): the first level below
-// the finest with at most kCoarseNodes nodes, when the bottom uses the dense inverse and the tail fits
-// the kernel's level table; -1 otherwise (every level on its own launches).
-int NodalSolver::coarse_first() const
+// The tail of the hierarchy that one cluster cycles: the first level small enough whose slabs fit, when the bottom
+// uses the dense inverse.
+void NodalSolver::plan_tail(Tail& t, long long most, int esize)
 {
-    if (!dense_bottom || !use_coarse) return -1;
-    for (int l = 1; l + 1 < (int)L.size(); ++l) {
+    t = Tail{};
+    const int ctas = dense_bottom ? tail_cluster_size() : 0;
+    if (!ctas) return;
+    for (int l = 0; l + 1 < (int)L.size(); ++l) {
         const NodalGeom& g = L[l].g;
-        if ((long long)g.nu[0] * g.nu[1] * g.nu[2] <= kCoarseNodes)
-            return ((int)L.size() - l <= kCoarseMaxLevels) ? l : -1;
+        if ((long long)g.nu[0] * g.nu[1] * g.nu[2] > most) continue;
+        std::vector<int> planes, elems;
+        std::vector<long long> nodes;
+        for (size_t q = l; q < L.size(); ++q) {
+            planes.push_back(L[q].g.nu[2]);
+            elems.push_back((int)L[q].g.sz);
+            nodes.push_back((long long)L[q].g.nu[0] * L[q].g.nu[1] * L[q].g.nu[2]);
+        }
+        if (tail_layout((int)planes.size(), planes.data(), g.per[2], elems.data(), nodes.data(), 4, esize, nbottom,
+                        esize == 4 ? kSoloNodes32 : kSoloNodes64, ctas, &t.t)) {
+            t.first = l;
+            return;
+        }
     }
-    return -1;
 }
+
+template <>
+const NodalSolver::Tail& NodalSolver::tail<float>() const { return tail32; }
+template <>
+const NodalSolver::Tail& NodalSolver::tail<double>() const { return tail64; }
 
 // V-cycle for A x = b on level l. zero: x starts at 0; otherwise from xres[l].
 template <typename T>
@@ -526,19 +550,23 @@ void NodalSolver::vcycle(int l, const T* b, bool zero)
         return;
     }
     // the small levels (this one down to the bottom) in one cluster-resident launch
-    if (sizeof(T) == 4 && zero && l >= 1 && l == coarse_first()) {
-        CoarseCycle<T> c{};
-        c.nl = (int)L.size() - l;
+    const Tail& tl = tail<T>();
+    if (zero && l == tl.first && use_coarse && opt.nu1 >= 1 && opt.nu2 >= 1 && !(l == 0 && eb.on)) {
+        NodalTail<T> c{};
+        c.nl = tl.t.nl;
+        c.ctas = tl.t.ctas;
+        c.solo = tl.t.solo;
+        c.tab_ints = tl.t.tab_ints;
         for (int q = 0; q < c.nl; ++q) {
-            const NodalLevel& v = L[l + q];
-            c.g[q] = v.g;
-            c.s[q] = B::s(v);
-            c.x[q] = B::x(v);
-            c.t[q] = B::t(v);
-            c.b[q] = B::b(v);
-            c.r[q] = B::r(v);
+            c.g[q] = L[l + q].g;
+            c.s[q] = B::s(L[l + q]);
+            c.np[q] = tl.t.np[q];
+            c.off[q] = tl.t.off[q];
+            c.own[q] = tl.t.own[q];
+            c.copies[q] = tl.t.copies[q];
         }
-        c.b[0] = const_cast<T*>(b);
+        c.b0 = b;
+        c.xout = B::x(lv);
         c.M = dmat;
         c.singular = bsing ? 1 : 0;
         for (int q = 0; q < kSweepWeights; ++q) {
@@ -547,10 +575,13 @@ void NodalSolver::vcycle(int l, const T* b, bool zero)
         }
         c.nu1 = opt.nu1;
         c.nu2 = opt.nu2;
-        int rc = nodal_coarse_vcycle<T>(c, nodal_coarse_cluster_size(), s);
+        c.table = tl.table;
+        c.tab_off = tl.t.tab_off;
+        c.dense_off = tl.t.dense_off;
+        int rc = nodal_tail<T>(c, tl.t.bytes, s);
         if (rc && !launch_rc) launch_rc = rc;
         ++nk;
-        xres[l] = coarse_result_slot(opt.nu1, opt.nu2) ? B::t(lv) : B::x(lv);
+        xres[l] = B::x(lv);
         return;
     }
     T* x = zero ? B::x(lv) : (T*)xres[l];
@@ -1884,7 +1915,7 @@ int NodalSolver::check_level_kernels_on(float* A, float* C, double diff[4])
 int NodalSolver::check_coarse_cycle(double* diff)
 {
     const int lc = coarse_first();
-    if (lc < 1 || !sigma_ready) {
+    if (lc < 0 || !sigma_ready) {
         set_error("check_coarse_cycle: the plan has no cluster-cycled levels (levels " + std::to_string(L.size()) +
                   ", dense bottom " + std::to_string((int)dense_bottom) + " of " + std::to_string(nbottom) +
                   " nodes, cluster path " + std::to_string((int)use_coarse) + ") or no sigma (" +

@@ -13,6 +13,7 @@
 #include "nodal_kernels.h"
 #include "nodal_eb.h"
 #include "nodal_sweep.h"
+#include "tail.h"
 
 namespace gbp {
 
@@ -215,12 +216,21 @@ private:
     unsigned long long* dnorm = nullptr;  // [0] rhs norm, [1] residual norm
     unsigned long long* hnorm = nullptr;  // pinned mirror
     bool singular = false;        // the system has the constants as null space (consistent RHS, gauge)
-    // the FP32 levels with at most this many nodes (below the finest) run as one cluster launch per V-cycle
-    // (measured at 256^3: 11.92 ms per projection against 11.98 with per-level launches and 12.12 with the
-    // 33^3 level included; FP64 levels stay on per-level launches, which were faster there)
-    static constexpr long long kCoarseNodes = 5000;
+    // the levels from this many nodes down run as one cluster launch per V-cycle (tail.h): what fits the cluster's shared
+    // memory and, in FP64, what its 16 SMs' FP64 pipes do not take longer for than launches over the chip
+    static constexpr long long kTailNodes32 = 5000, kTailNodes64 = 1000;
+    // ... and by one CTA of it
+    static constexpr long long kSoloNodes32 = 1400, kSoloNodes64 = 130;
     bool use_coarse = true;
-    int coarse_first() const;
+    struct Tail {
+        int first = -1;  // its first level, -1: none
+        TailLayout t;
+        int* table = nullptr;
+    } tail32, tail64;
+    void plan_tail(Tail& t, long long most, int esize);
+    template <typename T>
+    const Tail& tail() const;
+    int coarse_first() const { return use_coarse && opt.nu1 >= 1 && opt.nu2 >= 1 ? tail32.first : -1; }
 public:
     // test hook: one FP32 V-cycle from the first cluster-cycled level on a seeded right-hand side, through
     // the per-level launches and through the cluster kernel; *diff = max |difference| / max |result|

@@ -100,3 +100,15 @@ def test_cluster_bottom_solve_mac(gpu_lib, n, lo, hi, precision):
     mp.setUMAC(ut)
     st = mp.project(rtol=1e-12, atol=0.0, phi=phi, phi_guess=False)
     assert st["status"] == 0 and rel_l2(phi.cpu().numpy(), phi_or) <= 1e-9
+
+
+# levels that one thread-block cluster cycles in shared memory: fewer planes than CTAs, planes that do not split evenly,
+# levels with one CTA's worth of points at once, periodic and bounded in z
+TAILS = [((16, 32, 8), (P, N, P), (P, D, P)), ((8, 12, 64), (N, P, P), (N, P, P)), ((32, 16, 56), (D, N, N), (N, I, N))]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,lo,hi", TAILS, ids=["x".join(map(str, c[0])) for c in TAILS])
+def test_cluster_tail(gpu_lib, n, lo, hi, precision):
+    _nodal(n, lo, hi, precision)
+    test_cluster_bottom_solve_mac(gpu_lib, n, lo, hi, precision)
