@@ -91,55 +91,100 @@ __global__ void __launch_bounds__(128) k_rows_mac(CellGeom g, const double* __re
 }
 
 // ------------------------------------------------------------------------------------------------ dense inverse
-// Gauss-Jordan in place (the matrix is symmetric positive definite: no pivoting)
+// Symmetric positive definite, so no pivoting, and Gauss-Jordan as the sweep operator (Goodnight 1979, The American
+// Statistician 33), which keeps the symmetry: one triangle in registers, the pivot's column passed through shared
+// memory, one division per pivot and two warps. One SM's FP64 pipe bounds it (16 cycles per warp and instruction): 64
+// unknowns took 243 us with the whole matrix and a division in every warp, now 75.
 __global__ void __launch_bounds__(1024) k_bottom_inverse(BottomRows r, int singular, double* __restrict__ M,
                                                          unsigned char* __restrict__ act, unsigned* bad)
 {
-    __shared__ double A[kDenseBottom][kDenseBottom];
-    __shared__ double row[kDenseBottom], col[kDenseBottom];
+    constexpr int kMost = (kDenseBottom * (kDenseBottom + 1) / 2 + 1023) / 1024;  // entries of a thread
+    __shared__ double A[kDenseBottom][kDenseBottom + 1];
+    __shared__ double col[2][kDenseBottom], scl[kDenseBottom], shift;
     const int N = r.n, t = threadIdx.x;
     for (int q = t; q < N * N; q += blockDim.x) A[q / N][q % N] = 0.0;
     __syncthreads();
     double tr = 0.0, na = 0.0;
-    for (int u = t; u < N; u += blockDim.x) {
-        const bool held = r.diag[u] == 0.0;
-        for (int q = 0; q < r.w; ++q) A[u][r.idx[(size_t)q * N + u]] += r.coef[(size_t)q * N + u];
-        if (held) A[u][u] = 1.0;
-        tr += held ? 0.0 : A[u][u];
-        na += held ? 0.0 : 1.0;
-        if (act) act[u] = !held;
-    }
-    if (singular) {
-        tr = block_sum_all(tr);
-        na = block_sum_all(na);
-        const double c = na > 0.0 ? tr / (na * na) : 0.0;
-        for (int q = t; q < N * N; q += blockDim.x)
-            if (r.diag[q / N] != 0.0 && r.diag[q % N] != 0.0) A[q / N][q % N] += c;
+    if (t < N) {
+        const bool held = r.diag[t] == 0.0;
+        for (int q = 0; q < r.w; ++q) A[t][r.idx[(size_t)q * N + t]] += r.coef[(size_t)q * N + t];
+        if (held) A[t][t] = 1.0;
+        tr = held ? 0.0 : A[t][t];
+        na = held ? 0.0 : 1.0;
+        scl[t] = tr;
+        col[0][t] = na;
+        if (act) act[t] = !held;
     }
     __syncthreads();
-    for (int c = 0; c < N; ++c) {
-        if (t < N) {
-            row[t] = A[c][t];
-            col[t] = A[t][c];
+    if (t < 32) {
+        tr = (t < N ? scl[t] : 0.0) + (t + 32 < N ? scl[t + 32] : 0.0);
+        na = (t < N ? col[0][t] : 0.0) + (t + 32 < N ? col[0][t + 32] : 0.0);
+        for (int o = 16; o > 0; o >>= 1) {
+            tr += __shfl_xor_sync(0xffffffffu, tr, o);
+            na += __shfl_xor_sync(0xffffffffu, na, o);
         }
-        __syncthreads();
-        const double piv = row[c];
+        if (t == 0) shift = singular && na > 0.0 ? tr / (na * na) : 0.0;
+    }
+    __syncthreads();
+    // entry e of the lower triangle: (u, v), v <= u, e = u (u + 1) / 2 + v
+    int eu[kMost], ev[kMost];
+    double a[kMost];
+#pragma unroll
+    for (int m = 0; m < kMost; ++m) {
+        const int e = t + 1024 * m;
+        int u = (int)((sqrtf(8.f * (float)e + 1.f) - 1.f) * 0.5f);
+        while (u * (u + 1) / 2 > e) --u;
+        while ((u + 1) * (u + 2) / 2 <= e) ++u;
+        eu[m] = u < N ? u : -1;
+        ev[m] = u < N ? e - u * (u + 1) / 2 : -1;
+        a[m] = 0.0;
+        if (u < N) {
+            a[m] = A[u][ev[m]];
+            if (r.diag[u] != 0.0 && r.diag[ev[m]] != 0.0) a[m] += shift;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < kMost; ++m)  // the first pivot's column
+        if (eu[m] >= 0 && ev[m] == 0) col[0][eu[m]] = a[m];
+    __syncthreads();
+    for (int c = 0; c < N; ++c) {
+        const double* cc = col[c & 1];
+        const double piv = cc[c];
         if (!(piv > 0.0)) {  // uniform
             if (t == 0) *bad = 1u;
             return;
         }
-        const double inv = 1.0 / piv;
-        for (int q = t; q < N * N; q += blockDim.x) {
-            const int u = q / N, v = q % N;
-            if (u == c)
-                A[u][v] = v == c ? inv : row[v] * inv;
+        if (t < ((N + 31) & ~31)) {
+            const double inv = 1.0 / piv;
+            if (t < N) scl[t] = t == c ? -inv : cc[t] * inv;
+        }
+        __syncthreads();
+        // a_uv -= a_uc a_cv / a_cc; the pivot's row and column a_uc / a_cc; the pivot -1 / a_cc: minus the inverse
+        double* nx = col[(c + 1) & 1];
+#pragma unroll
+        for (int m = 0; m < kMost; ++m) {
+            const int u = eu[m], v = ev[m];
+            if (u < 0) continue;
+            if (u == c || v == c)
+                a[m] = scl[u == c ? v : u];
             else
-                A[u][v] = v == c ? -col[u] * inv : A[u][v] - col[u] * inv * row[v];
+                a[m] = fma(-cc[u], scl[v], a[m]);
+            if (u == c + 1)
+                nx[v] = a[m];
+            else if (v == c + 1)
+                nx[u] = a[m];
         }
         __syncthreads();
     }
-    for (int q = t; q < N * N; q += blockDim.x)
-        M[q] = r.diag[q / N] != 0.0 && r.diag[q % N] != 0.0 ? A[q % N][q / N] : 0.0;
+#pragma unroll
+    for (int m = 0; m < kMost; ++m) {
+        const int u = eu[m], v = ev[m];
+        if (u < 0) continue;
+        const double x = r.diag[u] != 0.0 && r.diag[v] != 0.0 ? -a[m] : 0.0;
+        M[u * N + v] = x;
+        M[v * N + u] = x;
+    }
 }
 
 // ------------------------------------------------------------------------------------------------ conjugate gradients

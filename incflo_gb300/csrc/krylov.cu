@@ -58,37 +58,104 @@ __device__ __forceinline__ long long vec_at(const KrylovBox& b, unsigned t, unsi
     return pidx(b.sy, b.sz, i, (int)(row - k * (unsigned)b.n[1]), (int)k);
 }
 
-// The last block to get here sums the nb partial pairs in order and returns true in every thread, with the sums.
-__device__ __forceinline__ bool fold_last(double v0, double v1, double* part, unsigned* done, double& s0, double& s1)
+// A sum carried by a thread: FP64 as it is, FP32 as an unevaluated pair hi + lo (Knuth's two-sum, about 48 bits: the
+// FP64 pipe takes 16 cycles per warp for an addition or a conversion, the FP32 pipe takes the six additions of a
+// two-sum in less).
+template <typename T>
+struct Sum;
+template <>
+struct Sum<double> {
+    double v = 0.0;
+};
+template <>
+struct Sum<float> {
+    float hi = 0.f, lo = 0.f;
+    __device__ __forceinline__ void add(float h, float l)
+    {
+        const float s = __fadd_rn(hi, h), t = __fsub_rn(s, hi);
+        const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, t)), __fsub_rn(h, t));
+        hi = s;
+        lo = __fadd_rn(lo, __fadd_rn(l, e));
+    }
+    __device__ __forceinline__ void warp()
+    {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            add(__shfl_xor_sync(0xffffffffu, hi, o), __shfl_xor_sync(0xffffffffu, lo, o));
+    }
+};
+
+// Block sums of NV values per thread in a fixed order; the result lies in out[0 .. NV) after the next __syncthreads.
+// FP64: one warp per value adds the threads' values (every warp reducing its own lanes would cost the pipe 8 times that).
+template <int NV>
+__device__ __forceinline__ void block_sums(const Sum<double> (&v)[NV], double* tab, double* out)
 {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) tab[q * kT + threadIdx.x] = v[q].v;
+    __syncthreads();
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (wid < NV) {
+        const double* t = tab + wid * kT + lane;
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < kT / 32; w += 4) s += (t[32 * w] + t[32 * w + 32]) + (t[32 * w + 64] + t[32 * w + 96]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) out[wid] = s;
+    }
+}
+template <int NV>
+__device__ __forceinline__ void block_sums(Sum<float> (&v)[NV], double* tab, double* out)
+{
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+        v[q].warp();
+        if (lane == 0) tab[q * kT + wid] = (double)v[q].hi + (double)v[q].lo;
+    }
+    __syncthreads();
+    if (wid < NV) {
+        double s = lane < kT / 32 ? tab[wid * kT + lane] : 0.0;
+#pragma unroll
+        for (int o = kT / 64; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) out[wid] = s;
+    }
+}
+
+// The last block to get here sums the blocks' partial sums in order and returns true in every thread, with the sums in out.
+template <typename T, int NV>
+__device__ __forceinline__ bool fold_last(Sum<T> (&v)[NV], double* part, unsigned* done, double* out)
+{
+    __shared__ double tab[NV * kT];
     __shared__ bool last;
-    v0 = block_sum_all(v0);
-    v1 = block_sum_all(v1);
+    block_sums(v, tab, out);
+    __syncthreads();
     if (threadIdx.x == 0) {
-        part[2 * blockIdx.x] = v0;
-        part[2 * blockIdx.x + 1] = v1;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) part[2 * blockIdx.x + q] = out[q];
         __threadfence();
         last = atomicAdd(done, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    v0 = v1 = 0.0;
-    for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) {
-        v0 += __ldcg(part + 2 * q);
-        v1 += __ldcg(part + 2 * q + 1);
-    }
-    s0 = block_sum_all(v0);
-    s1 = block_sum_all(v1);
+    Sum<double> f[NV];
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += kT)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) f[q].v += __ldcg(part + 2 * b + q);
+    block_sums(f, tab, out);
+    __syncthreads();
     if (threadIdx.x == 0) *done = 0;
     return true;
 }
 
 // a.b and a.c (c may be null) over the unique points. FP32 vectors are summed in FP32 per thread (a few hundred
-// terms) and in FP64 from there: the FP64 pipe is 64 times slower than the FP32 one.
+// terms), as pairs over the block and in FP64 from there. Latency and the FP64 pipe bound it below some 10^6 points:
+// with FP64 sums in every warp 17.2 us (r.z, 10^6 points FP32), 13.9 us (64^3 FP64), 9.8 us (16^3 FP64); now 10.5, 11.3
+// and 7.2 us.
 template <typename T, int WHAT>
-__global__ void __launch_bounds__(kT) k_dots(KrylovBox b, const T* __restrict__ a, const T* __restrict__ v,
-                                             const T* __restrict__ w, double* __restrict__ part, KrylovState* s)
+__global__ void __launch_bounds__(kT) k_dots(KrylovBox b, const T* __restrict__ a, const T* __restrict__ c,
+                                             const T* __restrict__ d, double* __restrict__ part, KrylovState* s)
 {
     constexpr int N = Vec<T>::N;
     const unsigned vr = (unsigned)(b.n[0] + N - 1) / N;
@@ -100,8 +167,8 @@ __global__ void __launch_bounds__(kT) k_dots(KrylovBox b, const T* __restrict__ 
         const long long p = vec_at<T>(b, t, vr, i);
         T x[N], y[N], z[N];
         ldv<T>(a + p, x);
-        ldv<T>(v + p, y);
-        if (two) ldv<T>(w + p, z);
+        ldv<T>(c + p, y);
+        if (two) ldv<T>(d + p, z);
 #pragma unroll
         for (int e = 0; e < N; ++e) {
             if (i + e >= b.n[0]) continue;
@@ -109,13 +176,21 @@ __global__ void __launch_bounds__(kT) k_dots(KrylovBox b, const T* __restrict__ 
             if (two) acc1[e] += y[e] * z[e];
         }
     }
-    double s0 = 0.0, s1 = 0.0;
+    constexpr int NV = WHAT == 0 ? 2 : 1;
+    __shared__ double out[2];
+    Sum<T> v[NV];
 #pragma unroll
     for (int e = 0; e < N; ++e) {
-        s0 += (double)acc0[e];
-        s1 += (double)acc1[e];
+        if constexpr (sizeof(T) == 4) {
+            v[0].add(acc0[e], 0.f);
+            if (NV == 2) v[NV - 1].add(acc1[e], 0.f);
+        } else {
+            v[0].v += acc0[e];
+            if (NV == 2) v[NV - 1].v += acc1[e];
+        }
     }
-    if (!fold_last(s0, s1, part, s->done + WHAT, s0, s1) || threadIdx.x) return;
+    if (!fold_last<T, NV>(v, part, s->done + WHAT, out) || threadIdx.x) return;
+    const double s0 = out[0], s1 = out[NV - 1];
     if (WHAT == 0) {
         s->rz = s0;
         double beta = 0.0;
@@ -154,38 +229,66 @@ __global__ void __launch_bounds__(kT) k_direction(long long nvec, const T* __res
     stv<T>(p + t * N, x);
 }
 
-// one thread per vector of the padded array: x everywhere, r where the position is a unique point
-template <typename T>
+// One thread per vector of the padded array: x everywhere, r where the position is a unique point. NORM: also the max
+// of |r| / V, as integer keys of |r| (the points on non-periodic sides of a nodal box have half the volume per side: a
+// power of two) and one multiplication per block; a pass over r of its own
+// took 252 us at 256^3 (16 us at 64^3), the keys add 25 us (2 us).
+template <typename T, bool NORM>
 __global__ void __launch_bounds__(kT) k_update(KrylovBox b, long long nvec, const T* __restrict__ p,
                                                const T* __restrict__ q, T* __restrict__ x, T* __restrict__ r,
-                                               const KrylovState* s)
+                                               const KrylovState* s, KrylovNorm nm)
 {
     constexpr int N = Vec<T>::N;
     const long long t = blockIdx.x * (long long)kT + threadIdx.x;
-    if (t >= nvec) return;
-    const T alpha = (T)s->alpha;
-    const unsigned rowv = (unsigned)(b.sy / N), rows = (unsigned)(b.sz / b.sy);
-    const unsigned row = (unsigned)(t / rowv), k = row / rows;
-    const int i = (int)(t - (long long)row * rowv) * N - kOX, j = (int)(row - k * rows) - 1;
-    T u[N], v[N];
-    ldv<T>(p + t * N, u);
-    ldv<T>(x + t * N, v);
+    unsigned long long key = 0;
+    if (t < nvec) {
+        const T alpha = (T)s->alpha;
+        const unsigned rowv = (unsigned)(b.sy / N), rows = (unsigned)(b.sz / b.sy);
+        const unsigned row = (unsigned)(t / rowv), kp = row / rows;
+        const int i = (int)(t - (long long)row * rowv) * N - kOX, j = (int)(row - kp * rows) - 1, k = (int)kp - 1;
+        T u[N], v[N];
+        ldv<T>(p + t * N, u);
+        ldv<T>(x + t * N, v);
 #pragma unroll
-    for (int e = 0; e < N; ++e) v[e] += alpha * u[e];
-    stv<T>(x + t * N, v);
-    if (j < 0 || j >= b.n[1] || k < 1 || (int)k - 1 >= b.n[2] || i + N <= 0 || i >= b.n[0]) return;
-    ldv<T>(q + t * N, u);
-    ldv<T>(r + t * N, v);
+        for (int e = 0; e < N; ++e) v[e] += alpha * u[e];
+        stv<T>(x + t * N, v);
+        if (j >= 0 && j < b.n[1] && k >= 0 && k < b.n[2] && i + N > 0 && i < b.n[0]) {
+            ldv<T>(q + t * N, u);
+            ldv<T>(r + t * N, v);
 #pragma unroll
-    for (int e = 0; e < N; ++e)
-        if (i + e >= 0 && i + e < b.n[0]) v[e] += alpha * u[e];
-    stv<T>(r + t * N, v);
+            for (int e = 0; e < N; ++e) {
+                if (i + e < 0 || i + e >= b.n[0]) continue;
+                v[e] += alpha * u[e];
+                if constexpr (NORM) {
+                    const int at[3] = {i + e, j, k};
+                    int halves = 0;
+                    bool held = nm.mask && !nm.mask[t * N + e];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        const bool lo = at[d] == 0, hi = at[d] == b.n[d] - 1;
+                        halves += (nm.nodal[d] && (lo || hi)) ? 1 : 0;
+                        held = held || (lo && nm.dlo[d]) || (hi && nm.dhi[d]);
+                    }
+                    const unsigned long long kv =
+                        held ? 0 : abs_key(halves == 0 ? (double)v[e] : (double)v[e] * (double)(1 << halves));
+                    key = kv > key ? kv : key;
+                }
+            }
+            stv<T>(r + t * N, v);
+        }
+    }
+    if constexpr (NORM) {
+        key = block_max_key(key);
+        if (threadIdx.x == 0) atomic_max_nonneg(nm.norm, key_value(key) * nm.ivol);
+    }
 }
 
 unsigned dot_blocks(const KrylovBox& b, int vec)
 {
     const long long nv = (long long)((b.n[0] + vec - 1) / vec) * b.n[1] * b.n[2];
-    return (unsigned)std::max<long long>(1, std::min<long long>((nv + kT - 1) / kT, kKrylovBlocks));
+    // a vector per thread until every SM has a block, then four (fewer blocks to sum in FP64), up to the scratch
+    const long long blocks = std::max(std::min<long long>((nv + kT - 1) / kT, 152), (nv + 4 * kT - 1) / (4 * kT));
+    return (unsigned)std::max<long long>(1, std::min<long long>(blocks, kKrylovBlocks));
 }
 
 }  // namespace
@@ -207,17 +310,23 @@ void krylov_pq(const KrylovBox& b, const T* p, const T* q, double* part, KrylovS
     k_dots<T, 1><<<dot_blocks(b, Vec<T>::N), kT, 0, st>>>(b, p, q, nullptr, part, s);
 }
 template <typename T>
-void krylov_update(const KrylovBox& b, const T* p, const T* q, T* x, T* r, const KrylovState* s, cudaStream_t st)
+void krylov_update(const KrylovBox& b, const T* p, const T* q, T* x, T* r, const KrylovState* s, cudaStream_t st,
+                   const KrylovNorm* norm)
 {
     const long long nv = b.count / Vec<T>::N;
-    k_update<T><<<(unsigned)((nv + kT - 1) / kT), kT, 0, st>>>(b, nv, p, q, x, r, s);
+    const unsigned nb = (unsigned)((nv + kT - 1) / kT);
+    if (norm)
+        k_update<T, true><<<nb, kT, 0, st>>>(b, nv, p, q, x, r, s, *norm);
+    else
+        k_update<T, false><<<nb, kT, 0, st>>>(b, nv, p, q, x, r, s, KrylovNorm{});
 }
 
 #define GBP_KRYLOV(T)                                                                                               \
     template void krylov_rz<T>(const KrylovBox&, const T*, const T*, const T*, double*, KrylovState*, cudaStream_t); \
     template void krylov_direction<T>(const KrylovBox&, const T*, T*, const KrylovState*, cudaStream_t);             \
     template void krylov_pq<T>(const KrylovBox&, const T*, const T*, double*, KrylovState*, cudaStream_t);           \
-    template void krylov_update<T>(const KrylovBox&, const T*, const T*, T*, T*, const KrylovState*, cudaStream_t);
+    template void krylov_update<T>(const KrylovBox&, const T*, const T*, T*, T*, const KrylovState*, cudaStream_t,        \
+                                   const KrylovNorm*);
 GBP_KRYLOV(double)
 GBP_KRYLOV(float)
 

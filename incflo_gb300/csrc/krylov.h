@@ -43,8 +43,17 @@ void krylov_direction(const KrylovBox& b, const T* z, T* p, const KrylovState* s
 // alpha = rz / (p.Ap), q = -A p
 template <typename T>
 void krylov_pq(const KrylovBox& b, const T* p, const T* q, double* part, KrylovState* s, cudaStream_t st);
+// The max of |r| / V over the points that are not held, for krylov_update: *norm = max(*norm, it). nodal[d]: the points
+// on the sides of direction d have half the volume; dlo / dhi: held sides; mask: 0 on held points (padded), or null.
+struct KrylovNorm {
+    unsigned long long* norm;
+    int nodal[3], dlo[3], dhi[3];
+    const unsigned char* mask;
+    double ivol;
+};
 // x += alpha p over the whole padded array, r += alpha q on the unique points
 template <typename T>
-void krylov_update(const KrylovBox& b, const T* p, const T* q, T* x, T* r, const KrylovState* s, cudaStream_t st);
+void krylov_update(const KrylovBox& b, const T* p, const T* q, T* x, T* r, const KrylovState* s, cudaStream_t st,
+                   const KrylovNorm* norm = nullptr);
 
 }  // namespace gbp

@@ -579,13 +579,23 @@ __global__ void __launch_bounds__(256) k_mac_norm(CellGeom g, const double* __re
         if (threadIdx.x == 0) atomic_max_nonneg(norm, key_value(key) * (1.0 / g.vol));
         return;
     }
-    double nv = 0.0;
+    // the cut-cell operator divides by the volume fraction; whole cells as above (the FP64 maxima and a division per cell
+    // bound it: 59 us for 10^6 cells against 14.7)
+    unsigned long long whole = 0, cut = 0;
     if (decode_cell(g, blockIdx.x * (long long)blockDim.x + threadIdx.x, i, j, k)) {
         const long long p = pidx(g.sy, g.sz, i, j, k);
-        if (kap[p] > 0.0) nv = fabs(v[p]) / (kap[p] * g.vol);  // the cut-cell operator divides by the volume fraction
+        const double f = kap[p];
+        if (f == 1.0)
+            whole = abs_key(v[p]);
+        else if (f > 0.0)
+            cut = abs_key(fabs(v[p]) / (f * g.vol));
     }
-    nv = block_max(nv);
-    if (threadIdx.x == 0) atomic_max_nonneg(norm, nv);
+    whole = block_max_key(whole);
+    cut = block_max_key(cut);
+    if (threadIdx.x == 0) {
+        const double w = key_value(whole) * (1.0 / g.vol);
+        atomic_max_nonneg(norm, nanmax(w, key_value(cut)));
+    }
 }
 
 // per-block sums of v (kap != null and weighted: of kap * v): each thread sums its cells of a grid-stride

@@ -859,7 +859,7 @@ void MacSolver::resid64(const double* x, const double* b, double* r, unsigned lo
 
 // q = -A p, then the vector passes (krylov.h)
 template <typename T>
-void MacSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s)
+void MacSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s, const KrylovNorm* norm)
 {
     using B = MacBufs<T>;
     const MacLevel& l0 = L[0];
@@ -874,7 +874,7 @@ void MacSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s)
         mac_resid<T>(l0.g, be[0], be[1], be[2], p, nullptr, q, nullptr, s);
         if (eb.on) eb_cells<T>(l0.g, eb.cells, eb.ncells, eb.faces, B::cb(eb), p, q, q, s);
         krylov_pq<T>(kbox, p, q, kpart, kstate, s);
-        krylov_update<T>(kbox, p, q, x, r, kstate, s);
+        krylov_update<T>(kbox, p, q, x, r, kstate, s, c == m - 1 ? norm : nullptr);
     }
 }
 
@@ -894,8 +894,9 @@ void MacSolver::record_iteration(int m)
         mac_add_correction<float>(l0.g, phi, e, 1.0, s, kstate);
         resid64(phi, rhs0, res, dnorm + 1, s);
     } else {
-        krylov_steps<double>(1, phi, res, s);
-        mac_norm(l0.g, res, dnorm + 1, s, eb.on ? eb.m.kap : nullptr);
+        const KrylovNorm nm{dnorm + 1, {}, {}, {}, nullptr, 1.0 / l0.g.vol};
+        krylov_steps<double>(1, phi, res, s, eb.on ? nullptr : &nm);
+        if (eb.on) mac_norm(l0.g, res, dnorm + 1, s, eb.m.kap);
     }
     cudaMemcpyAsync(hnorm + 1, dnorm + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
 }

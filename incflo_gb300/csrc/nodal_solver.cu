@@ -695,7 +695,7 @@ void NodalSolver::apply_neg<float>(const float* p, float* q, cudaStream_t s)
 }
 
 template <typename T>
-void NodalSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s)
+void NodalSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s, const KrylovNorm* norm)
 {
     T* p = reinterpret_cast<T*>(kp);
     T* q = reinterpret_cast<T*>(kq);
@@ -706,7 +706,7 @@ void NodalSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s)
         krylov_direction<T>(kbox, z, p, kstate, s);
         apply_neg<T>(p, q, s);
         krylov_pq<T>(kbox, p, q, kpart, kstate, s);
-        krylov_update<T>(kbox, p, q, x, r, kstate, s);
+        krylov_update<T>(kbox, p, q, x, r, kstate, s, c == m - 1 ? norm : nullptr);
         nk += 5;
     }
 }
@@ -754,12 +754,17 @@ void NodalSolver::record_iteration(int m)
         }
         nk += 2;
     } else {
-        krylov_steps<double>(1, phi, res, s);
-        if (eb.on)
+        KrylovNorm nm{dnorm + 1, {}, {}, {}, l0.g.mask, l0.g.ivol};
+        for (int d = 0; d < 3; ++d) {
+            nm.nodal[d] = !l0.g.per[d];
+            nm.dlo[d] = l0.g.dlo[d];
+            nm.dhi[d] = l0.g.dhi[d];
+        }
+        krylov_steps<double>(1, phi, res, s, eb.on ? nullptr : &nm);
+        if (eb.on) {
             eb_norm(l0.g, res, eb.ivol, dnorm + 1, s);
-        else
-            nodal_norm(l0.g, res, dnorm + 1, s);
-        ++nk;
+            ++nk;
+        }
     }
     cudaMemcpyAsync(hnorm + 1, dnorm + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
     step_kernels = nk - nk0;

@@ -178,7 +178,7 @@ private:
                cudaStream_t s_);
     // m iterations of the accelerated V-cycle (krylov.h) for A x = r: x and r in place
     template <typename T>
-    void krylov_steps(int m, T* x, T* r, cudaStream_t s);
+    void krylov_steps(int m, T* x, T* r, cudaStream_t s, const KrylovNorm* norm = nullptr);
     template <typename T>
     void apply_neg(const T* p, T* q, cudaStream_t s);  // q = -A p on level 0
     bool accelerated() const;
