@@ -4,7 +4,8 @@
 // once per geometry) in a table. Nodes that touch a cut cell ("EB nodes", about 1 % of the nodes around
 // a body) are recomputed by the node-centric kernels below after the level kernel has run, from the
 // same input, so the level kernel's output there is simply overwritten:
-//   k_eb_node<MODE>   Jacobi update (MODE 0) or residual (MODE 1) of the EB nodes over their 8 cells
+//   k_eb_rows         the 27 entries of every EB node's row, whenever sigma is set
+//   k_eb_node<MODE>   Jacobi update (MODE 0) or residual (MODE 1) of the EB nodes with those rows
 //   k_eb_rhs          the cut cells' int u . grad N added to the right-hand side of the EB nodes
 //   k_eb_correct      u -= sigma grad phi at the fluid centroid of every cut cell, gp / grad phi out
 #include <cuda_runtime.h>
@@ -28,57 +29,75 @@ __device__ __forceinline__ long long corner_off(const NodalGeom& g, int b)
     return (long long)(b & 1) + ((b >> 1) & 1) * g.sy + ((b >> 2) & 1) * g.sz;
 }
 
-template <typename T>
-__device__ __forceinline__ const T* sig_true(const EbNodal& e);
-template <>
-__device__ __forceinline__ const double* sig_true<double>(const EbNodal& e) { return e.sig64; }
-template <>
-__device__ __forceinline__ const float* sig_true<float>(const EbNodal& e) { return e.sig32; }
+// offset (-1, 0, 1 per direction) of entry q of a row
+__device__ __forceinline__ long long row_off(long long sy, long long sz, int q)
+{
+    return (q % 3 - 1) + (q / 3 % 3 - 1) * sy + (q / 9 - 1) * sz;
+}
 
+// one thread per entry: the sum of sigma K over the (at most 8) cells that hold both nodes, in FP64
+__global__ void __launch_bounds__(128) k_eb_rows(NodalGeom g, EbNodal e)
+{
+    const int t = blockIdx.x * 128 + threadIdx.x, q = blockIdx.y;
+    if (t >= e.nnodes) return;
+    const EbNodeEntry nd = e.nodes[t];
+    const long long p = pidx(g.sy, g.sz, nd.i, nd.j, nd.k);
+    const int qx = q % 3, qy = q / 3 % 3, qz = q / 9;
+    double v = 0.0;
+    for (int c = 0; c < 8; ++c) {
+        // cell c = (i - 1 + dx, j - 1 + dy, k - 1 + dz): this node is its corner a, the other one its corner b
+        const int dx = c & 1, dy = (c >> 1) & 1, dz = c >> 2, cc = nd.cell[c];
+        if (cc == kEbCovered || (unsigned)(qx - dx) > 1u || (unsigned)(qy - dy) > 1u || (unsigned)(qz - dz) > 1u) continue;
+        const int a = (1 - dx) | ((1 - dy) << 1) | ((1 - dz) << 2), b = (qx - dx) | ((qy - dy) << 1) | ((qz - dz) << 2);
+        v += e.sig64[p - corner_off(g, a)] * (cc == kEbRegular ? g.K[a ^ b] : e.cells[cc].K[8 * a + b]);
+    }
+    e.row64[(size_t)q * e.pitch + t] = v;
+    e.row32[(size_t)q * e.pitch + t] = (float)v;
+    if (q == 13) {
+        const double rd = v > 0.0 ? 1.0 / v : 0.0;
+        e.row64[(size_t)27 * e.pitch + t] = rd;
+        e.row32[(size_t)27 * e.pitch + t] = (float)rd;
+    }
+}
+
+template <typename T>
+__device__ __forceinline__ const T* eb_row(const EbNodal& e);
+template <>
+__device__ __forceinline__ const double* eb_row<double>(const EbNodal& e) { return e.row64; }
+template <>
+__device__ __forceinline__ const float* eb_row<float>(const EbNodal& e) { return e.row32; }
+
+// Latency bounds it (some 10^4 nodes): all 54 loads of a node are independent. Over the node's cells and their element
+// matrices, 8 dependent steps of 17 loads and as many conversions, 18.9 us per call around the cylinder of a 256 x 64 x
+// 64 channel; 6.2 us (sweep) and 7.7 us (residual) with rows, whose set-up takes 6.9 us once per sigma (some 60 calls per
+// projection).
 template <typename T, int MODE>
 __global__ void __launch_bounds__(128) k_eb_node(NodalGeom g, EbNodal e, const T* __restrict__ x, const T* __restrict__ b,
                                                  T* out, T omega)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= e.nnodes) return;
-    const EbNodeEntry nd = e.nodes[t];
+    const EbNodeEntry& nd = e.nodes[t];
+    const int i = nd.i, j = nd.j, k = nd.k;
     T v = T(0);
-    if (!node_is_dirichlet(g, nd.i, nd.j, nd.k)) {
-        const long long p = pidx(g.sy, g.sz, nd.i, nd.j, nd.k);
-        const T* sg = sig_true<T>(e);
-        // damped Jacobi with the row's own diagonal, as the level kernels do on the regular nodes
-        T ax = T(0), diag = T(0);
-        for (int c = 0; c < 8; ++c) {
-            const int cc = nd.cell[c];
-            if (cc == kEbCovered) continue;
-            // cell c = (i - 1 + dx, j - 1 + dy, k - 1 + dz); this node is its corner a
-            const int dx = c & 1, dy = (c >> 1) & 1, dz = c >> 2;
-            const int a = (1 - dx) | ((1 - dy) << 1) | ((1 - dz) << 2);
-            const long long p0 = p - corner_off(g, a);  // the cell's low corner (and the cell's index)
-            const T s = sg[p0];
-            if (cc == kEbRegular) {
-                for (int q = 0; q < 8; ++q) {
-                    const T kq = s * (T)g.K[a ^ q];
-                    if (x) ax += kq * x[p0 + corner_off(g, q)];
-                    if (q == a) diag += kq;
-                }
-            } else {
-                const double* K = e.cells[cc].K + 8 * a;
-                for (int q = 0; q < 8; ++q) {
-                    const T kq = s * (T)K[q];
-                    if (x) ax += kq * x[p0 + corner_off(g, q)];
-                    if (q == a) diag += kq;
-                }
-            }
+    if (!node_is_dirichlet(g, i, j, k)) {
+        const long long p = pidx(g.sy, g.sz, i, j, k);
+        const T* row = eb_row<T>(e) + t;
+        T ax = T(0), xc = T(0);  // x == nullptr: a zero start
+        if (x) {
+            T part[3] = {T(0), T(0), T(0)};
+#pragma unroll
+            for (int q = 0; q < 27; ++q) part[q % 3] += row[(size_t)q * e.pitch] * x[p + row_off(g.sy, g.sz, q)];
+            ax = part[0] + part[1] + part[2];
+            xc = x[p];
         }
-        // x == nullptr: a zero start
-        const T xc = x ? x[p] : T(0);
+        // damped Jacobi with the row's own diagonal, as the level kernels do on the regular nodes
         if (MODE == 0)
-            v = diag > T(0) ? xc + omega * (b[p] - ax) / diag : xc;
+            v = xc + omega * (b[p] - ax) * row[(size_t)27 * e.pitch];
         else
             v = (b ? b[p] : T(0)) - ax;
     }
-    store_node(out, g, nd.i, nd.j, nd.k, v);
+    store_node(out, g, i, j, k, v);
 }
 
 __global__ void __launch_bounds__(128) k_eb_rhs(NodalGeom g, EbNodal e, RhsArgs a, double* __restrict__ rhs)
@@ -169,14 +188,12 @@ __global__ void k_eb_pack(gbp_array4 in, int c, int n0, int n1, int n2, double* 
 }
 
 __global__ void k_eb_sigma(long long count, const double* __restrict__ s, const double* __restrict__ kap,
-                           const unsigned char* __restrict__ reg, double* __restrict__ st64, float* __restrict__ st32,
-                           double* __restrict__ s64, float* __restrict__ s32, double* __restrict__ sk)
+                           const unsigned char* __restrict__ reg, double* __restrict__ st64, double* __restrict__ s64, float* __restrict__ s32, double* __restrict__ sk)
 {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= count) return;
     const double v = s[t];
     st64[t] = v;
-    st32[t] = (float)v;
     const double r = reg[t] ? v : 0.0;
     s64[t] = r;
     s32[t] = (float)r;
@@ -224,8 +241,8 @@ void eb_sigma(const NodalGeom& g, const EbNodal& e, const double* s_in, double* 
               cudaStream_t st)
 {
     k_eb_sigma<<<(unsigned)((g.count + 255) / 256), 256, 0, st>>>(g.count, s_in, e.kap, e.reg,
-                                                                  const_cast<double*>(e.sig64),
-                                                                  const_cast<float*>(e.sig32), s64, s32, sk);
+                                                                  const_cast<double*>(e.sig64), s64, s32, sk);
+    if (e.nnodes > 0) k_eb_rows<<<dim3((unsigned)((e.nnodes + 127) / 128), 27), 128, 0, st>>>(g, e);
 }
 
 }  // namespace gbp

@@ -33,7 +33,11 @@ struct EbNodal {
     const EbNodeCell* cells;
     int nnodes, ncells;
     const double* sig64;       // true sigma of the level (padded cells, aliases)
-    const float* sig32;
+    // the EB nodes' rows: entry q at [q * pitch + node] (node + offset q % 3 - 1, q / 3 % 3 - 1, q / 9 - 1), 1 / diagonal
+    // (0 where there is none) at q = 27
+    double* row64;
+    float* row32;
+    int pitch;
     const double* kap;         // volume fraction (padded cells, aliases)
     const unsigned char* reg;  // 1 on regular cells (volume fraction 1)
     // EB inflow: F_c N_b(x_b) for corner b of cut cell c (8 per cell), F_c the EB inflow velocity's flux
@@ -53,7 +57,7 @@ void eb_rhs(const NodalGeom& g, const EbNodal& e, const RhsArgs& a, double* rhs,
 void eb_inflow_shares(const NodalGeom& g, const EbNodal& e, const gbp_array4& eb_vel, const gbp_array4& dap,
                       const gbp_array4& bcent, double* out, cudaStream_t st);
 void eb_correct(const NodalGeom& g, const EbNodal& e, const CorrArgs& a, const double* phi, cudaStream_t st);
-// s_in (the level's sigma as set) -> true sigma (e.sig64 / sig32), s64 / s32 = sigma on regular cells,
+// s_in (the level's sigma as set) -> true sigma (e.sig64) and the EB nodes' rows, s64 / s32 = sigma on regular cells,
 // sk = sigma x volume fraction (the coarsening source)
 void eb_sigma(const NodalGeom& g, const EbNodal& e, const double* s_in, double* s64, float* s32, double* sk,
               cudaStream_t st);

@@ -1336,9 +1336,11 @@ int NodalSolver::set_eb(const gbp_array4* M)
     add(g.count, 1);
     for (size_t l = 0; l < L.size(); ++l) add(L[l].g.count, 1);
     add(g.count, 8);
-    add(g.count, 4);
     add(g.count, 8);
     add(8 * cells.size() + 8, 8);
+    const size_t pitch = (nodes.size() + 31) & ~size_t(31);
+    add(28 * pitch + 1, 8);
+    add(28 * pitch + 1, 4);
     need += 4096;
     rc = eb.pool.reserve(need);
     if (rc) return rc;
@@ -1348,9 +1350,11 @@ int NodalSolver::set_eb(const gbp_array4* M)
     unsigned char* dr = eb.pool.take<unsigned char>(g.count);
     for (size_t l = 0; l < L.size(); ++l) eb.active8[l] = eb.pool.take<unsigned char>(L[l].g.count);
     double* s64t = eb.pool.take<double>(g.count);
-    float* s32t = eb.pool.take<float>(g.count);
     eb.ivol = eb.pool.take<double>(g.count);
     eb.inflow_buf = eb.pool.take<double>(8 * cells.size() + 8);
+    eb.e.row64 = eb.pool.take<double>(28 * pitch + 1);
+    eb.e.row32 = eb.pool.take<float>(28 * pitch + 1);
+    eb.e.pitch = (int)pitch;
     if (!nodes.empty())
         GBP_CUDA(cudaMemcpyAsync(dn, nodes.data(), sizeof(EbNodeEntry) * nodes.size(), cudaMemcpyHostToDevice, st));
     if (!cells.empty())
@@ -1361,14 +1365,14 @@ int NodalSolver::set_eb(const gbp_array4* M)
         GBP_CUDA(cudaMemcpyAsync(eb.active8[l], act_lv[l].data(), L[l].g.count, cudaMemcpyHostToDevice, st));
     GBP_CUDA(cudaMemcpyAsync(eb.ivol, ivol_p.data(), sizeof(double) * g.count, cudaMemcpyHostToDevice, st));
     GBP_CUDA(cudaMemsetAsync(s64t, 0, sizeof(double) * g.count, st));
-    GBP_CUDA(cudaMemsetAsync(s32t, 0, sizeof(float) * g.count, st));
+    GBP_CUDA(cudaMemsetAsync(eb.e.row64, 0, sizeof(double) * 28 * pitch, st));
+    GBP_CUDA(cudaMemsetAsync(eb.e.row32, 0, sizeof(float) * 28 * pitch, st));
     GBP_CUDA(cudaStreamSynchronize(st));  // the host vectors go out of scope
     eb.e.nodes = dn;
     eb.e.cells = dc;
     eb.e.nnodes = (int)nodes.size();
     eb.e.ncells = (int)cells.size();
     eb.e.sig64 = s64t;
-    eb.e.sig32 = s32t;
     eb.e.kap = dk;
     eb.e.reg = dr;
     eb.has_inactive = inactive;
