@@ -480,20 +480,23 @@ __global__ void k_amr_zero_nondof_fine(NodalGeom gf, const unsigned char* __rest
 }
 
 // composite max norm |v| / V over the unknowns of both levels (per-level node volumes)
+// (these and the sums walk z: a block per few nodes spent its time on the block reduction, 326 us for 5 10^7 nodes against
+// 146, and 1300 against 217 us for the sums)
 __global__ void k_amr_norm_c(NodalGeom gc, const unsigned char* __restrict__ ccls, const double* __restrict__ v,
                              unsigned long long* norm)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z * blockDim.z + threadIdx.z;
     unsigned long long key = 0;  // as in k_amr_norm_f
-    if (i < gc.nu[0] && j < gc.nu[1] && k < gc.nu[2]) {
+    for (int k = blockIdx.z * blockDim.z + threadIdx.z; i < gc.nu[0] && j < gc.nu[1] && k < gc.nu[2];
+         k += gridDim.z * blockDim.z) {
         const long long p = pidx(gc.sy, gc.sz, i, j, k);
         const unsigned char c = ccls[p];
         if (c == C_DOF || c == C_IFACE) {
             const int e = (!gc.per[0] && (i == 0 || i == gc.n[0])) + (!gc.per[1] && (j == 0 || j == gc.n[1])) +
                           (!gc.per[2] && (k == 0 || k == gc.n[2]));
-            key = e == 0 ? abs_key(v[p]) : abs_key(v[p] * (double)(1 << e));
+            const unsigned long long kv = e == 0 ? abs_key(v[p]) : abs_key(v[p] * (double)(1 << e));
+            key = kv > key ? kv : key;
         }
     }
     key = block_max_key(key);
@@ -504,16 +507,17 @@ __global__ void k_amr_norm_f(NodalGeom gf, const unsigned char* __restrict__ fcl
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z * blockDim.z + threadIdx.z;
     // max |v| / node volume as an integer key of |v| 2^e (volume V / 2^e on e non-periodic boundary
     // planes): no FP64 instruction on interior nodes, one multiplication by 1/V per block
     unsigned long long key = 0;
-    if (i < gf.nu[0] && j < gf.nu[1] && k < gf.nu[2]) {
+    for (int k = blockIdx.z * blockDim.z + threadIdx.z; i < gf.nu[0] && j < gf.nu[1] && k < gf.nu[2];
+         k += gridDim.z * blockDim.z) {
         const long long p = pidx(gf.sy, gf.sz, i, j, k);
         if (fcls[p] == F_DOF) {
             const int e = (!gf.per[0] && (i == 0 || i == gf.n[0])) + (!gf.per[1] && (j == 0 || j == gf.n[1])) +
                           (!gf.per[2] && (k == 0 || k == gf.n[2]));
-            key = e == 0 ? abs_key(v[p]) : abs_key(v[p] * (double)(1 << e));
+            const unsigned long long kv = e == 0 ? abs_key(v[p]) : abs_key(v[p] * (double)(1 << e));
+            key = kv > key ? kv : key;
         }
     }
     key = block_max_key(key);
@@ -627,73 +631,94 @@ __global__ void k_amr_inject(NodalGeom gc, NodalGeom gf, const unsigned char* __
     store_node(pc, gc, i, j, k, pf[pidx(gf.sy, gf.sz, m[0], m[1], m[2])]);
 }
 
-// sums over the unknowns of v and of the node volumes (consistency of a singular system)
+// sums over the unknowns of v and of the node volumes (consistency of a singular system); the volumes V / 2^e as whole
+// eighths
+__device__ __forceinline__ int half_sides(const NodalGeom& g, int i, int j, int k)
+{
+    return (!g.per[0] && (i == 0 || i == g.n[0])) + (!g.per[1] && (j == 0 || j == g.n[1])) +
+           (!g.per[2] && (k == 0 || k == g.n[2]));
+}
+__device__ __forceinline__ void add_sums(const NodalGeom& g, double a, int eighths, double* part)
+{
+    a = block_sum_all(a);
+    const double b = block_sum_all((double)eighths);
+    if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
+        atomicAdd(part, a);
+        atomicAdd(part + 1, b * (0.125 * g.vol));
+    }
+}
 __global__ void k_amr_sums_c(NodalGeom gc, const unsigned char* __restrict__ ccls, const double* __restrict__ v,
                              double* __restrict__ part)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z * blockDim.z + threadIdx.z;
-    double a = 0.0, b = 0.0;
-    if (i < gc.nu[0] && j < gc.nu[1] && k < gc.nu[2]) {
+    double a = 0.0;
+    int b = 0;
+    for (int k = blockIdx.z * blockDim.z + threadIdx.z; i < gc.nu[0] && j < gc.nu[1] && k < gc.nu[2];
+         k += gridDim.z * blockDim.z) {
         const long long p = pidx(gc.sy, gc.sz, i, j, k);
         const unsigned char c = ccls[p];
         if (c == C_DOF || c == C_IFACE) {
-            a = v[p];
-            b = node_volume(gc, i, j, k);
+            a += v[p];
+            b += 8 >> half_sides(gc, i, j, k);
         }
     }
-    a = block_sum_all(a);
-    b = block_sum_all(b);
-    if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
-        const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-        atomicAdd(part, a);
-        atomicAdd(part + 1, b);
-        (void)bid;
-    }
+    add_sums(gc, a, b, part);
 }
 __global__ void k_amr_sums_f(NodalGeom gf, const unsigned char* __restrict__ fcls, const double* __restrict__ v,
                              double* __restrict__ part)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z * blockDim.z + threadIdx.z;
-    double a = 0.0, b = 0.0;
-    if (i < gf.nu[0] && j < gf.nu[1] && k < gf.nu[2]) {
+    double a = 0.0;
+    int b = 0;
+    for (int k = blockIdx.z * blockDim.z + threadIdx.z; i < gf.nu[0] && j < gf.nu[1] && k < gf.nu[2];
+         k += gridDim.z * blockDim.z) {
         const long long p = pidx(gf.sy, gf.sz, i, j, k);
         if (fcls[p] == F_DOF) {
-            a = v[p];
-            b = node_volume(gf, i, j, k);
+            a += v[p];
+            b += 8 >> half_sides(gf, i, j, k);
         }
     }
-    a = block_sum_all(a);
-    b = block_sum_all(b);
-    if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
-        atomicAdd(part, a);
-        atomicAdd(part + 1, b);
-    }
+    add_sums(gf, a, b, part);
 }
-// v -= V_node * (sum v / sum V) on the unknowns
+// v -= V_node * (sum v / sum V) on the unknowns; the quotient once per block (an FP64 division per node bound it: 770 us
+// for 5 10^7 nodes against 214)
+__device__ __forceinline__ double mean_shift(const NodalGeom& g, const double* part)
+{
+    __shared__ double c;
+    if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) c = g.vol * (part[0] / part[1]);
+    __syncthreads();
+    return c;
+}
 __global__ void k_amr_consistent_c(NodalGeom gc, const unsigned char* __restrict__ ccls, const double* __restrict__ part,
                                    double* __restrict__ v)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z * blockDim.z + threadIdx.z;
-    if (i >= gc.nu[0] || j >= gc.nu[1] || k >= gc.nu[2]) return;
-    const long long p = pidx(gc.sy, gc.sz, i, j, k);
-    const unsigned char c = ccls[p];
-    if (c == C_DOF || c == C_IFACE) v[p] -= node_volume(gc, i, j, k) * (part[0] / part[1]);
+    const double m = mean_shift(gc, part);
+    for (int k = blockIdx.z * blockDim.z + threadIdx.z; i < gc.nu[0] && j < gc.nu[1] && k < gc.nu[2];
+         k += gridDim.z * blockDim.z) {
+        const long long p = pidx(gc.sy, gc.sz, i, j, k);
+        const unsigned char c = ccls[p];
+        if (c != C_DOF && c != C_IFACE) continue;
+        const int e = half_sides(gc, i, j, k);
+        v[p] -= e == 0 ? m : m / (double)(1 << e);
+    }
 }
 __global__ void k_amr_consistent_f(NodalGeom gf, const unsigned char* __restrict__ fcls, const double* __restrict__ part,
                                    double* __restrict__ v)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z * blockDim.z + threadIdx.z;
-    if (i >= gf.nu[0] || j >= gf.nu[1] || k >= gf.nu[2]) return;
-    const long long p = pidx(gf.sy, gf.sz, i, j, k);
-    if (fcls[p] == F_DOF) v[p] -= node_volume(gf, i, j, k) * (part[0] / part[1]);
+    const double m = mean_shift(gf, part);
+    for (int k = blockIdx.z * blockDim.z + threadIdx.z; i < gf.nu[0] && j < gf.nu[1] && k < gf.nu[2];
+         k += gridDim.z * blockDim.z) {
+        const long long p = pidx(gf.sy, gf.sz, i, j, k);
+        if (fcls[p] != F_DOF) continue;
+        const int e = half_sides(gf, i, j, k);
+        v[p] -= e == 0 ? m : m / (double)(1 << e);
+    }
 }
 // fine phi -= c on the region's nodes (the gauge shift of the coarse level)
 __global__ void k_amr_shift_f(NodalGeom gf, const unsigned char* __restrict__ fcls, const double* __restrict__ scal,
@@ -720,6 +745,8 @@ __global__ void k_amr_fine_nodes(NodalGeom gf, const double* __restrict__ pf, do
 inline dim3 g3(int a, int b, int c) { return dim3((a + 31) / 32, (b + 3) / 4, (c + 1) / 2); }
 const dim3 kB3(32, 4, 2);
 inline dim3 gnodes(const NodalGeom& g) { return g3(g.nu[0], g.nu[1], g.nu[2]); }
+// for kernels that walk z
+inline dim3 gwalk(const NodalGeom& g) { return g3(g.nu[0], g.nu[1], std::min(g.nu[2], 16)); }
 inline double bits_to_double(unsigned long long b)
 {
     double v;
@@ -729,11 +756,19 @@ inline double bits_to_double(unsigned long long b)
 
 }  // namespace
 
+void CompositeNodal::drop_steps()
+{
+    for (auto& g : gsteps) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+}
+
 CompositeNodal::~CompositeNodal()
 {
     if (iface) cudaFree(iface);
     if (st) cudaStreamSynchronize(st);
-    if (gstep) cudaGraphExecDestroy(gstep);
+    drop_steps();
     if (capst) cudaStreamDestroy(capst);
     if (hnorm) cudaFreeHost(hnorm);
     if (dboxes) cudaFree(dboxes);
@@ -752,8 +787,7 @@ int CompositeNodal::set_options(const gbp_options& o)
     int rc = crs.set_options(o);
     if (!rc) rc = fin.set_options(o);
     if (!rc) opt = o;
-    if (gstep) cudaGraphExecDestroy(gstep);  // the step's kernels depend on the options
-    gstep = nullptr;
+    drop_steps();  // the step's kernels depend on the options
     return rc;
 }
 
@@ -1044,8 +1078,8 @@ void CompositeNodal::composite_residual(const double* bc, const double* bf, unsi
     resid_c(phi_c, bc, r_c);
     sync(r_c, r_f);
     if (norm) {
-        k_amr_norm_c<<<gnodes(gc), kB3, 0, st>>>(gc, ccls, r_c, norm);
-        k_amr_norm_f<<<gnodes(gf), kB3, 0, st>>>(gf, fcls, r_f, norm);
+        k_amr_norm_c<<<gwalk(gc), kB3, 0, st>>>(gc, ccls, r_c, norm);
+        k_amr_norm_f<<<gwalk(gf), kB3, 0, st>>>(gf, fcls, r_f, norm);
     }
 }
 
@@ -1130,10 +1164,10 @@ void CompositeNodal::resid32(const NodalGeom& g, const float* s, const float* x,
 }
 
 // One refinement step of the mixed form: the FP64 composite residual (r_c, r_f), scaled into FP32, is the
-// right-hand side of the correction equation A e = r, which kInner two-level steps solve in FP32
+// right-hand side of the correction equation A e = r, which `inner` two-level steps solve in FP32
 // arithmetic (the same steps as issue_step on e, with FP32 composite residuals between them); then
 // phi += e / scale on both levels in FP64 and the FP64 composite residual with its norm.
-void CompositeNodal::issue_outer32(double scale32)
+void CompositeNodal::issue_outer32(double scale32, int inner)
 {
     const unsigned ncb = (unsigned)((gc.count + kT - 1) / kT), nfb_ = (unsigned)((gf.count + kT - 1) / kT);
     k_amr_to32<<<ncb, kT, 0, st>>>(gc.count, r_c, scale32, bc32);
@@ -1147,7 +1181,7 @@ void CompositeNodal::issue_outer32(double scale32)
         resid32(gc, scm32, ec32, bc32, rc32);
         k_amr_sync<<<gnodes(gc), kB3, 0, st>>>(gc, gf, ccls, fcls, off[0], off[1], off[2], (const float*)rm32, rc32);
     };
-    for (int q = 0; q < kInner; ++q) {
+    for (int q = 0; q < inner; ++q) {
         const float* rc = q == 0 ? bc32 : rc32;
         const float* rf = q == 0 ? bf32 : rf32;
         const int o0 = off[0] / 2, o1 = off[1] / 2, o2 = off[2] / 2;
@@ -1171,18 +1205,21 @@ void CompositeNodal::issue_outer32(double scale32)
             if (niface > 0)
                 k_amr_fill_fine_list<<<(unsigned)((niface + kT - 1) / kT), kT, 0, st>>>(
                     gc, gf, off[0], off[1], off[2], (const int4*)iface, niface, (const float*)ec32, ef32);
-            resid32(gf, fin.sigma32(), ef32, bf32, rf32);  // the fine unknowns only (the mask holds the rest)
         } else {
             k_amr_fill_fine<<<gnodes(gf), kB3, 0, st>>>(gc, gf, fcls, off[0], off[1], off[2], (const float*)ec32,
                                                         ef32);
-            resid32(gf_nomask, fin.sigma32(), ef32, bf32, rf32);
         }
-        if (kFineSweeps > 0)
-            fin.smooth32(rf32, kFineSweeps, st);
-        else
-            fin.apply_vcycles32(rf32, 1, st);
-        k_amr_add32<<<nfb_, kT, 0, st>>>(gf.count, fin.correction32(), ef32);
-        if (q + 1 < kInner) {
+        // the fine sweeps on e_f itself, which the mask holds on the interface: sweeps from zero on its residual and
+        // their sum are the same step with three passes more (residual 196, first sweep 279, sum 152 of 780 us)
+        if (kFineSweeps == 0 || !fin.sweep32_in_place(bf32, ef32, kFineSweeps, st)) {
+            resid32(xfer1 ? gf : gf_nomask, fin.sigma32(), ef32, bf32, rf32);
+            if (kFineSweeps > 0)
+                fin.smooth32(rf32, kFineSweeps, st);
+            else
+                fin.apply_vcycles32(rf32, 1, st);
+            k_amr_add32<<<nfb_, kT, 0, st>>>(gf.count, fin.correction32(), ef32);
+        }
+        if (q + 1 < inner) {
             // FP32 composite residual of e (the interface values of e_f are those of e_c already)
             if (xfer1) {
                 // the fine unknowns' residuals, and the interface nodes' into rm32 for the coarse interface
@@ -1310,14 +1347,14 @@ int CompositeNodal::project(const AmrFields& f, gbp_stats* stats)
     k_amr_zero_nondof_fine<<<gnodes(gf), kB3, 0, st>>>(gf, fcls, b_f);
     if (singular) {
         GBP_CUDA(cudaMemsetAsync(part, 0, 2 * sizeof(double), st));
-        k_amr_sums_c<<<gnodes(gc), kB3, 0, st>>>(gc, ccls, b_c, part);
-        k_amr_sums_f<<<gnodes(gf), kB3, 0, st>>>(gf, fcls, b_f, part);
-        k_amr_consistent_c<<<gnodes(gc), kB3, 0, st>>>(gc, ccls, part, b_c);
-        k_amr_consistent_f<<<gnodes(gf), kB3, 0, st>>>(gf, fcls, part, b_f);
+        k_amr_sums_c<<<gwalk(gc), kB3, 0, st>>>(gc, ccls, b_c, part);
+        k_amr_sums_f<<<gwalk(gf), kB3, 0, st>>>(gf, fcls, b_f, part);
+        k_amr_consistent_c<<<gwalk(gc), kB3, 0, st>>>(gc, ccls, part, b_c);
+        k_amr_consistent_f<<<gwalk(gf), kB3, 0, st>>>(gf, fcls, part, b_f);
     }
     GBP_CUDA(cudaMemsetAsync(dnorm, 0, 2 * sizeof(unsigned long long), st));
-    k_amr_norm_c<<<gnodes(gc), kB3, 0, st>>>(gc, ccls, b_c, dnorm);
-    k_amr_norm_f<<<gnodes(gf), kB3, 0, st>>>(gf, fcls, b_f, dnorm);
+    k_amr_norm_c<<<gwalk(gc), kB3, 0, st>>>(gc, ccls, b_c, dnorm);
+    k_amr_norm_f<<<gwalk(gf), kB3, 0, st>>>(gf, fcls, b_f, dnorm);
     // initial_guess = previous: both levels start from the last converged composite phi of this box layout
     // (phi_c / phi_f keep it between calls); the tolerance refers to that start's residual, as in the
     // single-level solve
@@ -1347,9 +1384,10 @@ int CompositeNodal::project(const AmrFields& f, gbp_stats* stats)
     int it = 0, status = GBP_OK;
     const double r0 = rn;
     const bool mixed = opt.precision == GBP_PREC_MIXED;
+    int inner = mixed ? kInner : 1, steps = 0;
     auto issue = [&](double sc) {
         if (mixed)
-            issue_outer32(sc);
+            issue_outer32(sc, inner);
         else
             issue_step(sc);
     };
@@ -1359,11 +1397,11 @@ int CompositeNodal::project(const AmrFields& f, gbp_stats* stats)
             set_error("amr solve: maxiter reached before the tolerance");
             break;
         }
-        if (opt.use_graphs && (!gstep || gstep_scale != scale32 || gstep_prec != opt.precision)) {
+        if (gstep_scale != scale32 || gstep_prec != opt.precision) drop_steps();
+        cudaGraphExec_t& gstep = gsteps[inner];
+        if (opt.use_graphs && !gstep) {
             // capture the step once on a stream of its own (the caller's may be the legacy default
             // stream), with every kernel of the step issued there
-            if (gstep) cudaGraphExecDestroy(gstep);
-            gstep = nullptr;
             if (!capst) GBP_CUDA(cudaStreamCreateWithFlags(&capst, cudaStreamNonBlocking));
             cudaStream_t keep = st;
             st = capst;
@@ -1390,8 +1428,16 @@ int CompositeNodal::project(const AmrFields& f, gbp_stats* stats)
         GBP_CUDA(cudaStreamSynchronize(st));
         GBP_CUDA(cudaGetLastError());
         if ((rc = sweep_status())) return rc;
+        const double before = rn;
         rn = bits_to_double(hnorm[1]);
         ++it;
+        steps += inner;
+        if (mixed && rn > target && rn < before && target > 0.0) {
+            // one refinement step more costs an FP64 composite residual, one of kInner steps too many 2 ms each at 256^3
+            const double rate = log(rn / before) / inner, need = ceil(log(0.8 * target / rn) / rate);
+            inner = (int)std::min<double>(kMostInner, std::max(1.0, need));
+            if (need > kMostInner) inner = kInner;
+        }
         if (opt.verbose > 1) fprintf(stderr, "gbp amr: iter %d rel resid %.3e\n", it, bnorm > 0 ? rn / bnorm : rn);
         if (!isfinite(rn)) {
             status = GBP_NAN;
@@ -1459,7 +1505,7 @@ int CompositeNodal::project(const AmrFields& f, gbp_stats* stats)
         stats->prev_rel_resid = from_prev ? (bnorm > 0 ? r0 / bnorm : r0) : 0.0;
         // V-cycles: the coarse one of every two-level step, and the fine one where the fine correction is a
         // V-cycle (the plain form; the mixed form with kFineSweeps = 0)
-        stats->vcycles = it * (mixed ? kInner * (kFineSweeps > 0 ? 1 : 2) : 2);
+        stats->vcycles = steps * (mixed && kFineSweeps > 0 ? 1 : 2);
         stats->num_levels = 2;
         stats->rhs_norm = bnorm;
         stats->initial_rel_resid = bnorm > 0 ? r0 / bnorm : r0;

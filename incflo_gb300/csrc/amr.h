@@ -95,15 +95,15 @@ private:
     // and its norm read-back) captured as a CUDA graph and replayed; recaptured when the FP32 scale or
     // the options change
     void issue_step(double scale32);
-    // the mixed form's step: kInner FP32 two-level steps on the correction equation per FP64 composite
-    // residual
-    void issue_outer32(double scale32);
+    // the mixed form's step: FP32 two-level steps on the correction equation per FP64 composite residual: kInner in the
+    // first, then as many as the contraction so far asks for (at most kMostInner; a step may reduce the residual by 1e-6)
+    void issue_outer32(double scale32, int inner);
     template <typename T>
     void restrict_to_coarse(const T* rc, const T* rf, T* out);
 #ifndef GBP_AMR_INNER
 #define GBP_AMR_INNER 8
 #endif
-    static constexpr int kInner = GBP_AMR_INNER;
+    static constexpr int kInner = GBP_AMR_INNER, kMostInner = kInner + 2;
 #ifndef GBP_AMR_FINE_SWEEPS
 #define GBP_AMR_FINE_SWEEPS 2
 #endif
@@ -129,7 +129,8 @@ private:
     int launch_rc = 0;         // first launch error of a step (tensor-map set-up)
     int sweep_status();
     cudaStream_t capst = nullptr;
-    cudaGraphExec_t gstep = nullptr;
+    cudaGraphExec_t gsteps[kMostInner + 1] = {};  // by the number of inner steps
+    void drop_steps();
     double gstep_scale = 0.0;
     int gstep_prec = -1;
 };

@@ -219,40 +219,62 @@ __global__ void __launch_bounds__(256) k_prolong_block(NodalGeom gf, NodalGeom g
     const bool seam = (gf.per[0] && (2 * I <= 1 || 2 * I + 1 >= gf.n[0] - 1)) ||
                       (gf.per[1] && (2 * J <= 1 || 2 * J + 1 >= gf.n[1] - 1)) ||
                       (gf.per[2] && (2 * K <= 1 || 2 * K + 1 >= gf.n[2] - 1));
+    using V = typename Vec2<T>::type;
+    // coarse values interpolated to (., 2J+oy, 2K+oz) at x = 2I, 2I+1
+    auto at = [&](int oy, int oz, T& a0, T& a1) {
+        T e0 = c[0][0][0], e1 = c[0][0][1];
+        if (oy) {
+            e0 = T(0.5) * (e0 + c[0][1][0]);
+            e1 = T(0.5) * (e1 + c[0][1][1]);
+        }
+        if (oz) {
+            T f0 = c[1][0][0], f1 = c[1][0][1];
+            if (oy) {
+                f0 = T(0.5) * (f0 + c[1][1][0]);
+                f1 = T(0.5) * (f1 + c[1][1][1]);
+            }
+            e0 = T(0.5) * (e0 + f0);
+            e1 = T(0.5) * (e1 + f1);
+        }
+        a0 = e0;
+        a1 = T(0.5) * (e0 + e1);
+    };
+    const long long p0 = pidx(gf.sy, gf.sz, 2 * I, 2 * J, 2 * K);
+    if (!seam && vx && vy && vz) {
+        // all loads before the first store: one after another the four round trips were most of the kernel's time (277 us
+        // for 5 10^7 masked fine nodes, 127 us at once)
+        V v[4];
+        uchar2 m[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const long long p = p0 + (q & 1) * gf.sy + (q >> 1) * gf.sz;
+            v[q] = *reinterpret_cast<const V*>(xf + p);
+            m[q] = gf.mask ? *reinterpret_cast<const uchar2*>(gf.mask + p) : make_uchar2(1, 1);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            T a0, a1;
+            at(q & 1, q >> 1, a0, a1);
+            v[q].x += m[q].x ? a0 : T(0);
+            v[q].y += m[q].y ? a1 : T(0);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            *reinterpret_cast<V*>(xf + p0 + (q & 1) * gf.sy + (q >> 1) * gf.sz) = v[q];
+        return;
+    }
 #pragma unroll
     for (int oz = 0; oz < 2; ++oz) {
         if (oz && !vz) break;
 #pragma unroll
         for (int oy = 0; oy < 2; ++oy) {
             if (oy && !vy) break;
-            // coarse values interpolated to (., 2J+oy, 2K+oz) at x = I and I+1
-            T e0 = c[0][0][0], e1 = c[0][0][1];
-            if (oy) {
-                e0 = T(0.5) * (e0 + c[0][1][0]);
-                e1 = T(0.5) * (e1 + c[0][1][1]);
-            }
-            if (oz) {
-                T f0 = c[1][0][0], f1 = c[1][0][1];
-                if (oy) {
-                    f0 = T(0.5) * (f0 + c[1][1][0]);
-                    f1 = T(0.5) * (f1 + c[1][1][1]);
-                }
-                e0 = T(0.5) * (e0 + f0);
-                e1 = T(0.5) * (e1 + f1);
-            }
-            const T a0 = e0, a1 = T(0.5) * (e0 + e1);  // fine x = 2I, 2I+1
+            T a0, a1;
+            at(oy, oz, a0, a1);
             const int i = 2 * I, j = 2 * J + oy, k = 2 * K + oz;
-            const long long p = pidx(gf.sy, gf.sz, i, j, k);
-            if (!seam && vx && !gf.mask) {
-                using V = typename Vec2<T>::type;
-                V v = *reinterpret_cast<const V*>(xf + p);
-                v.x += a0;
-                v.y += a1;
-                *reinterpret_cast<V*>(xf + p) = v;
-            } else {
-                if (!(gf.mask && !gf.mask[p])) store_node(xf, gf, i, j, k, xf[p] + a0);
-                if (vx && !(gf.mask && !gf.mask[p + 1])) store_node(xf, gf, i + 1, j, k, xf[p + 1] + a1);
-            }
+            const long long p = p0 + oy * gf.sy + oz * gf.sz;
+            if (!(gf.mask && !gf.mask[p])) store_node(xf, gf, i, j, k, xf[p] + a0);
+            if (vx && !(gf.mask && !gf.mask[p + 1])) store_node(xf, gf, i + 1, j, k, xf[p + 1] + a1);
         }
     }
 }

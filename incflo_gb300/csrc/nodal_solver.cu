@@ -811,6 +811,20 @@ void NodalSolver::smooth32(const float* b32, int nu, cudaStream_t s)
     cap_or_st = st;
 }
 
+bool NodalSolver::sweep32_in_place(const float* b32, float* x, int nu, cudaStream_t s)
+{
+    const NodalLevel& l0 = L[0];
+    if (!use_tma || !vsweep32_supported(l0.g) || (nu & 1)) return false;
+    float* in = x;
+    float* out = l0.x32;
+    for (int q = 0; q < nu; ++q) {
+        const int rc = vsweep32(l0.g, 0, l0.s32, in, b32, out, (float)wpre[q % kSweepWeights], derr, s, true);
+        if (rc && !launch_rc) launch_rc = rc;
+        std::swap(in, out);
+    }
+    return true;
+}
+
 int NodalSolver::take_sweep_status(cudaStream_t s)
 {
     if (launch_rc) {

@@ -130,6 +130,9 @@ public:
     // nu FP32 Jacobi sweeps from zero on level 0 only (b32 scaled as for apply_vcycles32); the correction
     // stays in correction32()
     void smooth32(const float* b32, int nu, cudaStream_t s);
+    // the same nu sweeps on x itself (rows of the level's layout, values of the held nodes kept) with the right-hand side
+    // b32: x + the correction of its residual, without forming either. false: not on this level, nothing done
+    bool sweep32_in_place(const float* b32, float* x, int nu, cudaStream_t s);
     // For work issued through apply_vcycles / apply_vcycles32: GBP_OK, the first launch error (cleared), or
     // GBP_TIMEOUT when a bounded device wait of a level sweep ran out (the device error word is read and
     // cleared; synchronises s).

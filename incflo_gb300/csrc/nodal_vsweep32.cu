@@ -99,6 +99,7 @@ struct VsArgs {
     NodalGeom gc;   // the coarse level (restriction / prolongation modes)
     float* out;     // fine output (modes 0, 1, 3) or coarse right-hand side (mode 2)
     float k0, k3, omega;
+    bool hold;      // mode 0 with an overset mask: masked nodes keep their value (false: 0)
     int kchunk;     // node planes per CTA (even in mode 2)
     int rowlen;     // padded fine row length (floats)
     int crowlen;    // padded coarse row length (floats)
@@ -514,7 +515,8 @@ __global__ void __launch_bounds__(TXM * VsShape<MODE, TY, RPT>::TTR,
                         val = bb[q] - ax;
                     else
                         val = fmaf(a.omega * (bb[q] - ax), rcp_approx(a.k0 * (ss[r][q] + sgl)), cA);
-                    v[r][q] = (dk || (((dmask | mk) >> (r * 4 + q)) & 1u)) ? 0.f : val;
+                    const float held = MODE == 0 && a.hold ? cA : 0.f;
+                    v[r][q] = (dk || ((dmask >> (r * 4 + q)) & 1u)) ? 0.f : (((mk >> (r * 4 + q)) & 1u) ? held : val);
                 }
                 // node plane P (registers Bn) gets its lower half
                 acc[r][q] = fmaf(-2.f * (cB - cA), sgl, G) + xb;
@@ -635,7 +637,7 @@ int make_map4(const void* base, long long sy, long long sz, long long count, int
 
 template <int MODE, int TY, int TXM>
 int launch(const NodalGeom& g, const NodalGeom* gc, const float* s, const float* x, const float* b,
-           const float* e, float* out, float omega, unsigned* err, cudaStream_t st)
+           const float* e, float* out, float omega, unsigned* err, cudaStream_t st, bool hold = false)
 {
     constexpr int RPT = GBP_VS_RPT;
     using Sh = VsShape<MODE, TY, RPT>;
@@ -647,6 +649,7 @@ int launch(const NodalGeom& g, const NodalGeom* gc, const float* s, const float*
     a.k0 = (float)g.K[0];
     a.k3 = (float)g.K[3];
     a.omega = omega;
+    a.hold = hold;
     a.rowlen = (int)g.sy;
     a.crowlen = gc ? (int)gc->sy : 4;
     a.rstride = 4 * TX + 8;
@@ -719,18 +722,19 @@ bool vsweep32_transfer_supported(const NodalGeom& g, const NodalGeom& gc)
 // rows per CTA by the row width: 8 (<= 128 nodes), GBP_VS_TY_256 (<= 256), GBP_VS_TY_512 (<= 512)
 template <int MODE>
 static int launch_any(const NodalGeom& g, const NodalGeom* gc, const float* s, const float* x, const float* b,
-                      const float* e, float* out, float omega, unsigned* err, cudaStream_t st)
+                      const float* e, float* out, float omega, unsigned* err, cudaStream_t st,
+               bool hold = false)
 {
     const int TX = (g.nu[0] + 3) / 4;
-    if (TX <= 32) return launch<MODE, 8, 32>(g, gc, s, x, b, e, out, omega, err, st);
-    if (TX <= 64) return launch<MODE, GBP_VS_TY_256, 64>(g, gc, s, x, b, e, out, omega, err, st);
-    return launch<MODE, GBP_VS_TY_512, 128>(g, gc, s, x, b, e, out, omega, err, st);
+    if (TX <= 32) return launch<MODE, 8, 32>(g, gc, s, x, b, e, out, omega, err, st, hold);
+    if (TX <= 64) return launch<MODE, GBP_VS_TY_256, 64>(g, gc, s, x, b, e, out, omega, err, st, hold);
+    return launch<MODE, GBP_VS_TY_512, 128>(g, gc, s, x, b, e, out, omega, err, st, hold);
 }
 
 int vsweep32(const NodalGeom& g, int mode, const float* s, const float* x, const float* b, float* out, float omega,
-             unsigned* err, cudaStream_t st)
+             unsigned* err, cudaStream_t st, bool hold)
 {
-    return mode == 0 ? launch_any<0>(g, nullptr, s, x, b, nullptr, out, omega, err, st)
+    return mode == 0 ? launch_any<0>(g, nullptr, s, x, b, nullptr, out, omega, err, st, hold)
                      : launch_any<1>(g, nullptr, s, x, b, nullptr, out, omega, err, st);
 }
 
