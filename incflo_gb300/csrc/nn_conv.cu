@@ -1,14 +1,20 @@
 // BF16 3x3x3 convolutions of the warm-start U-Net as implicit GEMMs on tcgen05.
 //
-// Forward / data-gradient kernel (k_conv): a persistent CTA walks output tiles of 128 consecutive
-// rows of the zero-haloed channels-last grid. For each K step (input tensor, 16..64-channel chunk,
-// tap) warp 0 issues two TMA loads into a ring stage: the 128-row activation box at row p0 + off(tap)
-// (a K-major, swizzled A operand; rows outside the array read as zeros) and the N-row weight box of
-// that tap (the B operand). Warp 1 issues the MMAs (M = 128, N = output channels, K = 16 per
-// instruction) into one of two FP32 tensor-memory accumulators, so the epilogue of tile t overlaps
-// the MMAs of tile t+1. Warps 2..5 read the accumulator with tcgen05.ld (one row per thread), apply
-// bias + GELU (forward) or gradient accumulation + GELU derivative (backward), zero the halo rows
-// and store BF16.
+// Forward / data-gradient kernel (k_conv): a row of the GEMM is a group of G consecutive voxels of the zero-haloed
+// channels-last grid (G = 4 for 16 channels, 2 for 32: a row of 64 elements, 128 bytes), because a TMA box costs about 8
+// cycles per row however short the row is: with 32-byte rows the 16-channel convolutions at 128^3 ran at 13 k cycles per
+// 128 voxels, 728 us, all of it TMA rows. The G output voxels of a group take G N accumulator columns. A persistent CTA
+// walks output tiles of 128 groups. For each K step (input tensor, up to 64 channels, (dz, dy) of the taps) warp 0 issues
+// the TMA loads of the groups' 130-row activation boxes (K-major, swizzled A operands; rows outside the array read as
+// zeros); the weights lie in shared memory for the whole kernel where they fit, else they come with each step. Warp 1
+// issues the MMAs, all of G N columns (one shape and accumulator, whose MMAs run in order): input voxel vi of the group
+// feeds the output voxels vi - 1 to vi + 1, so its B operand is the stack of the three dx taps' weights at the rows of
+// those voxels, with rows of zeros above and below; moving the start in one stack padded by zeros serves every vi. The
+// group's last (first) voxel also feeds the first (last) output voxel of the next (previous) row: the box shifted by a
+// row. (A value that is not finite so reaches the other voxels of the groups next to it as well.) Two FP32 accumulators
+// in tensor memory: the epilogue of tile t overlaps the MMAs of tile t + 1.
+// Warps 2..5 read the accumulator with tcgen05.ld (one group per thread), apply bias + GELU (forward) or gradient
+// accumulation + GELU derivative (backward), zero the halo rows and store BF16.
 //
 // Weight-gradient kernel (k_wgrad): dw[tap][co][ci] = sum_p gout[p][co] in[p + off(tap)][ci] is a GEMM
 // with M = (taps x input channels) in blocks of 128, N = output channels and K = grid rows. Both
@@ -38,20 +44,18 @@ namespace {
 constexpr int kBM = 128;       // output rows per tile (MMA M)
 constexpr int kThreads = 192;  // warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 epilogue
 constexpr int kMaxStages = 32;
+constexpr int kMaxStepMmas = 24;  // G + 2 voxels of up to 4 slices of 16 channels
 constexpr int kWgradRows = 64;  // K rows per pipeline stage of the weight-gradient kernel
 
 struct ConvParams {
-    CUtensorMap amap[2];
+    CUtensorMap amap[2][2];  // per input: groups that start at voxel 0, at voxel `residue`
     CUtensorMap wmap[2];
-    int nin, ntaps, N, ntiles;
-    int cb[2], nchunk[2], wc0[2];
-    // K steps walk tap groups: a 3x3x3 convolution has 9 groups (dz, dy), each one activation box of
-    // kBM + 2 rows shared by its 3 dx taps (tap q starts tap_row[q] rows into the box); a 1x1x1 one
-    // has one group of one tap
-    int ngroups, gtaps, a_rows, wbox_rows;
-    int goff[9];
-    int tap_row[3];
-    int off[27];
+    int nin, ntaps, N, ntiles, G;
+    // per input: channels, channels of a K step, elements of a box row (voxels per box times those), boxes of a step
+    int cin[2], cb[2], ab[2], nbox[2], wc0[2];
+    // (dz, dy) of the taps: 9 of 3 taps (dx) each, or one of one; first box row relative to the tile's first group, and map
+    int ngroups, gtaps, a_rows, flip, wbox;  // wbox: taps per weight box (1, or all that lie in order)
+    int grow[9], gmap[9];
     int X, Y, Z;
     long long PX, PXY, R;
     int nseg, flags;
@@ -60,18 +64,12 @@ struct ConvParams {
     int seg_c0[2], seg_nc[2];
     const float* bias;
     unsigned* err;
-    int ns;
-    uint32_t a_bytes, stage_bytes, tmem_cols, idesc;
+    int ns, wres;
+    // weights of one (input, channel chunk, (dz, dy)): (G - 1) N rows of zeros, the taps' rows; zeros again at the end.
+    // Resident: start, offset of an input, bytes of a channel chunk, bytes loaded, all bytes (else w_in: within a stage)
+    uint32_t w_base, w_in[2], w_chunk[2], w_bytes, w_area;
+    uint32_t box_bytes, a_bytes, stage_bytes, tmem_cols, idesc;
 };
-
-__device__ __forceinline__ bool row_interior(long long p, int X, int Y, int Z, long long PX, long long PXY)
-{
-    const long long z = p / PXY;
-    const long long rem = p - z * PXY;
-    const long long y = rem / PX;
-    const long long x = rem - y * PX;
-    return x >= 1 && x <= X && y >= 1 && y <= Y && z >= 1 && z <= Z;
-}
 
 __device__ __forceinline__ void unpack16(const uint4 (&u)[2], float (&v)[16])
 {
@@ -115,14 +113,33 @@ __device__ __forceinline__ uint32_t aligned_smem_base(unsigned char* raw)
 __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ ConvParams P)
 {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], accf[2], acce[2], done;
+    __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], accf[2], acce[2], done, wfull;
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
+    __shared__ uint2 mtab[2][kMaxStepMmas];  // per input: the MMAs of a K step, operand addresses in 16-byte units
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t sbase = aligned_smem_base(smem_raw);
     unsigned char* sgen = smem_raw + (sbase - smem_u32(smem_raw));
+    const int mid = P.ntaps > 1 ? 1 : 0;                 // box row of the tile's first group
+    const uint32_t pad = (uint32_t)(P.G - 1);            // zero blocks of N rows before a weight stack
+    const uint32_t per = (uint32_t)P.gtaps + pad;        // blocks from one stack to the next
 
+    if (threadIdx.x < 2 * kMaxStepMmas) {
+        // Input voxels -mid .. G - 1 + mid of the group, in the order of the taps: every output voxel sums its taps in the
+        // same order whatever G is (the others add zeros), so the sums do not depend on it
+        const int i = threadIdx.x / kMaxStepMmas, t = threadIdx.x % kMaxStepMmas;
+        if (i < P.nin) {
+            const uint32_t rowa = P.ab[i] * 2u, roww = P.cb[i] * 2u;
+            const int ks = P.cb[i] / 16, vpb = P.ab[i] / P.cb[i], n = t / ks, kk = t % ks, G = P.G;
+            const int vi = P.flip ? G - 1 + mid - n : n - mid;
+            const int slot = vi < 0 ? G - 1 : (vi >= G ? 0 : vi), r = vi < 0 ? 0 : (vi == G ? 2 : mid);
+            // (G = 1 keeps the taps in the order in which they lie)
+            const int t0 = (int)pad + (G == 1 && !P.flip ? vi + mid : mid - vi);
+            mtab[i][t] = make_uint2(((uint32_t)(slot / vpb) * P.box_bytes + r * rowa + (slot % vpb) * roww + 32u * kk) >> 4,
+                                    ((uint32_t)t0 * P.N * roww + 32u * kk) >> 4);
+        }
+    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < P.ns; ++s) {
             mbar_init(&full[s], 1);
@@ -133,6 +150,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
             mbar_init(&acce[b], 4);
         }
         mbar_init(&done, 1);
+        mbar_init(&wfull, 1);
         abort_flag = 0;
         mbar_fence_init();
     }
@@ -140,34 +158,70 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
         tc::tmem_alloc(&tmem_slot, 2 * P.tmem_cols);
         tc::tmem_relinquish();
     }
+    if (P.G > 1) {
+        // the zero rows of the weight stacks (the loads fill in the rest)
+        const uint4 zero = make_uint4(0, 0, 0, 0);
+        const uint32_t from = P.wres ? P.w_base : P.a_bytes, area = P.wres ? P.w_area : P.stage_bytes - P.a_bytes;
+        for (int s = 0; s < (P.wres ? 1 : P.ns); ++s)
+            for (uint32_t q = threadIdx.x * 16u; q < area; q += kThreads * 16u)
+                *reinterpret_cast<uint4*>(sgen + s * P.stage_bytes + from + q) = zero;
+        fence_proxy_async();
+    }
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_slot;
-
     if (warp == 0) {
         if (lane == 0) {
-            uint32_t it = 0;
+            // the taps of a (dz, dy) in the order of the output voxels they feed: vi - 1, vi, vi + 1 (one voxel: as they lie)
+            auto load_taps = [&](unsigned char* w, uint64_t* bar, int i, int cc, int gq) {
+                const int x = P.wc0[i] + cc * P.cb[i], row0 = gq * P.gtaps * P.N;
+                if (P.wbox > 1 || P.gtaps == 1) {
+                    tma_load_2d(w, &P.wmap[i], bar, x, row0);
+                    return;
+                }
+                for (int t = 0; t < P.gtaps; ++t) {
+                    const int q = P.flip || P.G == 1 ? t : P.gtaps - 1 - t;
+                    tma_load_2d(w + (uint32_t)(t * P.N) * P.cb[i] * 2u, &P.wmap[i], bar, x, row0 + q * P.N);
+                }
+            };
+            if (P.wres) {
+                mbar_arrive_expect_tx(&wfull, P.w_bytes);
+                for (int i = 0; i < P.nin; ++i)
+                    for (int cc = 0; cc < P.cin[i] / P.cb[i]; ++cc)
+                        for (int gq = 0; gq < P.ngroups; ++gq)
+                            load_taps(sgen + P.w_base + P.w_in[i] + cc * P.w_chunk[i] +
+                                          (gq * per + pad) * (uint32_t)P.N * P.cb[i] * 2u,
+                                      &wfull, i, cc, gq);
+            }
+            uint32_t it = 0, s = 0, phase = 1;  // stage of the step, parity of its last release
             for (int tile = blockIdx.x; tile < P.ntiles && !abort_flag; tile += gridDim.x) {
                 const int p0 = tile * kBM;
-                for (int i = 0; i < P.nin; ++i)
-                    for (int j = 0; j < P.nchunk[i]; ++j)
+                for (int i = 0; i < P.nin; ++i) {
+                    const int nbox = P.nbox[i], ncc = P.cin[i] / P.cb[i], xstep = (P.ab[i] / P.cb[i]) * P.cin[i];
+                    const uint32_t bytes = (uint32_t)(nbox * P.a_rows * P.ab[i]) * 2u +
+                                           (P.wres ? 0u : (uint32_t)(P.gtaps * P.N) * P.cb[i] * 2u);
+                    const uint32_t w_at = P.a_bytes + P.w_in[i] + pad * (uint32_t)P.N * P.cb[i] * 2u;
+                    for (int cc = 0; cc < ncc; ++cc)
                         for (int gq = 0; gq < P.ngroups; ++gq) {
-                            const uint32_t s = it % P.ns;
-                            if (it >= (uint32_t)P.ns && !mbar_wait_bounded(&empty[s], ((it / P.ns) + 1) & 1, P.err)) {
+                            if (it >= (uint32_t)P.ns && !mbar_wait_bounded(&empty[s], phase, P.err)) {
                                 abort_flag = 1;
                                 goto produced;
                             }
-                            const uint32_t bytes = (uint32_t)(P.a_rows + P.gtaps * P.N) * P.cb[i] * 2u;
                             mbar_arrive_expect_tx(&full[s], bytes);
                             unsigned char* a = sgen + s * P.stage_bytes;
-                            tma_load_2d(a, &P.amap[i], &full[s], j * P.cb[i], p0 + P.goff[gq]);
-                            const int wrow0 = gq * P.gtaps * P.N;
-                            for (int r = 0; r < P.gtaps * P.N; r += P.wbox_rows)
-                                tma_load_2d(a + P.a_bytes + (uint32_t)r * P.cb[i] * 2u, &P.wmap[i], &full[s],
-                                            P.wc0[i] + j * P.cb[i], wrow0 + r);
+                            const int row = p0 + P.grow[gq];
+                            const CUtensorMap* map = &P.amap[i][P.gmap[gq]];
+                            for (int m = 0; m < nbox; ++m)
+                                tma_load_2d(a + m * P.box_bytes, map, &full[s], m * xstep + cc * P.cb[i], row);
+                            if (!P.wres) load_taps(a + w_at, &full[s], i, cc, gq);
                             ++it;
+                            if (++s == (uint32_t)P.ns) {
+                                s = 0;
+                                phase ^= 1u;
+                            }
                         }
+                }
             }
         produced:
             // drain: the last load into each stage must have landed before the CTA exits
@@ -175,10 +229,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
                 const uint32_t last = it - 1 - ((it - 1 - s) % P.ns);
                 (void)mbar_wait_bounded(&full[s], (last / P.ns) & 1, P.err);
             }
+            if (P.wres) (void)mbar_wait_bounded(&wfull, 0, P.err);
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            uint32_t it = 0, tl = 0;
+            uint32_t s = 0, phase = 0, tl = 0;
+            if (P.wres && !mbar_wait_bounded(&wfull, 0, P.err)) abort_flag = 1;
             for (int tile = blockIdx.x; tile < P.ntiles && !abort_flag; tile += gridDim.x, ++tl) {
                 const uint32_t buf = tl & 1;
                 if (tl >= 2 && !mbar_wait_bounded(&acce[buf], ((tl >> 1) + 1) & 1, P.err)) {
@@ -189,32 +245,36 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
                 const uint32_t d = tmem + buf * P.tmem_cols;
                 uint32_t acc = 0;
                 for (int i = 0; i < P.nin; ++i) {
-                    const uint32_t rowb = P.cb[i] * 2u;
-                    const int swz = tc::swizzle_code((int)rowb);
-                    for (int j = 0; j < P.nchunk[i]; ++j)
+                    // descriptors: the addresses (16-byte units) are added to the low words
+                    const uint32_t rowa = P.ab[i] * 2u, roww = P.cb[i] * 2u, stack = (per * (uint32_t)P.N * roww) >> 4;
+                    const uint64_t da = tc::sdesc(0, 16, 8 * rowa, tc::swizzle_code((int)rowa));
+                    const uint64_t dw = tc::sdesc(0, 16, 8 * roww, tc::swizzle_code((int)roww));
+                    const int nmma = (P.G + 2 * mid) * (P.cb[i] / 16), ncc = P.cin[i] / P.cb[i];
+                    const uint2* tab = mtab[i];
+                    for (int cc = 0; cc < ncc; ++cc) {
+                        uint32_t wr = (sbase + P.w_base + P.w_in[i] + cc * P.w_chunk[i]) >> 4;
                         for (int gq = 0; gq < P.ngroups; ++gq) {
-                            const uint32_t s = it % P.ns;
-                            if (!mbar_wait_bounded(&full[s], (it / P.ns) & 1, P.err)) {
+                            if (!mbar_wait_bounded(&full[s], phase, P.err)) {
                                 abort_flag = 1;
                                 goto issued;
                             }
                             tc::fence_after_sync();
-                            const uint32_t a = sbase + s * P.stage_bytes, b = a + P.a_bytes;
-                            for (int q = 0; q < P.gtaps; ++q) {
-                                // the tap's 128 rows start tap_row[q] rows into the shared box; the
-                                // swizzle follows the absolute shared-memory address, so a start on
-                                // any row of the 8-row pattern reads the rows TMA wrote there
-                                const uint32_t aq = a + (uint32_t)P.tap_row[q] * rowb;
-                                const uint32_t bq = b + (uint32_t)(q * P.N) * rowb;
-                                for (uint32_t kk = 0; kk < rowb / 32u; ++kk) {
-                                    tc::mma_bf16(d, tc::sdesc(aq + 32u * kk, 16, 8 * rowb, swz),
-                                                 tc::sdesc(bq + 32u * kk, 16, 8 * rowb, swz), P.idesc, acc);
-                                    acc = 1;
-                                }
+                            const uint32_t a = sbase + s * P.stage_bytes;
+                            const uint64_t ad = da + (a >> 4), wd = dw + (P.wres ? wr : (a + P.a_bytes + P.w_in[i]) >> 4);
+                            wr += stack;
+#pragma unroll 4
+                            for (int m = 0; m < nmma; ++m) {
+                                const uint2 t = tab[m];
+                                tc::mma_bf16(d, ad + t.x, wd + t.y, P.idesc, acc);
+                                acc = 1;
                             }
                             tc::mma_commit(&empty[s]);
-                            ++it;
+                            if (++s == (uint32_t)P.ns) {
+                                s = 0;
+                                phase ^= 1u;
+                            }
                         }
+                    }
                 }
                 tc::mma_commit(&accf[buf]);
             }
@@ -231,47 +291,59 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
             if (!mbar_wait_bounded(&accf[buf], (tl >> 1) & 1, P.err)) abort_flag = 1;
             if (__any_sync(0xffffffffu, abort_flag)) break;
             tc::fence_after_sync();
-            const long long p = (long long)tile * kBM + row;
-            const bool valid = p < P.R;
-            const bool inside = valid && row_interior(p, P.X, P.Y, P.Z, P.PX, P.PXY);
+            const long long pg = ((long long)tile * kBM + row) * P.G;
+            const bool valid = pg < P.R;  // (R is a multiple of G, below 2^30)
+            const unsigned up = (unsigned)pg, pxy = (unsigned)P.PXY, px = (unsigned)P.PX;
+            int z = (int)(up / pxy), y = (int)((up - z * pxy) / px), x = (int)(up - z * pxy - y * px);
             const uint32_t taddr = tmem + buf * P.tmem_cols + ((uint32_t)(q * 32) << 16);
-            for (int sg = 0; sg < P.nseg; ++sg) {
-                const int nc = P.seg_nc[sg], c0 = P.seg_c0[sg];
-                __nv_bfloat16* orow = P.out[sg] + p * nc;
-                __nv_bfloat16* arow = P.aux[sg] ? P.aux[sg] + p * nc : nullptr;
-                for (int c = 0; c < nc; c += 16) {
-                    float v[16];
-                    tc::tmem_ld16(taddr + (uint32_t)(c0 + c), v);
-                    if (!valid) continue;
-                    if (!inside) {
+            for (int vo = 0; vo < P.G; ++vo) {
+                const long long p = pg + vo;
+                const bool inside = x >= 1 && x <= P.X && y >= 1 && y <= P.Y && z >= 1 && z <= P.Z;
+                if (++x == (int)px) {
+                    x = 0;
+                    if (++y == (int)(pxy / px)) {
+                        y = 0;
+                        ++z;
+                    }
+                }
+                for (int sg = 0; sg < P.nseg; ++sg) {
+                    const int nc = P.seg_nc[sg], c0 = P.seg_c0[sg];
+                    __nv_bfloat16* orow = P.out[sg] + p * nc;
+                    __nv_bfloat16* arow = P.aux[sg] ? P.aux[sg] + p * nc : nullptr;
+                    for (int c = 0; c < nc; c += 16) {
+                        float v[16];
+                        tc::tmem_ld16(taddr + (uint32_t)(vo * P.N + c0 + c), v);
+                        if (!valid) continue;
+                        if (!inside) {
 #pragma unroll
-                        for (int e = 0; e < 16; ++e) v[e] = 0.f;
+                            for (int e = 0; e < 16; ++e) v[e] = 0.f;
+                            store16(orow + c, v);
+                            if (arow && (P.flags & kGelu)) store16(arow + c, v);
+                            continue;
+                        }
+                        if (P.bias) {
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) v[e] += __ldg(P.bias + c0 + c + e);
+                        }
+                        if (P.flags & kAccum) {
+                            float o[16];
+                            load16(orow + c, o);
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) v[e] += o[e];
+                        }
+                        if (P.flags & kDGelu) {
+                            float a[16];
+                            load16(arow + c, a);
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) v[e] *= dgelu_f(a[e]);
+                        }
+                        if (P.flags & kGelu) {
+                            if (arow) store16(arow + c, v);
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) v[e] = gelu_f(v[e]);
+                        }
                         store16(orow + c, v);
-                        if (arow && (P.flags & kGelu)) store16(arow + c, v);
-                        continue;
                     }
-                    if (P.bias) {
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) v[e] += __ldg(P.bias + c0 + c + e);
-                    }
-                    if (P.flags & kAccum) {
-                        float o[16];
-                        load16(orow + c, o);
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) v[e] += o[e];
-                    }
-                    if (P.flags & kDGelu) {
-                        float a[16];
-                        load16(arow + c, a);
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) v[e] *= dgelu_f(a[e]);
-                    }
-                    if (P.flags & kGelu) {
-                        if (arow) store16(arow + c, v);
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) v[e] = gelu_f(v[e]);
-                    }
-                    store16(orow + c, v);
                 }
             }
             tc::fence_before_sync();
@@ -309,6 +381,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad(const __grid_constant__ W
     __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], accf;
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
+    __shared__ int2 atab[8];  // the A atoms of a K step: first channel, row offset
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t sbase = aligned_smem_base(smem_raw);
@@ -318,6 +391,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad(const __grid_constant__ W
     const int k_begin = blockIdx.y * P.k_steps_per_cta;
     const int k_end = min(P.k_steps_total, k_begin + P.k_steps_per_cta);
 
+    if ((int)threadIdx.x < P.natom_a) {
+        const int m = threadIdx.x, chunks = P.cin / P.ca, tap = mt * taps_per_tile + m / chunks;
+        // taps past the last one load a valid tap (their rows of D are never stored)
+        atab[m] = make_int2(m % chunks * P.ca, P.off[tap < P.ntaps ? tap : P.ntaps - 1]);
+    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < P.ns; ++s) {
             mbar_init(&full[s], 1);
@@ -340,26 +418,28 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad(const __grid_constant__ W
 
     if (warp == 0) {
         if (lane == 0) {
-            uint32_t it = 0;
+            uint32_t it = 0, s = 0, phase = 1;  // stage of the step, parity of its last release
+            const uint32_t bytes = a_atom_bytes * P.natom_a + g_atom_bytes * P.natom_g;
             for (int ks = k_begin; ks < k_end; ++ks, ++it) {
-                const uint32_t s = it % P.ns;
-                if (it >= (uint32_t)P.ns && !mbar_wait_bounded(&empty[s], ((it / P.ns) + 1) & 1, P.err)) {
+                if (it >= (uint32_t)P.ns && !mbar_wait_bounded(&empty[s], phase, P.err)) {
                     abort_flag = 1;
                     break;
                 }
                 const int q0 = ks * kWgradRows;
-                mbar_arrive_expect_tx(&full[s], a_atom_bytes * P.natom_a + g_atom_bytes * P.natom_g);
+                mbar_arrive_expect_tx(&full[s], bytes);
                 unsigned char* a = sgen + s * P.stage_bytes;
-                const int chunks = P.cin / P.ca;
-                for (int m = 0; m < P.natom_a; ++m) {
-                    const int tap = mt * taps_per_tile + m / chunks;
-                    const int ch = m % chunks;
-                    // taps past the last one load a valid tap (their rows of D are never stored)
-                    const int tt = tap < P.ntaps ? tap : P.ntaps - 1;
-                    tma_load_2d(a + m * a_atom_bytes, &P.amap, &full[s], ch * P.ca, q0 + P.off[tt]);
+                const int natom_a = P.natom_a, natom_g = P.natom_g;
+#pragma unroll 4
+                for (int m = 0; m < natom_a; ++m) {
+                    const int2 t = atab[m];
+                    tma_load_2d(a + m * a_atom_bytes, &P.amap, &full[s], t.x, q0 + t.y);
                 }
-                for (int m = 0; m < P.natom_g; ++m)
-                    tma_load_2d(a + P.a_bytes + m * g_atom_bytes, &P.gmap, &full[s], m * P.cg, q0);
+                a += P.a_bytes;
+                for (int m = 0; m < natom_g; ++m) tma_load_2d(a + m * g_atom_bytes, &P.gmap, &full[s], m * P.cg, q0);
+                if (++s == (uint32_t)P.ns) {
+                    s = 0;
+                    phase ^= 1u;
+                }
             }
             for (uint32_t s = 0; s < (uint32_t)P.ns && s < it; ++s) {
                 const uint32_t last = it - 1 - ((it - 1 - s) % P.ns);
@@ -368,24 +448,31 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad(const __grid_constant__ W
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            const int swa = tc::swizzle_code(P.ca * 2), swg = tc::swizzle_code(P.cg * 2);
-            uint32_t it = 0, acc = 0;
-            for (int ks = k_begin; ks < k_end; ++ks, ++it) {
-                const uint32_t s = it % P.ns;
-                if (abort_flag || !mbar_wait_bounded(&full[s], (it / P.ns) & 1, P.err)) {
+            // MN-major swizzled operands: MN atoms at LBO = atom bytes, 8-row K groups at SBO
+            const uint64_t da = tc::sdesc(0, a_atom_bytes, 8u * P.ca * 2u, tc::swizzle_code(P.ca * 2));
+            const uint64_t dg = tc::sdesc(0, g_atom_bytes, 8u * P.cg * 2u, tc::swizzle_code(P.cg * 2));
+            const uint32_t stepa = 16u * P.ca * 2u >> 4, stepg = 16u * P.cg * 2u >> 4;
+            uint32_t s = 0, phase = 0, acc = 0;
+            for (int ks = k_begin; ks < k_end; ++ks) {
+                if (abort_flag || !mbar_wait_bounded(&full[s], phase, P.err)) {
                     abort_flag = 1;
                     break;
                 }
                 tc::fence_after_sync();
-                const uint32_t a = sbase + s * P.stage_bytes, b = a + P.a_bytes;
-                // MN-major swizzled operands: MN atoms at LBO = atom bytes, 8-row K groups at SBO
+                const uint32_t a = sbase + s * P.stage_bytes;
+                uint64_t ad = da + (a >> 4), bd = dg + ((a + P.a_bytes) >> 4);
+#pragma unroll
                 for (int kk = 0; kk < kWgradRows / 16; ++kk) {
-                    const uint64_t ad = tc::sdesc(a + kk * 16u * P.ca * 2u, a_atom_bytes, 8u * P.ca * 2u, swa);
-                    const uint64_t bd = tc::sdesc(b + kk * 16u * P.cg * 2u, g_atom_bytes, 8u * P.cg * 2u, swg);
                     tc::mma_bf16(tmem, ad, bd, P.idesc, acc);
                     acc = 1;
+                    ad += stepa;
+                    bd += stepg;
                 }
                 tc::mma_commit(&empty[s]);
+                if (++s == (uint32_t)P.ns) {
+                    s = 0;
+                    phase ^= 1u;
+                }
             }
             tc::mma_commit(&accf);
         }
@@ -478,17 +565,17 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
     }
     ConvParams P;
     memset(&P, 0, sizeof(P));
-    int cin_tot = 0, cbmax = 16;
+    int cin_tot = 0, cmin = 64;
     for (int i = 0; i < L.nin; ++i) {
         if (!L.in[i] || !channels_ok(L.cin[i]) || (reinterpret_cast<uintptr_t>(L.in[i]) & 15)) {
             set_error("conv3d: input channels must be 16, 32 or a multiple of 64, data 16-byte aligned");
             return GBP_BAD_ARG;
         }
+        P.cin[i] = L.cin[i];
         P.cb[i] = chunk_of(L.cin[i]);
-        P.nchunk[i] = L.cin[i] / P.cb[i];
         P.wc0[i] = cin_tot;
         cin_tot += L.cin[i];
-        cbmax = std::max(cbmax, P.cb[i]);
+        cmin = std::min(cmin, P.cb[i]);
     }
     int segsum = 0;
     for (int s = 0; s < L.nseg; ++s) {
@@ -510,27 +597,49 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
     P.nin = L.nin;
     P.ntaps = L.ntaps;
     P.N = L.N;
-    P.ntiles = (int)((L.g.R + kBM - 1) / kBM);
-    tap_offsets(L.g, L.ntaps, L.flip, P.off);
-    if (L.ntaps == 27) {
-        P.ngroups = 9;
-        P.gtaps = 3;
-        P.a_rows = kBM + 2;
-        for (int gq = 0; gq < 9; ++gq) P.goff[gq] = std::min(P.off[3 * gq], P.off[3 * gq + 2]);
-        // dx = -1, 0, +1 of a group sit at rows +0, +1, +2 of the box (+2, +1, +0 for flipped taps)
-        for (int q = 0; q < 3; ++q) P.tap_row[q] = P.off[q] - P.goff[0];
-    } else {
-        P.ngroups = 1;
-        P.gtaps = 1;
-        P.a_rows = kBM;
-        P.goff[0] = P.off[0];
-        P.tap_row[0] = 0;
+    P.flip = L.flip;
+    P.ngroups = L.ntaps == 27 ? 9 : 1;
+    P.gtaps = L.ntaps == 27 ? 3 : 1;
+    P.a_rows = L.ntaps == 27 ? kBM + 2 : kBM;
+    int off[27];
+    tap_offsets(L.g, L.ntaps, L.flip, off);
+    // voxels per GEMM row: rows of 64 elements (128 bytes) for the narrowest input, where the grid splits into such groups,
+    // the (dz, dy) offsets fall on at most two positions within a group and the columns stay within an MMA's 256 (twice
+    // that is the tensor memory)
+    int residue = 0;
+    for (P.G = 64 / cmin;; P.G >>= 1) {
+        bool ok = L.g.R % P.G == 0 && P.G * L.N <= 256;
+        residue = 0;
+        for (int gq = 0; gq < P.ngroups; ++gq) {
+            const int c = L.ntaps == 27 ? off[3 * gq + 1] : 0, r = ((c % P.G) + P.G) % P.G;
+            if (r && residue && r != residue) ok = false;
+            if (r) residue = r;
+            P.gmap[gq] = r ? 1 : 0;
+            P.grow[gq] = (c - r) / P.G - (L.ntaps == 27 ? 1 : 0);
+        }
+        if (ok || P.G == 1) break;
     }
-    P.wbox_rows = P.gtaps * L.N <= 256 ? P.gtaps * L.N : L.N;
+    P.ntiles = (int)((L.g.R / P.G + kBM - 1) / kBM);
+    P.wbox = (P.flip || P.G == 1) && P.gtaps * L.N <= 256 ? P.gtaps : 1;
+    uint32_t wres_bytes = 0;
+    int abmax = 16, nbmax = 1;
     for (int i = 0; i < L.nin; ++i) {
-        int rc = encode_rows(L.in[i], L.cin[i], L.g.R, P.cb[i], P.a_rows, &P.amap[i]);
-        if (!rc) rc = encode_rows(L.w, cin_tot, (long long)L.ntaps * L.N, P.cb[i], P.wbox_rows, &P.wmap[i]);
+        P.ab[i] = std::min(64, P.G * P.cb[i]);
+        P.nbox[i] = P.G * P.cb[i] / P.ab[i];
+        abmax = std::max(abmax, P.ab[i]);
+        nbmax = std::max(nbmax, P.nbox[i]);
+        for (int m = 0; m < 2; ++m) {
+            const int r = m ? residue : 0;
+            const int rc = encode_rows(L.in[i] + (size_t)r * L.cin[i], P.G * L.cin[i], (L.g.R - r) / P.G, P.ab[i], P.a_rows,
+                                       &P.amap[i][m]);
+            if (rc) return rc;
+        }
+        const int rc = encode_rows(L.w, cin_tot, (long long)L.ntaps * L.N, P.cb[i], P.wbox * L.N, &P.wmap[i]);
         if (rc) return rc;
+        P.w_in[i] = wres_bytes;
+        P.w_chunk[i] = ((uint32_t)((P.gtaps + P.G - 1) * P.ngroups + P.G - 1) * L.N * P.cb[i] * 2u + 1023u) & ~1023u;
+        wres_bytes += P.w_chunk[i] * (L.cin[i] / P.cb[i]);
+        P.w_bytes += (uint32_t)L.ntaps * L.N * L.cin[i] * 2u;
     }
     P.X = L.g.X;
     P.Y = L.g.Y;
@@ -542,20 +651,34 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
     P.flags = L.flags;
     P.bias = L.bias;
     P.err = L.err;
-    P.a_bytes = ((uint32_t)P.a_rows * cbmax * 2u + 1023u) & ~1023u;
-    P.stage_bytes = P.a_bytes + (((uint32_t)(P.gtaps * L.N) * cbmax * 2u + 1023u) & ~1023u);
-    P.tmem_cols = pow2_cols(L.N);
-    P.idesc = tc::idesc_bf16(kBM, L.N, 0, 0);
-    const int max_smem = 200 * 1024;
-    P.ns = std::min(kMaxStages, (int)((max_smem - 1024) / P.stage_bytes));
+    P.box_bytes = ((uint32_t)P.a_rows * abmax * 2u + 1023u) & ~1023u;
+    P.a_bytes = nbmax * P.box_bytes;
+    P.tmem_cols = pow2_cols(P.G * L.N);
+    P.idesc = tc::idesc_bf16(kBM, P.G * L.N, 0, 0);
+    P.w_area = wres_bytes;
+    // weights resident where at least 3 activation stages fit beside them, else with each step
+    const uint32_t max_smem = 220 * 1024;
+    P.wres = wres_bytes + 3 * P.a_bytes + 1024 <= max_smem;
+    P.stage_bytes = P.a_bytes;
+    if (!P.wres) {
+        uint32_t w = 0;
+        for (int i = 0; i < L.nin; ++i) {
+            const uint32_t stack = ((uint32_t)((P.gtaps + 2 * (P.G - 1)) * L.N) * P.cb[i] * 2u + 1023u) & ~1023u;
+            P.w_in[i] = P.G > 1 ? w : 0;  // (each input's zero rows stay where they are)
+            w = P.G > 1 ? w + stack : std::max(w, stack);
+        }
+        P.stage_bytes += w;
+    }
+    P.ns = std::min(kMaxStages, (int)((max_smem - 1024 - (P.wres ? wres_bytes : 0)) / P.stage_bytes));
     if (P.ns < 2) {
         set_error("conv3d: stage does not fit in shared memory");
         return GBP_BAD_ARG;
     }
-    const size_t smem = (size_t)P.ns * P.stage_bytes + 1024;
+    P.w_base = (uint32_t)P.ns * P.stage_bytes;
+    const size_t smem = (size_t)P.w_base + (P.wres ? wres_bytes : 0) + 1024;
     static bool attr_set = false;
     if (!attr_set) {
-        GBP_CUDA(cudaFuncSetAttribute(k_conv, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        GBP_CUDA(cudaFuncSetAttribute(k_conv, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         attr_set = true;
     }
     const int grid = std::min(P.ntiles, sm_count_cached());
