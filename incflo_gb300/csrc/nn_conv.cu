@@ -44,7 +44,7 @@ namespace {
 constexpr int kBM = 128;       // output rows per tile (MMA M)
 constexpr int kThreads = 192;  // warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 epilogue
 constexpr int kMaxStages = 32;
-constexpr int kMaxStepMmas = 24;  // G + 2 voxels of up to 4 slices of 16 channels
+constexpr int kMostVoxels = 6;  // G + 2 input voxels feed a group
 constexpr int kWgradRows = 64;  // K rows per pipeline stage of the weight-gradient kernel
 
 struct ConvParams {
@@ -54,6 +54,7 @@ struct ConvParams {
     // per input: channels, channels of a K step, elements of a box row (voxels per box times those), boxes of a step
     int cin[2], cb[2], ab[2], nbox[2], wc0[2];
     // (dz, dy) of the taps: 9 of 3 taps (dx) each, or one of one; first box row relative to the tile's first group, and map
+    int vsh[2];  // log2 of the voxels per box
     int ngroups, gtaps, a_rows, flip, wbox;  // wbox: taps per weight box (1, or all that lie in order)
     int grow[9], gmap[9];
     int X, Y, Z;
@@ -116,30 +117,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
     __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], accf[2], acce[2], done, wfull;
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
-    __shared__ uint2 mtab[2][kMaxStepMmas];  // per input: the MMAs of a K step, operand addresses in 16-byte units
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (uniform by construction, so that the issue loops' values live in uniform registers)
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t sbase = aligned_smem_base(smem_raw);
     unsigned char* sgen = smem_raw + (sbase - smem_u32(smem_raw));
     const int mid = P.ntaps > 1 ? 1 : 0;                 // box row of the tile's first group
     const uint32_t pad = (uint32_t)(P.G - 1);            // zero blocks of N rows before a weight stack
     const uint32_t per = (uint32_t)P.gtaps + pad;        // blocks from one stack to the next
 
-    if (threadIdx.x < 2 * kMaxStepMmas) {
-        // Input voxels -mid .. G - 1 + mid of the group, in the order of the taps: every output voxel sums its taps in the
-        // same order whatever G is (the others add zeros), so the sums do not depend on it
-        const int i = threadIdx.x / kMaxStepMmas, t = threadIdx.x % kMaxStepMmas;
-        if (i < P.nin) {
-            const uint32_t rowa = P.ab[i] * 2u, roww = P.cb[i] * 2u;
-            const int ks = P.cb[i] / 16, vpb = P.ab[i] / P.cb[i], n = t / ks, kk = t % ks, G = P.G;
-            const int vi = P.flip ? G - 1 + mid - n : n - mid;
-            const int slot = vi < 0 ? G - 1 : (vi >= G ? 0 : vi), r = vi < 0 ? 0 : (vi == G ? 2 : mid);
-            // (G = 1 keeps the taps in the order in which they lie)
-            const int t0 = (int)pad + (G == 1 && !P.flip ? vi + mid : mid - vi);
-            mtab[i][t] = make_uint2(((uint32_t)(slot / vpb) * P.box_bytes + r * rowa + (slot % vpb) * roww + 32u * kk) >> 4,
-                                    ((uint32_t)t0 * P.N * roww + 32u * kk) >> 4);
-        }
-    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < P.ns; ++s) {
             mbar_init(&full[s], 1);
@@ -172,116 +158,134 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
     tc::fence_after_sync();
     const uint32_t tmem = tmem_slot;
     if (warp == 0) {
-        if (lane == 0) {
-            // the taps of a (dz, dy) in the order of the output voxels they feed: vi - 1, vi, vi + 1 (one voxel: as they lie)
-            auto load_taps = [&](unsigned char* w, uint64_t* bar, int i, int cc, int gq) {
-                const int x = P.wc0[i] + cc * P.cb[i], row0 = gq * P.gtaps * P.N;
-                if (P.wbox > 1 || P.gtaps == 1) {
-                    tma_load_2d(w, &P.wmap[i], bar, x, row0);
-                    return;
-                }
-                for (int t = 0; t < P.gtaps; ++t) {
-                    const int q = P.flip || P.G == 1 ? t : P.gtaps - 1 - t;
-                    tma_load_2d(w + (uint32_t)(t * P.N) * P.cb[i] * 2u, &P.wmap[i], bar, x, row0 + q * P.N);
-                }
-            };
-            if (P.wres) {
-                mbar_arrive_expect_tx(&wfull, P.w_bytes);
-                for (int i = 0; i < P.nin; ++i)
-                    for (int cc = 0; cc < P.cin[i] / P.cb[i]; ++cc)
-                        for (int gq = 0; gq < P.ngroups; ++gq)
-                            load_taps(sgen + P.w_base + P.w_in[i] + cc * P.w_chunk[i] +
-                                          (gq * per + pad) * (uint32_t)P.N * P.cb[i] * 2u,
-                                      &wfull, i, cc, gq);
+        // the taps of a (dz, dy) in the order of the output voxels they feed: vi - 1, vi, vi + 1 (one voxel: as they lie)
+        auto load_taps = [&](unsigned char* w, uint64_t* bar, int i, int cc, int gq) {
+            const int x = P.wc0[i] + cc * P.cb[i], row0 = gq * P.gtaps * P.N;
+            if (P.wbox > 1 || P.gtaps == 1) {
+                tma_load_2d(w, &P.wmap[i], bar, x, row0);
+                return;
             }
-            uint32_t it = 0, s = 0, phase = 1;  // stage of the step, parity of its last release
-            for (int tile = blockIdx.x; tile < P.ntiles && !abort_flag; tile += gridDim.x) {
-                const int p0 = tile * kBM;
-                for (int i = 0; i < P.nin; ++i) {
-                    const int nbox = P.nbox[i], ncc = P.cin[i] / P.cb[i], xstep = (P.ab[i] / P.cb[i]) * P.cin[i];
-                    const uint32_t bytes = (uint32_t)(nbox * P.a_rows * P.ab[i]) * 2u +
-                                           (P.wres ? 0u : (uint32_t)(P.gtaps * P.N) * P.cb[i] * 2u);
-                    const uint32_t w_at = P.a_bytes + P.w_in[i] + pad * (uint32_t)P.N * P.cb[i] * 2u;
-                    for (int cc = 0; cc < ncc; ++cc)
-                        for (int gq = 0; gq < P.ngroups; ++gq) {
-                            if (it >= (uint32_t)P.ns && !mbar_wait_bounded(&empty[s], phase, P.err)) {
-                                abort_flag = 1;
-                                goto produced;
-                            }
+            for (int t = 0; t < P.gtaps; ++t) {
+                const int q = P.flip || P.G == 1 ? t : P.gtaps - 1 - t;
+                tma_load_2d(w + (uint32_t)(t * P.N) * P.cb[i] * 2u, &P.wmap[i], bar, x, row0 + q * P.N);
+            }
+        };
+        if (P.wres && tc::elect_one()) {
+            mbar_arrive_expect_tx(&wfull, P.w_bytes);
+            for (int i = 0; i < P.nin; ++i)
+                for (int cc = 0; cc < P.cin[i] / P.cb[i]; ++cc)
+                    for (int gq = 0; gq < P.ngroups; ++gq)
+                        load_taps(sgen + P.w_base + P.w_in[i] + cc * P.w_chunk[i] +
+                                      (gq * per + pad) * (uint32_t)P.N * P.cb[i] * 2u,
+                                  &wfull, i, cc, gq);
+        }
+        __syncwarp();
+        uint32_t it = 0, s = 0, phase = 1;  // stage of the step, parity of its last release
+        for (int tile = blockIdx.x; tile < P.ntiles && __all_sync(0xffffffffu, !abort_flag); tile += gridDim.x) {
+            const int p0 = tile * kBM;
+            for (int i = 0; i < P.nin; ++i) {
+                const int nbox = P.nbox[i], ncc = P.cin[i] / P.cb[i], xstep = (P.ab[i] / P.cb[i]) * P.cin[i];
+                const uint32_t bytes = (uint32_t)(nbox * P.a_rows * P.ab[i]) * 2u +
+                                       (P.wres ? 0u : (uint32_t)(P.gtaps * P.N) * P.cb[i] * 2u);
+                const uint32_t w_at = P.a_bytes + P.w_in[i] + pad * (uint32_t)P.N * P.cb[i] * 2u;
+                for (int cc = 0; cc < ncc; ++cc)
+                    for (int gq = 0; gq < P.ngroups; ++gq) {
+                        if (it >= (uint32_t)P.ns && !tc::warp_wait(&empty[s], phase, P.err)) {
+                            abort_flag = 1;
+                            goto produced;
+                        }
+                        if (tc::elect_one()) {
                             mbar_arrive_expect_tx(&full[s], bytes);
                             unsigned char* a = sgen + s * P.stage_bytes;
-                            const int row = p0 + P.grow[gq];
+                            const int arow = p0 + P.grow[gq];
                             const CUtensorMap* map = &P.amap[i][P.gmap[gq]];
                             for (int m = 0; m < nbox; ++m)
-                                tma_load_2d(a + m * P.box_bytes, map, &full[s], m * xstep + cc * P.cb[i], row);
+                                tma_load_2d(a + m * P.box_bytes, map, &full[s], m * xstep + cc * P.cb[i], arow);
                             if (!P.wres) load_taps(a + w_at, &full[s], i, cc, gq);
-                            ++it;
-                            if (++s == (uint32_t)P.ns) {
-                                s = 0;
-                                phase ^= 1u;
-                            }
                         }
-                }
+                        __syncwarp();
+                        ++it;
+                        if (++s == (uint32_t)P.ns) {
+                            s = 0;
+                            phase ^= 1u;
+                        }
+                    }
             }
-        produced:
-            // drain: the last load into each stage must have landed before the CTA exits
-            for (uint32_t s = 0; s < (uint32_t)P.ns && s < it; ++s) {
-                const uint32_t last = it - 1 - ((it - 1 - s) % P.ns);
-                (void)mbar_wait_bounded(&full[s], (last / P.ns) & 1, P.err);
-            }
-            if (P.wres) (void)mbar_wait_bounded(&wfull, 0, P.err);
         }
+    produced:
+        // drain: the last load into each stage must have landed before the CTA exits
+        for (uint32_t q = 0; q < (uint32_t)P.ns && q < it; ++q) {
+            const uint32_t last = it - 1 - ((it - 1 - q) % P.ns);
+            (void)tc::warp_wait(&full[q], (last / P.ns) & 1, P.err);
+        }
+        if (P.wres) (void)tc::warp_wait(&wfull, 0, P.err);
     } else if (warp == 1) {
-        if (lane == 0) {
-            uint32_t s = 0, phase = 0, tl = 0;
-            if (P.wres && !mbar_wait_bounded(&wfull, 0, P.err)) abort_flag = 1;
-            for (int tile = blockIdx.x; tile < P.ntiles && !abort_flag; tile += gridDim.x, ++tl) {
-                const uint32_t buf = tl & 1;
-                if (tl >= 2 && !mbar_wait_bounded(&acce[buf], ((tl >> 1) + 1) & 1, P.err)) {
-                    abort_flag = 1;
-                    break;
+        uint32_t s = 0, phase = 0, tl = 0;
+        if (P.wres && !tc::warp_wait(&wfull, 0, P.err)) abort_flag = 1;
+        const int G = P.G;
+        for (int tile = blockIdx.x; tile < P.ntiles && __all_sync(0xffffffffu, !abort_flag); tile += gridDim.x, ++tl) {
+            const uint32_t buf = tl & 1;
+            if (tl >= 2 && !tc::warp_wait(&acce[buf], ((tl >> 1) + 1) & 1, P.err)) {
+                abort_flag = 1;
+                break;
+            }
+            tc::fence_after_sync();
+            const uint32_t d = tmem + buf * P.tmem_cols;
+            uint32_t acc = 0;
+            for (int i = 0; i < P.nin; ++i) {
+                // descriptors: the addresses (16-byte units) are added to the low words
+                const uint32_t rowa = P.ab[i] * 2u, roww = P.cb[i] * 2u, blk = ((uint32_t)P.N * roww) >> 4;
+                const uint64_t da = tc::sdesc(0, 16, 8 * rowa, tc::swizzle_code((int)rowa));
+                const uint64_t dw = tc::sdesc(0, 16, 8 * roww, tc::swizzle_code((int)roww));
+                const int ks = P.cb[i] / 16, ncc = P.cin[i] / P.cb[i], vsh = P.vsh[i], vmask = (1 << vsh) - 1;
+                // Input voxels -mid .. G - 1 + mid of the group, in the order of the taps: every output voxel sums its taps in
+                // the same order whatever G is (the others add zeros), so the sums do not depend on it
+                const int nvox = G + 2 * mid;
+                uint32_t ao[kMostVoxels], wo[kMostVoxels];
+#pragma unroll
+                for (int n = 0; n < kMostVoxels; ++n) {
+                    const int vi = P.flip ? G - 1 + mid - n : n - mid;
+                    const int slot = vi < 0 ? G - 1 : (vi == G ? 0 : vi), r = vi < 0 ? 0 : (vi == G ? 2 : mid);
+                    // (G = 1 keeps the taps in the order in which they lie)
+                    const int t0 = (int)pad + (G == 1 && !P.flip ? vi + mid : mid - vi);
+                    ao[n] = ((uint32_t)(slot >> vsh) * P.box_bytes + (uint32_t)r * rowa + (uint32_t)(slot & vmask) * roww) >> 4;
+                    wo[n] = n < nvox ? (uint32_t)t0 * blk : 0;
                 }
-                tc::fence_after_sync();
-                const uint32_t d = tmem + buf * P.tmem_cols;
-                uint32_t acc = 0;
-                for (int i = 0; i < P.nin; ++i) {
-                    // descriptors: the addresses (16-byte units) are added to the low words
-                    const uint32_t rowa = P.ab[i] * 2u, roww = P.cb[i] * 2u, stack = (per * (uint32_t)P.N * roww) >> 4;
-                    const uint64_t da = tc::sdesc(0, 16, 8 * rowa, tc::swizzle_code((int)rowa));
-                    const uint64_t dw = tc::sdesc(0, 16, 8 * roww, tc::swizzle_code((int)roww));
-                    const int nmma = (P.G + 2 * mid) * (P.cb[i] / 16), ncc = P.cin[i] / P.cb[i];
-                    const uint2* tab = mtab[i];
-                    for (int cc = 0; cc < ncc; ++cc) {
-                        uint32_t wr = (sbase + P.w_base + P.w_in[i] + cc * P.w_chunk[i]) >> 4;
-                        for (int gq = 0; gq < P.ngroups; ++gq) {
-                            if (!mbar_wait_bounded(&full[s], phase, P.err)) {
-                                abort_flag = 1;
-                                goto issued;
-                            }
-                            tc::fence_after_sync();
-                            const uint32_t a = sbase + s * P.stage_bytes;
-                            const uint64_t ad = da + (a >> 4), wd = dw + (P.wres ? wr : (a + P.a_bytes + P.w_in[i]) >> 4);
-                            wr += stack;
-#pragma unroll 4
-                            for (int m = 0; m < nmma; ++m) {
-                                const uint2 t = tab[m];
-                                tc::mma_bf16(d, ad + t.x, wd + t.y, P.idesc, acc);
+                for (int cc = 0; cc < ncc; ++cc) {
+                    uint32_t wr = (sbase + P.w_base + P.w_in[i] + cc * P.w_chunk[i]) >> 4;
+                    for (int gq = 0; gq < P.ngroups; ++gq) {
+                        if (!tc::warp_wait(&full[s], phase, P.err)) {
+                            abort_flag = 1;
+                            goto issued;
+                        }
+                        tc::fence_after_sync();
+                        const uint32_t a = sbase + s * P.stage_bytes;
+                        const uint32_t w = P.wres ? wr : (a + P.a_bytes + P.w_in[i]) >> 4;
+                        wr += per * blk;
+                        const uint64_t ad = da + (a >> 4), wd = dw + w;
+#pragma unroll
+                        for (int n = 0; n < kMostVoxels; ++n) {
+                            if (n >= nvox) break;
+#pragma unroll
+                            for (int kk = 0; kk < 4; ++kk) {
+                                if (kk >= ks) break;
+                                tc::mma_bf16(d, ad + (ao[n] + 2u * kk), wd + (wo[n] + 2u * kk), P.idesc, acc);
                                 acc = 1;
                             }
-                            tc::mma_commit(&empty[s]);
-                            if (++s == (uint32_t)P.ns) {
-                                s = 0;
-                                phase ^= 1u;
-                            }
+                        }
+                        tc::mma_commit(&empty[s]);
+                        if (++s == (uint32_t)P.ns) {
+                            s = 0;
+                            phase ^= 1u;
                         }
                     }
                 }
-                tc::mma_commit(&accf[buf]);
             }
-        issued:
-            tc::mma_commit(&done);
-            (void)mbar_wait_bounded(&done, 0, P.err);
+            tc::mma_commit(&accf[buf]);
         }
+    issued:
+        tc::mma_commit(&done);
+        (void)tc::warp_wait(&done, 0, P.err);
     } else {
         const int q = warp & 3;  // tensor-memory lane quarter this warp may read
         const int row = q * 32 + lane;
@@ -383,7 +387,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad(const __grid_constant__ W
     __shared__ volatile int abort_flag;
     __shared__ int2 atab[8];  // the A atoms of a K step: first channel, row offset
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (uniform by construction, so that the issue loops' values live in uniform registers)
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t sbase = aligned_smem_base(smem_raw);
     unsigned char* sgen = smem_raw + (sbase - smem_u32(smem_raw));
     const int mt = blockIdx.x;  // M tile: taps [mt * taps_per_tile, ...)
@@ -417,14 +422,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad(const __grid_constant__ W
     const uint32_t g_atom_bytes = (uint32_t)kWgradRows * P.cg * 2u;
 
     if (warp == 0) {
-        if (lane == 0) {
-            uint32_t it = 0, s = 0, phase = 1;  // stage of the step, parity of its last release
-            const uint32_t bytes = a_atom_bytes * P.natom_a + g_atom_bytes * P.natom_g;
-            for (int ks = k_begin; ks < k_end; ++ks, ++it) {
-                if (it >= (uint32_t)P.ns && !mbar_wait_bounded(&empty[s], phase, P.err)) {
-                    abort_flag = 1;
-                    break;
-                }
+        uint32_t it = 0, s = 0, phase = 1;  // stage of the step, parity of its last release
+        const uint32_t bytes = a_atom_bytes * P.natom_a + g_atom_bytes * P.natom_g;
+        for (int ks = k_begin; ks < k_end; ++ks, ++it) {
+            if (it >= (uint32_t)P.ns && !tc::warp_wait(&empty[s], phase, P.err)) {
+                abort_flag = 1;
+                break;
+            }
+            if (tc::elect_one()) {
                 const int q0 = ks * kWgradRows;
                 mbar_arrive_expect_tx(&full[s], bytes);
                 unsigned char* a = sgen + s * P.stage_bytes;
@@ -436,46 +441,45 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad(const __grid_constant__ W
                 }
                 a += P.a_bytes;
                 for (int m = 0; m < natom_g; ++m) tma_load_2d(a + m * g_atom_bytes, &P.gmap, &full[s], m * P.cg, q0);
-                if (++s == (uint32_t)P.ns) {
-                    s = 0;
-                    phase ^= 1u;
-                }
             }
-            for (uint32_t s = 0; s < (uint32_t)P.ns && s < it; ++s) {
-                const uint32_t last = it - 1 - ((it - 1 - s) % P.ns);
-                (void)mbar_wait_bounded(&full[s], (last / P.ns) & 1, P.err);
+            __syncwarp();
+            if (++s == (uint32_t)P.ns) {
+                s = 0;
+                phase ^= 1u;
             }
+        }
+        for (uint32_t q = 0; q < (uint32_t)P.ns && q < it; ++q) {
+            const uint32_t last = it - 1 - ((it - 1 - q) % P.ns);
+            (void)tc::warp_wait(&full[q], (last / P.ns) & 1, P.err);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // MN-major swizzled operands: MN atoms at LBO = atom bytes, 8-row K groups at SBO
-            const uint64_t da = tc::sdesc(0, a_atom_bytes, 8u * P.ca * 2u, tc::swizzle_code(P.ca * 2));
-            const uint64_t dg = tc::sdesc(0, g_atom_bytes, 8u * P.cg * 2u, tc::swizzle_code(P.cg * 2));
-            const uint32_t stepa = 16u * P.ca * 2u >> 4, stepg = 16u * P.cg * 2u >> 4;
-            uint32_t s = 0, phase = 0, acc = 0;
-            for (int ks = k_begin; ks < k_end; ++ks) {
-                if (abort_flag || !mbar_wait_bounded(&full[s], phase, P.err)) {
-                    abort_flag = 1;
-                    break;
-                }
-                tc::fence_after_sync();
-                const uint32_t a = sbase + s * P.stage_bytes;
-                uint64_t ad = da + (a >> 4), bd = dg + ((a + P.a_bytes) >> 4);
-#pragma unroll
-                for (int kk = 0; kk < kWgradRows / 16; ++kk) {
-                    tc::mma_bf16(tmem, ad, bd, P.idesc, acc);
-                    acc = 1;
-                    ad += stepa;
-                    bd += stepg;
-                }
-                tc::mma_commit(&empty[s]);
-                if (++s == (uint32_t)P.ns) {
-                    s = 0;
-                    phase ^= 1u;
-                }
+        // MN-major swizzled operands: MN atoms at LBO = atom bytes, 8-row K groups at SBO
+        const uint64_t da = tc::sdesc(0, a_atom_bytes, 8u * P.ca * 2u, tc::swizzle_code(P.ca * 2));
+        const uint64_t dg = tc::sdesc(0, g_atom_bytes, 8u * P.cg * 2u, tc::swizzle_code(P.cg * 2));
+        const uint32_t stepa = 16u * P.ca * 2u >> 4, stepg = 16u * P.cg * 2u >> 4;
+        uint32_t s = 0, phase = 0, acc = 0;
+        for (int ks = k_begin; ks < k_end; ++ks) {
+            if (!tc::warp_wait(&full[s], phase, P.err)) {
+                abort_flag = 1;
+                break;
             }
-            tc::mma_commit(&accf);
+            tc::fence_after_sync();
+            const uint32_t a = sbase + s * P.stage_bytes;
+            uint64_t ad = da + (a >> 4), bd = dg + ((a + P.a_bytes) >> 4);
+#pragma unroll
+            for (int kk = 0; kk < kWgradRows / 16; ++kk) {
+                tc::mma_bf16(tmem, ad, bd, P.idesc, acc);
+                acc = 1;
+                ad += stepa;
+                bd += stepg;
+            }
+            tc::mma_commit(&empty[s]);
+            if (++s == (uint32_t)P.ns) {
+                s = 0;
+                phase ^= 1u;
+            }
         }
+        tc::mma_commit(&accf);
     } else {
         const int q = warp & 3;
         const int row = q * 32 + lane;  // M row = (tap in tile, input channel)
@@ -626,6 +630,8 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
     for (int i = 0; i < L.nin; ++i) {
         P.ab[i] = std::min(64, P.G * P.cb[i]);
         P.nbox[i] = P.G * P.cb[i] / P.ab[i];
+        for (P.vsh[i] = 0; P.cb[i] << P.vsh[i] < P.ab[i]; ++P.vsh[i]) {
+        }
         abmax = std::max(abmax, P.ab[i]);
         nbmax = std::max(nbmax, P.nbox[i]);
         for (int m = 0; m < 2; ++m) {
