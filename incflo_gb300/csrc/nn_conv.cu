@@ -1,9 +1,11 @@
 // BF16 3x3x3 convolutions of the warm-start U-Net as implicit GEMMs on tcgen05.
 //
 // Forward / data-gradient kernel (k_conv): a row of the GEMM is a group of G consecutive voxels of the zero-haloed
-// channels-last grid (G = 4 for 16 channels, 2 for 32: a row of 64 elements, 128 bytes), because a TMA box costs about 8
-// cycles per row however short the row is: with 32-byte rows the 16-channel convolutions at 128^3 ran at 13 k cycles per
-// 128 voxels, 728 us, all of it TMA rows. The G output voxels of a group take G N accumulator columns. A persistent CTA
+// channels-last grid (G = 4 for 16 channels, 2 for 32: a row of 64 elements, 128 bytes). With a voxel per row the
+// 16-channel convolutions at 128^3 took 728 us: 27 MMAs of 16 columns and 9 boxes of 32-byte rows per 128 voxels, every one
+// of them some 400 cycles of scalar issue code. Now 116 us: 54 MMAs of 64 columns and 3 boxes per 512 voxels, at 150 cycles
+// per MMA, which still bounds it (the tensor pipe is busy 21 %, DRAM 17 %). The G output voxels of a group take G N
+// accumulator columns. A persistent CTA
 // walks output tiles of 128 groups. For each K step (input tensor, up to 64 channels, (dz, dy) of the taps) warp 0 issues
 // the TMA loads of the groups' 130-row activation boxes (K-major, swizzled A operands; rows outside the array read as
 // zeros); the weights lie in shared memory for the whole kernel where they fit, else they come with each step. Warp 1
@@ -13,7 +15,7 @@
 // group's last (first) voxel also feeds the first (last) output voxel of the next (previous) row: the box shifted by a
 // row. (A value that is not finite so reaches the other voxels of the groups next to it as well.) Two FP32 accumulators
 // in tensor memory: the epilogue of tile t overlaps the MMAs of tile t + 1.
-// Warps 2..5 read the accumulator with tcgen05.ld (one group per thread), apply bias + GELU (forward) or gradient
+// The other warps read the accumulator with tcgen05.ld (one group per thread, 16 columns at a time), apply bias + GELU (forward) or gradient
 // accumulation + GELU derivative (backward), zero the halo rows and store BF16.
 //
 // Weight-gradient kernel (k_wgrad): dw[tap][co][ci] = sum_p gout[p][co] in[p + off(tap)][ci] is a GEMM
@@ -42,21 +44,26 @@ namespace nn {
 namespace {
 
 constexpr int kBM = 128;       // output rows per tile (MMA M)
-constexpr int kThreads = 192;  // warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 epilogue
+constexpr int kThreads = 192;  // weight gradient: warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 epilogue
+// convolution: four epilogue warps per lane quarter of tensor memory. The epilogue's chain (tensor-memory load, bias, GELU,
+// two stores) bounded the level-0 convolutions with one: 4.6 k cycles per tile without a GELU, about 11 k with it.
+constexpr int kEpiSets = 4, kConvThreads = 64 + 128 * kEpiSets;
 constexpr int kMaxStages = 32;
-constexpr int kMostVoxels = 6;  // G + 2 input voxels feed a group
 constexpr int kWgradRows = 64;  // K rows per pipeline stage of the weight-gradient kernel
 
 struct ConvParams {
-    CUtensorMap amap[2][2];  // per input: groups that start at voxel 0, at voxel `residue`
+    CUtensorMap amap[2];
     CUtensorMap wmap[2];
     int nin, ntaps, N, ntiles, G;
     // per input: channels, channels of a K step, elements of a box row (voxels per box times those), boxes of a step
     int cin[2], cb[2], ab[2], nbox[2], wc0[2];
     // (dz, dy) of the taps: 9 of 3 taps (dx) each, or one of one; first box row relative to the tile's first group, and map
     int vsh[2];  // log2 of the voxels per box
-    int ngroups, gtaps, a_rows, flip, wbox;  // wbox: taps per weight box (1, or all that lie in order)
-    int grow[9], gmap[9];
+    // K steps of an input and channel chunk: nstep boxes of a_rows rows, the first at row grow[step] relative to the tile's
+    // first group; a box holds the rows of ndy of the 9 (dz, dy), 3 taps (dx) each (a 1x1x1 convolution: one of one tap).
+    // yoff[dy]: the voxel offset of a dy from the group, ybase: the one that box row 0 starts at or before (ndy = 1: per dy)
+    int nstep, ndy, gtaps, a_rows, flip, wbox;  // wbox: taps per weight box (1, or all that lie in order)
+    int grow[9], yoff[3], ybase[3];
     int X, Y, Z;
     long long PX, PXY, R;
     int nseg, flags;
@@ -111,20 +118,40 @@ __device__ __forceinline__ uint32_t aligned_smem_base(unsigned char* raw)
     return (smem_u32(raw) + 1023u) & ~1023u;
 }
 
-__global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ ConvParams P)
+// the MMAs of NV input voxels, KS slices of 16 channels each; vstep / wstep: descriptor steps (mod 2^32) from one to the next
+template <int NV, int KS>
+__device__ __forceinline__ void mma_voxels(uint32_t leader, uint32_t d, uint64_t ad, uint64_t wd, uint32_t vstep,
+                                           uint32_t wstep, uint32_t idesc, uint32_t& acc)
+{
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+#pragma unroll
+        for (int kk = 0; kk < KS; ++kk) {
+            tc::mma_bf16(leader, d, ad + 2u * kk, wd + 2u * kk, idesc, acc);
+            acc = 1;
+        }
+        ad += (int32_t)vstep;
+        wd += (int32_t)wstep;
+    }
+}
+
+template <int G>
+__global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant__ ConvParams P)
 {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], accf[2], acce[2], done, wfull;
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
+    __shared__ __align__(16) float sbias[256];
 
     // (uniform by construction, so that the issue loops' values live in uniform registers)
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t sbase = aligned_smem_base(smem_raw);
     unsigned char* sgen = smem_raw + (sbase - smem_u32(smem_raw));
     const int mid = P.ntaps > 1 ? 1 : 0;                 // box row of the tile's first group
-    const uint32_t pad = (uint32_t)(P.G - 1);            // zero blocks of N rows before a weight stack
+    const uint32_t pad = (uint32_t)(G - 1);            // zero blocks of N rows before a weight stack
     const uint32_t per = (uint32_t)P.gtaps + pad;        // blocks from one stack to the next
+    const int nstack = P.nstep * P.ndy;                  // stacks of a channel chunk: the (dz, dy)
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < P.ns; ++s) {
@@ -133,7 +160,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&accf[b], 1);
-            mbar_init(&acce[b], 4);
+            mbar_init(&acce[b], 4 * kEpiSets);
         }
         mbar_init(&done, 1);
         mbar_init(&wfull, 1);
@@ -144,12 +171,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
         tc::tmem_alloc(&tmem_slot, 2 * P.tmem_cols);
         tc::tmem_relinquish();
     }
-    if (P.G > 1) {
+    if ((int)threadIdx.x < P.N) sbias[threadIdx.x] = P.bias ? P.bias[threadIdx.x] : 0.f;
+    if (G > 1) {
         // the zero rows of the weight stacks (the loads fill in the rest)
         const uint4 zero = make_uint4(0, 0, 0, 0);
         const uint32_t from = P.wres ? P.w_base : P.a_bytes, area = P.wres ? P.w_area : P.stage_bytes - P.a_bytes;
         for (int s = 0; s < (P.wres ? 1 : P.ns); ++s)
-            for (uint32_t q = threadIdx.x * 16u; q < area; q += kThreads * 16u)
+            for (uint32_t q = threadIdx.x * 16u; q < area; q += kConvThreads * 16u)
                 *reinterpret_cast<uint4*>(sgen + s * P.stage_bytes + from + q) = zero;
         fence_proxy_async();
     }
@@ -166,7 +194,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
                 return;
             }
             for (int t = 0; t < P.gtaps; ++t) {
-                const int q = P.flip || P.G == 1 ? t : P.gtaps - 1 - t;
+                const int q = P.flip || G == 1 ? t : P.gtaps - 1 - t;
                 tma_load_2d(w + (uint32_t)(t * P.N) * P.cb[i] * 2u, &P.wmap[i], bar, x, row0 + q * P.N);
             }
         };
@@ -174,7 +202,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
             mbar_arrive_expect_tx(&wfull, P.w_bytes);
             for (int i = 0; i < P.nin; ++i)
                 for (int cc = 0; cc < P.cin[i] / P.cb[i]; ++cc)
-                    for (int gq = 0; gq < P.ngroups; ++gq)
+                    for (int gq = 0; gq < nstack; ++gq)
                         load_taps(sgen + P.w_base + P.w_in[i] + cc * P.w_chunk[i] +
                                       (gq * per + pad) * (uint32_t)P.N * P.cb[i] * 2u,
                                   &wfull, i, cc, gq);
@@ -189,7 +217,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
                                        (P.wres ? 0u : (uint32_t)(P.gtaps * P.N) * P.cb[i] * 2u);
                 const uint32_t w_at = P.a_bytes + P.w_in[i] + pad * (uint32_t)P.N * P.cb[i] * 2u;
                 for (int cc = 0; cc < ncc; ++cc)
-                    for (int gq = 0; gq < P.ngroups; ++gq) {
+                    for (int gq = 0; gq < P.nstep; ++gq) {
                         if (it >= (uint32_t)P.ns && !tc::warp_wait(&empty[s], phase, P.err)) {
                             abort_flag = 1;
                             goto produced;
@@ -198,7 +226,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
                             mbar_arrive_expect_tx(&full[s], bytes);
                             unsigned char* a = sgen + s * P.stage_bytes;
                             const int arow = p0 + P.grow[gq];
-                            const CUtensorMap* map = &P.amap[i][P.gmap[gq]];
+                            const CUtensorMap* map = &P.amap[i];
                             for (int m = 0; m < nbox; ++m)
                                 tma_load_2d(a + m * P.box_bytes, map, &full[s], m * xstep + cc * P.cb[i], arow);
                             if (!P.wres) load_taps(a + w_at, &full[s], i, cc, gq);
@@ -221,8 +249,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
         if (P.wres) (void)tc::warp_wait(&wfull, 0, P.err);
     } else if (warp == 1) {
         uint32_t s = 0, phase = 0, tl = 0;
+        const uint32_t leader = tc::elect_one();
         if (P.wres && !tc::warp_wait(&wfull, 0, P.err)) abort_flag = 1;
-        const int G = P.G;
         for (int tile = blockIdx.x; tile < P.ntiles && __all_sync(0xffffffffu, !abort_flag); tile += gridDim.x, ++tl) {
             const uint32_t buf = tl & 1;
             if (tl >= 2 && !tc::warp_wait(&acce[buf], ((tl >> 1) + 1) & 1, P.err)) {
@@ -237,43 +265,62 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
                 const uint32_t rowa = P.ab[i] * 2u, roww = P.cb[i] * 2u, blk = ((uint32_t)P.N * roww) >> 4;
                 const uint64_t da = tc::sdesc(0, 16, 8 * rowa, tc::swizzle_code((int)rowa));
                 const uint64_t dw = tc::sdesc(0, 16, 8 * roww, tc::swizzle_code((int)roww));
-                const int ks = P.cb[i] / 16, ncc = P.cin[i] / P.cb[i], vsh = P.vsh[i], vmask = (1 << vsh) - 1;
-                // Input voxels -mid .. G - 1 + mid of the group, in the order of the taps: every output voxel sums its taps in
-                // the same order whatever G is (the others add zeros), so the sums do not depend on it
-                const int nvox = G + 2 * mid;
-                uint32_t ao[kMostVoxels], wo[kMostVoxels];
-#pragma unroll
-                for (int n = 0; n < kMostVoxels; ++n) {
-                    const int vi = P.flip ? G - 1 + mid - n : n - mid;
-                    const int slot = vi < 0 ? G - 1 : (vi == G ? 0 : vi), r = vi < 0 ? 0 : (vi == G ? 2 : mid);
-                    // (G = 1 keeps the taps in the order in which they lie)
-                    const int t0 = (int)pad + (G == 1 && !P.flip ? vi + mid : mid - vi);
-                    ao[n] = ((uint32_t)(slot >> vsh) * P.box_bytes + (uint32_t)r * rowa + (uint32_t)(slot & vmask) * roww) >> 4;
-                    wo[n] = n < nvox ? (uint32_t)t0 * blk : 0;
-                }
+                const int ks = P.cb[i] / 16, ncc = P.cin[i] / P.cb[i];
+                // first input voxel of a step's MMAs within the box, its step, and the same of the weight stacks. Every output
+                // voxel sums its taps in their order whatever G is (the others add zeros), so the sums do not depend on it.
+                // (G = 1 keeps the taps in the order in which they lie.)
+                const int vfirst = P.flip ? G - 1 + mid : -mid;
+                const uint32_t vstep = P.flip ? 0u - (roww >> 4) : roww >> 4, wstep = P.flip || G == 1 ? blk : 0u - blk;
+                const uint32_t wfirst = P.flip || G == 1 ? 0u : (pad + 2u * mid) * blk;
                 for (int cc = 0; cc < ncc; ++cc) {
                     uint32_t wr = (sbase + P.w_base + P.w_in[i] + cc * P.w_chunk[i]) >> 4;
-                    for (int gq = 0; gq < P.ngroups; ++gq) {
+                    for (int gq = 0, y1 = 0; gq < P.nstep; ++gq) {
                         if (!tc::warp_wait(&full[s], phase, P.err)) {
                             abort_flag = 1;
                             goto issued;
                         }
                         tc::fence_after_sync();
                         const uint32_t a = sbase + s * P.stage_bytes;
-                        const uint32_t w = P.wres ? wr : (a + P.a_bytes + P.w_in[i]) >> 4;
-                        wr += per * blk;
-                        const uint64_t ad = da + (a >> 4), wd = dw + w;
+                        for (int y = P.ndy == 1 ? y1 : 0, ye = P.ndy == 1 ? y1 + 1 : 3; y < ye; ++y) {
+                            const int v0 = P.yoff[y] - P.ybase[y] + vfirst;
+                            uint64_t wd = dw + ((P.wres ? wr : (a + P.a_bytes + P.w_in[i]) >> 4) + wfirst);
+                            wr += per * blk;
+                            if (P.nbox[i] == 1) {
+                                // one box: its rows follow one another, voxel v at v * roww
+                                uint64_t ad = da + ((a + (uint32_t)v0 * roww) >> 4);
+                                if (mid) {
+                                    if (ks == 4)
+                                        mma_voxels<G + 2, 4>(leader, d, ad, wd, vstep, wstep, P.idesc, acc);
+                                    else if (ks == 2)
+                                        mma_voxels<G + 2, 2>(leader, d, ad, wd, vstep, wstep, P.idesc, acc);
+                                    else
+                                        mma_voxels<G + 2, 1>(leader, d, ad, wd, vstep, wstep, P.idesc, acc);
+                                } else {
+                                    for (int kk = 0; kk < ks; ++kk)
+                                        mma_voxels<G, 1>(leader, d, ad + 2u * kk, wd + 2u * kk, vstep, wstep, P.idesc, acc);
+                                }
+                            } else {
+                                // voxel v in row v / G, box (v % G) / (voxels per box)
+                                const int vsh = P.vsh[i];
+                                const uint32_t boxes = P.box_bytes >> 4, a16 = a >> 4, ra = rowa >> 4, rw = roww >> 4;
 #pragma unroll
-                        for (int n = 0; n < kMostVoxels; ++n) {
-                            if (n >= nvox) break;
+                                for (int n = 0; n < G + 2; ++n) {
+                                    if (n >= G + 2 * mid) break;
+                                    const int v = P.flip ? v0 - n : v0 + n, slot = v & (G - 1);
+                                    const uint64_t ad = da + (a16 + (uint32_t)(slot >> vsh) * boxes + (uint32_t)(v / G) * ra +
+                                                              (uint32_t)(slot & ((1 << vsh) - 1)) * rw);
 #pragma unroll
-                            for (int kk = 0; kk < 4; ++kk) {
-                                if (kk >= ks) break;
-                                tc::mma_bf16(d, ad + (ao[n] + 2u * kk), wd + (wo[n] + 2u * kk), P.idesc, acc);
-                                acc = 1;
+                                    for (int kk = 0; kk < 4; ++kk) {
+                                        if (kk >= ks) break;
+                                        tc::mma_bf16(leader, d, ad + 2u * kk, wd + 2u * kk, P.idesc, acc);
+                                        acc = 1;
+                                    }
+                                    wd += (int32_t)wstep;
+                                }
                             }
                         }
-                        tc::mma_commit(&empty[s]);
+                        if (P.gtaps > 1 && ++y1 == 3) y1 = 0;
+                        tc::mma_commit(leader, &empty[s]);
                         if (++s == (uint32_t)P.ns) {
                             s = 0;
                             phase ^= 1u;
@@ -281,74 +328,80 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv(const __grid_constant__ Co
                     }
                 }
             }
-            tc::mma_commit(&accf[buf]);
+            tc::mma_commit(leader, &accf[buf]);
         }
     issued:
-        tc::mma_commit(&done);
+        tc::mma_commit(leader, &done);
         (void)tc::warp_wait(&done, 0, P.err);
     } else {
         const int q = warp & 3;  // tensor-memory lane quarter this warp may read
-        const int row = q * 32 + lane;
+        const int row = q * 32 + lane, set = (warp - 2) >> 2, cpv = P.N / 16, nchunk = G * cpv;
         uint32_t tl = 0;
         for (int tile = blockIdx.x; tile < P.ntiles; tile += gridDim.x, ++tl) {
             const uint32_t buf = tl & 1;
             if (!mbar_wait_bounded(&accf[buf], (tl >> 1) & 1, P.err)) abort_flag = 1;
             if (__any_sync(0xffffffffu, abort_flag)) break;
             tc::fence_after_sync();
-            const long long pg = ((long long)tile * kBM + row) * P.G;
+            const long long pg = ((long long)tile * kBM + row) * G;
             const bool valid = pg < P.R;  // (R is a multiple of G, below 2^30)
             const unsigned up = (unsigned)pg, pxy = (unsigned)P.PXY, px = (unsigned)P.PX;
-            int z = (int)(up / pxy), y = (int)((up - z * pxy) / px), x = (int)(up - z * pxy - y * px);
+            const int z0 = (int)(up / pxy), y0 = (int)((up - z0 * pxy) / px), x0 = (int)(up - z0 * pxy - y0 * px);
             const uint32_t taddr = tmem + buf * P.tmem_cols + ((uint32_t)(q * 32) << 16);
-            for (int vo = 0; vo < P.G; ++vo) {
-                const long long p = pg + vo;
-                const bool inside = x >= 1 && x <= P.X && y >= 1 && y <= P.Y && z >= 1 && z <= P.Z;
-                if (++x == (int)px) {
-                    x = 0;
-                    if (++y == (int)(pxy / px)) {
+            // 16 columns at a time, shared out over the sets of warps
+            for (int ch = set; ch < nchunk; ch += kEpiSets) {
+                const int vo = ch / cpv, col = 16 * (ch - vo * cpv);
+                float v[16];
+                tc::tmem_ld16(taddr + (uint32_t)(16 * ch), v);
+                if (!valid) continue;
+                int x = x0 + vo, y = y0, z = z0;
+                if (x >= (int)px) {  // (G <= 4 voxels cross the end of one row at most)
+                    x -= (int)px;
+                    if (++y == P.Y + 2) {
                         y = 0;
                         ++z;
                     }
                 }
-                for (int sg = 0; sg < P.nseg; ++sg) {
-                    const int nc = P.seg_nc[sg], c0 = P.seg_c0[sg];
-                    __nv_bfloat16* orow = P.out[sg] + p * nc;
-                    __nv_bfloat16* arow = P.aux[sg] ? P.aux[sg] + p * nc : nullptr;
-                    for (int c = 0; c < nc; c += 16) {
-                        float v[16];
-                        tc::tmem_ld16(taddr + (uint32_t)(vo * P.N + c0 + c), v);
-                        if (!valid) continue;
-                        if (!inside) {
+                const bool inside = x >= 1 && x <= P.X && y >= 1 && y <= P.Y && z >= 1 && z <= P.Z;
+                const int sg = P.nseg > 1 && col >= P.seg_c0[1] ? 1 : 0;
+                const int nc = P.seg_nc[sg], c = col - P.seg_c0[sg];
+                const long long at = (pg + vo) * nc + c;
+                __nv_bfloat16* orow = P.out[sg] + at;
+                __nv_bfloat16* arow = P.aux[sg] ? P.aux[sg] + at : nullptr;
+                if (!inside) {
 #pragma unroll
-                            for (int e = 0; e < 16; ++e) v[e] = 0.f;
-                            store16(orow + c, v);
-                            if (arow && (P.flags & kGelu)) store16(arow + c, v);
-                            continue;
-                        }
-                        if (P.bias) {
+                    for (int e = 0; e < 16; ++e) v[e] = 0.f;
+                    store16(orow, v);
+                    if (arow && (P.flags & kGelu)) store16(arow, v);
+                    continue;
+                }
+                if (P.bias) {
 #pragma unroll
-                            for (int e = 0; e < 16; ++e) v[e] += __ldg(P.bias + c0 + c + e);
-                        }
-                        if (P.flags & kAccum) {
-                            float o[16];
-                            load16(orow + c, o);
-#pragma unroll
-                            for (int e = 0; e < 16; ++e) v[e] += o[e];
-                        }
-                        if (P.flags & kDGelu) {
-                            float a[16];
-                            load16(arow + c, a);
-#pragma unroll
-                            for (int e = 0; e < 16; ++e) v[e] *= dgelu_f(a[e]);
-                        }
-                        if (P.flags & kGelu) {
-                            if (arow) store16(arow + c, v);
-#pragma unroll
-                            for (int e = 0; e < 16; ++e) v[e] = gelu_f(v[e]);
-                        }
-                        store16(orow + c, v);
+                    for (int e = 0; e < 16; e += 4) {
+                        const float4 bq = *reinterpret_cast<const float4*>(sbias + col + e);
+                        v[e] += bq.x;
+                        v[e + 1] += bq.y;
+                        v[e + 2] += bq.z;
+                        v[e + 3] += bq.w;
                     }
                 }
+                if (P.flags & kAccum) {
+                    float o[16];
+                    load16(orow, o);
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) v[e] += o[e];
+                }
+                if (P.flags & kDGelu) {
+                    float a[16];
+                    load16(arow, a);
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) v[e] *= dgelu_f(a[e]);
+                }
+                if (P.flags & kGelu) {
+                    if (arow) store16(arow, v);
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) v[e] = gelu_f(v[e]);
+                }
+                store16(orow, v);
             }
             tc::fence_before_sync();
             __syncwarp();
@@ -456,6 +509,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad(const __grid_constant__ W
         // MN-major swizzled operands: MN atoms at LBO = atom bytes, 8-row K groups at SBO
         const uint64_t da = tc::sdesc(0, a_atom_bytes, 8u * P.ca * 2u, tc::swizzle_code(P.ca * 2));
         const uint64_t dg = tc::sdesc(0, g_atom_bytes, 8u * P.cg * 2u, tc::swizzle_code(P.cg * 2));
+        const uint32_t leader = tc::elect_one();
         const uint32_t stepa = 16u * P.ca * 2u >> 4, stepg = 16u * P.cg * 2u >> 4;
         uint32_t s = 0, phase = 0, acc = 0;
         for (int ks = k_begin; ks < k_end; ++ks) {
@@ -468,18 +522,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad(const __grid_constant__ W
             uint64_t ad = da + (a >> 4), bd = dg + ((a + P.a_bytes) >> 4);
 #pragma unroll
             for (int kk = 0; kk < kWgradRows / 16; ++kk) {
-                tc::mma_bf16(tmem, ad, bd, P.idesc, acc);
+                tc::mma_bf16(leader, tmem, ad, bd, P.idesc, acc);
                 acc = 1;
                 ad += stepa;
                 bd += stepg;
             }
-            tc::mma_commit(&empty[s]);
+            tc::mma_commit(leader, &empty[s]);
             if (++s == (uint32_t)P.ns) {
                 s = 0;
                 phase ^= 1u;
             }
         }
-        tc::mma_commit(&accf);
+        tc::mma_commit(leader, &accf);
     } else {
         const int q = warp & 3;
         const int row = q * 32 + lane;  // M row = (tap in tile, input channel)
@@ -497,6 +551,153 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad(const __grid_constant__ W
 #pragma unroll
             for (int e = 0; e < 16; ++e) atomicAdd(dst + (long long)e * P.cin_tot, v[e]);
         }
+    }
+
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == 1) {
+        tc::fence_after_sync();
+        tc::tmem_dealloc(tmem, P.tmem_cols);
+    }
+}
+
+// The same for 16 and 32 input channels, with the groups of k_conv as K: A = the input's rows of G voxels (64 elements),
+// two rows (2 G voxels, M = 128), B = the gradient's rows (N = G cout). One MMA sums 16 groups for a (dz, dy): D[(w, ci)]
+// [(vo, co)], whose entries with the input voxel w next to the output voxel vo are the 3 taps dx. 3 boxes of 64 to 130 rows
+// of 128 bytes per 256 voxels and 12 MMAs, where the taps one by one took 36 boxes of 64 32-byte rows and 64 MMAs (451 us
+// for 16 x 16 channels at 128^3, now 70 us). The window of 2 G voxels starts at a voxel of one position within a group for
+// all three dy (base), so they share a box.
+struct WgradGroupParams {
+    CUtensorMap amap, gmap;
+    int cin, ci0, cin_tot, cout, G, ntaps, N;
+    int ndy, box_rows;             // dy of a step: 3, or 1 (a 1x1x1 convolution)
+    int row0[3];                   // per dz: first box row relative to the step's first group
+    int yrow[3], ydelta[3];        // per dy: its row within the box; the window's first voxel relative to the group
+    int cg, natom_g;
+    int k_steps_per_cta, k_steps_total;
+    float* dw;
+    unsigned* err;
+    int ns;
+    uint32_t a_bytes, g_atom_bytes, stage_bytes, tmem_cols, idesc;
+};
+
+__global__ void __launch_bounds__(kThreads, 1) k_wgrad_groups(const __grid_constant__ WgradGroupParams P)
+{
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], accf;
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile int abort_flag;
+
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const uint32_t sbase = aligned_smem_base(smem_raw);
+    unsigned char* sgen = smem_raw + (sbase - smem_u32(smem_raw));
+    const int dz = blockIdx.x;
+    const int k_begin = blockIdx.y * P.k_steps_per_cta;
+    const int k_end = min(P.k_steps_total, k_begin + P.k_steps_per_cta);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < P.ns; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(&accf, 1);
+        abort_flag = 0;
+        mbar_fence_init();
+    }
+    if (warp == 1) {
+        tc::tmem_alloc(&tmem_slot, P.tmem_cols);
+        tc::tmem_relinquish();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = tmem_slot;
+
+    if (warp == 0) {
+        uint32_t it = 0, s = 0, phase = 1;  // stage of the step, parity of its last release
+        const uint32_t bytes = (uint32_t)P.box_rows * 128u + P.g_atom_bytes * P.natom_g;
+        const int row0 = P.row0[dz];
+        for (int ks = k_begin; ks < k_end; ++ks, ++it) {
+            if (it >= (uint32_t)P.ns && !tc::warp_wait(&empty[s], phase, P.err)) {
+                abort_flag = 1;
+                break;
+            }
+            if (tc::elect_one()) {
+                const int q0 = ks * kWgradRows;
+                mbar_arrive_expect_tx(&full[s], bytes);
+                unsigned char* a = sgen + s * P.stage_bytes;
+                tma_load_2d(a, &P.amap, &full[s], 0, q0 + row0);
+                for (int m = 0; m < P.natom_g; ++m)
+                    tma_load_2d(a + P.a_bytes + m * P.g_atom_bytes, &P.gmap, &full[s], m * P.cg, q0);
+            }
+            __syncwarp();
+            if (++s == (uint32_t)P.ns) {
+                s = 0;
+                phase ^= 1u;
+            }
+        }
+        for (uint32_t q = 0; q < (uint32_t)P.ns && q < it; ++q) {
+            const uint32_t last = it - 1 - ((it - 1 - q) % P.ns);
+            (void)tc::warp_wait(&full[q], (last / P.ns) & 1, P.err);
+        }
+    } else if (warp == 1) {
+        // MN-major operands: the second atom of A is the next row (LBO one row), 8-row K groups at SBO
+        const uint32_t leader = tc::elect_one();
+        const uint64_t da = tc::sdesc(0, 128, 1024, tc::kSwizzle128);
+        const uint64_t dg = tc::sdesc(0, P.g_atom_bytes, 8u * P.cg * 2u, tc::swizzle_code(P.cg * 2));
+        const uint32_t stepg = 16u * P.cg * 2u >> 4;
+        const int ndy = P.ndy;
+        const uint32_t y0 = (uint32_t)P.yrow[0] * 8u, y1 = (uint32_t)P.yrow[1] * 8u, y2 = (uint32_t)P.yrow[2] * 8u;
+        uint32_t s = 0, phase = 0, acc = 0;
+        for (int ks = k_begin; ks < k_end; ++ks) {
+            if (!tc::warp_wait(&full[s], phase, P.err)) {
+                abort_flag = 1;
+                break;
+            }
+            tc::fence_after_sync();
+            const uint32_t a = sbase + s * P.stage_bytes;
+            const uint64_t ad = da + (a >> 4);
+            uint64_t bd = dg + ((a + P.a_bytes) >> 4);
+#pragma unroll
+            for (int kk = 0; kk < kWgradRows / 16; ++kk) {
+                tc::mma_bf16(leader, tmem, ad + (y0 + 128u * kk), bd, P.idesc, acc);
+                if (ndy > 1) {
+                    tc::mma_bf16(leader, tmem + P.N, ad + (y1 + 128u * kk), bd, P.idesc, acc);
+                    tc::mma_bf16(leader, tmem + 2 * P.N, ad + (y2 + 128u * kk), bd, P.idesc, acc);
+                }
+                acc = 1;
+                bd += stepg;
+            }
+            tc::mma_commit(leader, &empty[s]);
+            if (++s == (uint32_t)P.ns) {
+                s = 0;
+                phase ^= 1u;
+            }
+        }
+        tc::mma_commit(leader, &accf);
+    } else {
+        const int q = warp & 3;
+        const int row = q * 32 + lane;  // M row = (window voxel, input channel)
+        const bool ok = tc::warp_wait(&accf, 0, P.err) && k_end > k_begin;
+        tc::fence_after_sync();
+        const int w = row / P.cin, ci = row % P.cin;
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16);
+        const bool good = __all_sync(0xffffffffu, ok && !abort_flag);
+        for (int y = 0; y < P.ndy; ++y)
+            for (int vo = 0; vo < P.G; ++vo) {
+                const int dx = P.ydelta[y] + w - vo;
+                const bool store = good && (P.ntaps == 1 ? dx == 0 : dx >= -1 && dx <= 1);
+                if (!__any_sync(0xffffffffu, store)) continue;
+                const int tap = P.ntaps == 1 ? 0 : 9 * dz + 3 * y + dx + 1;
+                for (int c = 0; c < P.cout; c += 16) {
+                    float v[16];
+                    tc::tmem_ld16(taddr + (uint32_t)(y * P.N + vo * P.cout + c), v);
+                    if (!store) continue;
+                    float* dst = P.dw + ((long long)tap * P.cout + c) * P.cin_tot + P.ci0 + ci;
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) atomicAdd(dst + (long long)e * P.cin_tot, v[e]);
+                }
+            }
     }
 
     tc::fence_before_sync();
@@ -602,27 +803,15 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
     P.ntaps = L.ntaps;
     P.N = L.N;
     P.flip = L.flip;
-    P.ngroups = L.ntaps == 27 ? 9 : 1;
     P.gtaps = L.ntaps == 27 ? 3 : 1;
-    P.a_rows = L.ntaps == 27 ? kBM + 2 : kBM;
+    const int nstack = L.ntaps == 27 ? 9 : 1;
     int off[27];
     tap_offsets(L.g, L.ntaps, L.flip, off);
-    // voxels per GEMM row: rows of 64 elements (128 bytes) for the narrowest input, where the grid splits into such groups,
-    // the (dz, dy) offsets fall on at most two positions within a group and the columns stay within an MMA's 256 (twice
-    // that is the tensor memory)
-    int residue = 0;
-    for (P.G = 64 / cmin;; P.G >>= 1) {
-        bool ok = L.g.R % P.G == 0 && P.G * L.N <= 256;
-        residue = 0;
-        for (int gq = 0; gq < P.ngroups; ++gq) {
-            const int c = L.ntaps == 27 ? off[3 * gq + 1] : 0, r = ((c % P.G) + P.G) % P.G;
-            if (r && residue && r != residue) ok = false;
-            if (r) residue = r;
-            P.gmap[gq] = r ? 1 : 0;
-            P.grow[gq] = (c - r) / P.G - (L.ntaps == 27 ? 1 : 0);
-        }
-        if (ok || P.G == 1) break;
-    }
+    // voxels per GEMM row: rows of 64 elements (128 bytes) for the narrowest input, where the grid and its planes split into
+    // such groups and the columns stay within an MMA's 256 (twice that is the tensor memory)
+    for (P.G = 64 / cmin; P.G > 1; P.G >>= 1)
+        if (L.g.R % P.G == 0 && L.g.PXY % P.G == 0 && P.G * L.N <= 256) break;
+    auto rows_of = [&](int v) { return (int)((v >= 0 ? v : v - P.G + 1) / P.G); };  // floor
     P.ntiles = (int)((L.g.R / P.G + kBM - 1) / kBM);
     P.wbox = (P.flip || P.G == 1) && P.gtaps * L.N <= 256 ? P.gtaps : 1;
     uint32_t wres_bytes = 0;
@@ -634,16 +823,10 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
         }
         abmax = std::max(abmax, P.ab[i]);
         nbmax = std::max(nbmax, P.nbox[i]);
-        for (int m = 0; m < 2; ++m) {
-            const int r = m ? residue : 0;
-            const int rc = encode_rows(L.in[i] + (size_t)r * L.cin[i], P.G * L.cin[i], (L.g.R - r) / P.G, P.ab[i], P.a_rows,
-                                       &P.amap[i][m]);
-            if (rc) return rc;
-        }
         const int rc = encode_rows(L.w, cin_tot, (long long)L.ntaps * L.N, P.cb[i], P.wbox * L.N, &P.wmap[i]);
         if (rc) return rc;
         P.w_in[i] = wres_bytes;
-        P.w_chunk[i] = ((uint32_t)((P.gtaps + P.G - 1) * P.ngroups + P.G - 1) * L.N * P.cb[i] * 2u + 1023u) & ~1023u;
+        P.w_chunk[i] = ((uint32_t)((P.gtaps + P.G - 1) * nstack + P.G - 1) * L.N * P.cb[i] * 2u + 1023u) & ~1023u;
         wres_bytes += P.w_chunk[i] * (L.cin[i] / P.cb[i]);
         P.w_bytes += (uint32_t)L.ntaps * L.N * L.cin[i] * 2u;
     }
@@ -657,14 +840,46 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
     P.flags = L.flags;
     P.bias = L.bias;
     P.err = L.err;
-    P.box_bytes = ((uint32_t)P.a_rows * abmax * 2u + 1023u) & ~1023u;
-    P.a_bytes = nbmax * P.box_bytes;
     P.tmem_cols = pow2_cols(P.G * L.N);
     P.idesc = tc::idesc_bf16(kBM, P.G * L.N, 0, 0);
     P.w_area = wres_bytes;
     // weights resident where at least 3 activation stages fit beside them, else with each step
     const uint32_t max_smem = 220 * 1024;
+    auto box = [&](int rows) {
+        P.a_rows = rows;
+        P.box_bytes = ((uint32_t)rows * abmax * 2u + 1023u) & ~1023u;
+        P.a_bytes = nbmax * P.box_bytes;
+    };
+    const int PX = (int)L.g.PX, mid = L.ntaps == 27 ? 1 : 0;
+    box(kBM + (mid ? 2 + (P.G > 1) : 0));
     P.wres = wres_bytes + 3 * P.a_bytes + 1024 <= max_smem;
+    P.ndy = 1;
+    if (mid && P.wres) {
+        // one box for the three dy of a dz where its rows fit a TMA box and two stages stay: the rows of neighbouring dy
+        // overlap (194 rows instead of 3 x 130 at 128^3), and L2 reads bounded the level-0 convolutions at 5 TB/s
+        const int rows = kBM + rows_of(PX + P.G) - rows_of(-PX - 1), was = P.a_rows;
+        if (rows <= 256) {
+            box(rows);
+            P.ndy = 3;
+            if (wres_bytes + 2 * P.a_bytes + 1024 > max_smem) {
+                box(was);
+                P.ndy = 1;
+            }
+        }
+    }
+    P.nstep = nstack / P.ndy;
+    for (int y = 0; y < 3; ++y) {
+        P.yoff[y] = mid ? off[3 * (3 + y) + 1] : 0;  // dz = 0
+        P.ybase[y] = rows_of(P.ndy == 3 ? -PX - 1 : P.yoff[y] - mid) * P.G;
+    }
+    for (int q = 0; q < P.nstep; ++q) {
+        const int dz = mid ? off[3 * (3 * (q * P.ndy / 3) + 1) + 1] : 0;  // a multiple of G
+        P.grow[q] = dz / P.G + P.ybase[P.ndy == 3 ? 0 : (mid ? q % 3 : 0)] / P.G;
+    }
+    for (int i = 0; i < L.nin; ++i) {
+        const int rc = encode_rows(L.in[i], P.G * L.cin[i], L.g.R / P.G, P.ab[i], P.a_rows, &P.amap[i]);
+        if (rc) return rc;
+    }
     P.stage_bytes = P.a_bytes;
     if (!P.wres) {
         uint32_t w = 0;
@@ -684,12 +899,84 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
     const size_t smem = (size_t)P.w_base + (P.wres ? wres_bytes : 0) + 1024;
     static bool attr_set = false;
     if (!attr_set) {
-        GBP_CUDA(cudaFuncSetAttribute(k_conv, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+        for (auto k : {k_conv<1>, k_conv<2>, k_conv<4>})
+            GBP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         attr_set = true;
     }
     const int grid = std::min(P.ntiles, sm_count_cached());
-    k_conv<<<grid, kThreads, smem, st>>>(P);
+    (P.G == 4 ? k_conv<4> : P.G == 2 ? k_conv<2> : k_conv<1>)<<<grid, kConvThreads, smem, st>>>(P);
     GBP_CUDA(cudaGetLastError());
+    return GBP_OK;
+}
+
+// The grouped weight gradient for 16 and 32 input channels; *done = false: not for this grid, nothing launched
+static int wgrad_groups(const WgradLaunch& L, cudaStream_t st, bool* done)
+{
+    *done = false;
+    const int G = 64 / std::max(L.cin, 1), PX = (int)L.g.PX;
+    if ((L.cin != 16 && L.cin != 32) || L.g.R % G || L.g.PXY % G || 3 * G * L.cout > 512 || G * L.cout > 256) return GBP_OK;
+    WgradGroupParams P;
+    memset(&P, 0, sizeof(P));
+    auto rows_of = [&](int v) { return (v >= 0 ? v : v - G + 1) / G; };  // floor
+    const int mid = L.ntaps == 27 ? 1 : 0;
+    P.ndy = mid ? 3 : 1;
+    // the position within a group at which every dy's window of 2 G voxels can start: at or before its voxel -1, ending at or
+    // after its voxel G
+    int base = -1;
+    for (int b = 0; b < G && base < 0; ++b) {
+        bool all = true;
+        for (int y = 0; y < P.ndy; ++y) {
+            const int first = (mid ? (y - 1) * PX : 0) - mid;  // the window's start lies in (first - (G - 2 mid) - 1, first]
+            const int start = b + rows_of(first - b) * G;
+            all = all && start >= first - (G - 2 * mid);
+        }
+        if (all) base = b;
+    }
+    if (base < 0) return GBP_OK;
+    int start[3], lo = 0, hi = 0;
+    for (int y = 0; y < P.ndy; ++y) {
+        const int off = mid ? (y - 1) * PX : 0;
+        start[y] = rows_of(off - mid - base);
+        P.ydelta[y] = base + start[y] * G - off;
+        lo = y ? std::min(lo, start[y]) : start[y];
+        hi = y ? std::max(hi, start[y]) : start[y];
+    }
+    P.box_rows = kWgradRows + hi - lo + 1;
+    if (P.box_rows > 256) return GBP_OK;
+    for (int y = 0; y < P.ndy; ++y) P.yrow[y] = start[y] - lo;
+    for (int z = 0; z < 3; ++z) P.row0[z] = mid ? (int)((z - 1) * (L.g.PXY / G)) + lo : lo;
+    P.cin = L.cin;
+    P.ci0 = L.ci0;
+    P.cin_tot = L.cin_tot;
+    P.cout = L.cout;
+    P.G = G;
+    P.ntaps = L.ntaps;
+    P.N = G * L.cout;
+    P.cg = std::min(64, P.N);
+    P.natom_g = P.N / P.cg;
+    int rc = encode_rows(L.in + (size_t)base * L.cin, 64, (L.g.R - base) / G, 64, P.box_rows, &P.amap);
+    if (!rc) rc = encode_rows(L.gout, P.N, L.g.R / G, P.cg, kWgradRows, &P.gmap);
+    if (rc) return rc;
+    P.dw = L.dw;
+    P.err = L.err;
+    P.a_bytes = ((uint32_t)P.box_rows * 128u + 1023u) & ~1023u;
+    P.g_atom_bytes = (uint32_t)kWgradRows * P.cg * 2u;
+    P.stage_bytes = P.a_bytes + ((P.g_atom_bytes * P.natom_g + 1023u) & ~1023u);
+    P.tmem_cols = pow2_cols(P.ndy * P.N);
+    P.idesc = tc::idesc_bf16(kBM, P.N, 1, 1);
+    P.ns = std::min(kMaxStages, (int)((200 * 1024 - 1024) / P.stage_bytes));
+    P.k_steps_total = (int)((L.g.R / G + kWgradRows - 1) / kWgradRows);
+    const int nz = mid ? 3 : 1, want = std::max(1, sm_count_cached() / nz);
+    P.k_steps_per_cta = std::max(8, (P.k_steps_total + want - 1) / want);
+    const int splits = (P.k_steps_total + P.k_steps_per_cta - 1) / P.k_steps_per_cta;
+    static bool attr_set = false;
+    if (!attr_set) {
+        GBP_CUDA(cudaFuncSetAttribute(k_wgrad_groups, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        attr_set = true;
+    }
+    k_wgrad_groups<<<dim3(nz, splits), kThreads, (size_t)P.ns * P.stage_bytes + 1024, st>>>(P);
+    GBP_CUDA(cudaGetLastError());
+    *done = true;
     return GBP_OK;
 }
 
@@ -701,6 +988,9 @@ int conv3d_wgrad(const WgradLaunch& L, cudaStream_t st)
         set_error("conv3d_wgrad: bad launch shape");
         return GBP_BAD_ARG;
     }
+    bool done = false;
+    const int grc = wgrad_groups(L, st, &done);
+    if (grc || done) return grc;
     WgradParams P;
     memset(&P, 0, sizeof(P));
     P.ca = chunk_of(L.cin);

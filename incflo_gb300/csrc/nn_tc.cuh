@@ -60,27 +60,29 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem] * B[smem]^T. Called by a whole warp, issued by one elected lane: descriptors and addresses are
-// uniform-register operands, which a value computed under a one-lane branch has to be moved into, one round trip each
-// (150 to 300 cycles per MMA; see k_conv).
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc)
+// D[tmem] (+)= A[smem] * B[smem]^T. Called by a whole warp, issued by the lane with leader != 0 (elect_one): descriptors
+// and addresses are uniform-register operands, which a value computed under a one-lane branch has to be moved into, one
+// round trip each (150 to 300 cycles per MMA; see k_conv).
+__device__ __forceinline__ void mma_bf16(uint32_t leader, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                         uint32_t acc)
 {
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc), "r"(leader)
         : "memory");
 }
 
-// arrive on *bar once every MMA issued so far by this warp's elected lane has completed (called by the whole warp)
-__device__ __forceinline__ void mma_commit(uint64_t* bar)
+// arrive on *bar once every MMA issued so far by the leader has completed (called by the whole warp)
+__device__ __forceinline__ void mma_commit(uint32_t leader, uint64_t* bar)
 {
     asm volatile(
         "{\n\t.reg .pred q;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
+        "r"(leader)
         : "memory");
 }
 
