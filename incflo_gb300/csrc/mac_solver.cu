@@ -390,11 +390,12 @@ void MacSolver::add_vcycle_correction(const double* r, double* e, double sc)
     }
 }
 
-void MacSolver::vcycles32(const float* b32)
+void MacSolver::vcycles32(const float* b32, cudaStream_t s)
 {
-    cap_or_st = st;
+    cap_or_st = s;
     vcycle<float>(0, b32, true);
     for (int c = 1; c < opt.ir_inner_cycles; ++c) vcycle<float>(0, b32, false);
+    cap_or_st = st;
 }
 
 void MacSolver::eb_refresh_beta()

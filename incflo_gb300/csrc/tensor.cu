@@ -383,6 +383,11 @@ TensorSolver::~TensorSolver()
     if (hnorm) cudaFreeHost(hnorm);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
+    if (fork) cudaEventDestroy(fork);
+    for (int q = 0; q < 2; ++q) {
+        if (join[q]) cudaEventDestroy(join[q]);
+        if (side[q]) cudaStreamDestroy(side[q]);
+    }
 }
 
 int TensorSolver::init(const gbp_geometry& g, const int bc_lo[9], const int bc_hi[9], const gbp_options& o,
@@ -455,6 +460,11 @@ int TensorSolver::init(const gbp_geometry& g, const int bc_lo[9], const int bc_h
     GBP_CUDA(cudaMallocHost(&hnorm, 4 * sizeof(unsigned long long)));
     GBP_CUDA(cudaEventCreate(&ev0));
     GBP_CUDA(cudaEventCreate(&ev1));
+    GBP_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    for (int q = 0; q < 2; ++q) {
+        GBP_CUDA(cudaStreamCreateWithFlags(&side[q], cudaStreamNonBlocking));
+        GBP_CUDA(cudaEventCreateWithFlags(&join[q], cudaEventDisableTiming));
+    }
     return GBP_OK;
 }
 
@@ -600,10 +610,17 @@ int TensorSolver::solve(const gbp_array4& rhs_in, gbp_array4& vel, gbp_stats* st
                 GBP_CUDA(cudaMemsetAsync(e32[c], 0, sizeof(float) * cnt, st));
             }
             for (int q = 0; q < kInner; ++q) {
+                // The blocks do not depend on one another and their small levels leave most of the chip idle (half of a V-cycle's
+                // time at 256 x 128 x 128): each on a stream of its own, all back on st before the next residual
+                GBP_CUDA(cudaEventRecord(fork, st));
                 for (int c = 0; c < 3; ++c) {
-                    comp[c].vcycles32(q == 0 ? b32[c] : r32[c]);
-                    k_tensor_acc32<<<nb, 256, 0, st>>>(cnt, comp[c].correction32(), e32[c]);
+                    const cudaStream_t s = c ? side[c - 1] : st;
+                    if (c) GBP_CUDA(cudaStreamWaitEvent(s, fork, 0));
+                    comp[c].vcycles32(q == 0 ? b32[c] : r32[c], s);
+                    k_tensor_acc32<<<nb, 256, 0, s>>>(cnt, comp[c].correction32(), e32[c]);
+                    if (c) GBP_CUDA(cudaEventRecord(join[c - 1], s));
                 }
+                for (int q2 = 0; q2 < 2; ++q2) GBP_CUDA(cudaStreamWaitEvent(st, join[q2], 0));
                 if (q + 1 < kInner) {
                     tensor_ghosts<float>(g, bclo, bchi, e32, vel, 1, st);
                     tensor_fluxes<float>(g, e32, eta32, fl32, st);

@@ -72,6 +72,9 @@ private:
     bool ready = false;
     unsigned long long *dnorm = nullptr, *hnorm = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    // the blocks' V-cycles of a step run side by side: component 0 on st, 1 and 2 on these
+    cudaStream_t side[2] = {};
+    cudaEvent_t fork = nullptr, join[2] = {};
 };
 
 }  // namespace gbp
