@@ -58,7 +58,7 @@ private:
     double* r[3] = {};
     double* eta[3] = {};
     double* fl[3][3] = {};  // [face direction][component]: tau_{c,d} on the faces of direction d
-    // the mixed form's FP32 inner steps: correction, scaled FP64 residual, FP32 residual, face eta, fluxes
+    // the mixed form's FP32 inner steps: correction, scaled FP64 residual, FP32 residual, face eta
 #ifndef GBP_TENSOR_INNER
 #define GBP_TENSOR_INNER 6
 #endif
@@ -67,7 +67,6 @@ private:
     float* b32[3] = {};
     float* r32[3] = {};
     float* eta32[3] = {};
-    float* fl32[3][3] = {};
     double alpha = 0.0, beta = 0.0;
     bool ready = false;
     unsigned long long *dnorm = nullptr, *hnorm = nullptr;
