@@ -150,9 +150,9 @@ __device__ __forceinline__ bool coarse_to_g1(const NodalGeom& g1, const int o[3]
 }
 
 // out (whole coarse level) = the coarse unknowns' own residual + the full weighting r1 of the fine
-// unknowns' residual (on g1, the fine box coarsened by 2), except on fixed nodes
+// unknowns' residual (on g1, the fine box coarsened by 2), except on fixed nodes, times relax
 __global__ void k_amr_combine(NodalGeom gc, NodalGeom g1, const unsigned char* __restrict__ ccls, int o0, int o1,
-                              int o2, const float* __restrict__ rc, const float* __restrict__ r1, float* out)
+                              int o2, const float* __restrict__ rc, const float* __restrict__ r1, float relax, float* out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -164,7 +164,7 @@ __global__ void k_amr_combine(NodalGeom gc, NodalGeom g1, const unsigned char* _
     const int o[3] = {o0, o1, o2}, I[3] = {i, j, k};
     int q[3];
     if (c != C_FIXED && coarse_to_g1(g1, o, I, q)) v += r1[pidx(g1.sy, g1.sz, q[0], q[1], q[2])];
-    store_node(out, gc, i, j, k, v);
+    store_node(out, gc, i, j, k, relax * v);
 }
 
 // x1 (g1, the fine box coarsened by 2) = the coarse-level values at the same positions (aliases written)
@@ -347,6 +347,13 @@ __global__ void k_amr_rhs32_fine(NodalGeom gf, const unsigned char* __restrict__
     if (i >= gf.nu[0] || j >= gf.nu[1] || k >= gf.nu[2]) return;
     const long long p = pidx(gf.sy, gf.sz, i, j, k);
     store_node(out, gf, i, j, k, fcls[p] == F_DOF ? (float)(scale * r[p]) : 0.f);
+}
+
+// r = b + w r over whole padded arrays (the right-hand side of a relaxed step's fine sweeps)
+__global__ void k_amr_relax(long long count, const float* __restrict__ b, float w, float* __restrict__ r)
+{
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t < count) r[t] = fmaf(w, r[t], b[t]);
 }
 
 // acc += e over whole padded arrays (the fine hierarchy's correction: zero on the masked nodes)
@@ -1181,14 +1188,18 @@ void CompositeNodal::issue_outer32(double scale32, int inner)
         resid32(gc, scm32, ec32, bc32, rc32);
         k_amr_sync<<<gnodes(gc), kB3, 0, st>>>(gc, gf, ccls, fcls, off[0], off[1], off[2], (const float*)rm32, rc32);
     };
+    const bool relaxed = xfer1 && kFineSweeps > 0 && fin.sweeps32_in_place(kFineSweeps);
     for (int q = 0; q < inner; ++q) {
+        // Relaxed steps (cheb_step; the error factors of a step lie in [0, 0.25]): the coarse right-hand side takes the weight,
+        // the fine sweeps the right-hand side b + (w - 1) r. The first keeps w = 1, next to its Chebyshev point.
+        const double w = relaxed && q > 0 ? cheb_step(q, inner, kRelaxLow, 1.0) : 1.0;
         const float* rc = q == 0 ? bc32 : rc32;
         const float* rf = q == 0 ? bf32 : rf32;
         const int o0 = off[0] / 2, o1 = off[1] / 2, o2 = off[2] / 2;
         if (xfer1) {
             // rf holds the fine unknowns' residuals and 0 elsewhere (bf32, or the masked fine residual)
             nodal_restrict<float>(gf_nomask, g1n, rf, x1_32, st);
-            k_amr_combine<<<gnodes(gc), kB3, 0, st>>>(gc, g1n, ccls, o0, o1, o2, rc, x1_32, rcf32);
+            k_amr_combine<<<gnodes(gc), kB3, 0, st>>>(gc, g1n, ccls, o0, o1, o2, rc, x1_32, (float)w, rcf32);
         } else {
             restrict_to_coarse(rc, rf, rcf32);
         }
@@ -1211,7 +1222,8 @@ void CompositeNodal::issue_outer32(double scale32, int inner)
         }
         // the fine sweeps on e_f itself, which the mask holds on the interface: sweeps from zero on its residual and
         // their sum are the same step with three passes more (residual 196, first sweep 279, sum 152 of 780 us)
-        if (kFineSweeps == 0 || !fin.sweep32_in_place(bf32, ef32, kFineSweeps, st)) {
+        if (w != 1.0) k_amr_relax<<<nfb_, kT, 0, st>>>(gf.count, bf32, (float)(w - 1.0), rf32);
+        if (kFineSweeps == 0 || !fin.sweep32_in_place(w != 1.0 ? rf32 : bf32, ef32, kFineSweeps, st)) {
             resid32(xfer1 ? gf : gf_nomask, fin.sigma32(), ef32, bf32, rf32);
             if (kFineSweeps > 0)
                 fin.smooth32(rf32, kFineSweeps, st);

@@ -101,9 +101,10 @@ private:
     template <typename T>
     void restrict_to_coarse(const T* rc, const T* rf, T* out);
 #ifndef GBP_AMR_INNER
-#define GBP_AMR_INNER 8
+#define GBP_AMR_INNER 5
 #endif
     static constexpr int kInner = GBP_AMR_INNER, kMostInner = kInner + 2;
+    static constexpr double kRelaxLow = 0.75;  // lowest eigenvalue of a two-level step times A that the relaxation aims at
 #ifndef GBP_AMR_FINE_SWEEPS
 #define GBP_AMR_FINE_SWEEPS 2
 #endif

@@ -349,6 +349,14 @@ __device__ __forceinline__ double node_inv_volume(const NodalGeom& g, int i, int
     return f * g.ivol;
 }
 
+// Relaxation of step k (0 .. m - 1) of m stationary steps e += w B (b - A e) whose B A has its eigenvalues in [lo, hi]: the
+// reciprocals of the Chebyshev points (Young 1953, J. Math. Phys. 32), from hi down, so that the error is 1 / T_m((hi + lo)
+// / (hi - lo)) instead of max(1 - lo, hi - 1)^m.
+inline double cheb_step(int k, int m, double lo, double hi)
+{
+    return 1.0 / (0.5 * (hi + lo) + 0.5 * (hi - lo) * cos((2 * k + 1) * 3.14159265358979323846 / (2 * m)));
+}
+
 // ---------------------------------------------------------------------------------------
 // error reporting
 void set_error(const std::string& msg);

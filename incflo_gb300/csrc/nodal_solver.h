@@ -133,6 +133,7 @@ public:
     // the same nu sweeps on x itself (rows of the level's layout, values of the held nodes kept) with the right-hand side
     // b32: x + the correction of its residual, without forming either. false: not on this level, nothing done
     bool sweep32_in_place(const float* b32, float* x, int nu, cudaStream_t s);
+    bool sweeps32_in_place(int nu) const;  // whether it is
     // For work issued through apply_vcycles / apply_vcycles32: GBP_OK, the first launch error (cleared), or
     // GBP_TIMEOUT when a bounded device wait of a level sweep ran out (the device error word is read and
     // cleared; synchronises s).
@@ -221,6 +222,7 @@ private:
     bool singular = false;        // the system has the constants as null space (consistent RHS, gauge)
     // the levels from this many nodes down run as one cluster launch per V-cycle (tail.h): what fits the cluster's shared
     // memory and, in FP64, what its 16 SMs' FP64 pipes do not take longer for than launches over the chip
+    static constexpr double kRelaxLow = 0.87;  // lowest eigenvalue of the V-cycle times A that the relaxation aims at
     static constexpr long long kTailNodes32 = 5000, kTailNodes64 = 1000;
     // ... and by one CTA of it
     static constexpr long long kSoloNodes32 = 1400, kSoloNodes64 = 130;

@@ -52,9 +52,10 @@ bool vsweep32_supported(const NodalGeom& g);
 // ... and whose coarse level is the standard coarsening by 2 (residual + restriction, prolongation + sweep),
 // neither of them with an overset mask
 bool vsweep32_transfer_supported(const NodalGeom& g, const NodalGeom& gc);
-// mode 0: Jacobi sweep, 1: residual; hold: masked nodes keep x in a Jacobi sweep instead of 0
+// mode 0: Jacobi sweep, 1: residual (mix != 1: mix b - (mix - 1) A x = b + (mix - 1) (b - A x)); hold: masked nodes keep x
+// in a Jacobi sweep instead of 0
 int vsweep32(const NodalGeom& g, int mode, const float* s, const float* x, const float* b, float* out, float omega,
-             unsigned* err, cudaStream_t st, bool hold = false);
+             unsigned* err, cudaStream_t st, bool hold = false, float mix = 1.f);
 // bc (the coarse right-hand side) = full-weighting restriction of b - A x
 int vsweep32_resid_restrict(const NodalGeom& g, const NodalGeom& gc, const float* s, const float* x, const float* b,
                             float* bc, unsigned* err, cudaStream_t st);

@@ -99,6 +99,7 @@ struct VsArgs {
     NodalGeom gc;   // the coarse level (restriction / prolongation modes)
     float* out;     // fine output (modes 0, 1, 3) or coarse right-hand side (mode 2)
     float k0, k3, omega;
+    float wb, wa;   // mode 1: out = wb b - wa A x
     bool hold;      // mode 0 with an overset mask: masked nodes keep their value (false: 0)
     int kchunk;     // node planes per CTA (even in mode 2)
     int rowlen;     // padded fine row length (floats)
@@ -511,7 +512,9 @@ __global__ void __launch_bounds__(TXM * VsShape<MODE, TY, RPT>::TTR,
                     // node plane P-1 (registers Ao) gets its upper half and is complete
                     const float ax = a.k3 * (acc[r][q] + (G + xa));
                     float val;
-                    if (MODE == 1 || MODE == 2)
+                    if (MODE == 1)
+                        val = fmaf(-a.wa, ax, a.wb * bb[q]);
+                    else if (MODE == 2)
                         val = bb[q] - ax;
                     else
                         val = fmaf(a.omega * (bb[q] - ax), rcp_approx(a.k0 * (ss[r][q] + sgl)), cA);
@@ -637,7 +640,7 @@ int make_map4(const void* base, long long sy, long long sz, long long count, int
 
 template <int MODE, int TY, int TXM>
 int launch(const NodalGeom& g, const NodalGeom* gc, const float* s, const float* x, const float* b,
-           const float* e, float* out, float omega, unsigned* err, cudaStream_t st, bool hold = false)
+           const float* e, float* out, float omega, unsigned* err, cudaStream_t st, bool hold = false, float mix = 1.f)
 {
     constexpr int RPT = GBP_VS_RPT;
     using Sh = VsShape<MODE, TY, RPT>;
@@ -650,6 +653,8 @@ int launch(const NodalGeom& g, const NodalGeom* gc, const float* s, const float*
     a.k3 = (float)g.K[3];
     a.omega = omega;
     a.hold = hold;
+    a.wb = mix;
+    a.wa = mix == 1.f ? 1.f : mix - 1.f;
     a.rowlen = (int)g.sy;
     a.crowlen = gc ? (int)gc->sy : 4;
     a.rstride = 4 * TX + 8;
@@ -723,19 +728,19 @@ bool vsweep32_transfer_supported(const NodalGeom& g, const NodalGeom& gc)
 template <int MODE>
 static int launch_any(const NodalGeom& g, const NodalGeom* gc, const float* s, const float* x, const float* b,
                       const float* e, float* out, float omega, unsigned* err, cudaStream_t st,
-               bool hold = false)
+               bool hold = false, float mix = 1.f)
 {
     const int TX = (g.nu[0] + 3) / 4;
-    if (TX <= 32) return launch<MODE, 8, 32>(g, gc, s, x, b, e, out, omega, err, st, hold);
-    if (TX <= 64) return launch<MODE, GBP_VS_TY_256, 64>(g, gc, s, x, b, e, out, omega, err, st, hold);
-    return launch<MODE, GBP_VS_TY_512, 128>(g, gc, s, x, b, e, out, omega, err, st, hold);
+    if (TX <= 32) return launch<MODE, 8, 32>(g, gc, s, x, b, e, out, omega, err, st, hold, mix);
+    if (TX <= 64) return launch<MODE, GBP_VS_TY_256, 64>(g, gc, s, x, b, e, out, omega, err, st, hold, mix);
+    return launch<MODE, GBP_VS_TY_512, 128>(g, gc, s, x, b, e, out, omega, err, st, hold, mix);
 }
 
 int vsweep32(const NodalGeom& g, int mode, const float* s, const float* x, const float* b, float* out, float omega,
-             unsigned* err, cudaStream_t st, bool hold)
+             unsigned* err, cudaStream_t st, bool hold, float mix)
 {
     return mode == 0 ? launch_any<0>(g, nullptr, s, x, b, nullptr, out, omega, err, st, hold)
-                     : launch_any<1>(g, nullptr, s, x, b, nullptr, out, omega, err, st);
+                     : launch_any<1>(g, nullptr, s, x, b, nullptr, out, omega, err, st, false, mix);
 }
 
 int vsweep32_resid_restrict(const NodalGeom& g, const NodalGeom& gc, const float* s, const float* x, const float* b,

@@ -331,11 +331,11 @@ __global__ void k_tensor_to32(long long count, const double* __restrict__ v, dou
     if (t < count) out[t] = (float)(scale * v[t]);
 }
 
-// acc += e over whole padded arrays
-__global__ void k_tensor_acc32(long long count, const float* __restrict__ e, float* __restrict__ acc)
+// acc += w e over whole padded arrays
+__global__ void k_tensor_acc32(long long count, const float* __restrict__ e, float w, float* __restrict__ acc)
 {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t < count) acc[t] += e[t];
+    if (t < count) acc[t] = fmaf(w, e[t], acc[t]);
 }
 
 // u += e / scale over whole padded arrays (FP32 correction into FP64)
@@ -624,7 +624,7 @@ int TensorSolver::solve(const gbp_array4& rhs_in, gbp_array4& vel, gbp_stats* st
         frexp(bnorm * g.vol, &ex);
         scale32 = ldexp(1.0, -ex);
     }
-    int it = 0, status = GBP_OK, steps = 0;
+    int it = 0, status = GBP_OK, steps = 0, inner = kInner;
     // mixed form: kInner block steps on the FP32 correction equation per FP64 residual (the residual of
     // the full operator in FP32 between them), as the single-level projections refine
     const bool inner32 = opt.precision == GBP_PREC_MIXED;
@@ -643,7 +643,9 @@ int TensorSolver::solve(const gbp_array4& rhs_in, gbp_array4& vel, gbp_stats* st
                 k_tensor_to32<<<nb, 256, 0, st>>>(cnt, r[c], scale32, b32[c]);
                 GBP_CUDA(cudaMemsetAsync(e32[c], 0, sizeof(float) * cnt, st));
             }
-            for (int q = 0; q < kInner; ++q) {
+            for (int q = 0; q < inner; ++q) {
+                // relaxed steps: the cross terms move the blocks' error factors to either side of 0
+                const float w = (float)cheb_step(q, inner, kRelaxLow, kRelaxHigh);
                 // The blocks do not depend on one another and their small levels leave most of the chip idle (half of a V-cycle's
                 // time at 256 x 128 x 128): each on a stream of its own, all back on st before the next residual
                 GBP_CUDA(cudaEventRecord(fork, st));
@@ -651,18 +653,18 @@ int TensorSolver::solve(const gbp_array4& rhs_in, gbp_array4& vel, gbp_stats* st
                     const cudaStream_t s = c ? side[c - 1] : st;
                     if (c) GBP_CUDA(cudaStreamWaitEvent(s, fork, 0));
                     comp[c].vcycles32(q == 0 ? b32[c] : r32[c], s);
-                    k_tensor_acc32<<<nb, 256, 0, s>>>(cnt, comp[c].correction32(), e32[c]);
+                    k_tensor_acc32<<<nb, 256, 0, s>>>(cnt, comp[c].correction32(), w, e32[c]);
                     if (c) GBP_CUDA(cudaEventRecord(join[c - 1], s));
                 }
                 for (int q2 = 0; q2 < 2; ++q2) GBP_CUDA(cudaStreamWaitEvent(st, join[q2], 0));
-                if (q + 1 < kInner) {
+                if (q + 1 < inner) {
                     tensor_ghosts<float>(g, bclo, bchi, e32, vel, 1, st);
                     k_tensor_resid32<<<cells_grid(g), kBlk, 0, st>>>(g, ce, eta32[0], eta32[1], eta32[2], face_k<float>(g),
                                                                      g.a32, (float)(beta * g.vol), cb32, rr32);
                 }
             }
             for (int c = 0; c < 3; ++c) k_tensor_add<<<nb, 256, 0, st>>>(cnt, e32[c], 1.0 / scale32, u[c]);
-            steps += kInner;
+            steps += inner;
         } else {
             for (int c = 0; c < 3; ++c) comp[c].add_vcycle_correction(r[c], u[c], scale32);
             ++steps;
@@ -675,8 +677,14 @@ int TensorSolver::solve(const gbp_array4& rhs_in, gbp_array4& vel, gbp_stats* st
         GBP_CUDA(cudaGetLastError());
         GBP_CUDA(cudaMemcpyAsync(hnorm + 1, dnorm + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
         GBP_CUDA(cudaStreamSynchronize(st));
+        const double before = rn;
         rn = bits_to_double(hnorm[1]);
         ++it;
+        if (inner32 && rn > target && rn < before && target > 0.0) {
+            // as many block steps as the contraction so far asks for; FP32 delivers about 1e-6 per refinement
+            const double need = ceil(log(std::max(0.8 * target / rn, 1e-6)) / (log(rn / before) / inner));
+            inner = (int)std::min<double>(kMostInner, std::max(1.0, need));
+        }
         if (opt.verbose > 1) fprintf(stderr, "gbp tensor: iter %d rel resid %.3e\n", it, bnorm > 0 ? rn / bnorm : rn);
         if (!std::isfinite(rn)) {
             status = GBP_NAN;

@@ -112,3 +112,21 @@ TAILS = [((16, 32, 8), (P, N, P), (P, D, P)), ((8, 12, 64), (N, P, P), (N, P, P)
 def test_cluster_tail(gpu_lib, n, lo, hi, precision):
     _nodal(n, lo, hi, precision)
     test_cluster_bottom_solve_mac(gpu_lib, n, lo, hi, precision)
+
+
+@pytest.mark.parametrize("n,lo,hi", [((128, 128, 72), (P, P, N), (P, P, N)), ((144, 100, 96), (N, D, P), (I, N, P))],
+                         ids=["128x128x72", "144x100x96"])
+def test_relaxed_vcycles(gpu_lib, n, lo, hi):
+    """FP32 V-cycles from the current iterate with Chebyshev weights (whole-row levels): the FP64 solve's phi within twice
+    the 1e-9 that either may be off, in at most a V-cycle more per refinement step than accelerated FP64 V-cycles."""
+    ext = tuple(v / n[0] for v in n)
+    g, sigma, vel = nodal_case(n, ext, lo, hi, seed=2)
+    phi, st = {}, {}
+    for p in ("fp64", "mixed"):
+        proj = NodalProjector(cuda(vel), cuda(sigma), Geometry(n, (0, 0, 0), ext), options=make_options(0, precision=p))
+        proj.setDomainBC(lo, hi)
+        st[p] = proj.project(rtol=1e-12, atol=0.0)
+        assert st[p]["status"] == 0 and st[p]["final_rel_resid"] <= 1e-12
+        phi[p] = unique_nodes(g, proj.getPhi().cpu().numpy())
+    assert rel_l2(phi["mixed"], phi["fp64"]) <= 2e-9
+    assert st["mixed"]["vcycles"] <= st["fp64"]["vcycles"] + st["mixed"]["outer_iters"]
