@@ -3,8 +3,8 @@
 // Forward / data-gradient kernel (k_conv): a row of the GEMM is a group of G consecutive voxels of the zero-haloed
 // channels-last grid (G = 4 for 16 channels, 2 for 32: a row of 64 elements, 128 bytes). With a voxel per row the
 // 16-channel convolutions at 128^3 took 728 us: 27 MMAs of 16 columns and 9 boxes of 32-byte rows per 128 voxels, every one
-// of them some 400 cycles of scalar issue code. Now 116 us: 54 MMAs of 64 columns and 3 boxes per 512 voxels, at 150 cycles
-// per MMA, which still bounds it (the tensor pipe is busy 21 %, DRAM 17 %). The G output voxels of a group take G N
+// of them some 400 cycles of scalar issue code. Now 81 us: 54 MMAs of 64 columns and 3 boxes per 512 voxels, at 150 cycles
+// per MMA and issuing warp, which still bounds it (one issuer at 116 us: tensor pipe busy 21 %, DRAM 17 %). The G output voxels of a group take G N
 // accumulator columns. A persistent CTA
 // walks output tiles of 128 groups. For each K step (input tensor, up to 64 channels, (dz, dy) of the taps) warp 0 issues
 // the TMA loads of the groups' 130-row activation boxes (K-major, swizzled A operands; rows outside the array read as
@@ -14,8 +14,10 @@
 // those voxels, with rows of zeros above and below; moving the start in one stack padded by zeros serves every vi. The
 // group's last (first) voxel also feeds the first (last) output voxel of the next (previous) row: the box shifted by a
 // row. (A value that is not finite so reaches the other voxels of the groups next to it as well.) Two FP32 accumulators
-// in tensor memory: the epilogue of tile t overlaps the MMAs of tile t + 1.
-// The other warps read the accumulator with tcgen05.ld (one group per thread, 16 columns at a time), apply bias + GELU (forward) or gradient
+// (or four) in tensor memory: the epilogue of a tile overlaps the MMAs of the next. Two producer and issuer pairs take
+// turns at the tiles where two rings of stages fit, since one warp's issue rate bounds a tile (116 us with one, 81 with two).
+// The other warps read the accumulator with tcgen05.ld (one group per thread, 16 columns at a time), apply bias + GELU
+// (forward) or gradient
 // accumulation + GELU derivative (backward), zero the halo rows and store BF16.
 //
 // Weight-gradient kernel (k_wgrad): dw[tap][co][ci] = sum_p gout[p][co] in[p + off(tap)][ci] is a GEMM
@@ -47,8 +49,9 @@ constexpr int kBM = 128;       // output rows per tile (MMA M)
 constexpr int kThreads = 192;  // weight gradient: warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 epilogue
 // convolution: four epilogue warps per lane quarter of tensor memory. The epilogue's chain (tensor-memory load, bias, GELU,
 // two stores) bounded the level-0 convolutions with one: 4.6 k cycles per tile without a GELU, about 11 k with it.
-constexpr int kEpiSets = 4, kConvThreads = 64 + 128 * kEpiSets;
+constexpr int kEpiSets = 4, kConvThreads = 128 + 128 * kEpiSets;
 constexpr int kMaxStages = 32;
+constexpr int kPairStages = kMaxStages / 2;  // stages of a producer / issuer pair of the convolution
 constexpr int kWgradRows = 64;  // K rows per pipeline stage of the weight-gradient kernel
 
 struct ConvParams {
@@ -72,7 +75,7 @@ struct ConvParams {
     int seg_c0[2], seg_nc[2];
     const float* bias;
     unsigned* err;
-    int ns, wres;
+    int ns, wres, npair, nbsh;  // stages of a pair, pairs (1 or 2), log2 of the accumulators (2 or 4)
     // weights of one (input, channel chunk, (dz, dy)): (G - 1) N rows of zeros, the taps' rows; zeros again at the end.
     // Resident: start, offset of an input, bytes of a channel chunk, bytes loaded, all bytes (else w_in: within a stage)
     uint32_t w_base, w_in[2], w_chunk[2], w_bytes, w_area;
@@ -139,7 +142,7 @@ template <int G>
 __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant__ ConvParams P)
 {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], accf[2], acce[2], done, wfull;
+    __shared__ __align__(8) uint64_t full_[2][kPairStages], empty_[2][kPairStages], accf[4], acce[4], done[2], wfull;
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
     __shared__ __align__(16) float sbias[256];
@@ -154,21 +157,23 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
     const int nstack = P.nstep * P.ndy;                  // stacks of a channel chunk: the (dz, dy)
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < P.ns; ++s) {
-            mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1);
-        }
-        for (int b = 0; b < 2; ++b) {
+        for (int s = 0; s < P.ns; ++s)
+            for (int b = 0; b < 2; ++b) {
+                mbar_init(&full_[b][s], 1);
+                mbar_init(&empty_[b][s], 1);
+            }
+        for (int b = 0; b < 4; ++b) {
             mbar_init(&accf[b], 1);
             mbar_init(&acce[b], 4 * kEpiSets);
         }
-        mbar_init(&done, 1);
+        mbar_init(&done[0], 1);
+        mbar_init(&done[1], 1);
         mbar_init(&wfull, 1);
         abort_flag = 0;
         mbar_fence_init();
     }
     if (warp == 1) {
-        tc::tmem_alloc(&tmem_slot, 2 * P.tmem_cols);
+        tc::tmem_alloc(&tmem_slot, P.tmem_cols << P.nbsh);
         tc::tmem_relinquish();
     }
     if ((int)threadIdx.x < P.N) sbias[threadIdx.x] = P.bias ? P.bias[threadIdx.x] : 0.f;
@@ -176,7 +181,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
         // the zero rows of the weight stacks (the loads fill in the rest)
         const uint4 zero = make_uint4(0, 0, 0, 0);
         const uint32_t from = P.wres ? P.w_base : P.a_bytes, area = P.wres ? P.w_area : P.stage_bytes - P.a_bytes;
-        for (int s = 0; s < (P.wres ? 1 : P.ns); ++s)
+        for (int s = 0; s < (P.wres ? 1 : P.npair * P.ns); ++s)
             for (uint32_t q = threadIdx.x * 16u; q < area; q += kConvThreads * 16u)
                 *reinterpret_cast<uint4*>(sgen + s * P.stage_bytes + from + q) = zero;
         fence_proxy_async();
@@ -185,7 +190,14 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_slot;
-    if (warp == 0) {
+    // producer and issuer of pair p: warps 2 p and 2 p + 1; its tiles: every npair-th of the CTA's
+    const int pair = warp >> 1 & 1;
+    uint64_t *full = full_[pair], *empty = empty_[pair];
+    const uint32_t ring = (uint32_t)(pair * P.ns) * P.stage_bytes;
+    const int tstep = P.npair * (int)gridDim.x;
+    if (warp < 4 && pair >= P.npair) {
+        // no second pair where its stages do not fit
+    } else if (warp < 4 && !(warp & 1)) {
         // the taps of a (dz, dy) in the order of the output voxels they feed: vi - 1, vi, vi + 1 (one voxel: as they lie)
         auto load_taps = [&](unsigned char* w, uint64_t* bar, int i, int cc, int gq) {
             const int x = P.wc0[i] + cc * P.cb[i], row0 = gq * P.gtaps * P.N;
@@ -198,7 +210,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
                 tma_load_2d(w + (uint32_t)(t * P.N) * P.cb[i] * 2u, &P.wmap[i], bar, x, row0 + q * P.N);
             }
         };
-        if (P.wres && tc::elect_one()) {
+        if (P.wres && pair == 0 && tc::elect_one()) {
             mbar_arrive_expect_tx(&wfull, P.w_bytes);
             for (int i = 0; i < P.nin; ++i)
                 for (int cc = 0; cc < P.cin[i] / P.cb[i]; ++cc)
@@ -209,7 +221,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
         }
         __syncwarp();
         uint32_t it = 0, s = 0, phase = 1;  // stage of the step, parity of its last release
-        for (int tile = blockIdx.x; tile < P.ntiles && __all_sync(0xffffffffu, !abort_flag); tile += gridDim.x) {
+        for (int tile = blockIdx.x + pair * gridDim.x; tile < P.ntiles && __all_sync(0xffffffffu, !abort_flag); tile += tstep) {
             const int p0 = tile * kBM;
             for (int i = 0; i < P.nin; ++i) {
                 const int nbox = P.nbox[i], ncc = P.cin[i] / P.cb[i], xstep = (P.ab[i] / P.cb[i]) * P.cin[i];
@@ -224,7 +236,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
                         }
                         if (tc::elect_one()) {
                             mbar_arrive_expect_tx(&full[s], bytes);
-                            unsigned char* a = sgen + s * P.stage_bytes;
+                            unsigned char* a = sgen + ring + s * P.stage_bytes;
                             const int arow = p0 + P.grow[gq];
                             const CUtensorMap* map = &P.amap[i];
                             for (int m = 0; m < nbox; ++m)
@@ -246,14 +258,15 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
             const uint32_t last = it - 1 - ((it - 1 - q) % P.ns);
             (void)tc::warp_wait(&full[q], (last / P.ns) & 1, P.err);
         }
-        if (P.wres) (void)tc::warp_wait(&wfull, 0, P.err);
-    } else if (warp == 1) {
-        uint32_t s = 0, phase = 0, tl = 0;
+        if (P.wres && pair == 0) (void)tc::warp_wait(&wfull, 0, P.err);
+    } else if (warp < 4) {
+        uint32_t s = 0, phase = 0, tl = pair;
         const uint32_t leader = tc::elect_one();
         if (P.wres && !tc::warp_wait(&wfull, 0, P.err)) abort_flag = 1;
-        for (int tile = blockIdx.x; tile < P.ntiles && __all_sync(0xffffffffu, !abort_flag); tile += gridDim.x, ++tl) {
-            const uint32_t buf = tl & 1;
-            if (tl >= 2 && !tc::warp_wait(&acce[buf], ((tl >> 1) + 1) & 1, P.err)) {
+        for (int tile = blockIdx.x + pair * gridDim.x; tile < P.ntiles && __all_sync(0xffffffffu, !abort_flag);
+             tile += tstep, tl += P.npair) {
+            const uint32_t buf = tl & ((1u << P.nbsh) - 1u), use = tl >> P.nbsh;
+            if (use > 0 && !tc::warp_wait(&acce[buf], (use + 1) & 1, P.err)) {
                 abort_flag = 1;
                 break;
             }
@@ -280,7 +293,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
                             goto issued;
                         }
                         tc::fence_after_sync();
-                        const uint32_t a = sbase + s * P.stage_bytes;
+                        const uint32_t a = sbase + ring + s * P.stage_bytes;
                         for (int y = P.ndy == 1 ? y1 : 0, ye = P.ndy == 1 ? y1 + 1 : 3; y < ye; ++y) {
                             const int v0 = P.yoff[y] - P.ybase[y] + vfirst;
                             uint64_t wd = dw + ((P.wres ? wr : (a + P.a_bytes + P.w_in[i]) >> 4) + wfirst);
@@ -331,15 +344,15 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
             tc::mma_commit(leader, &accf[buf]);
         }
     issued:
-        tc::mma_commit(leader, &done);
-        (void)tc::warp_wait(&done, 0, P.err);
+        tc::mma_commit(leader, &done[pair]);
+        (void)tc::warp_wait(&done[pair], 0, P.err);
     } else {
         const int q = warp & 3;  // tensor-memory lane quarter this warp may read
-        const int row = q * 32 + lane, set = (warp - 2) >> 2, cpv = P.N / 16, nchunk = G * cpv;
+        const int row = q * 32 + lane, set = (warp - 4) >> 2, cpv = P.N / 16, nchunk = G * cpv;
         uint32_t tl = 0;
         for (int tile = blockIdx.x; tile < P.ntiles; tile += gridDim.x, ++tl) {
-            const uint32_t buf = tl & 1;
-            if (!mbar_wait_bounded(&accf[buf], (tl >> 1) & 1, P.err)) abort_flag = 1;
+            const uint32_t buf = tl & ((1u << P.nbsh) - 1u);
+            if (!mbar_wait_bounded(&accf[buf], (tl >> P.nbsh) & 1, P.err)) abort_flag = 1;
             if (__any_sync(0xffffffffu, abort_flag)) break;
             tc::fence_after_sync();
             const long long pg = ((long long)tile * kBM + row) * G;
@@ -413,7 +426,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
     __syncthreads();
     if (warp == 1) {
         tc::fence_after_sync();
-        tc::tmem_dealloc(tmem, 2 * P.tmem_cols);
+        tc::tmem_dealloc(tmem, P.tmem_cols << P.nbsh);
     }
 }
 
@@ -890,12 +903,15 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
         }
         P.stage_bytes += w;
     }
-    P.ns = std::min(kMaxStages, (int)((max_smem - 1024 - (P.wres ? wres_bytes : 0)) / P.stage_bytes));
+    const int stages = (int)((max_smem - 1024 - (P.wres ? wres_bytes : 0)) / P.stage_bytes);
+    P.npair = stages >= 4 ? 2 : 1;
+    P.ns = std::min(kPairStages, stages / P.npair);
     if (P.ns < 2) {
         set_error("conv3d: stage does not fit in shared memory");
         return GBP_BAD_ARG;
     }
-    P.w_base = (uint32_t)P.ns * P.stage_bytes;
+    P.nbsh = P.npair == 2 && 4 * P.tmem_cols <= 512 ? 2 : 1;
+    P.w_base = (uint32_t)(P.npair * P.ns) * P.stage_bytes;
     const size_t smem = (size_t)P.w_base + (P.wres ? wres_bytes : 0) + 1024;
     static bool attr_set = false;
     if (!attr_set) {
