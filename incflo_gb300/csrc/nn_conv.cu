@@ -51,6 +51,7 @@ constexpr int kThreads = 192;  // weight gradient: warp 0 TMA producer, warp 1 M
 // two stores) bounded the level-0 convolutions with one: 4.6 k cycles per tile without a GELU, about 11 k with it.
 constexpr int kEpiSets = 4, kConvThreads = 128 + 128 * kEpiSets;
 constexpr int kMaxStages = 32;
+constexpr int kConvSmem = 225 * 1024;  // of the 227 KB of a CTA, beside the convolution's static part (2 KB)
 constexpr int kPairStages = kMaxStages / 2;  // stages of a producer / issuer pair of the convolution
 constexpr int kWgradRows = 64;  // K rows per pipeline stage of the weight-gradient kernel
 
@@ -857,7 +858,7 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
     P.idesc = tc::idesc_bf16(kBM, P.G * L.N, 0, 0);
     P.w_area = wres_bytes;
     // weights resident where at least 3 activation stages fit beside them, else with each step
-    const uint32_t max_smem = 220 * 1024;
+    const uint32_t max_smem = kConvSmem;
     auto box = [&](int rows) {
         P.a_rows = rows;
         P.box_bytes = ((uint32_t)rows * abmax * 2u + 1023u) & ~1023u;
@@ -870,11 +871,13 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
     if (mid && P.wres) {
         // one box for the three dy of a dz where its rows fit a TMA box and two stages stay: the rows of neighbouring dy
         // overlap (194 rows instead of 3 x 130 at 128^3), and L2 reads bounded the level-0 convolutions at 5 TB/s
+        // (two rings of single boxes go before one ring of these: 263 us with one, 193 with two for 32 + 16 -> 16 channels at 128^3)
         const int rows = kBM + rows_of(PX + P.G) - rows_of(-PX - 1), was = P.a_rows;
+        const bool two_rings = wres_bytes + 4 * P.a_bytes + 1024 <= max_smem;
         if (rows <= 256) {
             box(rows);
             P.ndy = 3;
-            if (wres_bytes + 2 * P.a_bytes + 1024 > max_smem) {
+            if (wres_bytes + (two_rings ? 4 : 2) * P.a_bytes + 1024 > max_smem) {
                 box(was);
                 P.ndy = 1;
             }
@@ -916,7 +919,7 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
     static bool attr_set = false;
     if (!attr_set) {
         for (auto k : {k_conv<1>, k_conv<2>, k_conv<4>})
-            GBP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+            GBP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem));
         attr_set = true;
     }
     const int grid = std::min(P.ntiles, sm_count_cached());
