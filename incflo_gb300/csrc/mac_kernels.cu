@@ -399,7 +399,10 @@ __device__ __forceinline__ double* a4p(const gbp_array4& a, int i, int j, int k,
 
 // Effective face beta of direction d for faces 0..n[d]: source 0 = array, 1 = constant,
 // 2 = dt / (0.5 (rho_lo + rho_hi)) (incflo: average_cellcenter_to_face then invert(dt)).
-__global__ void k_mac_beta(CellGeom g, int d, int source, gbp_array4 src, double cval, int bclo, int bchi,
+// (d is a template argument: index arrays subscripted by a run-time direction live in local memory; 285 us per direction
+// for 256^3 cells with a density, 82 us for 256 x 128 x 128 with a cell viscosity, now 98 and 43 us)
+template <int d>
+__global__ void __launch_bounds__(256) k_mac_beta(CellGeom g, int source, gbp_array4 src, double cval, int bclo, int bchi,
                            double* __restrict__ b64, float* __restrict__ b32, RobinFaces rb,
                            const double* __restrict__ ap, double mult)
 {
@@ -437,20 +440,20 @@ __global__ void k_mac_beta(CellGeom g, int d, int source, gbp_array4 src, double
             beta = a4(src, lo[0], lo[1], lo[2], 0);
         else
             beta = 0.5 * (a4(src, lo[0], lo[1], lo[2], 0) + a4(src, q[0], q[1], q[2], 0));
-    } else {
+    } else {  // cval over the face average
         int lo[3] = {q[0], q[1], q[2]};
         lo[d] -= 1;
         if (per && lo[d] < 0) lo[d] += g.n[d];
-        beta = cval / (0.5 * (a4(src, lo[0], lo[1], lo[2], 0) + a4(src, q[0], q[1], q[2], 0)));
+        beta = (2.0 * cval) / (a4(src, lo[0], lo[1], lo[2], 0) + a4(src, q[0], q[1], q[2], 0));
     }
-    beta *= mult;  // the ABecLaplacian's beta scalar times b (1 for the projections)
+    if (mult != 1.0) beta *= mult;  // the ABecLaplacian's beta scalar times b (1 for the projections)
     // Dirichlet face: the ghost value sits half a cell out, so the face weight doubles; Robin face
     // (a phi + b dphi/dn = 0): weight beta a h / (a h / 2 + b), with the raw beta kept for later factors
     double eff = beta;
     if (!per && (fd == 0 || fd == g.n[d])) {
         if (bside == GBP_BC_ROBIN) {
             const int q = 2 * d + (fd == 0 ? 0 : 1);
-            const int d1 = d == 0 ? 1 : 0, d2 = d == 2 ? 1 : 2;
+            constexpr int d1 = d == 0 ? 1 : 0, d2 = d == 2 ? 1 : 2;
             const long long fi = f[d1] + (long long)g.n[d1] * f[d2];
             rb.braw[q][fi] = beta;
             eff = beta * rb.rfac[q][fi];
@@ -520,7 +523,8 @@ __global__ void __launch_bounds__(256) k_mac_eb_inflow_flux(CellGeom g, gbp_arra
     flux[p] = f;
 }
 
-__global__ void __launch_bounds__(256) k_mac_correct(CellGeom g, int d, gbp_array4 u, const double* __restrict__ beta,
+template <int d>
+__global__ void __launch_bounds__(256) k_mac_correct(CellGeom g, gbp_array4 u, const double* __restrict__ beta,
                                                      const double* __restrict__ phi, const double* __restrict__ ap)
 {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -803,7 +807,8 @@ void mac_set_beta(const CellGeom& g, int d, int source, const gbp_array4* src, d
     if (src) a = *src;
     RobinFaces r{};
     if (rb) r = *rb;
-    k_mac_beta<<<nblk(nface(g, d), 256), 256, 0, st>>>(g, d, source, a, cval, bclo, bchi, b64, b32, r, ap, mult);
+    (d == 0 ? k_mac_beta<0> : d == 1 ? k_mac_beta<1> : k_mac_beta<2>)<<<nblk(nface(g, d), 256), 256, 0, st>>>(
+        g, source, a, cval, bclo, bchi, b64, b32, r, ap, mult);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -993,7 +998,8 @@ void mac_zero_faces(const CellGeom& g, int d, const gbp_array4& u, cudaStream_t 
 void mac_correct(const CellGeom& g, int d, const gbp_array4& u, const double* beta, const double* phi,
                  cudaStream_t st, const double* ap)
 {
-    k_mac_correct<<<nblk(nface(g, d), 256), 256, 0, st>>>(g, d, u, beta, phi, ap);
+    (d == 0 ? k_mac_correct<0> : d == 1 ? k_mac_correct<1> : k_mac_correct<2>)<<<nblk(nface(g, d), 256), 256, 0, st>>>(
+        g, u, beta, phi, ap);
 }
 void mac_load_phi(const CellGeom& g, const gbp_array4& in, double* phi, cudaStream_t st)
 {
