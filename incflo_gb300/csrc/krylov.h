@@ -1,5 +1,6 @@
-// Conjugate-gradient acceleration of the multigrid solves: the vector kernels between the V-cycle (the
-// preconditioner z = V r) and the operator q = -A p (the sign the residual kernels give with no right-hand side), on the padded layouts of the nodal and cell-centred levels.
+// Conjugate-gradient acceleration of the multigrid solves: the vector kernels between the V-cycle (the preconditioner
+// z = V r) and the operator q = -A p (the sign the residual kernels give with no right-hand side), on the padded layouts
+// of the nodal and cell-centred levels.
 //
 // Flexible form: beta = z.(r_new - r_old) / (r.z)_old = alpha q.z / (r.z)_old, which needs no symmetry of the
 // V-cycle beyond what rounding leaves of it, and costs one more dot product over vectors that are read anyway. The
@@ -8,8 +9,8 @@
 //
 // With a V-cycle that contracts the error by rho per application, the stationary iteration needs log(tol) / log(rho)
 // of them; the accelerated one removes the few slow modes that set rho (a density jump, cut cells, stretched cells):
-// V(2,2) cycles to 1e-10 on the 256^3 interface problem 10 -> 7
-// (nodal) and 11 -> 9 (MAC), to 1e-11 on cells of aspect 1 : 0.8 : 1.25 38 -> 16 (both).
+// V(2,2) cycles to 1e-10 on the 256^3 interface problem 10 -> 7 (nodal) and 11 -> 9 (MAC), to 1e-11 on cells of aspect
+// 1 : 0.8 : 1.25 38 -> 16 (both).
 #pragma once
 
 #include <cuda_runtime.h>

@@ -4,8 +4,8 @@
 // channels-last grid (G = 4 for 16 channels, 2 for 32: a row of 64 elements, 128 bytes). With a voxel per row the
 // 16-channel convolutions at 128^3 took 728 us: 27 MMAs of 16 columns and 9 boxes of 32-byte rows per 128 voxels, every one
 // of them some 400 cycles of scalar issue code. Now 81 us: 54 MMAs of 64 columns and 3 boxes per 512 voxels, at 150 cycles
-// per MMA and issuing warp, which still bounds it (one issuer at 116 us: tensor pipe busy 21 %, DRAM 17 %). The G output voxels of a group take G N
-// accumulator columns. A persistent CTA
+// per MMA and issuing warp, which still bounds it (one issuer at 116 us: tensor pipe busy 21 %, DRAM 17 %). The G output
+// voxels of a group take G N accumulator columns. A persistent CTA
 // walks output tiles of 128 groups. For each K step (input tensor, up to 64 channels, (dz, dy) of the taps) warp 0 issues
 // the TMA loads of the groups' 130-row activation boxes (K-major, swizzled A operands; rows outside the array read as
 // zeros); the weights lie in shared memory for the whole kernel where they fit, else they come with each step. Warp 1
@@ -17,8 +17,7 @@
 // (or four) in tensor memory: the epilogue of a tile overlaps the MMAs of the next. Two producer and issuer pairs take
 // turns at the tiles where two rings of stages fit, since one warp's issue rate bounds a tile (116 us with one, 81 with two).
 // The other warps read the accumulator with tcgen05.ld (one group per thread, 16 columns at a time), apply bias + GELU
-// (forward) or gradient
-// accumulation + GELU derivative (backward), zero the halo rows and store BF16.
+// (forward) or gradient accumulation + GELU derivative (backward), zero the halo rows and store BF16.
 //
 // Weight-gradient kernel (k_wgrad): dw[tap][co][ci] = sum_p gout[p][co] in[p + off(tap)][ci] is a GEMM
 // with M = (taps x input channels) in blocks of 128, N = output channels and K = grid rows. Both
@@ -871,7 +870,8 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
     if (mid && P.wres) {
         // one box for the three dy of a dz where its rows fit a TMA box and two stages stay: the rows of neighbouring dy
         // overlap (194 rows instead of 3 x 130 at 128^3), and L2 reads bounded the level-0 convolutions at 5 TB/s
-        // (two rings of single boxes go before one ring of these: 263 us with one, 193 with two for 32 + 16 -> 16 channels at 128^3)
+        // (two rings of single boxes go before one ring of these: 32 + 16 -> 16 channels at 128^3 263 us with one ring, 193
+        // with two)
         const int rows = kBM + rows_of(PX + P.G) - rows_of(-PX - 1), was = P.a_rows;
         const bool two_rings = wres_bytes + 4 * P.a_bytes + 1024 <= max_smem;
         if (rows <= 256) {
