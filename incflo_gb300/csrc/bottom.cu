@@ -93,32 +93,35 @@ __global__ void __launch_bounds__(128) k_rows_mac(CellGeom g, const double* __re
 // ------------------------------------------------------------------------------------------------ dense inverse
 // Symmetric positive definite, so no pivoting, and Gauss-Jordan as the sweep operator (Goodnight 1979, The American
 // Statistician 33), which keeps the symmetry: one triangle in registers, the pivot's column passed through shared
-// memory, one division per pivot and two warps. One SM's FP64 pipe bounds it (16 cycles per warp and instruction): 64
+// memory, one division per pivot in the warps that hold the column. One SM's FP64 pipe bounds it (16 cycles per warp and instruction): 64
 // unknowns took 243 us with the whole matrix and a division in every warp, now 75.
 __global__ void __launch_bounds__(1024) k_bottom_inverse(BottomRows r, int singular, double* __restrict__ M,
                                                          unsigned char* __restrict__ act, unsigned* bad)
 {
     constexpr int kMost = (kDenseBottom * (kDenseBottom + 1) / 2 + 1023) / 1024;  // entries of a thread
-    __shared__ double A[kDenseBottom][kDenseBottom + 1];
     __shared__ double col[2][kDenseBottom], scl[kDenseBottom], shift;
     const int N = r.n, t = threadIdx.x;
-    for (int q = t; q < N * N; q += blockDim.x) A[q / N][q % N] = 0.0;
-    __syncthreads();
+    // entry (u, v) of the matrix
+    auto entry = [&](int u, int v) {
+        if (r.diag[u] == 0.0) return u == v ? 1.0 : 0.0;
+        double sum = 0.0;
+        for (int q = 0; q < r.w; ++q)
+            if (r.idx[(size_t)q * N + u] == v) sum += r.coef[(size_t)q * N + u];
+        return sum;
+    };
     double tr = 0.0, na = 0.0;
     if (t < N) {
         const bool held = r.diag[t] == 0.0;
-        for (int q = 0; q < r.w; ++q) A[t][r.idx[(size_t)q * N + t]] += r.coef[(size_t)q * N + t];
-        if (held) A[t][t] = 1.0;
-        tr = held ? 0.0 : A[t][t];
-        na = held ? 0.0 : 1.0;
-        scl[t] = tr;
-        col[0][t] = na;
+        scl[t] = held ? 0.0 : entry(t, t);
+        col[0][t] = held ? 0.0 : 1.0;
         if (act) act[t] = !held;
     }
     __syncthreads();
     if (t < 32) {
-        tr = (t < N ? scl[t] : 0.0) + (t + 32 < N ? scl[t + 32] : 0.0);
-        na = (t < N ? col[0][t] : 0.0) + (t + 32 < N ? col[0][t + 32] : 0.0);
+        for (int u = t; u < N; u += 32) {
+            tr += scl[u];
+            na += col[0][u];
+        }
         for (int o = 16; o > 0; o >>= 1) {
             tr += __shfl_xor_sync(0xffffffffu, tr, o);
             na += __shfl_xor_sync(0xffffffffu, na, o);
@@ -139,7 +142,7 @@ __global__ void __launch_bounds__(1024) k_bottom_inverse(BottomRows r, int singu
         ev[m] = u < N ? e - u * (u + 1) / 2 : -1;
         a[m] = 0.0;
         if (u < N) {
-            a[m] = A[u][ev[m]];
+            a[m] = entry(u, ev[m]);
             if (r.diag[u] != 0.0 && r.diag[ev[m]] != 0.0) a[m] += shift;
         }
     }

@@ -10,10 +10,12 @@
 
 namespace gbp {
 
-// 64 unknowns: the inverse costs 64 x 64 x 64 FP64 multiply-adds on one SM (2 per clock: about 75 us) per coefficient
-// set, and a product 1 us per V-cycle, where the cluster's conjugate gradients take 25 to 60 us per V-cycle. (The
-// inverse of up to 216 unknowns by the host took 0.3 to 10 ms per coefficient set.)
-constexpr int kDenseBottom = 64;
+// n unknowns: the inverse costs n^3 / 2 FP64 multiply-adds on one SM (2 per clock: about 75 us for 64, 230 us for 108) per
+// coefficient set and a product of 1 to 3 us per V-cycle, where the cluster's conjugate gradients take 25 to 100 us per
+// V-cycle; and a dense bottom lets the cluster tail cycle the small levels (MAC 112 x 16 x 24 cells, 84 unknowns: 3.7 ms
+// per projection without, 1.5 with; 48 x 24 x 48, 108 unknowns: 1.84 and 1.27; nodal 112 x 48 x 48, 128 unknowns: 1.65 and
+// 1.90). (The inverse of up to 216 unknowns by the host took 0.3 to 10 ms per coefficient set.)
+constexpr int kDenseBottom = 112;
 // most unknowns of the cluster solver: the search direction is replicated in every CTA's shared memory
 constexpr int kClusterBottom = 16384;
 constexpr int kBottomThreads = 1024;

@@ -130,3 +130,12 @@ def test_relaxed_vcycles(gpu_lib, n, lo, hi):
         phi[p] = unique_nodes(g, proj.getPhi().cpu().numpy())
     assert rel_l2(phi["mixed"], phi["fp64"]) <= 2e-9
     assert st["mixed"]["vcycles"] <= st["fp64"]["vcycles"] + st["mixed"]["outer_iters"]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,lo,hi", [((48, 24, 48), (N, N, N), (N, N, N)), ((56, 32, 16), (N, P, D), (D, P, N))],
+                         ids=["48x24x48", "56x32x16"])
+def test_dense_bottoms(gpu_lib, n, lo, hi, precision):
+    """Dense inverses of several entries per thread (108 and 112 cells), singular and not, and nodal bottoms beside them."""
+    test_cluster_bottom_solve_mac(gpu_lib, n, lo, hi, precision)
+    _nodal(n, lo, hi, precision)
