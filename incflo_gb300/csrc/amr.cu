@@ -1317,10 +1317,12 @@ int CompositeNodal::project(const AmrFields& f, gbp_stats* stats)
     sa.nstride = (long long)ncf;
     rc = fin.set_sigma(&sa, 0.0);
     if (rc) return rc;
-    if (qsw) {
-        fin.qweights0();  // the fine part shares its solver's weights (a mask does not enter them)
-        nodal_qweights64(gc, sc_m, qwc, st);
-    }
+    // The sums of the new sigma that the FP64 kernels of a step read, before the first of them: a captured step replays
+    // its kernels without the host code around them. (The composite operator takes the fine solver's: a mask does not
+    // enter them.)
+    if (opt.precision != GBP_PREC_MIXED) crs.ensure_qweights();
+    if (opt.precision != GBP_PREC_MIXED || qsw) fin.ensure_qweights();
+    if (qsw) nodal_qweights64(gc, sc_m, qwc, st);
     // right-hand sides: leaf cells of each level, then the fine interface into the coarse interface
     const bool sub_old = f.incremental && f.vel_old_c;
     auto cellsf = [&](double* d, int nc_) {

@@ -405,12 +405,6 @@ void NodalSolver::ensure_qweights()
         }
 }
 
-const QWeights& NodalSolver::qweights0()
-{
-    ensure_qweights();
-    return L[0].qw;
-}
-
 int NodalSolver::level_of(const NodalGeom& g) const
 {
     for (size_t l = 0; l < L.size(); ++l)
@@ -789,7 +783,6 @@ void NodalSolver::apply_vcycles(const double* r, double* x, int m, double scale,
 {
     const NodalLevel& l0 = L[0];
     cap_or_st = s;
-    if (opt.precision != GBP_PREC_MIXED) ensure_qweights();
     if (opt.precision == GBP_PREC_MIXED) {
         nodal_to_f32(l0.g, r, l0.b32, scale, s);
         vcycle<float>(0, l0.b32, true);

@@ -121,7 +121,8 @@ public:
 
     // Preconditioner for a composite (two-level) driver: x += m V-cycles from zero on the FP64 level-0
     // residual r, in the plan's precision (FP32 V-cycles on r * scale in the mixed form). r and x are
-    // level-0 arrays in the padded layout; r is not modified.
+    // level-0 arrays in the padded layout; r is not modified. Both may be issued into a capture: in the plain form
+    // ensure_qweights comes before, after every new sigma.
     void apply_vcycles(const double* r, double* x, int m, double scale, cudaStream_t s);
     // The same on an FP32 level-0 right-hand side already scaled (mixed form only): m FP32 V-cycles from
     // zero on b32; the correction stays in correction32() until the next V-cycle of this solver.
@@ -139,8 +140,12 @@ public:
     // cleared; synchronises s).
     int take_sweep_status(cudaStream_t s);
     float* sigma32() const { return L[0].s32; }
-    // level-0 weights of the shared-sum FP64 sweep for the present sigma (w5 == nullptr: not a level it supports)
-    const QWeights& qweights0();
+    // The weights of the shared-sum FP64 sweep for the present sigma, on the levels it runs on: level 0, and with FP64
+    // V-cycles the others. Issued on the plan's stream, never from inside a captured step, whose replays would leave them
+    // out (with the sums of a density whose interface has since moved by half a cell, FP64 V-cycles diverge).
+    void ensure_qweights();
+    // level 0's (w5 == nullptr: not a level it supports)
+    const QWeights& qweights0() const { return L[0].qw; }
 
     void reset_count() { nk = 0; }
     long long kernel_count() const { return nk; }
@@ -240,6 +245,7 @@ public:
     // test hook: one FP32 V-cycle from the first cluster-cycled level on a seeded right-hand side, through
     // the per-level launches and through the cluster kernel; *diff = max |difference| / max |result|
     int check_coarse_cycle(double* diff);
+
 private:
     double omega_eff = 0.85;  // the fixed smoother weight (see set_omega)
     // weights of the pre- and post-smoothing sweeps of a V-cycle level (sweep p: [p % kSweepWeights])
@@ -249,8 +255,6 @@ private:
     bool singular_faces = false;  // singular from the boundary types alone (no overset mask)
     int rebuild_masks();
     int finish_sigma();
-    // the shared-sum FP64 sweep's weights of the levels it runs on: level 0, and with FP64 V-cycles the others
-    void ensure_qweights();
     int level_of(const NodalGeom& g) const;
     void resid0(const double* x, const double* b, double* r, unsigned long long* norm, cudaStream_t s);
     unsigned user_zeros = 0;
