@@ -1804,7 +1804,8 @@ namespace gbp {
 
 namespace {
 
-__global__ void k_maxdiff(const float* __restrict__ a, const float* __restrict__ ref, long long n,
+template <typename T>
+__global__ void k_maxdiff(const T* __restrict__ a, const T* __restrict__ ref, long long n,
                           unsigned long long* out)
 {
     double d = 0.0, m = 0.0;
@@ -1822,7 +1823,8 @@ __global__ void k_maxdiff(const float* __restrict__ a, const float* __restrict__
 }
 
 // seeded values in [-1, 1) on the unique nodes (with their periodic aliases when `aliases`)
-__global__ void k_fill_seeded(NodalGeom g, float* __restrict__ a, unsigned seed, int aliases)
+template <typename T>
+__global__ void k_fill_seeded(NodalGeom g, T* __restrict__ a, unsigned seed, int aliases)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
     if (i >= g.nu[0]) return;
@@ -1830,7 +1832,7 @@ __global__ void k_fill_seeded(NodalGeom g, float* __restrict__ a, unsigned seed,
     h ^= h >> 15;
     h *= 2246822519u;
     h ^= h >> 13;
-    const float v = (float)(h & 0xffffff) * (2.0f / 16777216.0f) - 1.0f;
+    const T v = (T)((float)(h & 0xffffff) * (2.0f / 16777216.0f) - 1.0f);
     if (aliases)
         store_node(a, g, i, j, k, v);
     else
@@ -1944,33 +1946,27 @@ int NodalSolver::check_level_kernels_on(float* A, float* C, double diff[4])
     return GBP_OK;
 }
 
-int NodalSolver::check_coarse_cycle(double* diff)
+template <typename T>
+int NodalSolver::tail_difference(int lc, double* diff)
 {
-    const int lc = coarse_first();
-    if (lc < 0 || !sigma_ready) {
-        set_error("check_coarse_cycle: the plan has no cluster-cycled levels (levels " + std::to_string(L.size()) +
-                  ", dense bottom " + std::to_string((int)dense_bottom) + " of " + std::to_string(nbottom) +
-                  " nodes, cluster path " + std::to_string((int)use_coarse) + ") or no sigma (" +
-                  std::to_string((int)sigma_ready) + ")");
-        return GBP_BAD_ARG;
-    }
+    using B = LevelBufs<T>;
     const NodalLevel& v = L[lc];
     const NodalGeom& g = v.g;
-    const size_t bytes = sizeof(float) * g.count;
-    float* C = nullptr;
+    const size_t bytes = sizeof(T) * g.count;
+    T* C = nullptr;
     GBP_CUDA(cudaMalloc(&C, bytes));
     cap_or_st = st;
     // the same seeded right-hand side through the per-level launches and through the cluster kernel
-    GBP_CUDA(cudaMemsetAsync(v.b32, 0, bytes, st));
-    k_fill_seeded<<<dim3((g.nu[0] + 127) / 128, g.nu[1], g.nu[2]), 128, 0, st>>>(g, v.b32, 53u, 0);
+    GBP_CUDA(cudaMemsetAsync(B::b(v), 0, bytes, st));
+    k_fill_seeded<<<dim3((g.nu[0] + 127) / 128, g.nu[1], g.nu[2]), 128, 0, st>>>(g, B::b(v), 53u, 0);
     use_coarse = false;
-    vcycle<float>(lc, v.b32, true);
+    vcycle<T>(lc, B::b(v), true);
     cudaMemcpyAsync(C, xres[lc], bytes, cudaMemcpyDeviceToDevice, st);
     use_coarse = true;
-    vcycle<float>(lc, v.b32, true);
+    vcycle<T>(lc, B::b(v), true);
     unsigned long long* dm = reinterpret_cast<unsigned long long*>(dscal + 4);
     cudaMemsetAsync(dm, 0, 2 * sizeof(unsigned long long), st);
-    k_maxdiff<<<592, 256, 0, st>>>((const float*)xres[lc], C, (long long)g.count, dm);
+    k_maxdiff<<<592, 256, 0, st>>>((const T*)xres[lc], C, (long long)g.count, dm);
     unsigned long long h[2] = {0, 0};
     cudaMemcpyAsync(h, dm, sizeof(h), cudaMemcpyDeviceToHost, st);
     cudaError_t e = cudaStreamSynchronize(st);
@@ -1982,8 +1978,24 @@ int NodalSolver::check_coarse_cycle(double* diff)
     double d, m;
     memcpy(&d, &h[0], 8);
     memcpy(&m, &h[1], 8);
-    *diff = m > 0 ? d / m : d;
+    *diff = std::max(*diff, m > 0 ? d / m : d);
     return GBP_OK;
+}
+
+int NodalSolver::check_coarse_cycle(double* diff)
+{
+    const int lc = coarse_first();
+    if (lc < 0 || !sigma_ready) {
+        set_error("check_coarse_cycle: the plan has no cluster-cycled levels (levels " + std::to_string(L.size()) +
+                  ", dense bottom " + std::to_string((int)dense_bottom) + " of " + std::to_string(nbottom) +
+                  " nodes, cluster path " + std::to_string((int)use_coarse) + ") or no sigma (" +
+                  std::to_string((int)sigma_ready) + ")");
+        return GBP_BAD_ARG;
+    }
+    *diff = 0.0;
+    const int rc = tail_difference<float>(lc, diff);
+    if (rc || opt.precision == GBP_PREC_MIXED || tail64.first < 0) return rc;
+    return tail_difference<double>(tail64.first, diff);
 }
 
 }  // namespace gbp

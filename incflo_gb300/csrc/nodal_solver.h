@@ -243,10 +243,13 @@ private:
     int coarse_first() const { return use_coarse && opt.nu1 >= 1 && opt.nu2 >= 1 ? tail32.first : -1; }
 public:
     // test hook: one FP32 V-cycle from the first cluster-cycled level on a seeded right-hand side, through
-    // the per-level launches and through the cluster kernel; *diff = max |difference| / max |result|
+    // the per-level launches and through the cluster kernel; *diff = max |difference| / max |result| (of the FP64 V-cycle
+    // as well where the plan runs one through the cluster: the larger one)
     int check_coarse_cycle(double* diff);
 
 private:
+    template <typename T>
+    int tail_difference(int lc, double* diff);
     double omega_eff = 0.85;  // the fixed smoother weight (see set_omega)
     // weights of the pre- and post-smoothing sweeps of a V-cycle level (sweep p: [p % kSweepWeights])
     double wpre[kSweepWeights] = {}, wpost[kSweepWeights] = {};

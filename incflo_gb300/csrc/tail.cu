@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "bottom.h"
 #include "nodal_op.cuh"
 
 namespace gbp {
@@ -329,8 +330,10 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_nodal_tail(const __grid_con
                 // x = M b (a singular system's right-hand side made consistent over the free nodes first), by the first
                 // warps: an FP64 instruction costs the SM 16 cycles per warp
                 if (threadIdx.x < 32 && a.singular) {
-                    double sb = 0.0, sv = 0.0, vu[2] = {};
-                    for (int h = 0; h < 2; ++h) {
+                    constexpr int kOwn = (kDenseBottom + 31) / 32;  // unknowns of a lane
+                    double sb = 0.0, sv = 0.0, vu[kOwn] = {};
+#pragma unroll
+                    for (int h = 0; h < kOwn; ++h) {
                         const int u = threadIdx.x + 32 * h;
                         if (u >= N) break;
                         int ui, uj, uk;
@@ -345,7 +348,8 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_nodal_tail(const __grid_con
                         sv += __shfl_xor_sync(0xffffffffu, sv, o);
                     }
                     const double m = sv > 0.0 ? sb / sv : 0.0;
-                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int h = 0; h < kOwn; ++h)
                         if (threadIdx.x + 32 * h < N) bb[threadIdx.x + 32 * h] -= m * vu[h];
                 }
                 __syncthreads();

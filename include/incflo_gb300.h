@@ -404,10 +404,11 @@ int gbp_plan_time_kernel(gbp_plan* plan, int which, int reps, double* ms_per_lau
 int gbp_plan_check_level_kernels(gbp_plan* plan, double diff[4]);
 
 /* No counterpart in the reference: a test hook. One FP32 V-cycle from the first level that a plan cycles
- * in one thread-block-cluster launch (the FP32 levels of at most 5000 nodes (nodal) / 40000 cells (MAC)
- * below the finest, with the dense bottom), on a seeded right-hand side, once through the per-level launches and
- * once through the cluster kernel; *diff = max |cluster - per-level| / max |per-level| over every padded
- * position. GBP_BAD_ARG when the plan has no such levels. */
+ * in one thread-block-cluster launch (the FP32 levels of at most 5000 nodes or cells, with the dense bottom), on
+ * a seeded right-hand side, once through the per-level launches and once through the cluster kernel; *diff =
+ * max |cluster - per-level| / max |per-level| over every padded position. A nodal plan with precision = fp64
+ * does the same with the FP64 V-cycle (levels of at most 1000 nodes), and *diff is the larger one.
+ * GBP_BAD_ARG when the plan has no such levels. */
 int gbp_plan_check_coarse_cycle(gbp_plan* plan, double* diff);
 
 /* MacProjector::setLevelBC(lev, nullptr, robin_a, robin_b, robin_f) for the GBP_BC_ROBIN sides
