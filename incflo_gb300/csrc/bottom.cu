@@ -18,7 +18,9 @@ namespace {
 __host__ __device__ inline size_t up(size_t v) { return (v + 255) & ~size_t(255); }
 
 // ------------------------------------------------------------------------------------------------ rows
-__global__ void __launch_bounds__(128) k_rows_nodal(NodalGeom g, const double* __restrict__ s, BottomRows r)
+// *empty += unknowns whose row is 0
+__global__ void __launch_bounds__(128) k_rows_nodal(NodalGeom g, const double* __restrict__ s, BottomRows r,
+                                                    unsigned* empty)
 {
     const int u = blockIdx.x * 128 + threadIdx.x;
     if (u >= r.n) return;
@@ -58,6 +60,7 @@ __global__ void __launch_bounds__(128) k_rows_nodal(NodalGeom g, const double* _
     }
     r.diag[u] = held ? 0.0 : a[13];
     r.weight[u] = held ? 0.0 : node_volume(g, i, j, k);
+    if (!held && a[13] == 0.0) atomicAdd(empty, 1u);
 }
 
 __global__ void __launch_bounds__(128) k_rows_mac(CellGeom g, const double* __restrict__ bx, const double* __restrict__ by,
@@ -91,9 +94,10 @@ __global__ void __launch_bounds__(128) k_rows_mac(CellGeom g, const double* __re
 }
 
 // ------------------------------------------------------------------------------------------------ dense inverse
-// Symmetric positive definite, so no pivoting, and Gauss-Jordan as the sweep operator (Goodnight 1979, The American
-// Statistician 33), which keeps the symmetry: one triangle in registers, the pivot's column passed through shared
-// memory, one division per pivot in the warps that hold the column. One SM's FP64 pipe bounds it (16 cycles per warp and instruction): 64
+// Symmetric and, for coefficients of one sign, definite, so no pivoting, and Gauss-Jordan as the sweep operator (Goodnight
+// 1979, The American Statistician 33), which keeps the symmetry: one triangle in registers, the pivot's column passed
+// through shared memory, one division per pivot in the warps that hold the column. (Coefficients of both signs or NaN go
+// through as well: the inverse is a preconditioner, and the solve's residual decides.) One SM's FP64 pipe bounds it (16 cycles per warp and instruction): 64
 // unknowns took 243 us with the whole matrix and a division in every warp, now 75.
 __global__ void __launch_bounds__(1024) k_bottom_inverse(BottomRows r, int singular, double* __restrict__ M,
                                                          unsigned char* __restrict__ act, unsigned* bad)
@@ -103,7 +107,7 @@ __global__ void __launch_bounds__(1024) k_bottom_inverse(BottomRows r, int singu
     const int N = r.n, t = threadIdx.x;
     // entry (u, v) of the matrix
     auto entry = [&](int u, int v) {
-        if (r.diag[u] == 0.0) return u == v ? 1.0 : 0.0;
+        if (r.weight[u] == 0.0) return u == v ? 1.0 : 0.0;
         double sum = 0.0;
         for (int q = 0; q < r.w; ++q)
             if (r.idx[(size_t)q * N + u] == v) sum += r.coef[(size_t)q * N + u];
@@ -111,7 +115,7 @@ __global__ void __launch_bounds__(1024) k_bottom_inverse(BottomRows r, int singu
     };
     double tr = 0.0, na = 0.0;
     if (t < N) {
-        const bool held = r.diag[t] == 0.0;
+        const bool held = r.weight[t] == 0.0;
         scl[t] = held ? 0.0 : entry(t, t);
         col[0][t] = held ? 0.0 : 1.0;
         if (act) act[t] = !held;
@@ -143,7 +147,7 @@ __global__ void __launch_bounds__(1024) k_bottom_inverse(BottomRows r, int singu
         a[m] = 0.0;
         if (u < N) {
             a[m] = entry(u, ev[m]);
-            if (r.diag[u] != 0.0 && r.diag[ev[m]] != 0.0) a[m] += shift;
+            if (r.weight[u] != 0.0 && r.weight[ev[m]] != 0.0) a[m] += shift;
         }
     }
     __syncthreads();
@@ -154,7 +158,7 @@ __global__ void __launch_bounds__(1024) k_bottom_inverse(BottomRows r, int singu
     for (int c = 0; c < N; ++c) {
         const double* cc = col[c & 1];
         const double piv = cc[c];
-        if (!(piv > 0.0)) {  // uniform
+        if (piv == 0.0) {  // uniform
             if (t == 0) *bad = 1u;
             return;
         }
@@ -184,7 +188,7 @@ __global__ void __launch_bounds__(1024) k_bottom_inverse(BottomRows r, int singu
     for (int m = 0; m < kMost; ++m) {
         const int u = eu[m], v = ev[m];
         if (u < 0) continue;
-        const double x = r.diag[u] != 0.0 && r.diag[v] != 0.0 ? -a[m] : 0.0;
+        const double x = r.weight[u] != 0.0 && r.weight[v] != 0.0 ? -a[m] : 0.0;
         M[u * N + v] = x;
         M[v * N + u] = x;
     }
@@ -473,9 +477,9 @@ void BottomRows::carve(char* base)
     weight = reinterpret_cast<double*>(take(sizeof(double) * n));
 }
 
-void bottom_rows_nodal(const NodalGeom& g, const double* s64, const BottomRows& r, cudaStream_t st)
+void bottom_rows_nodal(const NodalGeom& g, const double* s64, const BottomRows& r, unsigned* empty, cudaStream_t st)
 {
-    k_rows_nodal<<<(r.n + 127) / 128, 128, 0, st>>>(g, s64, r);
+    k_rows_nodal<<<(r.n + 127) / 128, 128, 0, st>>>(g, s64, r, empty);
 }
 void bottom_rows_mac(const CellGeom& g, const double* bx, const double* by, const double* bz, const BottomRows& r,
                      cudaStream_t st)

@@ -24,18 +24,18 @@ struct BottomRows {
     int n = 0, w = 0;          // unknowns, entries per row (27 nodal, 7 cell-centred)
     double* coef = nullptr;    // [w][n]
     int* idx = nullptr;        // [w][n] unknown of each entry
-    double* diag = nullptr;    // [n], 0: no equation (held at 0)
-    double* weight = nullptr;  // [n] null-space weight of each unknown (node volume / 1), 0 where held
+    double* diag = nullptr;    // [n]
+    double* weight = nullptr;  // [n] null-space weight of each unknown (node volume / 1), 0: no equation (held at 0)
     size_t bytes() const { return (size_t)n * w * 12 + (size_t)n * 16 + 1024; }
     void carve(char* base);    // sets the arrays inside `bytes()` bytes at base (256-byte aligned)
 };
 
-void bottom_rows_nodal(const NodalGeom& g, const double* s64, const BottomRows& r, cudaStream_t st);
+// *empty += unknowns that are not held but have an empty row (sigma 0 in all their cells)
+void bottom_rows_nodal(const NodalGeom& g, const double* s64, const BottomRows& r, unsigned* empty, cudaStream_t st);
 void bottom_rows_mac(const CellGeom& g, const double* bx, const double* by, const double* bz, const BottomRows& r,
                      cudaStream_t st);
 // M (n x n) = inverse of the rows' matrix (singular: of A + c 1 1^T over the unknowns that carry an equation), rows and
-// columns of held unknowns 0; act (may be null): 1 where an unknown carries an equation. *bad = 1 when a pivot is not
-// positive.
+// columns of held unknowns 0; act (may be null): 1 where an unknown carries an equation. *bad = 1 when a pivot is 0.
 void bottom_inverse(const BottomRows& r, int singular, double* M, unsigned char* act, unsigned* bad, cudaStream_t st);
 
 struct BottomCG {

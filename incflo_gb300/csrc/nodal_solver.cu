@@ -416,15 +416,16 @@ int NodalSolver::level_of(const NodalGeom& g) const
 int NodalSolver::build_bottom()
 {
     if (!brows.n) return GBP_OK;
-    bottom_rows_nodal(L.back().g, L.back().s64, brows, st);
-    if (!dense_bottom) return GBP_OK;
-    unsigned* bad = reinterpret_cast<unsigned*>(dinfo + 12);
-    GBP_CUDA(cudaMemsetAsync(bad, 0, sizeof(unsigned), st));
-    bottom_inverse(brows, bsing ? 1 : 0, dmat, nullptr, bad, st);
-    unsigned h = 0;
-    GBP_CUDA(cudaMemcpyAsync(&h, bad, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    unsigned* bad = reinterpret_cast<unsigned*>(dinfo + 12);  // a pivot of 0, and the number of empty rows
+    GBP_CUDA(cudaMemsetAsync(bad, 0, 2 * sizeof(unsigned), st));
+    bottom_rows_nodal(L.back().g, L.back().s64, brows, bad + 1, st);
+    if (dense_bottom) bottom_inverse(brows, bsing ? 1 : 0, dmat, nullptr, bad, st);
+    if (nbottom > kCheckedBottom) return GBP_OK;
+    unsigned h[2] = {0, 0};
+    GBP_CUDA(cudaMemcpyAsync(h, bad, sizeof(h), cudaMemcpyDeviceToHost, st));
     GBP_CUDA(cudaStreamSynchronize(st));
-    if (h) {
+    // (the constants of a singular system make up for one empty row)
+    if (h[0] || h[1] > (bsing ? 1u : 0u)) {
         set_error("nodal plan: the coarsest operator is singular beyond its constant null space");
         return GBP_BAD_ARG;
     }

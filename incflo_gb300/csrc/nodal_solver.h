@@ -281,6 +281,8 @@ private:
     int gexec_prec = -1;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     int nbottom = 0;
+    // up to this many unknowns, sigma that leaves the coarsest operator singular beyond its constants is refused when it is set
+    static constexpr int kCheckedBottom = 216;
     bool dense_bottom = false;
     double* dmat = nullptr;      // dense inverse of the coarsest operator (transposed)
     double* dscal = nullptr;     // device scalars of the mean / gauge corrections
