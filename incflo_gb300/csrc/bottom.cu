@@ -368,7 +368,8 @@ __global__ void __launch_bounds__(kBottomThreads) k_bottom_cg(G g, BottomCG c, c
             if (vec)
                 for (int u = threadIdx.x; u < nr; u += vstep) pq += p[u0 + u] * qv[u];
             sum(pq, unused);
-            if (!(pq > 0.0)) break;
+            // (with the sign of r.z: the operator is negative for negative coefficients)
+            if (!(__hiloint2double(__double2hiint(pq) ^ (__double2hiint(rz) & (int)0x80000000u), __double2loint(pq)) > 0.0)) break;
             double rz2 = 0.0;
             rr = 0.0;
             if (vec) {

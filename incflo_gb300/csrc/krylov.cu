@@ -194,18 +194,20 @@ __global__ void __launch_bounds__(kT) k_dots(KrylovBox b, const T* __restrict__ 
     if (WHAT == 0) {
         s->rz = s0;
         double beta = 0.0;
-        if (two && !s->restart && s->rz_old > 0.0) {
+        if (two && !s->restart && s->rz_old != 0.0) {
             beta = s->alpha * s1 / s->rz_old;
             if (!(beta > 0.0 && beta < 1e30)) beta = 0.0;
         }
         s->beta = beta;
         s->rz_old = s0;
     } else {
-        // a breakdown (rounding has the last word) takes the plain V-cycle step, or starts the directions again
+        // r.z and p.Ap have one sign, that of the operator (coefficients may be negative throughout). A breakdown (rounding
+        // has the last word) takes the plain V-cycle step, or starts the directions again.
         const double pap = -s0;
-        const bool ok = pap > 0.0 && s->rz > 0.0;
+        const double alpha = s->rz / pap;
+        const bool ok = alpha > 0.0 && alpha < 1e30;
         s->pq = pap;
-        s->alpha = ok ? s->rz / pap : (s->beta == 0.0 ? 1.0 : 0.0);
+        s->alpha = ok ? alpha : (s->beta == 0.0 ? 1.0 : 0.0);
         s->restart = !ok;
         s->it += 1;
     }
