@@ -1,6 +1,6 @@
-// Vector kernels of the conjugate-gradient acceleration (krylov.h). HBM bounds them on large levels: the dot product
-// of three vectors, the direction and the update move 3, 3 and 6 vectors once each with 16-byte accesses; on small
-// levels each is one launch.
+// Vector kernels of the conjugate-gradient acceleration (krylov.h). HBM bounds them on large levels: the two dot
+// products, the direction and the update move 2, 3, 3 and 6 vectors once each with 16-byte accesses; on small levels each is
+// one launch.
 #include "krylov.h"
 
 #include <algorithm>
@@ -149,10 +149,10 @@ __device__ __forceinline__ bool fold_last(Sum<T> (&v)[NV], double* part, unsigne
     return true;
 }
 
-// a.b and a.c (c may be null) over the unique points. FP32 vectors are summed in FP32 per thread (a few hundred
-// terms), as pairs over the block and in FP64 from there. Latency and the FP64 pipe bound it below some 10^6 points:
-// with FP64 sums in every warp 17.2 us (r.z, 10^6 points FP32), 13.9 us (64^3 FP64), 9.8 us (16^3 FP64); now 10.5, 11.3
-// and 7.2 us.
+// a.b (WHAT 0: z.q and beta) or a.b and a.c (WHAT 1: p.q, p.r and alpha) over the unique points. FP32 vectors are summed in
+// FP32 per thread (a few hundred terms), as pairs over the block and in FP64 from there. Latency and the FP64 pipe bound it
+// below some 10^6 points: with FP64 sums in every warp 17.2 us (two products, 10^6 points FP32), 13.9 us (64^3 FP64), 9.8 us
+// (16^3 FP64); now 10.5, 11.3 and 7.2 us.
 template <typename T, int WHAT>
 __global__ void __launch_bounds__(kT) k_dots(KrylovBox b, const T* __restrict__ a, const T* __restrict__ c,
                                              const T* __restrict__ d, double* __restrict__ part, KrylovState* s)
@@ -160,23 +160,23 @@ __global__ void __launch_bounds__(kT) k_dots(KrylovBox b, const T* __restrict__ 
     constexpr int N = Vec<T>::N;
     const unsigned vr = (unsigned)(b.n[0] + N - 1) / N;
     const unsigned total = vr * (unsigned)b.n[1] * (unsigned)b.n[2];
-    const bool two = WHAT == 0 && s->it > 0;
     T acc0[N] = {}, acc1[N] = {};
-    for (unsigned t = blockIdx.x * kT + threadIdx.x; t < total; t += gridDim.x * kT) {
-        int i;
-        const long long p = vec_at<T>(b, t, vr, i);
-        T x[N], y[N], z[N];
-        ldv<T>(a + p, x);
-        ldv<T>(c + p, y);
-        if (two) ldv<T>(d + p, z);
+    if (WHAT == 1 || s->it > 0)
+        for (unsigned t = blockIdx.x * kT + threadIdx.x; t < total; t += gridDim.x * kT) {
+            int i;
+            const long long p = vec_at<T>(b, t, vr, i);
+            T x[N], y[N], z[N];
+            ldv<T>(a + p, x);
+            ldv<T>(c + p, y);
+            if (WHAT == 1) ldv<T>(d + p, z);
 #pragma unroll
-        for (int e = 0; e < N; ++e) {
-            if (i + e >= b.n[0]) continue;
-            acc0[e] += x[e] * y[e];
-            if (two) acc1[e] += y[e] * z[e];
+            for (int e = 0; e < N; ++e) {
+                if (i + e >= b.n[0]) continue;
+                acc0[e] += x[e] * y[e];
+                if (WHAT == 1) acc1[e] += x[e] * z[e];
+            }
         }
-    }
-    constexpr int NV = WHAT == 0 ? 2 : 1;
+    constexpr int NV = WHAT == 1 ? 2 : 1;
     __shared__ double out[2];
     Sum<T> v[NV];
 #pragma unroll
@@ -192,21 +192,15 @@ __global__ void __launch_bounds__(kT) k_dots(KrylovBox b, const T* __restrict__ 
     if (!fold_last<T, NV>(v, part, s->done + WHAT, out) || threadIdx.x) return;
     const double s0 = out[0], s1 = out[NV - 1];
     if (WHAT == 0) {
-        s->rz = s0;
-        double beta = 0.0;
-        if (two && !s->restart && s->rz_old != 0.0) {
-            beta = s->alpha * s1 / s->rz_old;
-            if (!(beta > 0.0 && beta < 1e30)) beta = 0.0;
-        }
+        double beta = s->it > 0 && !s->restart ? s0 / s->pap : 0.0;
+        if (!(beta > 0.0 && beta < 1e30)) beta = 0.0;
         s->beta = beta;
-        s->rz_old = s0;
     } else {
-        // r.z and p.Ap have one sign, that of the operator (coefficients may be negative throughout). A breakdown (rounding
+        // p.r and p.Ap have one sign, that of the operator (coefficients may be negative throughout). A breakdown (rounding
         // has the last word) takes the plain V-cycle step, or starts the directions again.
-        const double pap = -s0;
-        const double alpha = s->rz / pap;
+        const double pap = -s0, alpha = s1 / pap;
         const bool ok = alpha > 0.0 && alpha < 1e30;
-        s->pq = pap;
+        s->pap = pap;
         s->alpha = ok ? alpha : (s->beta == 0.0 ? 1.0 : 0.0);
         s->restart = !ok;
         s->it += 1;
@@ -296,9 +290,9 @@ unsigned dot_blocks(const KrylovBox& b, int vec)
 }  // namespace
 
 template <typename T>
-void krylov_rz(const KrylovBox& b, const T* r, const T* z, const T* q, double* part, KrylovState* s, cudaStream_t st)
+void krylov_beta(const KrylovBox& b, const T* z, const T* q, double* part, KrylovState* s, cudaStream_t st)
 {
-    k_dots<T, 0><<<dot_blocks(b, Vec<T>::N), kT, 0, st>>>(b, r, z, q, part, s);
+    k_dots<T, 0><<<dot_blocks(b, Vec<T>::N), kT, 0, st>>>(b, z, q, nullptr, part, s);
 }
 template <typename T>
 void krylov_direction(const KrylovBox& b, const T* z, T* p, const KrylovState* s, cudaStream_t st)
@@ -307,9 +301,9 @@ void krylov_direction(const KrylovBox& b, const T* z, T* p, const KrylovState* s
     k_direction<T><<<(unsigned)((nv + kT - 1) / kT), kT, 0, st>>>(nv, z, p, s);
 }
 template <typename T>
-void krylov_pq(const KrylovBox& b, const T* p, const T* q, double* part, KrylovState* s, cudaStream_t st)
+void krylov_alpha(const KrylovBox& b, const T* p, const T* q, const T* r, double* part, KrylovState* s, cudaStream_t st)
 {
-    k_dots<T, 1><<<dot_blocks(b, Vec<T>::N), kT, 0, st>>>(b, p, q, nullptr, part, s);
+    k_dots<T, 1><<<dot_blocks(b, Vec<T>::N), kT, 0, st>>>(b, p, q, r, part, s);
 }
 template <typename T>
 void krylov_update(const KrylovBox& b, const T* p, const T* q, T* x, T* r, const KrylovState* s, cudaStream_t st,
@@ -324,10 +318,11 @@ void krylov_update(const KrylovBox& b, const T* p, const T* q, T* x, T* r, const
 }
 
 #define GBP_KRYLOV(T)                                                                                               \
-    template void krylov_rz<T>(const KrylovBox&, const T*, const T*, const T*, double*, KrylovState*, cudaStream_t); \
+    template void krylov_beta<T>(const KrylovBox&, const T*, const T*, double*, KrylovState*, cudaStream_t);         \
     template void krylov_direction<T>(const KrylovBox&, const T*, T*, const KrylovState*, cudaStream_t);             \
-    template void krylov_pq<T>(const KrylovBox&, const T*, const T*, double*, KrylovState*, cudaStream_t);           \
-    template void krylov_update<T>(const KrylovBox&, const T*, const T*, T*, T*, const KrylovState*, cudaStream_t,        \
+    template void krylov_alpha<T>(const KrylovBox&, const T*, const T*, const T*, double*, KrylovState*,             \
+                                  cudaStream_t);                                                                     \
+    template void krylov_update<T>(const KrylovBox&, const T*, const T*, T*, T*, const KrylovState*, cudaStream_t,   \
                                    const KrylovNorm*);
 GBP_KRYLOV(double)
 GBP_KRYLOV(float)

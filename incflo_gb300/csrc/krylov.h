@@ -2,10 +2,14 @@
 // z = V r) and the operator q = -A p (the sign the residual kernels give with no right-hand side), on the padded layouts
 // of the nodal and cell-centred levels.
 //
-// Flexible form: beta = z.(r_new - r_old) / (r.z)_old = alpha q.z / (r.z)_old, which needs no symmetry of the
-// V-cycle beyond what rounding leaves of it, and costs one more dot product over vectors that are read anyway. The
-// scalars stay on the device (no host round trip inside an iteration); the dot products are folded in a fixed order
-// by the last block to finish, so a solve is reproducible bit by bit.
+// Flexible form: beta = (z.q) / (p.Ap) of the last direction makes the new one conjugate to it, and alpha = (r.p) / (p.Ap)
+// is the exact minimum along it. Neither assumes that r is orthogonal to the last direction (as alpha = r.z / p.Ap and
+// beta = z.(r_new - r_old) / (r.z)_old do): between two refinement steps of an FP32 solve the recursion's residual is
+// replaced by the true one, and a solve that reached its rounding has lost the orthogonality anyway. With those forms the
+// iteration kept its wrong steps from there on: 20 to 40 V-cycles instead of 8 on 2^3 cells, where a V-cycle is an exact
+// solve, or a residual that grew from step to step. The scalars stay on the device (no host round trip inside an
+// iteration); the dot products are folded in a fixed order by the last block to finish, so a solve is reproducible bit by
+// bit.
 //
 // With a V-cycle that contracts the error by rho per application, the stationary iteration needs log(tol) / log(rho)
 // of them; the accelerated one removes the few slow modes that set rho (a density jump, cut cells, stretched cells):
@@ -24,7 +28,7 @@ struct KrylovBox {
 };
 
 struct KrylovState {
-    double rz, rz_old, qz, pq, alpha, beta;
+    double pap, alpha, beta;
     int it, restart;
     unsigned done[2];  // blocks that finished a dot product (reset by the last one)
     // power-of-two scale of an FP32 right-hand side, and its inverse: read on the device, so that a captured step
@@ -35,15 +39,15 @@ struct KrylovState {
 // most blocks of a dot product (2 partial sums each in the scratch)
 constexpr int kKrylovBlocks = 608;
 
-// rz = r.z and, after the first iteration, beta; q: the last iteration's -A p
+// beta = (z.q) / (p.Ap) of the last iteration (the first: 0); q: its -A p
 template <typename T>
-void krylov_rz(const KrylovBox& b, const T* r, const T* z, const T* q, double* part, KrylovState* s, cudaStream_t st);
+void krylov_beta(const KrylovBox& b, const T* z, const T* q, double* part, KrylovState* s, cudaStream_t st);
 // p = z + beta p over the whole padded array (z carries its periodic aliases)
 template <typename T>
 void krylov_direction(const KrylovBox& b, const T* z, T* p, const KrylovState* s, cudaStream_t st);
-// alpha = rz / (p.Ap), q = -A p
+// alpha = (r.p) / (p.Ap), q = -A p
 template <typename T>
-void krylov_pq(const KrylovBox& b, const T* p, const T* q, double* part, KrylovState* s, cudaStream_t st);
+void krylov_alpha(const KrylovBox& b, const T* p, const T* q, const T* r, double* part, KrylovState* s, cudaStream_t st);
 // The max of |r| / V over the points that are not held, for krylov_update: *norm = max(*norm, it). nodal[d]: the points
 // on the sides of direction d have half the volume; dlo / dhi: held sides; mask: 0 on held points (padded), or null.
 struct KrylovNorm {

@@ -870,11 +870,11 @@ void MacSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s, const KrylovNorm
     for (int c = 0; c < m; ++c) {
         vcycle<T>(0, r, true);
         const T* z = B::x(l0);
-        krylov_rz<T>(kbox, r, z, q, kpart, kstate, s);
+        krylov_beta<T>(kbox, z, q, kpart, kstate, s);
         krylov_direction<T>(kbox, z, p, kstate, s);
         mac_resid<T>(l0.g, be[0], be[1], be[2], p, nullptr, q, nullptr, s);
         if (eb.on) eb_cells<T>(l0.g, eb.cells, eb.ncells, eb.faces, B::cb(eb), p, q, q, s);
-        krylov_pq<T>(kbox, p, q, kpart, kstate, s);
+        krylov_alpha<T>(kbox, p, q, r, kpart, kstate, s);
         krylov_update<T>(kbox, p, q, x, r, kstate, s, c == m - 1 ? norm : nullptr);
     }
 }

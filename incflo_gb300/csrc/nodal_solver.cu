@@ -702,10 +702,10 @@ void NodalSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s, const KrylovNo
     for (int c = 0; c < m; ++c) {
         vcycle<T>(0, r, true);
         const T* z = (const T*)xres[0];
-        krylov_rz<T>(kbox, r, z, q, kpart, kstate, s);
+        krylov_beta<T>(kbox, z, q, kpart, kstate, s);
         krylov_direction<T>(kbox, z, p, kstate, s);
         apply_neg<T>(p, q, s);
-        krylov_pq<T>(kbox, p, q, kpart, kstate, s);
+        krylov_alpha<T>(kbox, p, q, r, kpart, kstate, s);
         krylov_update<T>(kbox, p, q, x, r, kstate, s, c == m - 1 ? norm : nullptr);
         nk += 5;
     }
