@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kT) k_dots(KrylovBox b, const T* __restrict__ 
     if (!fold_last<T, NV>(v, part, s->done + WHAT, out) || threadIdx.x) return;
     const double s0 = out[0], s1 = out[NV - 1];
     if (WHAT == 0) {
-        double beta = s->it > 0 && !s->restart ? s0 / s->pap : 0.0;
+        double beta = s->it > 0 && !s->restart && !s->plain ? s0 / s->pap : 0.0;
         if (!(beta > 0.0 && beta < 1e30)) beta = 0.0;
         s->beta = beta;
     } else {
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kT) k_dots(KrylovBox b, const T* __restrict__ 
         const double pap = -s0, alpha = s1 / pap;
         const bool ok = alpha > 0.0 && alpha < 1e30;
         s->pap = pap;
-        s->alpha = ok ? alpha : (s->beta == 0.0 ? 1.0 : 0.0);
+        s->alpha = ok && !s->plain ? alpha : (s->beta == 0.0 ? 1.0 : 0.0);
         s->restart = !ok;
         s->it += 1;
     }

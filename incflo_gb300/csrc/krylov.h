@@ -30,6 +30,7 @@ struct KrylovBox {
 struct KrylovState {
     double pap, alpha, beta;
     int it, restart;
+    int plain;  // 1: stationary steps (beta 0, alpha 1)
     unsigned done[2];  // blocks that finished a dot product (reset by the last one)
     // power-of-two scale of an FP32 right-hand side, and its inverse: read on the device, so that a captured step
     // serves every right-hand side
