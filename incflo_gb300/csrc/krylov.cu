@@ -132,7 +132,7 @@ __device__ __forceinline__ bool fold_last(Sum<T> (&v)[NV], double* part, unsigne
     __syncthreads();
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int q = 0; q < NV; ++q) part[2 * blockIdx.x + q] = out[q];
+        for (int q = 0; q < NV; ++q) part[kKrylovSums * blockIdx.x + q] = out[q];
         __threadfence();
         last = atomicAdd(done, 1u) == gridDim.x - 1;
     }
@@ -142,7 +142,7 @@ __device__ __forceinline__ bool fold_last(Sum<T> (&v)[NV], double* part, unsigne
     Sum<double> f[NV];
     for (unsigned b = threadIdx.x; b < gridDim.x; b += kT)
 #pragma unroll
-        for (int q = 0; q < NV; ++q) f[q].v += __ldcg(part + 2 * b + q);
+        for (int q = 0; q < NV; ++q) f[q].v += __ldcg(part + kKrylovSums * b + q);
     block_sums(f, tab, out);
     __syncthreads();
     if (threadIdx.x == 0) *done = 0;
@@ -153,14 +153,16 @@ __device__ __forceinline__ bool fold_last(Sum<T> (&v)[NV], double* part, unsigne
 // FP32 per thread (a few hundred terms), as pairs over the block and in FP64 from there. Latency and the FP64 pipe bound it
 // below some 10^6 points: with FP64 sums in every warp 17.2 us (two products, 10^6 points FP32), 13.9 us (64^3 FP64), 9.8 us
 // (16^3 FP64); now 10.5, 11.3 and 7.2 us.
-template <typename T, int WHAT>
+// NULLSPACE (WHAT 1, singular systems): p.r without the constants of either, p.r - (sum p)(sum r) / n. In FP64 the two sums
+// more bind it (117 against 62 us at 256^3, and 5 us more per launch on small levels).
+template <typename T, int WHAT, bool NULLSPACE>
 __global__ void __launch_bounds__(kT) k_dots(KrylovBox b, const T* __restrict__ a, const T* __restrict__ c,
                                              const T* __restrict__ d, double* __restrict__ part, KrylovState* s)
 {
-    constexpr int N = Vec<T>::N;
+    constexpr int N = Vec<T>::N, NV = WHAT == 0 ? 1 : (NULLSPACE ? 4 : 2);
     const unsigned vr = (unsigned)(b.n[0] + N - 1) / N;
     const unsigned total = vr * (unsigned)b.n[1] * (unsigned)b.n[2];
-    T acc0[N] = {}, acc1[N] = {};
+    T acc[NV][N] = {};
     if (WHAT == 1 || s->it > 0)
         for (unsigned t = blockIdx.x * kT + threadIdx.x; t < total; t += gridDim.x * kT) {
             int i;
@@ -172,33 +174,36 @@ __global__ void __launch_bounds__(kT) k_dots(KrylovBox b, const T* __restrict__ 
 #pragma unroll
             for (int e = 0; e < N; ++e) {
                 if (i + e >= b.n[0]) continue;
-                acc0[e] += x[e] * y[e];
-                if (WHAT == 1) acc1[e] += x[e] * z[e];
+                acc[0][e] += x[e] * y[e];
+                if constexpr (WHAT == 1) acc[1][e] += x[e] * z[e];
+                if constexpr (NULLSPACE) {
+                    acc[2][e] += x[e];
+                    acc[3][e] += z[e];
+                }
             }
         }
-    constexpr int NV = WHAT == 1 ? 2 : 1;
-    __shared__ double out[2];
+    __shared__ double out[NV];
     Sum<T> v[NV];
 #pragma unroll
-    for (int e = 0; e < N; ++e) {
-        if constexpr (sizeof(T) == 4) {
-            v[0].add(acc0[e], 0.f);
-            if (NV == 2) v[NV - 1].add(acc1[e], 0.f);
-        } else {
-            v[0].v += acc0[e];
-            if (NV == 2) v[NV - 1].v += acc1[e];
+    for (int q = 0; q < NV; ++q)
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+            if constexpr (sizeof(T) == 4)
+                v[q].add(acc[q][e], 0.f);
+            else
+                v[q].v += acc[q][e];
         }
-    }
     if (!fold_last<T, NV>(v, part, s->done + WHAT, out) || threadIdx.x) return;
-    const double s0 = out[0], s1 = out[NV - 1];
-    if (WHAT == 0) {
-        double beta = s->it > 0 && !s->restart && !s->plain ? s0 / s->pap : 0.0;
+    if constexpr (WHAT == 0) {
+        double beta = s->it > 0 && !s->restart && !s->plain ? out[0] / s->pap : 0.0;
         if (!(beta > 0.0 && beta < 1e30)) beta = 0.0;
         s->beta = beta;
     } else {
         // p.r and p.Ap have one sign, that of the operator (coefficients may be negative throughout). A breakdown (rounding
         // has the last word) takes the plain V-cycle step, or starts the directions again.
-        const double pap = -s0, alpha = s1 / pap;
+        double rp = out[1];
+        if constexpr (NULLSPACE) rp -= out[2] * out[3] * b.null_inv;
+        const double pap = -out[0], alpha = rp / pap;
         const bool ok = alpha > 0.0 && alpha < 1e30;
         s->pap = pap;
         s->alpha = ok && !s->plain ? alpha : (s->beta == 0.0 ? 1.0 : 0.0);
@@ -292,7 +297,7 @@ unsigned dot_blocks(const KrylovBox& b, int vec)
 template <typename T>
 void krylov_beta(const KrylovBox& b, const T* z, const T* q, double* part, KrylovState* s, cudaStream_t st)
 {
-    k_dots<T, 0><<<dot_blocks(b, Vec<T>::N), kT, 0, st>>>(b, z, q, nullptr, part, s);
+    k_dots<T, 0, false><<<dot_blocks(b, Vec<T>::N), kT, 0, st>>>(b, z, q, nullptr, part, s);
 }
 template <typename T>
 void krylov_direction(const KrylovBox& b, const T* z, T* p, const KrylovState* s, cudaStream_t st)
@@ -303,7 +308,8 @@ void krylov_direction(const KrylovBox& b, const T* z, T* p, const KrylovState* s
 template <typename T>
 void krylov_alpha(const KrylovBox& b, const T* p, const T* q, const T* r, double* part, KrylovState* s, cudaStream_t st)
 {
-    k_dots<T, 1><<<dot_blocks(b, Vec<T>::N), kT, 0, st>>>(b, p, q, r, part, s);
+    (b.null_inv != 0.0 ? k_dots<T, 1, true> : k_dots<T, 1, false>)<<<dot_blocks(b, Vec<T>::N), kT, 0, st>>>(b, p, q, r, part,
+                                                                                                           s);
 }
 template <typename T>
 void krylov_update(const KrylovBox& b, const T* p, const T* q, T* x, T* r, const KrylovState* s, cudaStream_t st,

@@ -25,6 +25,7 @@ namespace gbp {
 struct KrylovBox {
     int n[3];
     long long sy, sz, count;
+    double null_inv;  // 1 / the number of unknowns of a system whose null space are the constants, or 0 (krylov_alpha)
 };
 
 struct KrylovState {
@@ -37,8 +38,10 @@ struct KrylovState {
     double scale, inv_scale;
 };
 
-// most blocks of a dot product (2 partial sums each in the scratch)
-constexpr int kKrylovBlocks = 608;
+constexpr double kNearRounding = 1e-12;
+
+// most blocks of a dot product, and partial sums of each in the scratch
+constexpr int kKrylovBlocks = 608, kKrylovSums = 4;
 
 // beta = (z.q) / (p.Ap) of the last iteration (the first: 0); q: its -A p
 template <typename T>
@@ -46,7 +49,11 @@ void krylov_beta(const KrylovBox& b, const T* z, const T* q, double* part, Krylo
 // p = z + beta p over the whole padded array (z carries its periodic aliases)
 template <typename T>
 void krylov_direction(const KrylovBox& b, const T* z, T* p, const KrylovState* s, cudaStream_t st);
-// alpha = (r.p) / (p.Ap), q = -A p
+// alpha = (r.p) / (p.Ap), q = -A p. In a singular system r carries the constant that its rounding errors sum up to, which no
+// iteration removes, and p an arbitrary one; their product would drive alpha up without limit once the rest of r is smaller:
+// run on below its rounding a 32 x 24 x 16 FP64 solve went from 3e-18 back to 0.06, and FP32 inner solves of strong V-cycles (8
+// sweeps) spoiled a refinement step by a factor of 10 to 10^5. So r.p leaves the constants out (box.null_inv): always in FP32,
+// and in FP64 below kNearRounding of the right-hand side, where the constant is still far smaller than r.
 template <typename T>
 void krylov_alpha(const KrylovBox& b, const T* p, const T* q, const T* r, double* part, KrylovState* s, cudaStream_t st);
 // The max of |r| / V over the points that are not held, for krylov_update: *norm = max(*norm, it). nodal[d]: the points

@@ -159,7 +159,7 @@ int MacSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc_h
     }
     const CellGeom& G0 = L[0].g;
     for (int q = 0; q < 5; ++q) add(G0.count, 8);
-    add(2 * kKrylovBlocks, 8);
+    add(kKrylovSums * kKrylovBlocks, 8);
     add(1, sizeof(KrylovState));
     add(mac_partials_needed(G0) + 64, 8);
     brows = BottomRows{};
@@ -203,9 +203,9 @@ int MacSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc_h
     res = pool.take<double>(G0.count);
     kp = pool.take<double>(G0.count);
     kq = pool.take<double>(G0.count);
-    kpart = pool.take<double>(2 * kKrylovBlocks);
+    kpart = pool.take<double>(kKrylovSums * kKrylovBlocks);
     kstate = pool.take<KrylovState>(1);
-    kbox = KrylovBox{{G0.n[0], G0.n[1], G0.n[2]}, G0.sy, G0.sz, G0.count};
+    kbox = KrylovBox{{G0.n[0], G0.n[1], G0.n[2]}, G0.sy, G0.sz, G0.count, 0.0};
     partials = pool.take<double>(mac_partials_needed(G0) + 64);
     bscr = nullptr;
     if (brows.n) {
@@ -477,6 +477,7 @@ int MacSolver::set_eb(const gbp_array4* vfrac, const gbp_array4* const area[3], 
     auto cid = [&](int i, int j, int k) { return i + (long long)n[0] * (j + (long long)n[1] * k); };
     auto fid = [&](int d, int i, int j, int k) { return i + (long long)fn[d][0] * (j + (long long)fn[d][1] * k); };
     double ksum = 0.0;
+    long long fluid = 0;
     for (long long c = 0; c < ncell; ++c) {
         const double v = kapH[(size_t)c];
         if (!(v >= 0.0 && v <= 1.0)) {
@@ -484,6 +485,7 @@ int MacSolver::set_eb(const gbp_array4* vfrac, const gbp_array4* const area[3], 
             return GBP_BAD_ARG;
         }
         ksum += v;
+        fluid += v > 0.0;
     }
     if (!(ksum > 0.0)) {
         set_error("mac_set_eb: every cell is covered");
@@ -616,6 +618,7 @@ int MacSolver::set_eb(const gbp_array4* vfrac, const gbp_array4* const area[3], 
     eb.nfaces = (int)F.size();
     eb.ncells = (int)C.size();
     eb.kap_sum = ksum;
+    eb.fluid_cells = fluid;
     if (!F.empty()) GBP_CUDA(cudaMemcpyAsync(eb.faces, F.data(), sizeof(EbFace) * F.size(), cudaMemcpyHostToDevice, st));
     if (!C.empty()) GBP_CUDA(cudaMemcpyAsync(eb.cells, C.data(), sizeof(EbCell) * C.size(), cudaMemcpyHostToDevice, st));
     mac_load_eb(g, *vfrac, area, eb.m, st);
@@ -867,15 +870,17 @@ void MacSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s, const KrylovNorm
     T* const* be = B::b(l0);
     T* p = reinterpret_cast<T*>(kp);
     T* q = reinterpret_cast<T*>(kq);
+    KrylovBox box = kbox;
+    if (singular && (sizeof(T) == 4 || near_rounding)) box.null_inv = 1.0 / (eb.on ? (double)eb.fluid_cells : (double)l0.g.n[0] * l0.g.n[1] * l0.g.n[2]);
     for (int c = 0; c < m; ++c) {
         vcycle<T>(0, r, true);
         const T* z = B::x(l0);
-        krylov_beta<T>(kbox, z, q, kpart, kstate, s);
-        krylov_direction<T>(kbox, z, p, kstate, s);
+        krylov_beta<T>(box, z, q, kpart, kstate, s);
+        krylov_direction<T>(box, z, p, kstate, s);
         mac_resid<T>(l0.g, be[0], be[1], be[2], p, nullptr, q, nullptr, s);
         if (eb.on) eb_cells<T>(l0.g, eb.cells, eb.ncells, eb.faces, B::cb(eb), p, q, q, s);
-        krylov_alpha<T>(kbox, p, q, r, kpart, kstate, s);
-        krylov_update<T>(kbox, p, q, x, r, kstate, s, c == m - 1 ? norm : nullptr);
+        krylov_alpha<T>(box, p, q, r, kpart, kstate, s);
+        krylov_update<T>(box, p, q, x, r, kstate, s, c == m - 1 ? norm : nullptr);
     }
 }
 
@@ -916,7 +921,8 @@ int MacSolver::run_iteration(int m)
         drop_graphs();
         gexec_prec = opt.precision;
     }
-    cudaGraphExec_t& ge = gexec[m];
+    const int slot = near_rounding ? 0 : m;  // (the plain form has m = 1)
+    cudaGraphExec_t& ge = gexec[slot];
     if (!ge) {
         cudaGraph_t graph = nullptr;
         cap_or_st = cap;
@@ -996,6 +1002,7 @@ int MacSolver::solve(bool have_guess, gbp_stats* stats)
             set_error("solve: maxiter reached before the tolerance");
             break;
         }
+        near_rounding = !mixed && singular && rn < kNearRounding * bnorm;
         int rc = run_iteration(m);
         if (rc) return rc;
         GBP_CUDA(cudaStreamSynchronize(st));

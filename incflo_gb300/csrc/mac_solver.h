@@ -106,6 +106,7 @@ private:
     double *kp = nullptr, *kq = nullptr, *kpart = nullptr;
     KrylovState *kstate = nullptr, *hstate = nullptr;
     KrylovBox kbox{};
+    bool near_rounding = false;  // FP64 steps of a singular system whose residual is close to its rounding (krylov.h)
     template <typename T>
     void krylov_steps(int m, T* x, T* r, cudaStream_t s, const KrylovNorm* norm = nullptr);
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
@@ -144,6 +145,7 @@ private:
         double* beff64 = nullptr;  // finest-level right-hand side with the lagged cut-face terms
         float* beff32 = nullptr;
         double kap_sum = 0.0;
+        long long fluid_cells = 0;  // not covered
         bool on = false;
     } eb;
 };

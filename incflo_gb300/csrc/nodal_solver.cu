@@ -278,7 +278,7 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
     }
     const NodalGeom& G0 = L[0].g;
     for (int q = 0; q < 5; ++q) add(G0.count, 8);
-    add(2 * kKrylovBlocks, 8);
+    add(kKrylovSums * kKrylovBlocks, 8);
     add(1, sizeof(KrylovState));
     for (auto& lv : L)
         if (qsweep_supported(lv.g))
@@ -324,9 +324,9 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
     res = pool.take<double>(G0.count);
     kp = pool.take<double>(G0.count);
     kq = pool.take<double>(G0.count);
-    kpart = pool.take<double>(2 * kKrylovBlocks);
+    kpart = pool.take<double>(kKrylovSums * kKrylovBlocks);
     kstate = pool.take<KrylovState>(1);
-    kbox = KrylovBox{{G0.nu[0], G0.nu[1], G0.nu[2]}, G0.sy, G0.sz, G0.count};
+    kbox = KrylovBox{{G0.nu[0], G0.nu[1], G0.nu[2]}, G0.sy, G0.sz, G0.count, 0.0};
     for (auto& lv : L)
         if (qsweep_supported(lv.g))
             for (double** w : {&lv.qw.w5, &lv.qw.rd, &lv.qw.wx, &lv.qw.wy, &lv.qw.wz}) *w = pool.take<double>(lv.g.count);
@@ -699,14 +699,16 @@ void NodalSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s, const KrylovNo
 {
     T* p = reinterpret_cast<T*>(kp);
     T* q = reinterpret_cast<T*>(kq);
+    KrylovBox box = kbox;
+    if (singular && (sizeof(T) == 4 || near_rounding)) box.null_inv = 1.0 / (eb.on ? (double)eb.active_nodes : (double)kbox.n[0] * kbox.n[1] * kbox.n[2]);
     for (int c = 0; c < m; ++c) {
         vcycle<T>(0, r, true);
         const T* z = (const T*)xres[0];
-        krylov_beta<T>(kbox, z, q, kpart, kstate, s);
-        krylov_direction<T>(kbox, z, p, kstate, s);
+        krylov_beta<T>(box, z, q, kpart, kstate, s);
+        krylov_direction<T>(box, z, p, kstate, s);
         apply_neg<T>(p, q, s);
-        krylov_alpha<T>(kbox, p, q, r, kpart, kstate, s);
-        krylov_update<T>(kbox, p, q, x, r, kstate, s, c == m - 1 ? norm : nullptr);
+        krylov_alpha<T>(box, p, q, r, kpart, kstate, s);
+        krylov_update<T>(box, p, q, x, r, kstate, s, c == m - 1 ? norm : nullptr);
         nk += 5;
     }
 }
@@ -865,7 +867,8 @@ int NodalSolver::run_iteration(int m)
         drop_graphs();
         gexec_prec = opt.precision;
     }
-    cudaGraphExec_t& ge = gexec[m];
+    const int slot = near_rounding ? 0 : m;  // (the plain form has m = 1)
+    cudaGraphExec_t& ge = gexec[slot];
     if (!ge) {
         cudaGraph_t graph = nullptr;
         cap_or_st = cap;
@@ -885,10 +888,10 @@ int NodalSolver::run_iteration(int m)
             return cuda_fail(e, "cudaGraphInstantiate(refinement step)");
         }
         nk -= step_kernels;  // capture issued nothing; the launch below runs them
-        step_kernels_m[m] = step_kernels;
+        step_kernels_m[slot] = step_kernels;
     }
     GBP_CUDA(cudaGraphLaunch(ge, st));
-    nk += step_kernels_m[m];
+    nk += step_kernels_m[slot];
     return GBP_OK;
 }
 
@@ -982,6 +985,7 @@ int NodalSolver::solve(bool have_guess, gbp_stats* stats, bool from_prev)
             set_error("solve: maxiter reached before the tolerance");
             break;
         }
+        near_rounding = !mixed && singular && rn < kNearRounding * bnorm;
         int rc = run_iteration(m);
         if (rc) return rc;
         GBP_CUDA(cudaStreamSynchronize(st));
@@ -1400,6 +1404,7 @@ int NodalSolver::set_eb(const gbp_array4* M)
     eb.e.kap = dk;
     eb.e.reg = dr;
     eb.has_inactive = inactive;
+    eb.active_nodes = std::count(act_u.begin(), act_u.end(), 1);
     eb.on = true;
     set_omega();
     return rebuild_masks();

@@ -218,6 +218,7 @@ private:
     KrylovState* kstate = nullptr;
     KrylovState* hstate = nullptr;  // pinned: the state a solve starts from
     KrylovBox kbox{};
+    bool near_rounding = false;  // FP64 steps of a singular system whose residual is close to its rounding (krylov.h)
     double* partials = nullptr;  // reduction scratch
     double* bscr = nullptr;      // scratch of the single-CTA bottom CG (coarsest levels beyond the cluster's)
     BottomRows brows;            // the coarsest operator's rows
@@ -271,6 +272,7 @@ private:
         double* ivol = nullptr;            // 1 / fluid volume of each node's dual cell (level 0)
         double* inflow_buf = nullptr;      // 8 EB inflow shares per cut cell (e.inflow when set)
         bool has_inactive = false;
+        long long active_nodes = 0;        // unique nodes of level 0 that touch fluid
         bool on = false;
     } eb;
     bool sigma_ready = false;
