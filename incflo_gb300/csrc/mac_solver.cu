@@ -996,8 +996,22 @@ int MacSolver::solve(bool have_guess, gbp_stats* stats)
     constexpr double kStall = 0.75;
     int window = 0;
     double rwindow = rn, rate[2] = {0.0, 0.0};
+    // as NodalSolver's
+    auto true_residual = [&]() -> int {
+        GBP_CUDA(cudaMemsetAsync(dnorm + 1, 0, sizeof(unsigned long long), st));
+        resid64(phi, rhs0, res, dnorm + 1, st);
+        GBP_CUDA(cudaMemcpyAsync(hnorm + 1, dnorm + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+        GBP_CUDA(cudaStreamSynchronize(st));
+        rn = bits_to_double(hnorm[1]);
+        return GBP_OK;
+    };
     while (rn > target) {
         if (it >= opt.maxiter) {
+            if (!mixed && it > 0) {
+                const int rc = true_residual();
+                if (rc) return rc;
+                if (rn <= target) break;
+            }
             status = GBP_NOT_CONVERGED;
             set_error("solve: maxiter reached before the tolerance");
             break;
@@ -1010,14 +1024,7 @@ int MacSolver::solve(bool have_guess, gbp_stats* stats)
         rn = bits_to_double(hnorm[1]);
         ++it;
         vcycles += m;
-        if (!mixed && rn <= target) {
-            // the recursion's residual meets the tolerance: the true one decides, and the solve goes on from it
-            GBP_CUDA(cudaMemsetAsync(dnorm + 1, 0, sizeof(unsigned long long), st));
-            resid64(phi, rhs0, res, dnorm + 1, st);
-            GBP_CUDA(cudaMemcpyAsync(hnorm + 1, dnorm + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-            GBP_CUDA(cudaStreamSynchronize(st));
-            rn = bits_to_double(hnorm[1]);
-        }
+        if (!mixed && rn <= target && (rc = true_residual())) return rc;  // the solve goes on from the true one
         window += m;
         if (eb.on && window >= kWindow && rn > target) {
             const int now = hstate->plain;

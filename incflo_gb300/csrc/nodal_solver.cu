@@ -979,8 +979,23 @@ int NodalSolver::solve(bool have_guess, gbp_stats* stats, bool from_prev)
         GBP_CUDA(cudaEventCreate(&evi1));
     }
     GBP_CUDA(cudaEventRecord(evi0, st));
+    // the plain form's residual between two steps is the recursion's; the true one, which decides and is reported
+    auto true_residual = [&]() -> int {
+        GBP_CUDA(cudaMemsetAsync(dnorm + 1, 0, sizeof(unsigned long long), st));
+        resid0(phi, rhs0, res, dnorm + 1, st);
+        ++nk;
+        GBP_CUDA(cudaMemcpyAsync(hnorm + 1, dnorm + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+        GBP_CUDA(cudaStreamSynchronize(st));
+        rn = bits_to_double(hnorm[1]);
+        return GBP_OK;
+    };
     while (rn > target) {
         if (it >= opt.maxiter) {
+            if (!mixed && it > 0) {
+                const int rc = true_residual();
+                if (rc) return rc;
+                if (rn <= target) break;
+            }
             status = GBP_NOT_CONVERGED;
             set_error("solve: maxiter reached before the tolerance");
             break;
@@ -993,15 +1008,7 @@ int NodalSolver::solve(bool have_guess, gbp_stats* stats, bool from_prev)
         rn = bits_to_double(hnorm[1]);
         ++it;
         vcycles += m;
-        if (!mixed && rn <= target) {
-            // the recursion's residual meets the tolerance: the true one decides, and the solve goes on from it
-            GBP_CUDA(cudaMemsetAsync(dnorm + 1, 0, sizeof(unsigned long long), st));
-            resid0(phi, rhs0, res, dnorm + 1, st);
-            ++nk;
-            GBP_CUDA(cudaMemcpyAsync(hnorm + 1, dnorm + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-            GBP_CUDA(cudaStreamSynchronize(st));
-            rn = bits_to_double(hnorm[1]);
-        }
+        if (!mixed && rn <= target && (rc = true_residual())) return rc;  // the solve goes on from the true one
         if (mixed && rn > target && rn < rprev && rn > 0.0) {
             // next inner solve: as many V-cycles as the observed per-cycle contraction says the
             // remaining reduction needs (+1/4 cycle of margin), capped by ir_inner_cycles and by
