@@ -892,7 +892,18 @@ void MacSolver::record_iteration(int m)
     const MacLevel& l0 = L[0];
     const cudaStream_t s = cap_or_st;
     cudaMemsetAsync(dnorm + 1, 0, sizeof(unsigned long long), s);
-    if (opt.precision == GBP_PREC_MIXED) {
+    if (!accelerated()) {
+        // the coarsest level's solve alone: m = 1
+        if (opt.precision == GBP_PREC_MIXED) {
+            mac_to_f32(l0.g, res, l0.rhs32, 1.0, s, kstate);
+            vcycle<float>(0, l0.rhs32, true);
+            mac_add_correction<float>(l0.g, phi, l0.x32, 1.0, s, kstate);
+        } else {
+            vcycle<double>(0, res, true);
+            mac_add_correction<double>(l0.g, phi, l0.x64, 1.0, s);
+        }
+        resid64(phi, rhs0, res, dnorm + 1, s);
+    } else if (opt.precision == GBP_PREC_MIXED) {
         float* e = reinterpret_cast<float*>(kp) + l0.g.count;
         mac_to_f32(l0.g, res, l0.rhs32, 1.0, s, kstate);
         cudaMemsetAsync(e, 0, sizeof(float) * l0.g.count, s);
@@ -982,7 +993,9 @@ int MacSolver::solve(bool have_guess, gbp_stats* stats)
     int it = 0, status = GBP_OK, vcycles = 0;
     const double r0 = rn;
     const bool mixed = opt.precision == GBP_PREC_MIXED;
-    int m = mixed ? std::min(opt.ir_inner_cycles, 5) : 1;
+    const bool recursion = !mixed && accelerated();  // the residual between two steps is the recursion's
+    const int mmax = accelerated() ? opt.ir_inner_cycles : 1;
+    int m = mixed ? std::min(mmax, 5) : 1;
     memset(hstate, 0, sizeof(KrylovState));
     hstate->scale = scale32;
     hstate->inv_scale = 1.0 / scale32;
@@ -1007,7 +1020,7 @@ int MacSolver::solve(bool have_guess, gbp_stats* stats)
     };
     while (rn > target) {
         if (it >= opt.maxiter) {
-            if (!mixed && it > 0) {
+            if (recursion && it > 0) {
                 const int rc = true_residual();
                 if (rc) return rc;
                 if (rn <= target) break;
@@ -1016,7 +1029,7 @@ int MacSolver::solve(bool have_guess, gbp_stats* stats)
             set_error("solve: maxiter reached before the tolerance");
             break;
         }
-        near_rounding = !mixed && singular && rn < kNearRounding * bnorm;
+        near_rounding = recursion && singular && rn < kNearRounding * bnorm;
         int rc = run_iteration(m);
         if (rc) return rc;
         GBP_CUDA(cudaStreamSynchronize(st));
@@ -1024,9 +1037,9 @@ int MacSolver::solve(bool have_guess, gbp_stats* stats)
         rn = bits_to_double(hnorm[1]);
         ++it;
         vcycles += m;
-        if (!mixed && rn <= target && (rc = true_residual())) return rc;  // the solve goes on from the true one
+        if (recursion && rn <= target && (rc = true_residual())) return rc;  // the solve goes on from the true one
         window += m;
-        if (eb.on && window >= kWindow && rn > target) {
+        if (eb.on && accelerated() && window >= kWindow && rn > target) {
             const int now = hstate->plain;
             rate[now] = pow(rn / rwindow, 1.0 / window);
             if (rate[now] > kStall && rate[1 - now] < rate[now]) {
@@ -1042,7 +1055,7 @@ int MacSolver::solve(bool have_guess, gbp_stats* stats)
             // inner solve delivers (about 1e-6 of its right-hand side)
             const double rho = std::min(0.9, std::max(1e-3, pow(rn / rprev, 1.0 / m)));
             const double need = log(std::max(target / rn, 1e-6)) / log(rho);
-            m = std::max(1, std::min(opt.ir_inner_cycles, (int)ceil(need + 0.25)));
+            m = std::max(1, std::min(mmax, (int)ceil(need + 0.25)));
         }
         if (opt.verbose > 1) fprintf(stderr, "gbp mac: iter %d rel resid %.3e\n", it, bnorm > 0 ? rn / bnorm : rn);
         if (!isfinite(rn)) {

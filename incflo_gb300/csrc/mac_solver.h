@@ -83,6 +83,7 @@ private:
     // 1 / diag of every level for the FP64 half sweeps
     void ensure_idiag();
     bool idiag_ready = false;
+    bool accelerated() const { return L.size() > 1 || eb.on; }  // as NodalSolver::accelerated
     void record_iteration(int m);  // m V-cycles per refinement step
     int run_iteration(int m);
     int solve(bool have_guess, gbp_stats* stats);

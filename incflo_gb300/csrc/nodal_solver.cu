@@ -717,10 +717,13 @@ void NodalSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s, const KrylovNo
 // the vector kernels are 4 % of a V-cycle there). FP32 V-cycles: except on the levels of the whole-row sweeps, whose
 // V-cycle from the current iterate costs 0.78 ms at 256^3 where the accelerated one, from zero and with its five vector
 // passes, costs 1.12 ms (13.0 against 12.0 ms per projection with 8 against 10 V-cycles); cut cells (22 -> 12 V-cycles
-// on the cylinder channel) and stretched cells gain several times more than that.
+// on the cylinder channel) and stretched cells gain several times more than that. Never on a hierarchy of one level, whose
+// "V-cycle" is the coarsest level's solve: one of them per step, and nothing to accelerate (with the vector passes and the
+// inner solve's further V-cycles 2^3 cells took 310 to 560 us per projection, without 270 to 350).
 bool NodalSolver::accelerated() const
 {
-    return opt.precision != GBP_PREC_MIXED || eb.on || !(use_tma && vsweep32_supported(L[0].g));
+    if (eb.on) return true;  // (the coarsest level's rows do not carry the cut cells)
+    return L.size() > 1 && (opt.precision != GBP_PREC_MIXED || !(use_tma && vsweep32_supported(L[0].g)));
 }
 
 // One step of the solve, issued on cap_or_st. Plain form: one accelerated V-cycle on phi and res, and res' max norm.
@@ -764,6 +767,11 @@ void NodalSolver::record_iteration(int m)
             nodal_to_f32(l0.g, res, l0.b32, 1.0, s, kstate);
             ++nk;
         }
+        nk += 2;
+    } else if (!accelerated()) {
+        vcycle<double>(0, res, true);
+        nodal_add_correction<double>(l0.g, phi, (const double*)xres[0], 1.0, s);
+        resid0(phi, rhs0, res, dnorm + 1, s);
         nk += 2;
     } else {
         KrylovNorm nm{dnorm + 1, {}, {}, {}, l0.g.mask, l0.g.ivol};
@@ -963,7 +971,8 @@ int NodalSolver::solve(bool have_guess, gbp_stats* stats, bool from_prev)
     int status = GBP_OK;
     const double r0 = rn;
     const bool mixed = opt.precision == GBP_PREC_MIXED;
-    const int mmax = std::min(opt.ir_inner_cycles, kMaxInner);
+    const int mmax = L.size() > 1 || eb.on ? std::min(opt.ir_inner_cycles, kMaxInner) : 1;
+    const bool recursion = !mixed && accelerated();  // the residual between two steps is the recursion's
     // V-cycles of the first inner solve: accelerated, about what FP32 delivers (1e-6) at the contraction of a smooth
     // problem (0.03 to 0.04 per V-cycle)
     int m = mixed ? std::min(mmax, 4) : 1;
@@ -979,7 +988,7 @@ int NodalSolver::solve(bool have_guess, gbp_stats* stats, bool from_prev)
         GBP_CUDA(cudaEventCreate(&evi1));
     }
     GBP_CUDA(cudaEventRecord(evi0, st));
-    // the plain form's residual between two steps is the recursion's; the true one, which decides and is reported
+    // the true residual, which decides and is reported
     auto true_residual = [&]() -> int {
         GBP_CUDA(cudaMemsetAsync(dnorm + 1, 0, sizeof(unsigned long long), st));
         resid0(phi, rhs0, res, dnorm + 1, st);
@@ -991,7 +1000,7 @@ int NodalSolver::solve(bool have_guess, gbp_stats* stats, bool from_prev)
     };
     while (rn > target) {
         if (it >= opt.maxiter) {
-            if (!mixed && it > 0) {
+            if (recursion && it > 0) {
                 const int rc = true_residual();
                 if (rc) return rc;
                 if (rn <= target) break;
@@ -1000,7 +1009,7 @@ int NodalSolver::solve(bool have_guess, gbp_stats* stats, bool from_prev)
             set_error("solve: maxiter reached before the tolerance");
             break;
         }
-        near_rounding = !mixed && singular && rn < kNearRounding * bnorm;
+        near_rounding = recursion && singular && rn < kNearRounding * bnorm;
         int rc = run_iteration(m);
         if (rc) return rc;
         GBP_CUDA(cudaStreamSynchronize(st));
@@ -1008,7 +1017,7 @@ int NodalSolver::solve(bool have_guess, gbp_stats* stats, bool from_prev)
         rn = bits_to_double(hnorm[1]);
         ++it;
         vcycles += m;
-        if (!mixed && rn <= target && (rc = true_residual())) return rc;  // the solve goes on from the true one
+        if (recursion && rn <= target && (rc = true_residual())) return rc;  // the solve goes on from the true one
         if (mixed && rn > target && rn < rprev && rn > 0.0) {
             // next inner solve: as many V-cycles as the observed per-cycle contraction says the
             // remaining reduction needs (+1/4 cycle of margin), capped by ir_inner_cycles and by
