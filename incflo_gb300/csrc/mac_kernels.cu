@@ -98,8 +98,8 @@ __device__ __forceinline__ T mac_Ax(const CellGeom& g, const T* __restrict__ x, 
 // the corrected other one, and the second replaces the other.
 // FP32: HBM bound on large levels. FP64: the pipe (2 lanes per clock and SM) bounds it, so 1 / diag comes from an array
 // (id) and each direction's weight multiplies once: 10 instructions per cell against about 36 with the division and six
-// weighted coefficients.
-template <typename T, int FROM>
+// weighted coefficients. (ID false: no such array, as in FP32.)
+template <typename T, int FROM, bool ID>
 __global__ void __launch_bounds__(256) k_mac_rbgs(CellGeom g, const T* __restrict__ bx, const T* __restrict__ by,
                                                   const T* __restrict__ bz, const T* __restrict__ b,
                                                   const T* __restrict__ id, T* x, int color, CellGeom gc,
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(256) k_mac_rbgs(CellGeom g, const T* __restric
     if (i >= g.n[0]) return;
     const long long p = pidx(g.sy, g.sz, i, j, k);
     T v;
-    if (sizeof(T) == 8 && FROM == 1) {
+    if (ID && FROM == 1) {
         v = b[p] * id[p];
     } else {
         const T wx = (T)g.w[0], wy = (T)g.w[1], wz = (T)g.w[2];
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(256) k_mac_rbgs(CellGeom g, const T* __restric
             acc += wy * (b2 * xs + b3 * xn);
             acc += wz * (b4 * xb + b5 * xt);
         }
-        if (sizeof(T) == 8) {
+        if (ID) {
             v = acc * id[p];
         } else {
             T diag = wx * (b0 + b1) + wy * (b2 + b3) + wz * (b4 + b5);
@@ -684,21 +684,36 @@ void mac_rbgs(const CellGeom& g, const T* bx, const T* by, const T* bz, const T*
               cudaStream_t st)
 {
     const long long n = (long long)g.n[1] * g.n[2] * ((g.n[0] + 1) / 2);
-    k_mac_rbgs<T, 0><<<nblk(n, 256), 256, 0, st>>>(g, bx, by, bz, b, id, x, color, g, nullptr);
+    if constexpr (sizeof(T) == 8)
+        if (id) {
+            k_mac_rbgs<T, 0, true><<<nblk(n, 256), 256, 0, st>>>(g, bx, by, bz, b, id, x, color, g, nullptr);
+            return;
+        }
+    k_mac_rbgs<T, 0, false><<<nblk(n, 256), 256, 0, st>>>(g, bx, by, bz, b, id, x, color, g, nullptr);
 }
 template <typename T>
 void mac_rbgs_zero(const CellGeom& g, const T* bx, const T* by, const T* bz, const T* b, const T* id, T* x, int color,
                    cudaStream_t st)
 {
     const long long n = (long long)g.n[1] * g.n[2] * ((g.n[0] + 1) / 2);
-    k_mac_rbgs<T, 1><<<nblk(n, 256), 256, 0, st>>>(g, bx, by, bz, b, id, x, color, g, nullptr);
+    if constexpr (sizeof(T) == 8)
+        if (id) {
+            k_mac_rbgs<T, 1, true><<<nblk(n, 256), 256, 0, st>>>(g, bx, by, bz, b, id, x, color, g, nullptr);
+            return;
+        }
+    k_mac_rbgs<T, 1, false><<<nblk(n, 256), 256, 0, st>>>(g, bx, by, bz, b, id, x, color, g, nullptr);
 }
 template <typename T>
 void mac_rbgs_prolong(const CellGeom& g, const CellGeom& gc, const T* bx, const T* by, const T* bz, const T* b,
                       const T* id, const T* xc, T* x, int color, cudaStream_t st)
 {
     const long long n = (long long)g.n[1] * g.n[2] * ((g.n[0] + 1) / 2);
-    k_mac_rbgs<T, 2><<<nblk(n, 256), 256, 0, st>>>(g, bx, by, bz, b, id, x, color, gc, xc);
+    if constexpr (sizeof(T) == 8)
+        if (id) {
+            k_mac_rbgs<T, 2, true><<<nblk(n, 256), 256, 0, st>>>(g, bx, by, bz, b, id, x, color, gc, xc);
+            return;
+        }
+    k_mac_rbgs<T, 2, false><<<nblk(n, 256), 256, 0, st>>>(g, bx, by, bz, b, id, x, color, gc, xc);
 }
 void mac_idiag(const CellGeom& g, const double* bx, const double* by, const double* bz, double* id, cudaStream_t st)
 {

@@ -9,7 +9,7 @@ namespace gbp {
 
 struct KrylovState;
 
-// one red-black half sweep (colour 0 red, 1 black); id: 1 / diag (FP64 only); mac_rbgs_zero: from x = 0;
+// one red-black half sweep (colour 0 red, 1 black); id: 1 / diag (FP64 only; null: formed in the sweep); mac_rbgs_zero: from x = 0;
 // mac_rbgs_prolong: from x + the prolonged coarse correction xc on the other colour
 template <typename T>
 void mac_rbgs(const CellGeom& g, const T* bx, const T* by, const T* bz, const T* b, const T* id, T* x, int color,

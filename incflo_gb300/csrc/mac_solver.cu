@@ -53,6 +53,9 @@ void MacSolver::destroy()
     if (ev2) cudaEventDestroy(ev2);
     ev0 = ev1 = ev2 = nullptr;
     pool.release();
+    plain_pool.release();
+    kp = kq = kp_plain = nullptr;
+    form = -1;
     apool.release();
     dmat = nullptr;
     dact = nullptr;
@@ -79,7 +82,34 @@ int MacSolver::set_options(const gbp_options& o)
     opt = o;
     opt.max_coarsening_level = maxc;
     if (regraph) drop_graphs();
+    if (pool.base && form != opt.precision) choose_form();
     return GBP_OK;
+}
+
+// as NodalSolver::choose_form
+void MacSolver::choose_form()
+{
+    form = opt.precision;
+    const MacLevel& l0 = L[0];
+    kq = l0.rhs64;
+    if (form == GBP_PREC_MIXED) {
+        kp = l0.x64;
+        return;
+    }
+    cudaMemsetAsync(l0.x64, 0, sizeof(double) * l0.g.count, st);
+    cudaMemsetAsync(l0.rhs64, 0, sizeof(double) * l0.g.count, st);
+    if (!plain_pool.base) {
+        size_t need = 4096 + sizeof(double) * l0.g.count;
+        for (const auto& lv : L) need += sizeof(double) * lv.g.count + 256;
+        kp_plain = nullptr;
+        if (plain_pool.reserve(need) == GBP_OK && cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess) {
+            kp_plain = plain_pool.take<double>(l0.g.count);
+            for (auto& lv : L) lv.id64 = plain_pool.take<double>(lv.g.count);
+        }
+        cudaGetLastError();
+        idiag_ready = false;
+    }
+    kp = kp_plain;
 }
 
 int MacSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc_hi[3], const gbp_options& o,
@@ -154,11 +184,11 @@ int MacSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc_h
     size_t need = 0;
     auto add = [&](size_t cnt, size_t sz) { need = ((need + 255) & ~size_t(255)) + cnt * sz; };
     for (auto& lv : L) {
-        for (int q = 0; q < 7; ++q) add(lv.g.count, 8);
+        for (int q = 0; q < 6; ++q) add(lv.g.count, 8);
         for (int q = 0; q < 6; ++q) add(lv.g.count, 4);
     }
     const CellGeom& G0 = L[0].g;
-    for (int q = 0; q < 5; ++q) add(G0.count, 8);
+    for (int q = 0; q < 3; ++q) add(G0.count, 8);
     add(kKrylovSums * kKrylovBlocks, 8);
     add(1, sizeof(KrylovState));
     add(mac_partials_needed(G0) + 64, 8);
@@ -192,7 +222,6 @@ int MacSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc_h
         lv.x64 = pool.take<double>(lv.g.count);
         lv.rhs64 = pool.take<double>(lv.g.count);
         lv.r64 = pool.take<double>(lv.g.count);
-        lv.id64 = pool.take<double>(lv.g.count);
         for (int d = 0; d < 3; ++d) lv.b32[d] = pool.take<float>(lv.g.count);
         lv.x32 = pool.take<float>(lv.g.count);
         lv.rhs32 = pool.take<float>(lv.g.count);
@@ -201,8 +230,6 @@ int MacSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc_h
     phi = pool.take<double>(G0.count);
     rhs0 = pool.take<double>(G0.count);
     res = pool.take<double>(G0.count);
-    kp = pool.take<double>(G0.count);
-    kq = pool.take<double>(G0.count);
     kpart = pool.take<double>(kKrylovSums * kKrylovBlocks);
     kstate = pool.take<KrylovState>(1);
     kbox = KrylovBox{{G0.n[0], G0.n[1], G0.n[2]}, G0.sy, G0.sz, G0.count, 0.0};
@@ -235,6 +262,7 @@ int MacSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc_h
     GBP_CUDA(cudaEventCreate(&ev0));
     GBP_CUDA(cudaEventCreate(&ev1));
     GBP_CUDA(cudaEventCreate(&ev2));
+    choose_form();
     return GBP_OK;
 }
 
@@ -844,7 +872,7 @@ void MacSolver::vcycle(int l, const T* b, bool zero)
 
 void MacSolver::ensure_idiag()
 {
-    if (idiag_ready || opt.precision == GBP_PREC_MIXED) return;
+    if (idiag_ready || opt.precision == GBP_PREC_MIXED || !L[0].id64) return;
     for (auto& lv : L) mac_idiag(lv.g, lv.b64[0], lv.b64[1], lv.b64[2], lv.id64, st);
     idiag_ready = true;
 }

@@ -71,7 +71,7 @@ public:
     // correction32() until the next V-cycle of this solver
     void vcycles32(const float* b32, cudaStream_t s);
     const float* correction32() const { return L[0].x32; }
-    size_t device_bytes() const { return pool.bytes; }
+    size_t device_bytes() const { return pool.bytes + plain_pool.bytes; }
 
 private:
     template <typename T>
@@ -83,7 +83,8 @@ private:
     // 1 / diag of every level for the FP64 half sweeps
     void ensure_idiag();
     bool idiag_ready = false;
-    bool accelerated() const { return L.size() > 1 || eb.on; }  // as NodalSolver::accelerated
+    // as NodalSolver::accelerated
+    bool accelerated() const { return (L.size() > 1 || eb.on) && (opt.precision == GBP_PREC_MIXED || kp); }
     void record_iteration(int m);  // m V-cycles per refinement step
     int run_iteration(int m);
     int solve(bool have_guess, gbp_stats* stats);
@@ -103,8 +104,13 @@ private:
     cudaGraphExec_t gexec[kMaxGraphs + 1] = {};
     int gexec_prec = -1;
     void drop_graphs();
-    // conjugate-gradient vectors (as NodalSolver's)
+    // conjugate-gradient vectors, and what only the plain form needs (as NodalSolver's: p and 1 / diag; q lies in rhs64, or in the
+    // mixed form p and the inner solution in x64)
     double *kp = nullptr, *kq = nullptr, *kpart = nullptr;
+    DevicePool plain_pool;
+    double* kp_plain = nullptr;
+    int form = -1;
+    void choose_form();
     KrylovState *kstate = nullptr, *hstate = nullptr;
     KrylovBox kbox{};
     bool near_rounding = false;  // FP64 steps of a singular system whose residual is close to its rounding (krylov.h)

@@ -62,7 +62,8 @@ static void q1_element(const double h[3], double K[8])
     }
 }
 
-static NodalGeom make_geom(const int n[3], const double h[3], const int per[3], const int dlo[3], const int dhi[3])
+static NodalGeom make_geom(const int n[3], const double h[3], const int per[3], const int dlo[3], const int dhi[3],
+                           bool wide_rows)
 {
     NodalGeom g;
     memset(&g, 0, sizeof(g));
@@ -78,7 +79,7 @@ static NodalGeom make_geom(const int n[3], const double h[3], const int per[3], 
     // large levels with x walls: room for the last thread's columns of the whole-row sweeps, which read 4 nodes per thread
     // (without it every n0 = 8 m with walls in x fell back to a node per thread: 16.6 against 15.2 us per sweep on 145 x 81
     // x 113 nodes, and to accelerated V-cycles with their vector passes, 3.7 against 2.9 ms per solve)
-    if (!per[0] && (long long)g.nu[0] * g.nu[1] * g.nu[2] >= (1ll << 20))
+    if (wide_rows && !per[0] && (long long)g.nu[0] * g.nu[1] * g.nu[2] >= (1ll << 20))
         P0 = std::max<long long>(P0, round_up(4 * ((g.nu[0] + 3) / 4) + 5, 8));
     g.sy = P0;
     g.sz = P0 * (long long)(n[1] + 3);
@@ -135,6 +136,9 @@ void NodalSolver::destroy()
     umask8 = nullptr;
     user_zeros = 0;
     pool.release();
+    plain_pool.release();
+    kp = kq = kp_plain = nullptr;
+    form = -1;
     L.clear();
     sigma_ready = false;
 }
@@ -157,7 +161,43 @@ int NodalSolver::set_options(const gbp_options& o)
     if (regraph) {
         drop_graphs();
     }
+    if (pool.base && form != opt.precision) choose_form();
     return GBP_OK;
+}
+
+// The arrays of the form that opt.precision names (nodal_solver.h). Level 0's x64 and b64 hold other things in the mixed form:
+// cleared for the FP64 V-cycles, which rely on zeros beyond the walls.
+void NodalSolver::choose_form()
+{
+    form = opt.precision;
+    const NodalLevel& l0 = L[0];
+    kq = l0.b64;
+    if (form == GBP_PREC_MIXED) {
+        kp = l0.x64;
+        return;
+    }
+    cudaMemsetAsync(l0.x64, 0, sizeof(double) * l0.g.count, st);
+    cudaMemsetAsync(l0.b64, 0, sizeof(double) * l0.g.count, st);
+    if (!plain_pool.base) {
+        size_t need = 4096;
+        auto add = [&](const NodalLevel& lv, int arrays) { need += arrays * (sizeof(double) * lv.g.count + 256); };
+        add(l0, 1);
+        for (const auto& lv : L)
+            if (qsweep_supported(lv.g)) add(lv, &lv == &l0 ? 1 : 5);
+        kp_plain = nullptr;
+        if (plain_pool.reserve(need) == GBP_OK && cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess) {
+            kp_plain = plain_pool.take<double>(l0.g.count);
+            for (auto& lv : L) {
+                if (!qsweep_supported(lv.g)) continue;
+                lv.qw.rd = plain_pool.take<double>(lv.g.count);
+                if (&lv == &l0) continue;
+                for (double** w : {&lv.qw.w5, &lv.qw.wx, &lv.qw.wy, &lv.qw.wz}) *w = plain_pool.take<double>(lv.g.count);
+            }
+        }
+        cudaGetLastError();
+        for (auto& lv : L) lv.qw_ready = 0;
+    }
+    kp = kp_plain;
 }
 
 // The smoother's weights. The Jacobi-scaled operator has lambda_max(D^-1 A) <= lb = 1 + sum_{q != 0} |K_q| /
@@ -207,7 +247,7 @@ void NodalSolver::set_omega()
 }
 
 int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc_hi[3], const gbp_options& o,
-                      cudaStream_t stream)
+                      cudaStream_t stream, bool wide_rows)
 {
     destroy();
     opt = o;
@@ -251,7 +291,7 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
     double ch[3] = {h[0], h[1], h[2]};
     for (;;) {
         NodalLevel lv;
-        lv.g = make_geom(cn, ch, per, dlo, dhi);
+        lv.g = make_geom(cn, ch, per, dlo, dhi, wide_rows);
         L.push_back(lv);
         bool ok = (int)L.size() <= opt.max_coarsening_level && (int)L.size() < kMaxLevels;
         for (int d = 0; d < 3; ++d) ok = ok && (cn[d] % 2 == 0) && (cn[d] / 2 >= 2);
@@ -277,12 +317,11 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
         add(lv.g.count, 1);
     }
     const NodalGeom& G0 = L[0].g;
-    for (int q = 0; q < 5; ++q) add(G0.count, 8);
+    for (int q = 0; q < 3; ++q) add(G0.count, 8);
     add(kKrylovSums * kKrylovBlocks, 8);
     add(1, sizeof(KrylovState));
-    for (auto& lv : L)
-        if (qsweep_supported(lv.g))
-            for (int q = 0; q < 5; ++q) add(lv.g.count, 8);
+    if (qsweep_supported(G0))
+        for (int q = 0; q < 4; ++q) add(G0.count, 8);
     add(nodal_partials_needed(G0) + 64, 8);
     nbottom = B.g.nu[0] * B.g.nu[1] * B.g.nu[2];
     dense_bottom = nbottom <= kDenseBottom;
@@ -303,6 +342,10 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
     if (dense_bottom) add((size_t)nbottom * nbottom, 8);
     need += 4096;
     rc = pool.reserve(need);
+    if (rc && wide_rows) {
+        cudaGetLastError();
+        return init(geom, bc_lo, bc_hi, o, stream, false);  // up to 6 % less at 128 nodes per row
+    }
     if (rc) return rc;
     for (auto& lv : L) {
         lv.s64 = pool.take<double>(lv.g.count);
@@ -322,14 +365,11 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
     phi = pool.take<double>(G0.count);
     rhs0 = pool.take<double>(G0.count);
     res = pool.take<double>(G0.count);
-    kp = pool.take<double>(G0.count);
-    kq = pool.take<double>(G0.count);
     kpart = pool.take<double>(kKrylovSums * kKrylovBlocks);
     kstate = pool.take<KrylovState>(1);
     kbox = KrylovBox{{G0.nu[0], G0.nu[1], G0.nu[2]}, G0.sy, G0.sz, G0.count, 0.0};
-    for (auto& lv : L)
-        if (qsweep_supported(lv.g))
-            for (double** w : {&lv.qw.w5, &lv.qw.rd, &lv.qw.wx, &lv.qw.wy, &lv.qw.wz}) *w = pool.take<double>(lv.g.count);
+    if (qsweep_supported(G0))
+        for (double** w : {&L[0].qw.w5, &L[0].qw.wx, &L[0].qw.wy, &L[0].qw.wz}) *w = pool.take<double>(G0.count);
     partials = pool.take<double>(nodal_partials_needed(G0) + 64);
     bscr = nullptr;
     if (brows.n)
@@ -353,6 +393,7 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
     GBP_CUDA(cudaEventCreate(&ev0));
     GBP_CUDA(cudaEventCreate(&ev1));
     GBP_CUDA(cudaEventCreate(&ev2));
+    choose_form();
     return GBP_OK;
 }
 
@@ -394,8 +435,8 @@ void NodalSolver::ensure_qweights()
 {
     // the mixed form takes FP64 residuals of level 0 only, the plain form sweeps every level
     const bool mixed = opt.precision == GBP_PREC_MIXED;
-    const int need = mixed ? 1 : 2;
-    for (size_t l = 0; l < (mixed ? 1 : L.size()); ++l)
+    for (size_t l = 0; l < (mixed ? 1 : L.size()); ++l) {
+        const int need = mixed || !L[l].qw.rd ? 1 : 2;
         if (L[l].qw.w5 && L[l].qw_ready < need) {
             QWeights w = L[l].qw;
             if (mixed) w.rd = nullptr;
@@ -403,6 +444,7 @@ void NodalSolver::ensure_qweights()
             L[l].qw_ready = need;
             ++nk;
         }
+    }
 }
 
 int NodalSolver::level_of(const NodalGeom& g) const
@@ -722,6 +764,7 @@ void NodalSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s, const KrylovNo
 // inner solve's further V-cycles 2^3 cells took 310 to 560 us per projection, without 270 to 350).
 bool NodalSolver::accelerated() const
 {
+    if (opt.precision != GBP_PREC_MIXED && !kp) return false;  // no memory for it
     if (eb.on) return true;  // (the coarsest level's rows do not carry the cut cells)
     return L.size() > 1 && (opt.precision != GBP_PREC_MIXED || !(use_tma && vsweep32_supported(L[0].g)));
 }

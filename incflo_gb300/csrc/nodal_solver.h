@@ -81,8 +81,10 @@ class NodalSolver {
 public:
     static constexpr int kMaxInner = 8;  // FP32 V-cycles per refinement step, at most
 
+    // wide_rows: rows of large levels with x walls as long as the whole-row sweeps want them; shorter where the memory for that
+    // is not there
     int init(const gbp_geometry& geom, const int bc_lo[3], const int bc_hi[3], const gbp_options& opt,
-             cudaStream_t stream);
+             cudaStream_t stream, bool wide_rows = true);
     void destroy();
     ~NodalSolver() { destroy(); }
 
@@ -112,7 +114,7 @@ public:
 
     const NodalGeom& geom0() const { return L[0].g; }
     bool has_eb() const { return eb.on; }
-    size_t device_bytes() const { return pool.bytes; }
+    size_t device_bytes() const { return pool.bytes + plain_pool.bytes; }
     cudaStream_t stream() const { return st; }
     // solve A phi = g on the level-0 arrays already in place (used by project and tests)
     // from_prev: phi holds the plan's last solution (initial_guess = previous), a start the warm start
@@ -212,8 +214,15 @@ private:
     size_t net_prev_count = 0;
     double* rhs0 = nullptr;      // level-0 right-hand side (FP64, weak form)
     double* res = nullptr;       // level-0 outer residual (FP64)
-    // conjugate-gradient vectors: two FP64 arrays of level 0, or in the mixed form p, the inner solution, q and zeros
+    // Conjugate-gradient vectors. Mixed form: p and the inner solution, q and zeros, in two FP64 arrays of level 0 that only
+    // FP64 V-cycles use otherwise (x64, b64). Plain form: p and q, q in b64, which level 0's V-cycle does not touch.
     double *kp = nullptr, *kq = nullptr;
+    // What only the plain form needs, reserved when it is chosen: p and the weights of its FP64 sweeps. Without the memory for
+    // it its solves are stationary V-cycles with the level kernels that need none.
+    DevicePool plain_pool;
+    double* kp_plain = nullptr;
+    int form = -1;  // the precision that kp and kq are set for
+    void choose_form();
     double* kpart = nullptr;     // partial sums of its dot products
     KrylovState* kstate = nullptr;
     KrylovState* hstate = nullptr;  // pinned: the state a solve starts from
