@@ -13,7 +13,8 @@
 // feeds the output voxels vi - 1 to vi + 1, so its B operand is the stack of the three dx taps' weights at the rows of
 // those voxels, with rows of zeros above and below; moving the start in one stack padded by zeros serves every vi. The
 // group's last (first) voxel also feeds the first (last) output voxel of the next (previous) row: the box shifted by a
-// row. (A value that is not finite so reaches the other voxels of the groups next to it as well.) Two FP32 accumulators
+// row. A value that is not finite meets those zeros too and spoils the sums of the other voxels of its group and of the groups
+// next to it: the epilogue forms sums that are not finite once more, tap by tap (conv_at). Two FP32 accumulators
 // (or four) in tensor memory: the epilogue of a tile overlaps the MMAs of the next. Two producer and issuer pairs take
 // turns at the tiles where two rings of stages fit, since one warp's issue rate bounds a tile (116 us with one, 81 with two).
 // The other warps read the accumulator with tcgen05.ld (one group per thread, 16 columns at a time), apply bias + GELU
@@ -74,6 +75,8 @@ struct ConvParams {
     __nv_bfloat16* aux[2];
     int seg_c0[2], seg_nc[2];
     const float* bias;
+    const __nv_bfloat16 *in[2], *w;  // as the caller gave them (conv_at)
+    int cin_tot;
     unsigned* err;
     int ns, wres, npair, nbsh;  // stages of a pair, pairs (1 or 2), log2 of the accumulators (2 or 4)
     // weights of one (input, channel chunk, (dz, dy)): (G - 1) N rows of zeros, the taps' rows; zeros again at the end.
@@ -136,6 +139,27 @@ __device__ __forceinline__ void mma_voxels(uint32_t leader, uint32_t d, uint64_t
         ad += (int32_t)vstep;
         wd += (int32_t)wstep;
     }
+}
+
+// The sum of output channel n at row p, from the arrays themselves
+__device__ __noinline__ float conv_at(const ConvParams& P, long long p, int n)
+{
+    const int r = P.ntaps > 1 ? 1 : 0, sign = P.flip ? -1 : 1;
+    float sum = 0.f;
+    int t = 0;
+    for (int dz = -r; dz <= r; ++dz)
+        for (int dy = -r; dy <= r; ++dy)
+            for (int dx = -r; dx <= r; ++dx, ++t) {
+                const long long q = p + sign * (dz * P.PXY + dy * P.PX + dx);
+                if (q < 0 || q >= P.R) continue;
+                for (int i = 0; i < P.nin; ++i) {
+                    const __nv_bfloat16* a = P.in[i] + q * P.cin[i];
+                    const __nv_bfloat16* w = P.w + ((long long)t * P.N + n) * P.cin_tot + P.wc0[i];
+                    for (int c = 0; c < P.cin[i]; ++c) sum = fmaf(__bfloat162float(a[c]), __bfloat162float(w[c]), sum);
+                    if (sum != sum) return sum;  // NaN stays NaN
+                }
+            }
+    return sum;
 }
 
 template <int G>
@@ -364,6 +388,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
             for (int ch = set; ch < nchunk; ch += kEpiSets) {
                 const int vo = ch / cpv, col = 16 * (ch - vo * cpv);
                 float v[16];
+                if (G > 1) __syncwarp();  // (lanes may come from conv_at)
                 tc::tmem_ld16(taddr + (uint32_t)(16 * ch), v);
                 if (!valid) continue;
                 int x = x0 + vo, y = y0, z = z0;
@@ -386,6 +411,19 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
                     store16(orow, v);
                     if (arow && (P.flags & kGelu)) store16(arow, v);
                     continue;
+                }
+                if (G > 1) {
+                    float s = 0.f;
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) s = fmaf(v[e], 0.f, s);
+                    if (s != 0.f) {  // NaN: one of them is not finite
+#pragma unroll 1
+                        for (int e = 0; e < 16; ++e) {
+                            const float x = conv_at(P, pg + vo, col + e);
+#pragma unroll
+                            for (int f = 0; f < 16; ++f) v[f] = f == e ? x : v[f];
+                        }
+                    }
                 }
                 if (P.bias) {
 #pragma unroll
@@ -789,6 +827,7 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
             set_error("conv3d: input channels must be 16, 32 or a multiple of 64, data 16-byte aligned");
             return GBP_BAD_ARG;
         }
+        P.in[i] = L.in[i];
         P.cin[i] = L.cin[i];
         P.cb[i] = chunk_of(L.cin[i]);
         P.wc0[i] = cin_tot;
@@ -813,6 +852,8 @@ int conv3d(const ConvLaunch& L, cudaStream_t st)
         return GBP_BAD_ARG;
     }
     P.nin = L.nin;
+    P.w = L.w;
+    P.cin_tot = cin_tot;
     P.ntaps = L.ntaps;
     P.N = L.N;
     P.flip = L.flip;
