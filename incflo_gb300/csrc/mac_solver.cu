@@ -802,11 +802,13 @@ void MacSolver::vcycle(int l, const T* b, bool zero)
             c.tab_off = tail.t.tab_off;
             c.dense_off = tail.t.dense_off;
             int rc = mac_tail<T>(c, tail.t.bytes, s);
+            ++nk;
             if (rc && !launch_rc) launch_rc = rc;
             return;
         }
     }
     if (l == (int)L.size() - 1) {
+        ++nk;
         if (dense_bottom) {
             mac_bottom_dense<T>(lv.g, dmat, dact, b, x, singular ? 1 : 0, s);
         } else if (brows.n) {
@@ -830,6 +832,7 @@ void MacSolver::vcycle(int l, const T* b, bool zero)
             mac_rbgs<T>(lv.g, be[0], be[1], be[2], b, id, x, 1, s);
         }
         mac_resid_restrict<T>(lv.g, cv.g, be[0], be[1], be[2], x, b, B::rhs(cv), s);
+        nk += 2 * (opt.nu1 + opt.nu2) + 1;
         vcycle<T>(l + 1, B::rhs(cv), true);
         for (int q = 0; q < opt.nu2; ++q) {
             if (q == 0)
@@ -852,7 +855,9 @@ void MacSolver::vcycle(int l, const T* b, bool zero)
     }
     auto lag = [&]() {
         if (cut) eb_cells<T>(lv.g, eb.cells, eb.ncells, eb.faces, B::cb(eb), x, b, B::beff(eb), s);
+        nk += cut && eb.ncells > 0;
     };
+    nk += 2 * (opt.nu1 + opt.nu2) + 3 + (cut && eb.ncells > 0);
     for (int q = 0; q < opt.nu1; ++q) {
         if (!(zero && q == 0)) lag();  // (x = 0: nothing to lag)
         mac_rbgs<T>(lv.g, be[0], be[1], be[2], bs, id, x, 0, s);
@@ -874,16 +879,19 @@ void MacSolver::ensure_idiag()
 {
     if (idiag_ready || opt.precision == GBP_PREC_MIXED || !L[0].id64) return;
     for (auto& lv : L) mac_idiag(lv.g, lv.b64[0], lv.b64[1], lv.b64[2], lv.id64, st);
+    nk += (long long)L.size();
     idiag_ready = true;
 }
 
 void MacSolver::resid64(const double* x, const double* b, double* r, unsigned long long* norm, cudaStream_t s)
 {
     const MacLevel& l0 = L[0];
+    ++nk;
     if (!eb.on) {
         mac_resid<double>(l0.g, l0.b64[0], l0.b64[1], l0.b64[2], x, b, r, norm, s);
         return;
     }
+    nk += 1 + (eb.ncells > 0);
     mac_resid<double>(l0.g, l0.b64[0], l0.b64[1], l0.b64[2], x, b, r, nullptr, s);
     eb_cells<double>(l0.g, eb.cells, eb.ncells, eb.faces, eb.cb64, x, r, r, s);
     mac_norm(l0.g, r, norm, s, eb.m.kap);
@@ -907,6 +915,7 @@ void MacSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s, const KrylovNorm
         krylov_direction<T>(box, z, p, kstate, s);
         mac_resid<T>(l0.g, be[0], be[1], be[2], p, nullptr, q, nullptr, s);
         if (eb.on) eb_cells<T>(l0.g, eb.cells, eb.ncells, eb.faces, B::cb(eb), p, q, q, s);
+        nk += 5 + (eb.on && eb.ncells > 0);
         krylov_alpha<T>(box, p, q, r, kpart, kstate, s);
         krylov_update<T>(box, p, q, x, r, kstate, s, c == m - 1 ? norm : nullptr);
     }
@@ -919,6 +928,7 @@ void MacSolver::record_iteration(int m)
 {
     const MacLevel& l0 = L[0];
     const cudaStream_t s = cap_or_st;
+    const long long nk0 = nk;
     cudaMemsetAsync(dnorm + 1, 0, sizeof(unsigned long long), s);
     if (!accelerated()) {
         // the coarsest level's solve alone: m = 1
@@ -926,9 +936,11 @@ void MacSolver::record_iteration(int m)
             mac_to_f32(l0.g, res, l0.rhs32, 1.0, s, kstate);
             vcycle<float>(0, l0.rhs32, true);
             mac_add_correction<float>(l0.g, phi, l0.x32, 1.0, s, kstate);
+            nk += 2;
         } else {
             vcycle<double>(0, res, true);
             mac_add_correction<double>(l0.g, phi, l0.x64, 1.0, s);
+            ++nk;
         }
         resid64(phi, rhs0, res, dnorm + 1, s);
     } else if (opt.precision == GBP_PREC_MIXED) {
@@ -937,13 +949,16 @@ void MacSolver::record_iteration(int m)
         cudaMemsetAsync(e, 0, sizeof(float) * l0.g.count, s);
         krylov_steps<float>(m, e, l0.rhs32, s);
         mac_add_correction<float>(l0.g, phi, e, 1.0, s, kstate);
+        nk += 2;
         resid64(phi, rhs0, res, dnorm + 1, s);
     } else {
         const KrylovNorm nm{dnorm + 1, {}, {}, {}, nullptr, 1.0 / l0.g.vol};
         krylov_steps<double>(1, phi, res, s, eb.on ? nullptr : &nm);
         if (eb.on) mac_norm(l0.g, res, dnorm + 1, s, eb.m.kap);
+        nk += eb.on;
     }
     cudaMemcpyAsync(hnorm + 1, dnorm + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
+    step_kernels = nk - nk0;
 }
 
 int MacSolver::run_iteration(int m)
@@ -980,8 +995,11 @@ int MacSolver::run_iteration(int m)
             ge = nullptr;
             return cuda_fail(e, "cudaGraphInstantiate(mac refinement step)");
         }
+        nk -= step_kernels;  // capture issued nothing; the launch below runs them
+        step_kernels_m[slot] = step_kernels;
     }
     GBP_CUDA(cudaGraphLaunch(ge, st));
+    nk += step_kernels_m[slot];
     return GBP_OK;
 }
 
@@ -1002,6 +1020,7 @@ int MacSolver::solve(bool have_guess, gbp_stats* stats)
     GBP_CUDA(cudaMemsetAsync(dnorm, 0, 4 * sizeof(unsigned long long), st));
     mac_norm(l0.g, rhs0, dnorm, st, eb.on ? eb.m.kap : nullptr);
     resid64(phi, rhs0, res, dnorm + 1, st);
+    ++nk;
     GBP_CUDA(cudaMemcpyAsync(hnorm, dnorm, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
     GBP_CUDA(cudaStreamSynchronize(st));
     const double bnorm = bits_to_double(hnorm[0]);
@@ -1096,6 +1115,7 @@ int MacSolver::solve(bool have_guess, gbp_stats* stats)
         mac_remove_mean(l0.g, phi, partials, 1, st, eb.on ? eb.m.kap : nullptr, eb.kap_sum);
     else if (eb.on)
         eb_zero_covered(l0.g, eb.m.kap, phi, st);
+    nk += singular ? 3 : eb.on;
     GBP_CUDA(cudaEventRecord(ev2, st));
     GBP_CUDA(cudaGetLastError());
     if (stats) {
@@ -1144,12 +1164,14 @@ int MacSolver::project(gbp_array4* u[3], gbp_array4* phi_io, int phi_guess, gbp_
                              : "mac project: beta was never set on this plan");
         return GBP_BAD_ARG;
     }
+    nk = 0;
     const MacLevel& l0 = L[0];
     GBP_CUDA(cudaEventRecord(ev0, st));
     mac_rhs(l0.g, *u[0], *u[1], *u[2], rhs0, st, eb.on ? &eb.m : nullptr);
     if (singular) mac_remove_mean(l0.g, rhs0, partials, 0, st, eb.on ? eb.m.kap : nullptr, eb.kap_sum);
     const bool guess = phi_guess && phi_io && phi_io->data;
     if (guess) mac_load_phi(l0.g, *phi_io, phi, st);
+    nk += 1 + (singular ? 3 : 0) + guess;
     GBP_CUDA(cudaGetLastError());
     int status = solve(guess, stats);
     if (status != GBP_OK && status != GBP_NOT_CONVERGED) return status;
@@ -1160,6 +1182,7 @@ int MacSolver::project(gbp_array4* u[3], gbp_array4* phi_io, int phi_guess, gbp_
         eb_correct_u(l0.g, eb.faces, eb.nfaces, b, a, phi, u, st);
     }
     if (phi_io && phi_io->data) mac_store_phi(l0.g, *phi_io, phi, st);
+    nk += 3 + (eb.on && eb.nfaces > 0) + (phi_io && phi_io->data);
     GBP_CUDA(cudaEventRecord(ev2, st));
     GBP_CUDA(cudaGetLastError());
     if (stats) {
@@ -1167,17 +1190,7 @@ int MacSolver::project(gbp_array4* u[3], gbp_array4* phi_io, int phi_guess, gbp_
         float ms = 0.f;
         cudaEventElapsedTime(&ms, ev0, ev2);
         stats->ms_total = ms;
-        // kernels per V-cycle: 2 sweeps (red, black) per smoothing step, residual, restriction and
-        // prolongation on every level above the bottom, one bottom solve
-        const int cut = eb.on ? 1 : 0;
-        // with cut cells the finest level adds one cut-cell pass per smoothing step and one for its residual
-        const long long per_v =
-            (long long)(L.size() - 1) * (2LL * (opt.nu1 + opt.nu2) + 3) + 1 + cut * (opt.nu1 + opt.nu2 + 1);
-        const int mixed = opt.precision == GBP_PREC_MIXED;
-        const long long per_step = (mixed ? opt.ir_inner_cycles : 1) * per_v + 2 + mixed + 2 * cut;
-        const int steps = stats->outer_iters - 1;
-        stats->kernel_launches = 1 + (singular ? 4 : 0) + (guess ? 1 : 0) + 2 + 2 * cut + steps * per_step + 3 +
-                                 2 * cut + ((phi_io && phi_io->data) ? 1 : 0);
+        stats->kernel_launches = nk;
     }
     return status;
 }

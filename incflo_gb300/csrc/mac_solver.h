@@ -101,6 +101,8 @@ private:
     bool beta_ready = false;
     double scale32 = 1.0;
     static constexpr int kMaxGraphs = 8;  // captured steps of 1 to 8 inner V-cycles (more are launched directly)
+    long long nk = 0;  // kernels of the present projection (a captured step's at each launch)
+    long long step_kernels = 0, step_kernels_m[kMaxGraphs + 1] = {};
     cudaGraphExec_t gexec[kMaxGraphs + 1] = {};
     int gexec_prec = -1;
     void drop_graphs();

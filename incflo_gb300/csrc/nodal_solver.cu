@@ -420,6 +420,7 @@ int NodalSolver::finish_sigma()
     const double* src0 = L[0].s64;
     if (eb.on) {
         eb_sigma(L[0].g, eb.e, L[0].s64, L[0].s64, L[0].s32, L[0].t64, st);
+        nk += 1 + eb_kernel(true);
         src0 = L[0].t64;
     }
     for (size_t l = 1; l < L.size(); ++l)
@@ -462,6 +463,7 @@ int NodalSolver::build_bottom()
     GBP_CUDA(cudaMemsetAsync(bad, 0, 2 * sizeof(unsigned), st));
     bottom_rows_nodal(L.back().g, L.back().s64, brows, bad + 1, st);
     if (dense_bottom) bottom_inverse(brows, bsing ? 1 : 0, dmat, nullptr, bad, st);
+    nk += 1 + dense_bottom;
     if (nbottom > kCheckedBottom) return GBP_OK;
     unsigned h[2] = {0, 0};
     GBP_CUDA(cudaMemcpyAsync(h, bad, sizeof(h), cudaMemcpyDeviceToHost, st));
@@ -639,7 +641,7 @@ void NodalSolver::vcycle(int l, const T* b, bool zero)
             else
                 nodal_jacobi<T>(lv.g, B::s(lv), nullptr, b, x, wpre[0], true, s);
             if (cut) eb_nodes<T>(lv.g, eb.e, 0, nullptr, b, x, wpre[0], s);
-            ++nk;
+            nk += 1 + eb_kernel(cut);
             q0 = 1;
         } else {
             cudaMemsetAsync(x, 0, sizeof(T) * lv.g.count, s);
@@ -649,7 +651,7 @@ void NodalSolver::vcycle(int l, const T* b, bool zero)
         const double w = wpre[q % kSweepWeights];
         jacobi<T>(lv.g, B::s(lv), x, b, t, w, s);
         if (cut) eb_nodes<T>(lv.g, eb.e, 0, x, b, t, w, s);
-        ++nk;
+        nk += 1 + eb_kernel(cut);
         std::swap(x, t);
     }
     const NodalLevel& cv = L[l + 1];
@@ -679,7 +681,7 @@ void NodalSolver::vcycle(int l, const T* b, bool zero)
     resid<T>(lv.g, B::s(lv), x, b, B::r(lv), nullptr, s);
     if (cut) eb_nodes<T>(lv.g, eb.e, 1, x, b, B::r(lv), omega_eff, s);
     nodal_restrict<T>(lv.g, cv.g, B::r(lv), B::b(cv), s);
-    nk += 2;
+    nk += 2 + eb_kernel(cut);
     vcycle<T>(l + 1, B::b(cv), true);
     nodal_prolong_add<T>(lv.g, cv.g, (const T*)xres[l + 1], x, s);
     ++nk;
@@ -687,7 +689,7 @@ void NodalSolver::vcycle(int l, const T* b, bool zero)
         const double w = wpost[q % kSweepWeights];
         jacobi<T>(lv.g, B::s(lv), x, b, t, w, s);
         if (cut) eb_nodes<T>(lv.g, eb.e, 0, x, b, t, w, s);
-        ++nk;
+        nk += 1 + eb_kernel(cut);
         std::swap(x, t);
     }
     xres[l] = x;
@@ -704,6 +706,7 @@ void NodalSolver::resid0(const double* x, const double* b, double* r, unsigned l
     resid<double>(l0.g, l0.s64, x, b, r, nullptr, s);
     eb_nodes<double>(l0.g, eb.e, 1, x, b, r, omega_eff, s);
     if (norm) eb_norm(l0.g, r, eb.ivol, norm, s);
+    nk += eb_kernel(true) + (norm != nullptr);
 }
 
 void NodalSolver::drop_graphs()
@@ -751,7 +754,7 @@ void NodalSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s, const KrylovNo
         apply_neg<T>(p, q, s);
         krylov_alpha<T>(box, p, q, r, kpart, kstate, s);
         krylov_update<T>(box, p, q, x, r, kstate, s, c == m - 1 ? norm : nullptr);
-        nk += 5;
+        nk += 5 + eb_kernel(eb.on);
     }
 }
 
@@ -1024,6 +1027,7 @@ int NodalSolver::solve(bool have_guess, gbp_stats* stats, bool from_prev)
     hstate->inv_scale = 1.0 / scale32;
     GBP_CUDA(cudaMemcpyAsync(kstate, hstate, sizeof(KrylovState), cudaMemcpyHostToDevice, st));
     if (mixed) nodal_to_f32(l0.g, from_rhs ? rhs0 : res, l0.b32, scale32, st);
+    nk += mixed;
     if (mixed && accelerated())
         GBP_CUDA(cudaMemsetAsync(reinterpret_cast<float*>(kq) + l0.g.count, 0, sizeof(float) * l0.g.count, st));
     if (!evi0) {
@@ -1685,6 +1689,7 @@ int NodalSolver::project(const RhsArgs& rhs, const CorrArgs& corr, gbp_array4* p
         ++nk;
     }
     if (eb.on) eb_rhs(l0.g, eb.e, ra, rhs0, st);
+    nk += eb_kernel(eb.on) + eb.on;  // (and its norm)
     if (singular) {
         // consistent right-hand side, and its max norm (the relative-tolerance reference; with cut
         // cells taken again below over the fluid volumes)
@@ -1752,6 +1757,7 @@ int NodalSolver::project(const RhsArgs& rhs, const CorrArgs& corr, gbp_array4* p
         nodal_correct(l0.g, ca, l0.s64, phi, st);
         ++nk;
         if (eb.on) eb_correct(l0.g, eb.e, corr, phi, st);
+        nk += eb.on && eb.e.ncells > 0;
         if (out_slabs && out_slabs->nslabs > 0) {
             // cut cells: one copy after the whole correction
             const HostSlabs& o = *out_slabs;

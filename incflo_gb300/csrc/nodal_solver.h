@@ -284,6 +284,7 @@ private:
         long long active_nodes = 0;        // unique nodes of level 0 that touch fluid
         bool on = false;
     } eb;
+    int eb_kernel(bool cut) const { return cut && eb.e.nnodes > 0 ? 1 : 0; }  // the EB nodes' part of a sweep, as a kernel count
     bool sigma_ready = false;
     double scale32 = 1.0;
     // result buffer of each level's V-cycle (ping-pong aware)
