@@ -97,13 +97,15 @@ __global__ void __launch_bounds__(128) k_rows_mac(CellGeom g, const double* __re
 // Symmetric and, for coefficients of one sign, definite, so no pivoting, and Gauss-Jordan as the sweep operator (Goodnight
 // 1979, The American Statistician 33), which keeps the symmetry: one triangle in registers, the pivot's column passed
 // through shared memory, one division per pivot in the warps that hold the column. (Coefficients of both signs or NaN go
-// through as well: the inverse is a preconditioner, and the solve's residual decides.) One SM's FP64 pipe bounds it (16 cycles per warp and instruction): 64
+// through as well: the inverse is a preconditioner, and the solve's residual decides.) A pivot that is rounding against its
+// diagonal (up to 2e-13 with some 100 unknowns) closes a null space besides the constants, that of a region of fluid sealed off by covered cells: its unknown stays
+// unswept, held at 0 (a generalised inverse, exact for a right-hand side that is consistent in the region). One SM's FP64 pipe bounds it (16 cycles per warp and instruction): 64
 // unknowns took 243 us with the whole matrix and a division in every warp, now 75.
 __global__ void __launch_bounds__(1024) k_bottom_inverse(BottomRows r, int singular, double* __restrict__ M,
                                                          unsigned char* __restrict__ act, unsigned* bad)
 {
     constexpr int kMost = (kDenseBottom * (kDenseBottom + 1) / 2 + 1023) / 1024;  // entries of a thread
-    __shared__ double col[2][kDenseBottom], scl[kDenseBottom], shift;
+    __shared__ double col[2][kDenseBottom], scl[kDenseBottom], diag[kDenseBottom], shift;
     const int N = r.n, t = threadIdx.x;
     // entry (u, v) of the matrix
     auto entry = [&](int u, int v) {
@@ -153,7 +155,10 @@ __global__ void __launch_bounds__(1024) k_bottom_inverse(BottomRows r, int singu
     __syncthreads();
 #pragma unroll
     for (int m = 0; m < kMost; ++m)  // the first pivot's column
-        if (eu[m] >= 0 && ev[m] == 0) col[0][eu[m]] = a[m];
+        if (eu[m] >= 0) {
+            if (ev[m] == 0) col[0][eu[m]] = a[m];
+            if (ev[m] == eu[m]) diag[eu[m]] = fabs(a[m]);
+        }
     __syncthreads();
     for (int c = 0; c < N; ++c) {
         const double* cc = col[c & 1];
@@ -163,7 +168,7 @@ __global__ void __launch_bounds__(1024) k_bottom_inverse(BottomRows r, int singu
             return;
         }
         if (t < ((N + 31) & ~31)) {
-            const double inv = 1.0 / piv;
+            const double inv = fabs(piv) < 1e-12 * diag[c] ? 0.0 : 1.0 / piv;
             if (t < N) scl[t] = t == c ? -inv : cc[t] * inv;
         }
         __syncthreads();
