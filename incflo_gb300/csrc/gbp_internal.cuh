@@ -86,17 +86,6 @@ __device__ __forceinline__ int node_aliases(int i, int n, int per, int out[3])
     return m;
 }
 
-__device__ __forceinline__ int cell_aliases(int i, int n, int per, int out[3])
-{
-    out[0] = i;
-    int m = 1;
-    if (per) {
-        if (i == 0) out[m++] = n;
-        if (i == n - 1) out[m++] = -1;
-    }
-    return m;
-}
-
 // distance from unique node i to its padded alias along one direction, 0 when it has none (per, n >= 3: nodes 0
 // and 1 alias to n and n + 1, node n - 1 to -1)
 __device__ __forceinline__ int node_alias_step(int i, int n, int per)

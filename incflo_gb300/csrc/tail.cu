@@ -75,6 +75,7 @@ __device__ __forceinline__ void split(const Lev<T>&, unsigned row, unsigned plan
     j = m0 ? (int)__umulhi(r, m0) : (int)r;
     i = (int)(r - (unsigned)j * row);
 }
+// (p >= 4: a level above the bottom)
 __device__ __forceinline__ int node_step(int i, int p) { return !p ? 0 : (i <= 1 ? p : (i == p - 1 ? -p : 0)); }
 __device__ __forceinline__ int cell_step(int i, int p) { return !p ? 0 : (i == 0 ? p : (i == p - 1 ? -p : 0)); }
 
@@ -282,15 +283,6 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_nodal_tail(const __grid_con
                     // (a level of one CTA keeps planes -1 .. n of a periodic z, no plane n + 1)
                     const int ez = L.solo ? cell_step(kl, L.pz) * L.sz : 0;
                     put(out, L, kl + 1, at, node_step(i, L.px), node_step(j, L.py) * L.sy, ez, cp, all, v);
-                    if ((L.px == 2 && i == 1) || (L.py == 2 && j == 1)) {
-                        // a periodic x or y of 2 cells: node 1 is also node -1
-#pragma unroll 1
-                        for (int m = 1; m < 9; ++m) {
-                            const int ai = m % 3 == 0 ? i : (m % 3 == 1 ? (L.px ? i + node_step(i, L.px) : i) : (L.px == 2 && i == 1 ? -1 : i));
-                            const int aj = m / 3 == 0 ? j : (m / 3 == 1 ? (L.py ? j + node_step(j, L.py) : j) : (L.py == 2 && j == 1 ? -1 : j));
-                            put(out, L, kl + 1, (ai + kOX) + (aj + 1) * L.sy, 0, 0, ez, cp, all, v);
-                        }
-                    }
                 }
             } else if (op == kRestrict) {
                 // full weighting into the next level's right-hand side: its own slab's, or CTA 0's
