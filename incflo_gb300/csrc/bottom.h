@@ -1,6 +1,6 @@
 // The coarsest level of a multigrid hierarchy (nodal or cell-centred): its operator as rows of a fixed number of
 // entries, rebuilt on the device whenever the coefficients change, and the two solvers on it:
-//   - up to kDenseBottom unknowns: the dense FP64 inverse (Gauss-Jordan in one CTA), applied as one product;
+//   - up to kDenseBottom unknowns (nodal: kDenseNodal): the dense FP64 inverse (Gauss-Jordan in one CTA), applied as one product;
 //   - above: Jacobi-preconditioned conjugate gradients in FP64 by one thread-block cluster (bottom_cg).
 #pragma once
 
@@ -10,12 +10,14 @@
 
 namespace gbp {
 
-// n unknowns: the inverse costs n^3 / 2 FP64 multiply-adds on one SM (2 per clock: about 75 us for 64, 230 us for 108) per
-// coefficient set and a product of 1 to 3 us per V-cycle, where the cluster's conjugate gradients take 25 to 100 us per
+// n unknowns: the inverse costs n^3 / 2 FP64 multiply-adds on one SM (2 per clock: about 75 us for 64, 230 us for 108, 480 us for
+// 125) per coefficient set and a product of 1 to 3 us per V-cycle, where the cluster's conjugate gradients take 25 to 100 us per
 // V-cycle; and a dense bottom lets the cluster tail cycle the small levels (MAC 112 x 16 x 24 cells, 84 unknowns: 3.7 ms
-// per projection without, 1.5 with; 48 x 24 x 48, 108 unknowns: 1.84 and 1.27; nodal 112 x 48 x 48, 128 unknowns: 1.65 and
-// 1.90). (The inverse of up to 216 unknowns by the host took 0.3 to 10 ms per coefficient set.)
-constexpr int kDenseBottom = 112;
+// per projection without, 1.5 with; 48 x 24 x 48, 108 unknowns: 1.84 and 1.27; 40^3, 125 unknowns: 1.6 and 1.4, and 1.6 and 0.9
+// where the coefficients stay; nodal 112 x 48 x 48, 128 unknowns, whose sigma is set for every projection: 1.65 and 1.90). The
+// limit of the cell-centred hierarchies is what one thread block's registers hold without a spill. (The inverse of up to 216
+// unknowns by the host took 0.3 to 10 ms per coefficient set.)
+constexpr int kDenseBottom = 127, kDenseNodal = 112;
 // most unknowns of the cluster solver: the search direction is replicated in every CTA's shared memory
 constexpr int kClusterBottom = 16384;
 constexpr int kBottomThreads = 1024;

@@ -324,7 +324,7 @@ int NodalSolver::init(const gbp_geometry& geom, const int bc_lo[3], const int bc
         for (int q = 0; q < 4; ++q) add(G0.count, 8);
     add(nodal_partials_needed(G0) + 64, 8);
     nbottom = B.g.nu[0] * B.g.nu[1] * B.g.nu[2];
-    dense_bottom = nbottom <= kDenseBottom;
+    dense_bottom = nbottom <= kDenseNodal;
     brows = BottomRows{};
     if (nbottom <= kClusterBottom) {
         brows.n = nbottom;
