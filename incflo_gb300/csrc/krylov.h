@@ -13,8 +13,9 @@
 //
 // With a V-cycle that contracts the error by rho per application, the stationary iteration needs log(tol) / log(rho)
 // of them; the accelerated one removes the few slow modes that set rho (a density jump, cut cells, stretched cells):
-// V(2,2) cycles to 1e-10 on the 256^3 interface problem 10 -> 7 (nodal) and 11 -> 9 (MAC), to 1e-11 on cells of aspect
-// 1 : 0.8 : 1.25 38 -> 16 (both).
+// V(2,2) cycles on the 256^3 interface problem 10 -> 7 (nodal, FP64, to 1e-10) and 12 -> 9 (MAC, FP64; FP32 in FP64
+// 12 -> 10), to 1e-11 around a cylinder 22 -> 11 (nodal) and 13 -> 10 (MAC), on cells of aspect 1 : 0.8 : 1.25
+// 38 -> 16 (both).
 #pragma once
 
 #include <cuda_runtime.h>

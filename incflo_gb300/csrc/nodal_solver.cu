@@ -761,7 +761,7 @@ void NodalSolver::krylov_steps(int m, T* x, T* r, cudaStream_t s, const KrylovNo
 // Whether a solve accelerates its V-cycles. FP64 V-cycles: always (256^3 interface: 60.1 -> 44.9 ms, 10 -> 7 V-cycles;
 // the vector kernels are 4 % of a V-cycle there). FP32 V-cycles: except on the levels of the whole-row sweeps, whose
 // V-cycle from the current iterate costs 0.78 ms at 256^3 where the accelerated one, from zero and with its five vector
-// passes, costs 1.12 ms (13.0 against 12.0 ms per projection with 8 against 10 V-cycles); cut cells (22 -> 12 V-cycles
+// passes, costs 1.12 ms (13.0 against 12.0 ms per projection with 8 against 10 V-cycles); cut cells (22 -> 11 V-cycles
 // on the cylinder channel) and stretched cells gain several times more than that. Never on a hierarchy of one level, whose
 // "V-cycle" is the coarsest level's solve: one of them per step, and nothing to accelerate (with the vector passes and the
 // inner solve's further V-cycles 2^3 cells took 310 to 560 us per projection, without 270 to 350).
